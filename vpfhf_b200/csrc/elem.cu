@@ -4,6 +4,7 @@
 // atomics.  The element tables travel by value in the kernel parameters
 // (__grid_constant__): every thread of a warp reads the same entry, which the
 // constant bank broadcasts.
+#include <algorithm>
 #include <cmath>
 
 #include "elem.h"
@@ -723,6 +724,7 @@ __device__ __forceinline__ double mdz_t(const double (&m)[8], double tx, double 
   return ih * fma(fma(m[7], ty, m[5]), tx, fma(m[6], ty, m[4]));
 }
 
+// NOCOMPRESSION: all four quantities point by point.
 // One thread per element (grid-stride, fixed assignment), per-thread compensated
 // sums, pairwise tree in shared memory, per-block partials: deterministic.  The fields
 // at the 27 points come from their modal forms (the trilinear interpolants the
@@ -821,12 +823,265 @@ __global__ void __launch_bounds__(EN_THREADS, 3) energy_kernel(
   if (threadIdx.x < 4) partial[blockIdx.x * 4 + threadIdx.x] = red[threadIdx.x][0];
 }
 
-__global__ void energy_final_kernel(const double* __restrict__ partial, int nblocks,
-                                    double* __restrict__ out) {
-  if (threadIdx.x >= 4) return;
+// out[q] = compensated sum of partial[4 b + q] over the blocks: one warp per quantity, lane
+// l takes blocks l, l + 32, ..., the lanes join in a fixed tree.  (One thread per quantity
+// walking all 888 partials was a serial chain of 77 us.)
+__global__ void __launch_bounds__(128) energy_final_kernel(const double* __restrict__ partial,
+                                                           int nblocks, double* __restrict__ out) {
+  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   KSum s;
-  for (int b = 0; b < nblocks; b++) s.add(partial[b * 4 + threadIdx.x]);
-  out[threadIdx.x] = s.value();
+  for (int b = lane; b < nblocks; b += 32) s.add(partial[b * 4 + q]);
+  double r = s.value();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
+  if (lane == 0) out[q] = r;
+}
+
+// ---- energies by Gauss rows (the plain model).  Along a Gauss row (fixed gy, gz) every
+// trilinear field is linear in t = tx, so each integrand is a polynomial of degree <= 4 in
+// t and its 3-point sum follows from sum w = 1, sum w t^2 = 1/12, sum w t^4 = 1/80 (odd
+// sums vanish): the same Gauss sum as point by point from 9 rows instead of 27 points.
+// Where the 8 nodal v of the cell are equal and neither theta nor the Biot term enters,
+// v leaves the sum and the elastic terms are squares of polynomials of degree <= 1 per
+// axis, whose Gauss sums are closed (mean of t^2 = 1/12 per axis): no row is evaluated.
+// WANT selects the quantities a caller asked for (kEnElastic ...), so that each entry
+// point pays for its own.  A thread marches kEnLayers cells up a column and keeps the
+// nodes shared with the cell below.
+// The point-by-point kernel took 1.05 ms at 129^3 for every entry point (FP64 issue: 3500
+// operations per cell; 77 us more in a serial final sum); the three entry points one after
+// the other, each with its host read, measured 3.42 ms with it and 0.327 ms with these.
+constexpr int kEnLayers = 4;
+
+// Squared norm over the cell of a polynomial with coefficients c[m] of the monomials
+// m = px + 2 py + 4 pz of degree <= 1 per axis: weights 1, 1/12, 1/144 (no xyz term).
+__device__ __forceinline__ double en_sq(const double (&c)[7]) {
+  return fma(c[0], c[0],
+             fma(fma(c[1], c[1], fma(c[2], c[2], c[4] * c[4])), 1.0 / 12.0,
+                 fma(c[3], c[3], fma(c[5], c[5], c[6] * c[6])) * (1.0 / 144.0)));
+}
+
+template <int WANT>
+__global__ void __launch_bounds__(EN_THREADS, (WANT & kEnElastic) ? 3 : 4) energy_rows_kernel(
+    const __grid_constant__ ElemArgs E, const double* __restrict__ u, const double* __restrict__ v,
+    const double* __restrict__ theta, const double* __restrict__ thetaRef,
+    const double* __restrict__ p, double* __restrict__ partial, double* __restrict__ cellcov) {
+  constexpr bool EL = (WANT & kEnElastic) != 0, PW = EL, SU = (WANT & kEnSurface) != 0,
+                 CV = (WANT & kEnOpening) != 0, U = EL || CV;
+  __shared__ double red[4][EN_THREADS];
+  const int nex = E.nx - 1, ney = E.ny - 1, nez = E.nz - 1;
+  const int64_t ncol = (int64_t)nex * ney, nitem = ncol * ((nez + kEnLayers - 1) / kEnLayers);
+  const int64_t plane = (int64_t)E.nx * E.ny;
+  const double ih[3] = {1. / E.hx, 1. / E.hy, 1. / E.hz};
+  const double vol = E.hx * E.hy * E.hz;
+  KSum acc[4];
+  for (int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; it < nitem;
+       it += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t col = it % ncol;
+    const int ei = (int)(col % nex), ej = (int)(col / nex);
+    const int k0 = (int)(it / ncol) * kEnLayers, k1 = min(k0 + kEnLayers, nez);
+    double f[3][8], v8[8], th8[8], p8[8];  // [4 + j]: the upper nodes
+    auto load4 = [&](int k) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int64_t n = k * plane + (int64_t)(ej + (j >> 1)) * E.nx + ei + (j & 1);
+        if constexpr (U) {
+#pragma unroll
+          for (int c = 0; c < 3; c++) f[c][4 + j] = u[3 * n + c];
+        }
+        v8[4 + j] = v[n];
+        if constexpr (EL) {
+          th8[4 + j] = theta ? theta[n] - (thetaRef ? thetaRef[n] : 0.) : 0.;
+          p8[4 + j] = p ? p[n] : 0.;
+        }
+      }
+    };
+    load4(k0);
+#pragma unroll 1
+    for (int ek = k0; ek < k1; ek++) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        if constexpr (U) {
+#pragma unroll
+          for (int c = 0; c < 3; c++) f[c][j] = f[c][4 + j];
+        }
+        v8[j] = v8[4 + j];
+        if constexpr (EL) {
+          th8[j] = th8[4 + j];
+          p8[j] = p8[4 + j];
+        }
+      }
+      load4(ek + 1);
+      const CellMat mat = cell_mat(E, ei, ej, ek);
+      bool cst = true;
+#pragma unroll
+      for (int a = 1; a < 8; a++) cst = cst && v8[a] == v8[0];
+      double mv[8];
+      modal_of(v8, mv);
+      if constexpr (SU) {  // VF_AT1/AT2SurfaceEnergy3D_local (VFMech.c:2394-2465)
+        const double om = 1. - mv[0];
+        double lin = om;
+        if (E.atnum != 1)
+          lin = fma(om, om, (mv[1] * mv[1] + mv[2] * mv[2] + mv[4] * mv[4]) * (1. / 12.) +
+                                (mv[3] * mv[3] + mv[5] * mv[5] + mv[6] * mv[6]) * (1. / 144.) +
+                                mv[7] * mv[7] * (1. / 1728.));
+        auto g2 = [&](int a, int b, int c, double i) {
+          return i * i * (mv[a] * mv[a] + (mv[b] * mv[b] + mv[c] * mv[c]) * (1. / 12.) +
+                          mv[7] * mv[7] * (1. / 144.));
+        };
+        const double gr = (g2(1, 3, 5, ih[0]) + g2(2, 3, 6, ih[1])) + g2(4, 5, 6, ih[2]);
+        acc[2].add(vol * (lin / E.epsilon + gr * E.epsilon) * (mat.Gc / E.atcv * .25));
+      }
+      if constexpr (U) {
+        double m[3][8];
+#pragma unroll
+        for (int c = 0; c < 3; c++) modal_of(f[c], m[c]);
+        const double threekappa = 3. * mat.lambda + 2. * mat.mu;
+        const double cb = EL ? mat.beta / threekappa : 0.;
+        bool closed = cst;
+        if constexpr (EL) {
+          closed = closed && cb == 0.;
+#pragma unroll
+          for (int a = 0; a < 8; a++) closed = closed && th8[a] == 0.;
+        }
+        double el = 0., pw = 0., cv = 0.;
+        if (closed) {
+          if constexpr (EL) {
+            // gradient coefficients: d/dx of component c has the monomials 1, y, z, yz
+            // (modes 1, 3, 5, 7), d/dy 1, x, z, xz (2, 3, 6, 7), d/dz 1, x, y, xy (4, 5, 6, 7)
+            const double x1 = m[0][1] * ih[0], xy = m[0][3] * ih[0], xz = m[0][5] * ih[0], xyz = m[0][7] * ih[0];
+            const double y1 = m[1][2] * ih[1], yx = m[1][3] * ih[1], yz = m[1][6] * ih[1], yxz = m[1][7] * ih[1];
+            const double z1 = m[2][4] * ih[2], zx = m[2][5] * ih[2], zy = m[2][6] * ih[2], zxy = m[2][7] * ih[2];
+            const double tr[7] = {(x1 + y1) + z1, yx + zx, xy + zy, zxy, xz + yz, yxz, xyz};
+            double d0[7], d1[7], d2[7];
+            const double e0[7] = {x1, 0., xy, 0., xz, 0., xyz}, e1[7] = {y1, yx, 0., 0., yz, yxz, 0.};
+            const double e2[7] = {z1, zx, zy, zxy, 0., 0., 0.};
+#pragma unroll
+            for (int q = 0; q < 7; q++) {
+              d0[q] = fma(tr[q], -1. / 3., e0[q]);
+              d1[q] = fma(tr[q], -1. / 3., e1[q]);
+              d2[q] = fma(tr[q], -1. / 3., e2[q]);
+            }
+            // twice the shear strains: 12 = d/dx u_y + d/dy u_x, ...
+            const double s0[7] = {fma(m[1][1], ih[0], m[0][2] * ih[1]), m[0][3] * ih[1], m[1][3] * ih[0], 0.,
+                                  fma(m[1][5], ih[0], m[0][6] * ih[1]), m[0][7] * ih[1], m[1][7] * ih[0]};
+            const double s1[7] = {fma(m[2][2], ih[1], m[1][4] * ih[2]), fma(m[2][3], ih[1], m[1][5] * ih[2]),
+                                  m[1][6] * ih[2], m[1][7] * ih[2], m[2][6] * ih[1], m[2][7] * ih[1], 0.};
+            const double s2[7] = {fma(m[2][1], ih[0], m[0][4] * ih[2]), m[0][5] * ih[2],
+                                  fma(m[2][3], ih[0], m[0][6] * ih[2]), m[0][7] * ih[2], m[2][5] * ih[0], 0.,
+                                  m[2][7] * ih[0]};
+            const double dev = (en_sq(d0) + en_sq(d1)) + en_sq(d2) + .5 * ((en_sq(s0) + en_sq(s1)) + en_sq(s2));
+            const double tt = en_sq(tr), vv = v8[0] * v8[0];
+            el = vol * (dev * vv * (1. + E.eta) * mat.mu + threekappa / 6. * tt * (vv + E.eta));
+            // p only multiplies grad v = 0 here; a value that is not finite still shows
+#pragma unroll
+            for (int a = 0; a < 8; a++) pw += p8[a];
+            pw = 0. * pw;
+            el += pw;
+          }
+          if constexpr (CV) {  // u . grad v = 0; a displacement that is not finite still shows
+            double t = 0.;
+#pragma unroll
+            for (int c = 0; c < 3; c++) t += m[c][0];
+            cv = 0. * t;
+          }
+        } else {
+          double mp[8], mth[8];
+          if constexpr (EL) {
+            modal_of(p8, mp);
+            modal_of(th8, mth);
+          }
+#pragma unroll 1
+          for (int gz = 0; gz < 3; gz++) {
+            const double tz = gz == 1 ? 0. : (gz == 0 ? -VF_TAU : VF_TAU);
+#pragma unroll 1
+            for (int gy = 0; gy < 3; gy++) {
+              const double ty = gy == 1 ? 0. : (gy == 0 ? -VF_TAU : VF_TAU);
+              const double wr = vol * (w1(gy) * w1(gz));
+              // value and slope of a trilinear field along the row
+              auto row = [&](const double (&q)[8], double& r0, double& r1) {
+                r0 = fma(fma(q[6], tz, q[2]), ty, fma(q[4], tz, q[0]));
+                r1 = fma(fma(q[7], tz, q[3]), ty, fma(q[5], tz, q[1]));
+              };
+              // y and z derivatives along the row (value, slope)
+              auto dy = [&](const double (&q)[8], double& r0, double& r1) {
+                r0 = ih[1] * fma(q[6], tz, q[2]);
+                r1 = ih[1] * fma(q[7], tz, q[3]);
+              };
+              auto dz = [&](const double (&q)[8], double& r0, double& r1) {
+                r0 = ih[2] * fma(q[6], ty, q[4]);
+                r1 = ih[2] * fma(q[7], ty, q[5]);
+              };
+              double v0, v1;
+              row(mv, v0, v1);
+              double gy0, gy1, gz0, gz1;
+              dy(mv, gy0, gy1);
+              dz(mv, gz0, gz1);
+              const double gx0 = ih[0] * v1;
+              double ux0, ux1, uy0, uy1, uz0, uz1;
+              row(m[0], ux0, ux1);
+              row(m[1], uy0, uy1);
+              row(m[2], uz0, uz1);
+              // u . grad v = c0 + c1 t + c2 t^2
+              const double c0 = fma(ux0, gx0, fma(uy0, gy0, uz0 * gz0));
+              const double c2 = fma(uy1, gy1, uz1 * gz1);
+              if constexpr (CV) cv = fma(wr, fma(c2, 1. / 12., c0), cv);  // VolumetricCrackOpening3D_local
+              if constexpr (EL) {
+                double p0, p1, th0, th1;
+                row(mp, p0, p1);
+                row(mth, th0, th1);
+                if (E.hasCrackPressure) {  // VF_PressureWork3D_local (VFMech.c:920-974)
+                  const double c1 = fma(ux1, gx0, (uy0 * gy1 + uy1 * gy0) + (uz0 * gz1 + uz1 * gz0));
+                  pw = fma(wr, fma(c0, p0, fma(c1, p1, c2 * p0) * (1. / 12.)), pw);
+                }
+                // VF_ElasticEnergy3D_local (VFMech.c:725-809): v^2 (1 + eta) on the deviator
+                double ay[3], by[3], az[3], bz[3];
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                  dy(m[c], ay[c], by[c]);
+                  dz(m[c], az[c], bz[c]);
+                }
+                const double X0 = ih[0] * ux1, X1 = ih[0] * uy1, X2 = ih[0] * uz1;
+                const double T0 = (X0 + ay[1]) + az[2], T1 = by[1] + bz[2];
+                const double t0 = T0 * (1. / 3.), t1 = T1 * (1. / 3.);
+                const double d00 = X0 - t0, d11 = ay[1] - t0, d22 = az[2] - t0;
+                const double f11 = by[1] - t1, f22 = bz[2] - t1;
+                const double s01 = X1 + ay[0], s02 = X2 + az[0], s12 = ay[2] + az[1];
+                const double r12 = by[2] + bz[1];
+                const double q0 = fma(d00, d00, fma(d11, d11, d22 * d22)) +
+                                  .5 * fma(s01, s01, fma(s02, s02, s12 * s12));
+                const double q1 = 2. * (fma(d11, f11, d22 * f22) - d00 * t1) +
+                                  fma(s01, by[0], fma(s02, bz[0], s12 * r12));
+                const double q2 = fma(t1, t1, fma(f11, f11, f22 * f22)) +
+                                  .5 * fma(by[0], by[0], fma(bz[0], bz[0], r12 * r12));
+                const double a0 = v0 * v0, a1 = 2. * v0 * v1, a2 = v1 * v1;
+                const double dv = fma(a0, q0, fma(fma(a0, q2, fma(a1, q1, a2 * q0)), 1. / 12., a2 * q2 * (1. / 80.)));
+                // WD = (tr / 3 - alpha theta) v - cb p along the row
+                const double f0 = fma(-mat.alpha, th0, t0), f1 = fma(-mat.alpha, th1, t1);
+                const double b0 = fma(f0, v0, -(cb * p0)), b1 = fma(f0, v1, fma(f1, v0, -(cb * p1))), b2 = f1 * v1;
+                const double wd = fma(b0, b0, fma(fma(b1, b1, 2. * b0 * b2), 1. / 12., b2 * b2 * (1. / 80.)));
+                const double t2 = fma(T0, T0, T1 * T1 * (1. / 12.));
+                el = fma(wr, (dv * (1. + E.eta)) * mat.mu + fma(1.5 * threekappa, wd, threekappa / 6. * t2 * E.eta), el);
+              }
+            }
+          }
+        }
+        if constexpr (EL) acc[0].add(el);
+        if constexpr (PW) acc[1].add(E.hasCrackPressure ? pw : 0.);
+        if constexpr (CV) {
+          if (cellcov) cellcov[((int64_t)ek * ney + ej) * nex + ei] = cv / vol;
+          acc[3].add(cv);
+        }
+      }
+    }
+  }
+  for (int q = 0; q < 4; q++) red[q][threadIdx.x] = acc[q].value();
+  __syncthreads();
+  for (int st = EN_THREADS / 2; st > 0; st >>= 1) {
+    if (threadIdx.x < st)
+      for (int q = 0; q < 4; q++) red[q][threadIdx.x] += red[q][threadIdx.x + st];
+    __syncthreads();
+  }
+  if (threadIdx.x < 4) partial[blockIdx.x * 4 + threadIdx.x] = red[threadIdx.x][0];
 }
 
 template <typename K, typename... Args>
@@ -896,11 +1151,29 @@ cudaError_t launch_v_diag(const ElemArgs& E, const double* coef, double* d, cuda
 
 int energy_blocks() { return EN_BLOCKS; }
 
-cudaError_t launch_energies(const ElemArgs& E, const double* u, const double* v,
+cudaError_t launch_energies(const ElemArgs& E, int want, const double* u, const double* v,
                             const double* theta, const double* thetaRef, const double* p,
                             double* partial, double* out, double* cellcov, cudaStream_t s) {
-  energy_kernel<<<EN_BLOCKS, EN_THREADS, 0, s>>>(E, u, v, theta, thetaRef, p, partial, cellcov);
-  energy_final_kernel<<<1, 32, 0, s>>>(partial, EN_BLOCKS, out);
+  int blocks = EN_BLOCKS;
+  if (E.unilateral) {  // the spherical factor switches per point: point by point
+    energy_kernel<<<EN_BLOCKS, EN_THREADS, 0, s>>>(E, u, v, theta, thetaRef, p, partial, cellcov);
+  } else {
+    const int64_t items = (int64_t)(E.nx - 1) * (E.ny - 1) * ((E.nz - 1 + kEnLayers - 1) / kEnLayers);
+    blocks = (int)std::min<int64_t>(EN_BLOCKS, (items + EN_THREADS - 1) / EN_THREADS);
+    switch (want) {
+      case kEnElastic:
+        energy_rows_kernel<kEnElastic><<<blocks, EN_THREADS, 0, s>>>(E, u, v, theta, thetaRef, p, partial, cellcov);
+        break;
+      case kEnSurface:
+        energy_rows_kernel<kEnSurface><<<blocks, EN_THREADS, 0, s>>>(E, u, v, theta, thetaRef, p, partial, cellcov);
+        break;
+      case kEnOpening:
+        energy_rows_kernel<kEnOpening><<<blocks, EN_THREADS, 0, s>>>(E, u, v, theta, thetaRef, p, partial, cellcov);
+        break;
+      default: return cudaErrorInvalidValue;
+    }
+  }
+  energy_final_kernel<<<1, 128, 0, s>>>(partial, blocks, out);
   return cudaGetLastError();
 }
 

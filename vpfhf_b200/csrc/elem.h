@@ -50,9 +50,15 @@ cudaError_t launch_v_rhs(const ElemArgs& E, const double* u, const double* p, do
 cudaError_t launch_v_diag(const ElemArgs& E, const double* coef, double* d, cudaStream_t s);
 
 // Energies: out[0] elastic, out[1] pressure work, out[2] surface, out[3] crack
-// opening volume.  partial must hold 2*4*nblocks doubles; out is device memory.
+// opening volume, of which `want` (one of kEn*) names those the caller reads (the others
+// are 0 in the plain model, and all four are computed under NOCOMPRESSION).  cellcov (or
+// null) is written with kEnOpening.  partial must hold 4 * energy_blocks() doubles; out is
+// device memory.
+constexpr int kEnElastic = 1;  // out[0] and out[1]
+constexpr int kEnSurface = 2;  // out[2]
+constexpr int kEnOpening = 4;  // out[3]
 int energy_blocks();
-cudaError_t launch_energies(const ElemArgs& E, const double* u, const double* v,
+cudaError_t launch_energies(const ElemArgs& E, int want, const double* u, const double* v,
                             const double* theta, const double* thetaRef, const double* p,
                             double* partial, double* out, double* cellcov, cudaStream_t s);
 

@@ -758,7 +758,7 @@ int vfgpu_am_step(vfgpu_ctx* c, const vfgpu_solve_opts* o, double* errV, vfgpu_s
   return std::max(ru, rv);
 }
 
-static int energies(vfgpu_ctx* c, double* cellcov) {
+static int energies(vfgpu_ctx* c, int want, double* cellcov) {
   if (!c) return fail(VFGPU_ERR_INVALID, "null ctx");
   if (!c->have_mat) return fail(VFGPU_ERR_STATE, "material not set");
   cudaSetDevice(c->dev);
@@ -768,11 +768,11 @@ static int energies(vfgpu_ctx* c, double* cellcov) {
   const bool stage = cellcov && !is_device_ptr(cellcov);
   if (stage) cc = c->p64[8];
   ElemArgs E = elem_args(c);
-  cudaError_t e = launch_energies(E, c->f[VFGPU_FIELD_U], c->f[VFGPU_FIELD_V], c->f[VFGPU_FIELD_THETA],
-                                  c->f[VFGPU_FIELD_THETAREF], c->f[VFGPU_FIELD_PRESSURE],
+  cudaError_t e = launch_energies(E, want, c->f[VFGPU_FIELD_U], c->f[VFGPU_FIELD_V],
+                                  c->f[VFGPU_FIELD_THETA], c->f[VFGPU_FIELD_THETAREF], c->f[VFGPU_FIELD_PRESSURE],
                                   c->d_red + RED_BLOCKS * 4, c->d_out, cc, c->stream);
   // d_out[4] = in-situ work (partials in the CG part of d_red, idle outside solves)
-  if (e == cudaSuccess && c->has_insitu)
+  if (e == cudaSuccess && want == kEnElastic && c->has_insitu)
     e = launch_insitu_work(insitu_args(c), c->f[VFGPU_FIELD_U], c->d_red, c->d_out + 4, c->stream);
   else if (e == cudaSuccess)
     e = cudaMemsetAsync(c->d_out + 4, 0, sizeof(double), c->stream);
@@ -784,7 +784,7 @@ static int energies(vfgpu_ctx* c, double* cellcov) {
 }
 
 int vfgpu_u_energy(vfgpu_ctx* c, double* elastic, double* insitu, double* pressurework) {
-  int rc = energies(c, nullptr);
+  int rc = energies(c, kEnElastic, nullptr);
   if (rc) return rc;
   if (elastic) *elastic = c->h_out[0];
   if (insitu) *insitu = c->h_out[4];
@@ -793,14 +793,14 @@ int vfgpu_u_energy(vfgpu_ctx* c, double* elastic, double* insitu, double* pressu
 }
 
 int vfgpu_v_energy(vfgpu_ctx* c, double* surface) {
-  int rc = energies(c, nullptr);
+  int rc = energies(c, kEnSurface, nullptr);
   if (rc) return rc;
   if (surface) *surface = c->h_out[2];
   return VFGPU_OK;
 }
 
 int vfgpu_crack_opening(vfgpu_ctx* c, double* cov, double* cellcov) {
-  int rc = energies(c, cellcov);
+  int rc = energies(c, kEnOpening, cellcov);
   if (rc) return rc;
   if (cov) *cov = c->h_out[3];
   return VFGPU_OK;
