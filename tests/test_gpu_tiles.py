@@ -1,0 +1,69 @@
+"""GPU: the assembled V operator and the row-wise energies at the sizes where their tiles can
+go wrong (the smallest grids, one node past a block's 31 x 7 node columns, its multiples, a
+chunk's last planes), against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# (grid, AT1 / AT2, thermal strain, per-cell modulus, layers, NOCOMPRESSION)
+CASES = [((2, 2, 2), 1, False, False, False, 0), ((3, 8, 5), 2, True, False, True, 0),
+         ((31, 7, 9), 1, False, True, False, 0), ((32, 8, 6), 2, False, False, True, 0),
+         ((63, 15, 2), 1, True, False, False, 0), ((33, 9, 10), 2, True, True, False, 1),
+         ((62, 14, 17), 1, False, False, True, 1)]
+
+
+def _setup(oracle_mod, n, atnum, thermal, cellE, layers, unilateral):
+    import vpfhf_b200 as vg
+    rng = np.random.default_rng(sum(n) + atnum)
+    l = tuple(0.1 * (k - 1) * s for k, s in zip(n, (1.0, 1.2, 0.9)))
+    nlay, N = (2 if layers else 1), n[0] * n[1] * n[2]
+    E, nu, Gc = [1e10, 3e10][:nlay], [0.25, 0.2][:nlay], [100.0, 140.0][:nlay]
+    alpha = [1e-5 if thermal else 0.0] * nlay
+    lay = np.array([k % 2 for k in range(n[2] - 1)], np.int32) if layers else None
+    cE = None
+    if cellE:
+        cE = (1e10 * np.exp(0.5 * rng.standard_normal((n[0] - 1) * (n[1] - 1) * (n[2] - 1)))).astype(np.float32)
+        cE = cE.astype(np.float64)
+    kw = dict(epsilon=0.25, eta=1e-6, atnum=atnum)
+    o = oracle_mod.Oracle(n, l, E=E if layers else E[0], nu=nu if layers else nu[0],
+                          Gc=Gc if layers else Gc[0], alpha=alpha if layers else alpha[0],
+                          beta=0.7 if thermal else 0.0, layer=lay, cellE=cE, pressurize=True, unilateral=unilateral, **kw)
+    ctx = vg.VFContext(n, l, [dict(E=a, nu=b, Gc=g, alpha=t, beta=0.7 if thermal else 0.0) for a, b, g, t in zip(E, nu, Gc, alpha)],
+                       pressurize=True, layer=lay, **kw)
+    if cE is not None:
+        ctx.set_cell_modulus(cE)
+    if unilateral:
+        ctx.set_unilateral(1)
+    ctx.set_bc(vg.rollers())
+    v = np.ones(N)  # intact, a constant block, a random block
+    vv = v.reshape(n[2], n[1], n[0])
+    vv[: n[2] // 3, : n[1] // 2] = 0.4
+    blk = vv[n[2] // 2:, n[1] // 3:, n[0] // 3:]
+    blk[...] = rng.uniform(0, 1, blk.shape)
+    u, p = rng.standard_normal(3 * N) * 1e-4, rng.uniform(0.5, 1.5, N) * 1e6
+    theta = rng.uniform(0, 10, N) if thermal else np.zeros(N)
+    for name, f in (("U", u), ("V", v), ("VIrrev", v), ("pressure", p), ("theta", theta)):
+        ctx.set_field(name, f)
+    return o, ctx, u, v, p, theta
+
+
+@pytest.mark.parametrize("n,atnum,thermal,cellE,layers,unilateral", CASES)
+def test_v_residual_and_energies(cuda, oracle_mod, n, atnum, thermal, cellE, layers, unilateral):
+    """Residual entries sum at most 216 Gauss terms of one sign pattern and their rounding is
+    ~1e-15 of the largest: 1e-11 of it, as the other residual tests.  The energies are sums of
+    rounded terms (1e-13), of which the pressure work and the opening cancel by at most the
+    square root of the cells: 1e-10."""
+    o, ctx, u, v, p, theta = _setup(oracle_mod, n, atnum, thermal, cellE, layers, unilateral)
+    F = ctx.v_residual()
+    Fr = o.v_residual_ref(u, v, theta, None, p, v)
+    assert np.abs(F - Fr).max() <= 1e-11 * np.abs(Fr).max()
+    el_o, pw_o = o.u_energy(u, v, theta, None, p)
+    el, _, pw = ctx.u_energy()
+    cov, cc = ctx.crack_opening(cell=True)
+    cov_o, cc_o = o.cov(u, v, cell=True)
+    assert el == pytest.approx(el_o, rel=1e-10) and pw == pytest.approx(pw_o, rel=1e-10)
+    assert ctx.v_energy() == pytest.approx(o.v_energy(v), rel=1e-10)
+    assert cov == pytest.approx(cov_o, rel=1e-10) and ctx.crack_opening() == cov
+    assert np.abs(cc - cc_o).max() <= 1e-10 * np.abs(cc_o).max()
+    ctx.close()

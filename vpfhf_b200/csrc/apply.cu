@@ -1,4 +1,4 @@
-// apply.cu -- instantiations of the tile engine for the U and V operators.
+// apply.cu -- instantiations of the tile engine for the U operator.
 #include <mutex>
 #include <type_traits>
 
@@ -13,7 +13,7 @@ namespace vfgpu {
 #ifndef VFGPU_U64_TY
 #define VFGPU_U64_TY 8
 #endif
-constexpr int U_TY = 8, U64_TY = VFGPU_U64_TY, V_TY = kVTileY;
+constexpr int U_TY = 8, U64_TY = VFGPU_U64_TY;
 // Blocks per SM of the FP64 U operator: 1 (~250 registers, two corner-contribution
 // buffers) or, as a build option, 2 (128 registers: the row closed form of the
 // non-constant elements spills; one buffer and a second barrier per layer).
@@ -47,9 +47,6 @@ constexpr int U64C_MINB = VFGPU_U64C_MINB,
               U32C_MINB = kU32CPacked ? VFGPU_U32C2_MINB : VFGPU_U32C_MINB;
 using U32COp = std::conditional_t<kU32CPacked, UOpF2Const<false>, UOpConst<float>>;
 using U32COpC = std::conditional_t<kU32CPacked, UOpF2Const<true>, UOpConst<float, true>>;
-// V tiles carry 2 stages of 27 coefficients per cell in shared memory: 75 KB (FP32,
-// 2 CTAs per SM) or 150 KB (FP64, 1 CTA per SM).
-constexpr int V64_MINB = 1, V32_MINB = 2;
 // FP32 U operator: scalar UOp<float> (2 CTAs of 8 warps per SM) by default.  The
 // packed two-lane variant (UOpF2: two elements per thread, half the arithmetic
 // instructions) is kept as a build option; it needs 242 registers, so one CTA of
@@ -88,41 +85,7 @@ cudaError_t apply_kernel_attributes() {
   if (e == cudaSuccess) e = set_tile_attributes<U32OpC, U32_TY, U32_MINB>();
   if (e == cudaSuccess) e = set_tile_attributes<UOpNC<double>, U64_TY, 1>();
   if (e == cudaSuccess) e = set_tile_attributes<UOpNC<float>, U_TY, 2>();
-  if (e == cudaSuccess) e = set_tile_attributes<VOp<double>, V_TY, V64_MINB>();
-  if (e == cudaSuccess) e = set_tile_attributes<VOp<float>, V_TY, V32_MINB>();
   return e;
-}
-
-using TensorEncode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-// cuTensorMapEncodeTiled from the driver (null if it has none)
-static TensorEncode tensor_encode() {
-  static const TensorEncode fn = []() -> TensorEncode {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q{};
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      return nullptr;
-    return reinterpret_cast<TensorEncode>(f);
-  }();
-  return fn;
-}
-
-cudaError_t vcoef_tensor_map(CUtensorMap* map, const void* coef, int bytes, int nex, int ney, int nez) {
-  const TensorEncode encode = tensor_encode();
-  if (!encode) return cudaErrorNotSupported;
-  const int pitch = vcoef_pitch(nex);
-  const cuuint64_t dims[3] = {(cuuint64_t)nex, (cuuint64_t)ney, (cuuint64_t)27 * nez};
-  const cuuint64_t strides[2] = {(cuuint64_t)pitch * bytes, (cuuint64_t)pitch * ney * bytes};
-  const cuuint32_t box[3] = {32, (cuuint32_t)kVTileY, 27}, estride[3] = {1, 1, 1};
-  const CUresult r =
-      encode(map, bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
-             const_cast<void*>(coef), dims, strides, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 // One CTA waits on an mbarrier whose phase completes (complete = 1: the arrival is
@@ -384,50 +347,16 @@ TilePlan u_plan(int nx, int ny, int nz, int prec_bytes, int num_sms) {
   p.ncta0 = q.ncta;
   return p;
 }
-TilePlan v_plan(int nx, int ny, int nz, int prec_bytes, int num_sms) {
-  return tile_plan(nx, ny, nz, V_TY, 1, prec_bytes == 8 ? V64_MINB : V32_MINB, num_sms);
-}
-
-// The 1-D tensor maps of x (3N values) and v (N) that the fixed-weight wave copies its node
-// planes with (PlaneBox boxes, zeros beyond the ends); false where they cannot be made:
-// a pointer not 16-byte aligned, 3N past the 32-bit coordinates, no encoder.
-template <typename T> static bool u_plane_maps(UApplyArgs<T>& A) {
-  const int64_t N = (int64_t)A.nx * A.ny * A.nz;
-  const TensorEncode encode = tensor_encode();
-  if (!encode || 3 * N >= (int64_t)INT32_MAX || ((uintptr_t)A.x & 15) || ((uintptr_t)A.v & 15)) return false;
-  const CUtensorMapDataType dt = sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  const cuuint64_t dx[1] = {(cuuint64_t)(3 * N)}, dv[1] = {(cuuint64_t)N}, none[1] = {0};
-  const cuuint32_t bx[1] = {(cuuint32_t)PlaneBox<T>::XBOX}, bv[1] = {(cuuint32_t)PlaneBox<T>::VBOX}, es[1] = {1};
-  const CUresult r1 = encode(&A.xmap, dt, 1, const_cast<T*>(A.x), dx, none, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  const CUresult r2 = encode(&A.vmap, dt, 1, const_cast<T*>(A.v), dv, none, bv, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r1 == CUDA_SUCCESS && r2 == CUDA_SUCCESS;
-}
-
-// A split launch's operands (with the VFGPU_U_PLANES_TMA build option, the plane maps), or
-// false: then the apply runs one wave, with the second wave's x.y partials zeroed for a
-// caller that counts them.
-template <typename T> static bool split_args(const UApplyArgs<T>& A, const TilePlan& p, UApplyArgs<T>& B,
-                                             cudaStream_t s) {
-  B = A;
-  if (!VFGPU_U_PLANES_TMA || u_plane_maps(B)) return true;
-  if (A.dot) cudaMemsetAsync(A.dot + p.ncta + seam_blocks(p, A.nx, A.ny, A.nz), 0, p.ncta0 * sizeof(double), s);
-  return false;
-}
 
 template <>
 cudaError_t launch_u_apply<double>(const UApplyArgs<double>& A, const TilePlan& p,
                                    const LayerTable& L, cudaStream_t s) {
   if (A.cflag) return launch_tile_apply<UOpNC<double>, U64_TY, 1>(A, p, L, s);
-  UApplyArgs<double> B;
-  if (A.ur[0] && A.ur[1] && split_args(A, p, B, s)) {
+  if (A.ur[0] && A.ur[1]) {
     if (cubic(A))
       return launch_tile_apply_split<UOpConst<double, true>, UOp<double, true>, U64_TY, U64C_MINB, U64_MINB>(
-          B, p, L, s);
-    return launch_tile_apply_split<UOpConst<double>, UOp<double>, U64_TY, U64C_MINB, U64_MINB>(B, p, L, s);
+          A, p, L, s);
+    return launch_tile_apply_split<UOpConst<double>, UOp<double>, U64_TY, U64C_MINB, U64_MINB>(A, p, L, s);
   }
   if (cubic(A)) return launch_tile_apply<UOp<double, true>, U64_TY, U64_MINB>(A, p, L, s);
   return launch_tile_apply<UOp<double>, U64_TY, U64_MINB>(A, p, L, s);
@@ -439,27 +368,15 @@ cudaError_t launch_u_apply<float>(const UApplyArgs<float>& A, const TilePlan& p,
   // scalar tile (the packed build option keeps the plain operator packed)
   if (A.cflag) return launch_tile_apply<UOpNC<float>, U_TY, 2>(A, p, L, s);
   if constexpr (!kU32Packed) {
-    UApplyArgs<float> B;
-    if (A.ur[0] && A.ur[1] && split_args(A, p, B, s)) {
+    if (A.ur[0] && A.ur[1]) {
       if (cubic(A))
-        return launch_tile_apply_split<U32COpC, U32OpC, U32_TY, U32C_MINB, U32_MINB>(B, p, L, s);
-      return launch_tile_apply_split<U32COp, U32Op, U32_TY, U32C_MINB, U32_MINB>(B, p, L, s);
+        return launch_tile_apply_split<U32COpC, U32OpC, U32_TY, U32C_MINB, U32_MINB>(A, p, L, s);
+      return launch_tile_apply_split<U32COp, U32Op, U32_TY, U32C_MINB, U32_MINB>(A, p, L, s);
     }
   }
   if (cubic(A)) return launch_tile_apply<U32OpC, U32_TY, U32_MINB>(A, p, L, s);
   return launch_tile_apply<U32Op, U32_TY, U32_MINB>(A, p, L, s);
 }
-template <>
-cudaError_t launch_v_apply<double>(const VApplyArgs<double>& A, const TilePlan& p,
-                                   const LayerTable& L, cudaStream_t s) {
-  return launch_tile_apply<VOp<double>, V_TY, V64_MINB>(A, p, L, s);
-}
-template <>
-cudaError_t launch_v_apply<float>(const VApplyArgs<float>& A, const TilePlan& p,
-                                  const LayerTable& L, cudaStream_t s) {
-  return launch_tile_apply<VOp<float>, V_TY, V32_MINB>(A, p, L, s);
-}
-
 }  // namespace vfgpu
 
 extern "C" int vfgpu_wait_selftest(long long cycles, int complete, int* timed_out) {

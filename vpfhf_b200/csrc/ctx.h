@@ -57,9 +57,9 @@ struct vfgpu_ctx {
   bool v32_stale = true;  // (with ul_stale)
 
   // scratch
-  vfgpu::TilePlan plan64{}, plan32{}, vplan64{}, vplan32{};
+  vfgpu::TilePlan plan64{}, plan32{};
   double* d_dot = nullptr;   // block partials of the CG's p.w written by the operator applies
-  double* seam64 = nullptr;  // U and V seams FP64 (sized for the larger of the two plans)
+  double* seam64 = nullptr;
   float* seam32 = nullptr;
   double *t64a = nullptr, *t64b = nullptr;
   float *t32a = nullptr, *t32b = nullptr;
@@ -68,11 +68,8 @@ struct vfgpu_ctx {
   static constexpr int NP64 = 9, NP32 = 5;
   double* p64[NP64] = {nullptr};  // 3N + kPoolSlack doubles each
   float* p32[NP32] = {nullptr};   // 3N + kPoolSlack floats each
-  double* coef64 = nullptr;       // 27 per cell: V coupling coefficient (vcoef_index layout)
-  float* coef32 = nullptr;
-  CUtensorMap vmap64{}, vmap32{}; // coef64 / coef32 as the V apply's tensor copies see them
-  unsigned* d_cerr = nullptr;     // set by an apply whose bounded wait on a tensor copy (V
-                                  // coefficients, U node planes) gave up; held for the ctx's life
+  double* vmat64 = nullptr;       // couplings of the V operator (vmat.h), FP64 and FP32
+  float* vmat32 = nullptr;
   uint8_t* vmask = nullptr;       // N
   vfgpu::ETab h_tab{};            // element tables of the uniform element (kernel parameter)
   vfgpu::CGState* d_cg = nullptr; // device CG scalars

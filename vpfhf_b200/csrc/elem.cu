@@ -8,6 +8,7 @@
 #include <cmath>
 
 #include "elem.h"
+#include "vmat.h"
 
 namespace vfgpu {
 
@@ -119,10 +120,7 @@ __device__ __forceinline__ constexpr double bas(int i, int g) {
 __device__ __forceinline__ constexpr double w1(int g) { return g == 1 ? 8.0 / 18.0 : 5.0 / 18.0; }
 
 // Modal form of a trilinear field on the unit cell t in [-1/2, 1/2]^3: f = sum_p m_p t^p
-// (p = px + 2 py + 4 pz; m_0 the mean, m_1 the x slope, ...), and its value and
-// gradient at the Gauss point (gx, gy, gz), t = -tau, 0, +tau.  With the point
-// indices known at compile time (unrolled loops) each is a short chain of FMAs, and
-// the compiler shares the partial sums between points.
+// (p = px + 2 py + 4 pz; m_0 the mean, m_1 the x slope, ...).
 __device__ __forceinline__ void modal_of(const double (&f)[8], double (&m)[8]) {
   double a[8], b[8];
 #pragma unroll
@@ -145,23 +143,6 @@ __device__ __forceinline__ void modal_of(const double (&f)[8], double (&m)[8]) {
     m[q + 4] = hi - lo;
   }
 }
-__device__ __forceinline__ double mlin(int g, double a, double b) {
-  return g == 1 ? a : (g == 0 ? fma(b, -VF_TAU, a) : fma(b, VF_TAU, a));
-}
-__device__ __forceinline__ double mval(const double (&m)[8], int gx, int gy, int gz) {
-  return mlin(gz, mlin(gy, mlin(gx, m[0], m[1]), mlin(gx, m[2], m[3])),
-              mlin(gy, mlin(gx, m[4], m[5]), mlin(gx, m[6], m[7])));
-}
-__device__ __forceinline__ double mdx(const double (&m)[8], int gx, int gy, int gz, double ih) {
-  return ih * mlin(gy, mlin(gz, m[1], m[5]), mlin(gz, m[3], m[7]));
-}
-__device__ __forceinline__ double mdy(const double (&m)[8], int gx, int gy, int gz, double ih) {
-  return ih * mlin(gx, mlin(gz, m[2], m[6]), mlin(gz, m[3], m[7]));
-}
-__device__ __forceinline__ double mdz(const double (&m)[8], int gx, int gy, int gz, double ih) {
-  return ih * mlin(gx, mlin(gy, m[4], m[6]), mlin(gy, m[5], m[7]));
-}
-
 // Trilinear field at the 27 points, g = gx + 3 gy + 9 gz.
 __device__ __forceinline__ void interp27(const double (&f)[8], double (&o)[27]) {
   double fx[4][3], fy[2][3][3];
@@ -212,35 +193,6 @@ __device__ __forceinline__ void contract27(const double (&q)[27], double (&out)[
       for (int i = 0; i < 2; i++)
         out[i + 2 * j + 4 * k] =
             (bas(k, 0) * cy[i][j][0] + bas(k, 1) * cy[i][j][1]) + bas(k, 2) * cy[i][j][2];
-}
-
-// out[i + 2j + 4k] = sum_g q_g b_i(gx)^2 b_j(gy)^2 b_k(gz)^2
-__device__ __forceinline__ void contract27sq(const double (&q)[27], double (&out)[8]) {
-  auto f = [](int p, int g) { return bas(p, g) * bas(p, g); };
-  double cx[2][3][3], cy[2][2][3];
-#pragma unroll
-  for (int i = 0; i < 2; i++)
-#pragma unroll
-    for (int gz = 0; gz < 3; gz++)
-#pragma unroll
-      for (int gy = 0; gy < 3; gy++) {
-        const int b = 3 * gy + 9 * gz;
-        cx[i][gy][gz] = (f(i, 0) * q[b] + f(i, 1) * q[b + 1]) + f(i, 2) * q[b + 2];
-      }
-#pragma unroll
-  for (int i = 0; i < 2; i++)
-#pragma unroll
-    for (int j = 0; j < 2; j++)
-#pragma unroll
-      for (int gz = 0; gz < 3; gz++)
-        cy[i][j][gz] = (f(j, 0) * cx[i][0][gz] + f(j, 1) * cx[i][1][gz]) + f(j, 2) * cx[i][2][gz];
-#pragma unroll
-  for (int k = 0; k < 2; k++)
-#pragma unroll
-    for (int j = 0; j < 2; j++)
-#pragma unroll
-      for (int i = 0; i < 2; i++)
-        out[i + 2 * j + 4 * k] = (f(k, 0) * cy[i][j][0] + f(k, 1) * cy[i][j][1]) + f(k, 2) * cy[i][j][2];
 }
 
 // Integrals of q against the squared or plain basis products that carry no factor
@@ -524,84 +476,215 @@ __global__ void bc_diag_kernel(const uint8_t* __restrict__ bcbits, double* __res
   }
 }
 
-// ElasticEnergyDensity3D_local (VFMech.c:32-106) at every Gauss point, times 2 and
-// the Gauss weight, plus the AT2 mass coefficient (VFMech.c:2040-2058).  The strain at
-// the points comes from the modal form of u (the same trilinear interpolant the
-// reference's basis-function sums evaluate).
-__global__ void __launch_bounds__(128) v_coef_kernel(const __grid_constant__ ElemArgs E,
-                                                     const double* __restrict__ u,
-                                                     const double* __restrict__ theta,
-                                                     const double* __restrict__ thetaRef,
-                                                     double* __restrict__ coef,
-                                                     float* __restrict__ coef32) {
-  const int64_t NCELL = (int64_t)(E.nx - 1) * (E.ny - 1) * (E.nz - 1);
-  const int64_t cell = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (cell >= NCELL) return;
-  const int ei = (int)(cell % (E.nx - 1));
-  const int ej = (int)((cell / (E.nx - 1)) % (E.ny - 1));
-  const int ek = (int)(cell / ((int64_t)(E.nx - 1) * (E.ny - 1)));
-  const int pitch = vcoef_pitch(E.nx - 1);
-  const ETab& e = E.tab;
-  int64_t n[8];
-  cell_nodes(E, ei, ej, ek, n);
-  double mu3[3][8], mth[8];
-  {
-    double f[3][8], th8[8];
+// ---- the assembled V operator (vmat.h): 14 couplings per node.
+//
+// Along a Gauss row the strain is linear in t = tx, so twice the energy density (the
+// coupling coefficient 2 W, ElasticEnergyDensity3D_local, VFMech.c:32-106, plus the AT2 mass
+// coefficient, VFMech.c:2040-2058) is c0 + c1 t + c2 t^2 there and its row moments against
+// 1, t, t^2 follow from mean t^2 = 1/12, mean t^4 = 1/80 (odd means vanish): the reference's
+// 3-point sums.  Products of two 1-D basis functions are 1/4 - t + t^2 (both at the low
+// node), 1/4 - t^2 (one each) and 1/4 + t + t^2 (both high), so the cell's element matrix has
+// 27 distinct entries, one per product type and axis, built by sum factorisation; the
+// stiffness part (Gc / 2 c_w) eps grad . grad is a constant per type.  NOCOMPRESSION
+// (VFMech.c:115-218, 2125-2153) evaluates the row's three points instead (sign per point).
+__device__ __forceinline__ void v_cell_types(const ElemArgs& E, const CellMat& mat,
+                                             const double (&m)[3][8], const double (&mth)[8],
+                                             double (&M)[27]) {
+  const double ih[3] = {1. / E.hx, 1. / E.hy, 1. / E.hz};
+  const double vol = E.hx * E.hy * E.hz;
+  const double mass = E.atnum == 2 ? mat.Gc / E.atcv * .5 / E.epsilon : 0.;
+  const double lam = mat.lambda, mu = mat.mu;
+  // product of the basis functions of type p (0: low low, 1: low high, 2: high high) at point g
+  auto bb = [](int p, int g) { return bas(p == 2 ? 1 : 0, g) * bas(p == 0 ? 0 : 1, g); };
 #pragma unroll
-    for (int a = 0; a < 8; a++) {
+  for (int t = 0; t < 27; t++) M[t] = 0.;
 #pragma unroll
-      for (int c = 0; c < 3; c++) f[c][a] = u[3 * n[a] + c];
-      th8[a] = theta ? theta[n[a]] - (thetaRef ? thetaRef[n[a]] : 0.) : 0.;
+  for (int gz = 0; gz < 3; gz++) {
+    const double tz = gz == 1 ? 0. : (gz == 0 ? -VF_TAU : VF_TAU);
+    double cxy[3][3];  // [py][px]
+#pragma unroll
+    for (int q = 0; q < 9; q++) cxy[q / 3][q % 3] = 0.;
+#pragma unroll
+    for (int gy = 0; gy < 3; gy++) {
+      const double ty = gy == 1 ? 0. : (gy == 0 ? -VF_TAU : VF_TAU);
+      double X[3], ay[3], by[3], az[3], bz[3];
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        X[c] = ih[0] * fma(fma(m[c][7], tz, m[c][3]), ty, fma(m[c][5], tz, m[c][1]));
+        ay[c] = ih[1] * fma(m[c][6], tz, m[c][2]);
+        by[c] = ih[1] * fma(m[c][7], tz, m[c][3]);
+        az[c] = ih[2] * fma(m[c][6], ty, m[c][4]);
+        bz[c] = ih[2] * fma(m[c][7], ty, m[c][5]);
+      }
+      const double a0 = mat.alpha * fma(fma(mth[6], tz, mth[2]), ty, fma(mth[4], tz, mth[0]));
+      const double a1 = mat.alpha * fma(fma(mth[7], tz, mth[3]), ty, fma(mth[5], tz, mth[1]));
+      // twice the shear strains, value and slope along the row
+      const double s01 = X[1] + ay[0], s02 = X[2] + az[0], s12 = ay[2] + az[1], r12 = by[2] + bz[1];
+      double S0, S1, S2;  // row moments of the coefficient against 1, t, t^2
+      if (E.unilateral) {
+        S0 = S1 = S2 = 0.;
+        const double kappa = lam + 2. * mu / 3.;
+#pragma unroll
+        for (int gx = 0; gx < 3; gx++) {
+          const double t = gx == 1 ? 0. : (gx == 0 ? -VF_TAU : VF_TAU);
+          const double exx = X[0], eyy = fma(by[1], t, ay[1]), ezz = fma(bz[2], t, az[2]);
+          const double at = fma(a1, t, a0);
+          const double g01 = fma(by[0], t, s01), g02 = fma(bz[0], t, s02), g12 = fma(r12, t, s12);
+          // W = sigma(eps - e0) : eps, less (kappa/2) tr^2 where tr < 0
+          const double tr = exx + eyy + ezz, te = tr - 3. * at;
+          const double Wf = .5 * (lam * te * tr + 2. * mu * ((exx - at) * exx + (eyy - at) * eyy + (ezz - at) * ezz)) +
+                            .5 * mu * (g01 * g01 + g02 * g02 + g12 * g12);
+          const double S = tr < 0. ? 0. : kappa * tr * tr * .5, D = Wf - kappa * tr * tr * .5;
+          const double c = w1(gx) * (2. * (S + D) + mass);
+          S0 += c;
+          S1 = fma(t, c, S1);
+          S2 = fma(t * t, c, S2);
+        }
+      } else {
+        const double e0 = X[0] - a0, e1 = ay[1] - a0, e2 = az[2] - a0;
+        const double f0 = -a1, f1 = by[1] - a1, f2 = bz[2] - a1;
+        const double T0 = (e0 + e1) + e2, T1 = (f0 + f1) + f2;
+        const double c0 = fma(lam * T0, T0, fma(2. * mu, fma(e0, e0, fma(e1, e1, e2 * e2)),
+                                                mu * fma(s01, s01, fma(s02, s02, s12 * s12)))) + mass;
+        const double c1 = 2. * fma(lam * T0, T1, fma(2. * mu, fma(e0, f0, fma(e1, f1, e2 * f2)),
+                                                     mu * fma(s01, by[0], fma(s02, bz[0], s12 * r12))));
+        const double c2 = fma(lam * T1, T1, fma(2. * mu, fma(f0, f0, fma(f1, f1, f2 * f2)),
+                                                mu * fma(by[0], by[0], fma(bz[0], bz[0], r12 * r12))));
+        S0 = fma(c2, 1. / 12., c0);
+        S1 = c1 * (1. / 12.);
+        S2 = fma(c2, 1. / 80., c0 * (1. / 12.));
+      }
+      const double q = fma(S0, .25, S2);
+      const double px[3] = {q - S1, fma(S0, .25, -S2), q + S1};
+#pragma unroll
+      for (int py = 0; py < 3; py++)
+#pragma unroll
+        for (int x = 0; x < 3; x++) cxy[py][x] = fma(w1(gy) * bb(py, gy), px[x], cxy[py][x]);
     }
 #pragma unroll
-    for (int c = 0; c < 3; c++) modal_of(f[c], mu3[c]);
-    modal_of(th8, mth);
+    for (int pz = 0; pz < 3; pz++)
+#pragma unroll
+      for (int py = 0; py < 3; py++)
+#pragma unroll
+        for (int x = 0; x < 3; x++)
+          M[x + 3 * py + 9 * pz] = fma(w1(gz) * bb(pz, gz), cxy[py][x], M[x + 3 * py + 9 * pz]);
   }
-  const double ihx = 1. / E.hx, ihy = 1. / E.hy, ihz = 1. / E.hz;
-  const CellMat m = cell_mat(E, ei, ej, ek);
-  const double mass = E.atnum == 2 ? m.Gc / E.atcv * .5 / E.epsilon : 0.;
-  const double l = m.lambda, mu = m.mu;
+  const double kx = mat.Gc / E.atcv * .5 * E.epsilon * vol;
+  const double ix = kx * ih[0] * ih[0], iy = kx * ih[1] * ih[1], iz = kx * ih[2] * ih[2];
+  constexpr double st[3] = {1., -1., 1.}, ms[3] = {1. / 3., 1. / 6., 1. / 3.};
 #pragma unroll
-  for (int gz = 0; gz < 3; gz++)
+  for (int pz = 0; pz < 3; pz++)
 #pragma unroll
-    for (int gy = 0; gy < 3; gy++)
+    for (int py = 0; py < 3; py++)
 #pragma unroll
-      for (int gx = 0; gx < 3; gx++) {
-        const int g = gx + 3 * gy + 9 * gz;
-        const double uxx = mdx(mu3[0], gx, gy, gz, ihx), uyy = mdy(mu3[1], gx, gy, gz, ihy);
-        const double uzz = mdz(mu3[2], gx, gy, gz, ihz);
-        const double e12 = (mdx(mu3[1], gx, gy, gz, ihx) + mdy(mu3[0], gx, gy, gz, ihy)) * .5;
-        const double e23 = (mdy(mu3[2], gx, gy, gz, ihy) + mdz(mu3[1], gx, gy, gz, ihz)) * .5;
-        const double e13 = (mdx(mu3[2], gx, gy, gz, ihx) + mdz(mu3[0], gx, gy, gz, ihz)) * .5;
-        const double at = m.alpha * mval(mth, gx, gy, gz);
-        double cgv;
-        if (E.unilateral) {
-          // ElasticEnergyDensitySphericalDeviatoricNoCompression3D_local (VFMech.c:115-218):
-          // W = sigma(eps - e0) : eps, less (kappa/2) tr^2 where tr < 0
-          const double kappa = l + 2. * mu / 3.;
-          const double s11 = (l + 2. * mu) * (uxx - at) + l * (uyy - at) + l * (uzz - at);
-          const double s22 = l * (uxx - at) + (l + 2. * mu) * (uyy - at) + l * (uzz - at);
-          const double s33 = l * (uxx - at) + l * (uyy - at) + (l + 2. * mu) * (uzz - at);
-          const double Wf = (s11 * uxx + s22 * uyy + s33 * uzz) * .5 +
-                            2. * mu * (e12 * e12 + e23 * e23 + e13 * e13);
-          const double tr = uxx + uyy + uzz;
-          const double S = tr < 0. ? 0. : kappa * tr * tr * .5, D = Wf - kappa * tr * tr * .5;
-          cgv = e.w[g] * (2. * (S + D) + mass);
-        } else {
-          const double e11 = uxx - at, e22 = uyy - at, e33 = uzz - at;
-          const double s11 = (l + 2. * mu) * e11 + l * e22 + l * e33;
-          const double s22 = l * e11 + (l + 2. * mu) * e22 + l * e33;
-          const double s33 = l * e11 + l * e22 + (l + 2. * mu) * e33;
-          const double W = (s11 * e11 + s22 * e22 + s33 * e33) * .5 +
-                           2. * mu * (e12 * e12 + e23 * e23 + e13 * e13);
-          cgv = e.w[g] * (2. * W + mass);
-        }
-        const int64_t ci = vcoef_index(g, ei, ej, ek, pitch, E.ny - 1);
-        coef[ci] = cgv;
-        if (coef32) coef32[ci] = (float)cgv;
+      for (int x = 0; x < 3; x++) {
+        const double k = fma(ix, st[x] * ms[py] * ms[pz], fma(iy, ms[x] * st[py] * ms[pz], iz * (ms[x] * ms[py] * st[pz])));
+        M[x + 3 * py + 9 * pz] = fma(vol, M[x + 3 * py + 9 * pz], k);
       }
 }
 
+// Assembles the couplings.  A block owns 31 x 7 node columns and the 32 x 8 cell columns
+// around them, and marches up a chunk of node planes: per element layer each thread writes its
+// cell's 27 entries to shared memory, then its node gathers them from the 4 cells around it
+// (entry high-high in z of layer k - 1 carried in registers), so every coupling is summed in
+// one fixed order with no atomics and no colours.  The cells on the seams of the blocks are
+// computed twice (18 %).  FP64 issue bounds it.  It replaces the 27 coefficients per cell (in
+// both precisions) and the diagonal's 8 coloured passes over them: 0.60 ms per StepV at
+// 129^3, 0.41 ms now.
+constexpr int VM_NX = 31, VM_NY = 7;
+__global__ void __launch_bounds__(256, 1) v_assemble_kernel(const __grid_constant__ ElemArgs E,
+                                                            const double* __restrict__ u,
+                                                            const double* __restrict__ theta,
+                                                            const double* __restrict__ thetaRef,
+                                                            double* __restrict__ a64,
+                                                            float* __restrict__ a32, int64_t stride, int zc) {
+  extern __shared__ double vm_s[];  // [27][8][32]
+  const int l = threadIdx.x, w = threadIdx.y;
+  const int nx = E.nx, ny = E.ny, nz = E.nz;
+  const int ex = blockIdx.x * VM_NX - 1 + l, ey = blockIdx.y * VM_NY - 1 + w;
+  const bool cell = ex >= 0 && ex < nx - 1 && ey >= 0 && ey < ny - 1;
+  const bool node = l > 0 && w > 0 && ex < nx && ey < ny;  // owns node column (ex, ey)
+  const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);
+  const int64_t plane = (int64_t)nx * ny;
+  const int64_t base = cell ? (int64_t)ey * nx + ex : 0;
+  double f[3][8], th8[8], carry[5];
+#pragma unroll
+  for (int q = 0; q < 5; q++) carry[q] = 0.;
+  auto load4 = [&](int k) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int64_t n = base + k * plane + (j >> 1) * nx + (j & 1);
+#pragma unroll
+      for (int c = 0; c < 3; c++) f[c][4 + j] = cell ? u[3 * n + c] : 0.;
+      th8[4 + j] = (cell && theta) ? theta[n] - (thetaRef ? thetaRef[n] : 0.) : 0.;
+    }
+  };
+  const int k0 = max(z0 - 1, 0);
+  load4(k0);
+  for (int k = k0; k < z1; k++) {
+    double* s = vm_s + w * 32 + l;
+    if (k < nz - 1) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) f[c][j] = f[c][4 + j];
+        th8[j] = th8[4 + j];
+      }
+      load4(k + 1);
+      double M[27];
+      if (cell) {
+        double m[3][8], mth[8];
+#pragma unroll
+        for (int c = 0; c < 3; c++) modal_of(f[c], m[c]);
+        modal_of(th8, mth);
+        v_cell_types(E, cell_mat(E, ex, ey, k), m, mth, M);
+      } else {
+#pragma unroll
+        for (int t = 0; t < 27; t++) M[t] = 0.;
+      }
+#pragma unroll
+      for (int t = 0; t < 27; t++) s[t * 256] = M[t];
+    }
+    __syncthreads();
+    if (node) {
+      // the coupling (dx, dy) of z type pz over the 4 cells: lanes l - 1 (the node is the
+      // cell's high x corner) and l, rows w - 1 and w
+      auto gather = [&](int dx, int dy, int pz) {
+        double r = 0.;
+#pragma unroll
+        for (int yy = 0; yy < 2; yy++) {
+          if ((yy == 0 && dy > 0) || (yy == 1 && dy < 0)) continue;
+          const int py = dy ? 1 : (yy == 0 ? 2 : 0);
+#pragma unroll
+          for (int xx = 0; xx < 2; xx++) {
+            if ((xx == 0 && dx > 0) || (xx == 1 && dx < 0)) continue;
+            const int px = dx ? 1 : (xx == 0 ? 2 : 0);
+            r += s[(px + 3 * py + 9 * pz) * 256 + (yy - 1) * 32 + xx - 1];
+          }
+        }
+        return r;
+      };
+      const bool layer = k < nz - 1;
+      if (k >= z0) {
+        const int64_t n = (int64_t)k * plane + (int64_t)ey * nx + ex;
+        auto put = [&](int d, double v) {
+          a64[d * stride + n] = v;
+          if (a32) a32[d * stride + n] = (float)v;
+        };
+#pragma unroll
+        for (int q = 0; q < 5; q++)
+          put(q, carry[q] + (layer ? gather(kVForward[q][0], kVForward[q][1], 0) : 0.));
+#pragma unroll
+        for (int q = 5; q < kVCouplings; q++)
+          put(q, layer ? gather(kVForward[q][0], kVForward[q][1], 1) : 0.);
+      }
+      if (layer)
+#pragma unroll
+        for (int q = 0; q < 5; q++) carry[q] = gather(kVForward[q][0], kVForward[q][1], 2);
+    }
+    __syncthreads();  // the next layer rewrites the entries
+  }
+}
 
 // V load (VF_ResidualVAT1/AT23D_local and VF_ResidualVCrackPressure3D_local,
 // VFMech.c:2294-2384) in tensor form: the AT term coef sum_g w phi_a = coef vol / 8 per
@@ -655,45 +738,6 @@ __global__ void v_rhs_tp_kernel(const __grid_constant__ ElemArgs E, int color,
   }
 #pragma unroll
   for (int a = 0; a < 8; a++) b[n[a]] += rl[a];
-}
-
-// Diagonal of K_V (the AT forms VF_BilinearFormVAT1/AT23D_local, VFMech.c:2040-2090,
-// plus the coupling VF_BilinearFormVCoupling3D_local, :2093-2122) in tensor form:
-// aeps sum_g w |grad phi_a|^2 from the face moments of w, plus sum_g coef_g phi_a^2 as
-// a contraction against the squared basis.
-__global__ void v_diag_tp_kernel(const __grid_constant__ ElemArgs E, int color,
-                                 const double* __restrict__ coef, double* __restrict__ d) {
-  int ei, ej, ek;
-  if (!colour_cell(E, color, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, ei, ej, ek)) return;
-  int64_t n[8];
-  cell_nodes(E, ei, ej, ek, n);
-  const CellMat m = cell_mat(E, ei, ej, ek);
-  const double aeps = m.Gc / E.atcv * .5 * E.epsilon;
-  const double vol = E.hx * E.hy * E.hz;
-  const int pitch = vcoef_pitch(E.nx - 1);
-  double w27[27], c27[27], J[3][2][2], M[8];
-#pragma unroll
-  for (int gz = 0; gz < 3; gz++)
-#pragma unroll
-    for (int gy = 0; gy < 3; gy++)
-#pragma unroll
-      for (int gx = 0; gx < 3; gx++) {
-        const int g = gx + 3 * gy + 9 * gz;
-        w27[g] = vol * (w1(gx) * w1(gy) * w1(gz));
-        c27[g] = coef[vcoef_index(g, ei, ej, ek, pitch, E.ny - 1)];
-      }
-  face_moments<true>(w27, J);
-  contract27sq(c27, M);
-  const double ih2[3] = {1. / (E.hx * E.hx), 1. / (E.hy * E.hy), 1. / (E.hz * E.hz)};
-#pragma unroll
-  for (int k = 0; k < 2; k++)
-#pragma unroll
-    for (int j = 0; j < 2; j++)
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const double lap = (J[0][j][k] * ih2[0] + J[1][i][k] * ih2[1]) + J[2][i][j] * ih2[2];
-        d[n[i + 2 * j + 4 * k]] += fma(aeps, lap, M[i + 2 * j + 4 * k]);
-      }
 }
 
 // Neumaier-compensated accumulation.
@@ -1127,10 +1171,19 @@ cudaError_t launch_u_diag(const ElemArgs& E, const double* v, const uint8_t* bcb
   return e;
 }
 
-cudaError_t launch_v_coef(const ElemArgs& E, const double* u, const double* theta,
-                          const double* thetaRef, double* coef, float* coef32, cudaStream_t s) {
-  const int64_t NCELL = (int64_t)(E.nx - 1) * (E.ny - 1) * (E.nz - 1);
-  v_coef_kernel<<<(int)((NCELL + 127) / 128), 128, 0, s>>>(E, u, theta, thetaRef, coef, coef32);
+cudaError_t launch_v_assemble(const ElemArgs& E, const double* u, const double* theta,
+                              const double* thetaRef, double* a64, float* a32, cudaStream_t s) {
+  constexpr size_t smem = 27 * 256 * sizeof(double);
+  cudaError_t e = cudaFuncSetAttribute(v_assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const int gx = ceil_div(E.nx, VM_NX), gy = ceil_div(E.ny, VM_NY);
+  if (gy > 65535) return cudaErrorInvalidValue;
+  // planes of a chunk: four waves of one block per SM on large grids (each chunk computes the
+  // layer below it again), at least 4 planes on small ones, at most 65535 chunks
+  int zc = (int)std::max<int64_t>(4, ((int64_t)gx * gy * E.nz + 591) / 592);
+  zc = std::max(std::min(zc, E.nz), ceil_div(E.nz, 65535));
+  v_assemble_kernel<<<dim3(gx, gy, ceil_div(E.nz, zc)), dim3(32, 8), smem, s>>>(
+      E, u, theta, thetaRef, a64, a32, vmat_stride((int64_t)E.nx * E.ny * E.nz), zc);
   return cudaGetLastError();
 }
 
@@ -1140,13 +1193,6 @@ cudaError_t launch_v_rhs(const ElemArgs& E, const double* u, const double* p, do
   cudaError_t e = cudaMemsetAsync(b, 0, N * sizeof(double), s);
   if (e != cudaSuccess) return e;
   return colours(E, v_rhs_tp_kernel, s, u, p, b);
-}
-
-cudaError_t launch_v_diag(const ElemArgs& E, const double* coef, double* d, cudaStream_t s) {
-  const int64_t N = (int64_t)E.nx * E.ny * E.nz;
-  cudaError_t e = cudaMemsetAsync(d, 0, N * sizeof(double), s);
-  if (e != cudaSuccess) return e;
-  return colours(E, v_diag_tp_kernel, s, coef, d);
 }
 
 int energy_blocks() { return EN_BLOCKS; }

@@ -1,5 +1,5 @@
 // elem.h -- once-per-solve element kernels (FP64): load vectors, Jacobi diagonals,
-// the V coupling coefficient, energies and crack opening.
+// the V operator's assembly, energies and crack opening.
 #pragma once
 
 #include "common.cuh"
@@ -38,16 +38,13 @@ cudaError_t launch_u_diag(const ElemArgs& E, const double* v, const uint8_t* bcb
                           cudaStream_t s, const double* u0 = nullptr);
 // NOCOMPRESSION sign pattern: flags[cell] bit g = (tr(eps(u)) < 0 at Gauss point g).
 cudaError_t launch_nc_flags(const ElemArgs& E, const double* u, uint32_t* flags, cudaStream_t s);
-// coef (27 per cell in the vcoef_index layout: per element layer, 27 planes of the
-// layer's cells, so that a tile's values are one box of a 3-D tensor copy) = w_g
-// (2 W_g(u,theta) [+ Gc/(2c_w)/eps for AT2]) in FP64 and, if coef32 is not null, FP32.
-cudaError_t launch_v_coef(const ElemArgs& E, const double* u, const double* theta,
-                          const double* thetaRef, double* coef, float* coef32, cudaStream_t s);
+// The V operator's couplings (vmat.h) at u, in FP64 and, if a32 is not null, FP32; the
+// first array is the operator's diagonal.
+cudaError_t launch_v_assemble(const ElemArgs& E, const double* u, const double* theta,
+                              const double* thetaRef, double* a64, float* a32, cudaStream_t s);
 // b (N) = AT linear term + crack pressure term (VFMech.c:2294-2384).  Overwrites b.
 cudaError_t launch_v_rhs(const ElemArgs& E, const double* u, const double* p, double* b,
                          cudaStream_t s);
-// d (N) = diag K_V.  Overwrites d.
-cudaError_t launch_v_diag(const ElemArgs& E, const double* coef, double* d, cudaStream_t s);
 
 // Energies: out[0] elastic, out[1] pressure work, out[2] surface, out[3] crack
 // opening volume, of which `want` (one of kEn*) names those the caller reads (the others

@@ -2,29 +2,11 @@
 //
 //   UOp: y = K(v) x, the degraded elasticity operator of VF_BilinearFormU3D_local
 //        (VFMech.c:227-290) with Dirichlet rows identity (VFCartFE.c:1147-1296).
-//   VOp: y = K_V x, the damage operator of VF_BilinearFormVAT1/AT23D_local +
-//        VF_BilinearFormVCoupling3D_local (VFMech.c:2040-2115):
-//        (Gc/(2 c_w)) eps int grad(phi_a).grad(phi_b) + int c(x) phi_a phi_b,
-//        c = 2 W(u) [+ Gc/(2 c_w)/eps for AT2], with c premultiplied by the Gauss
-//        weight and stored per element and Gauss point (vfgpu v_coef kernel); the
-//        tile engine stages each element layer's 27 values per cell into shared
-//        memory with one 3-D tensor copy (cmap), two layers ahead of use.
-//        An optional mask removes dofs (row and column) for the reduced-space
-//        solves of the VI Newton method and the rows+columns Dirichlet/irreversibility
-//        treatment (VFCartFE.c:1305-1454, VFMech.c:2637-2682).
 #pragma once
 
 #include "f2.cuh"
 #include "tile_engine.cuh"
 #include "u_apply.cuh"
-
-// Build option: the fixed-weight U wave copies its node planes with 1-D tensor copies, two
-// per tile row (PlaneBox), instead of one cp.async per value.  Bit-identical; measured
-// slower on B200 at 129^3 on the penny field (FP64 apply 0.1223 ms against 0.1167, FP32
-// 0.0872 against 0.0855; with one thread waiting on each plane's mbarrier 0.1236 ms).
-#ifndef VFGPU_U_PLANES_TMA
-#define VFGPU_U_PLANES_TMA 0
-#endif
 
 namespace vfgpu {
 
@@ -32,9 +14,8 @@ namespace vfgpu {
 template <typename T_, bool CUBIC = false> struct UOp {
   using T = T_;
   using Args = UApplyArgs<T>;
-  static constexpr int NC = 3, NIN = 4, EPT = 1, CV = 0;
+  static constexpr int NC = 3, NIN = 4, EPT = 1;
   static constexpr int LIST = 1;  // the unit list this operator takes in a split launch
-  static constexpr bool PLANES_TMA = false;  // node planes by cp.async values
   __device__ __forceinline__ static void node_src(const Args& A, int64_t n, const T* (&src)[NIN]) {
     src[0] = A.x + 3 * n;
     src[1] = A.x + 3 * n + 1;
@@ -136,7 +117,6 @@ template <typename T_, bool CUBIC = false> struct UOpConst : UOp<T_, CUBIC> {
   using T = T_;
   using Args = UApplyArgs<T>;
   static constexpr int LIST = 0;
-  static constexpr bool PLANES_TMA = VFGPU_U_PLANES_TMA != 0;  // node planes by tensor copies
   __device__ __forceinline__ static void element(const Args& A, const LayerTable& L, int ex,
                                                  int ey, int ez, const T (&in)[8][Base::NIN],
                                                  T (&out)[8][Base::NC]) {
@@ -149,9 +129,8 @@ template <typename T_, bool CUBIC = false> struct UOpConst : UOp<T_, CUBIC> {
 template <typename T_> struct UOpNC {
   using T = T_;
   using Args = UApplyArgs<T>;
-  static constexpr int NC = 3, NIN = 4, EPT = 1, CV = 0;
+  static constexpr int NC = 3, NIN = 4, EPT = 1;
   static constexpr int LIST = -1;
-  static constexpr bool PLANES_TMA = false;
   __device__ __forceinline__ static void node_src(const Args& A, int64_t n, const T* (&src)[NIN]) {
     UOp<T>::node_src(A, n, src);
   }
@@ -201,9 +180,8 @@ template <typename T_> struct UOpNC {
 struct UOpF2 {
   using T = float;
   using Args = UApplyArgs<float>;
-  static constexpr int NC = 3, NIN = 4, EPT = 2, CV = 0;
+  static constexpr int NC = 3, NIN = 4, EPT = 2;
   static constexpr int LIST = -1;
-  static constexpr bool PLANES_TMA = false;
   __device__ __forceinline__ static void node_src(const Args& A, int64_t n, const T* (&src)[NIN]) {
     UOp<float>::node_src(A, n, src);
   }
@@ -263,9 +241,8 @@ struct UOpF2 {
 template <bool CUBIC = false> struct UOpF2Const {
   using T = float;
   using Args = UApplyArgs<float>;
-  static constexpr int NC = 3, NIN = 4, EPT = 2, CV = 0;
+  static constexpr int NC = 3, NIN = 4, EPT = 2;
   static constexpr int LIST = 0;
-  static constexpr bool PLANES_TMA = VFGPU_U_PLANES_TMA != 0;
   __device__ __forceinline__ static void node_src(const Args& A, int64_t n, const T* (&src)[NIN]) {
     UOp<float>::node_src(A, n, src);
   }
@@ -316,165 +293,6 @@ template <bool CUBIC = false> struct UOpF2Const {
   template <bool DOT>
   __device__ __forceinline__ static double finish_node(const Args& A, int64_t n, const T (&val)[NC]) {
     return UOp<float>::template finish_node<DOT>(A, n, val);
-  }
-};
-
-template <typename T> struct VApplyArgs {
-  CUtensorMap cmap;                   // the coefficient as a 3-D tensor (ex, ey, 27 ez + g),
-                                      // box 32 x TY x 27 (vcoef_index layout)
-  unsigned* __restrict__ cerr;        // set to 1 when a coefficient copy was not seen in time
-  const T* __restrict__ x;            // N input; must be 0 on masked dofs (the reduced-space
-                                      // CG keeps its directions 0 there), which makes the
-                                      // masked columns drop out
-  T* __restrict__ y;                  // N output
-  const uint8_t* __restrict__ mask;   // N: nonzero => dof removed (y = 0); or null
-  const uint8_t* __restrict__ elayer; // nz-1 or null
-  T* __restrict__ seamX;
-  T* __restrict__ seamY;
-  const int* __restrict__ skip;       // if non-null and *skip != 0 the launch does nothing
-  const DevParams* __restrict__ P;    // Gc/(2 c_w) eps per layer
-  double* __restrict__ dot;           // if non-null: per-block partials of x.y
-  int nx, ny, nz, ntx, nty;
-  T ihx, ihy, ihz, vol;
-};
-
-// A[s1][s2] = q0 + s1 q1 + s2 q2 + s1 s2 q3, s = -1 (index 0) or +1 (index 1).
-template <typename T>
-__device__ __forceinline__ void butterfly4(T q0, T q1, T q2, T q3, T (&A)[2][2]) {
-  const T r0m = q0 - q2, r0p = q0 + q2, r1m = q1 - q3, r1p = q1 + q3;
-  A[0][0] = r0m - r1m;
-  A[1][0] = r0m + r1m;
-  A[0][1] = r0p - r1p;
-  A[1][1] = r0p + r1p;
-}
-
-// y[a] = (K_V,e x_e)[a] for one element, in the modal form x = sum_p m_p t^p on the
-// unit cell t in [-1/2, 1/2]^3 (modal8, as u_element):
-//  - stiffness aeps int grad(phi_a).grad(x): the x-derivative is ihx (m1 + m3 ty +
-//    m5 tz + m7 ty tz), and its moments against {1, ty, tz, ty tz} are exactly
-//    {m1, m3 / 12, m5 / 12, m7 / 144} ihx (<t> = 0, <t^2> = 1/12), which is what the
-//    reference's 27-point Gauss sum gives for this integrand (VF_BilinearFormVAT1/
-//    AT23D_local, VFMech.c:2040-2115; 3 points per axis are exact for it), so the
-//    closed form replaces the sum; likewise y and z;
-//  - mass int c phi_a x with c given per Gauss point: x at the 27 points by sum
-//    factorisation of the modal form, psi_g = c_g x_g, and the moments
-//    M_p = sum_g psi_g t^p by sum factorisation along x, then y, then z.
-template <typename T>
-__device__ __forceinline__ void v_element(const T (&xn)[8], const T* __restrict__ cg, int cs,
-                                          T aeps, T ihx, T ihy, T ihz, T vol, T (&y)[8]) {
-  T m[8];
-  modal8(xn, m);
-  const T av = aeps * vol;
-  const T kx = av * ihx * ihx, ky = av * ihy * ihy, kz = av * ihz * ihz;
-  const T c4 = T(0.25), c24 = T(1.0 / 24.0), c144 = T(1.0 / 144.0);
-  T AX[2][2], AY[2][2], AZ[2][2];
-  butterfly4((kx * c4) * m[1], (kx * c24) * m[3], (kx * c24) * m[5], (kx * c144) * m[7], AX);
-  butterfly4((ky * c4) * m[2], (ky * c24) * m[3], (ky * c24) * m[6], (ky * c144) * m[7], AY);
-  butterfly4((kz * c4) * m[4], (kz * c24) * m[5], (kz * c24) * m[6], (kz * c144) * m[7], AZ);
-  // per gz: sums over the (gx, gy) points of psi {1, ty, tx, tx ty}, each t as its sign
-  T P00[3], P01[3], P10[3], P11[3];
-#pragma unroll
-  for (int gz = 0; gz < 3; gz++) {
-    const T p0 = lin(gz, m[0], m[4]), p1 = lin(gz, m[1], m[5]);
-    const T p2 = lin(gz, m[2], m[6]), p3 = lin(gz, m[3], m[7]);
-    T L0[3], L1[3];
-#pragma unroll
-    for (int gy = 0; gy < 3; gy++) {
-      const T q0 = lin(gy, p0, p2), q1 = lin(gy, p1, p3);
-      T psi[3];
-#pragma unroll
-      for (int gx = 0; gx < 3; gx++) psi[gx] = cg[(gx + 3 * gy + 9 * gz) * cs] * lin(gx, q0, q1);
-      L0[gy] = (psi[0] + psi[1]) + psi[2];
-      L1[gy] = psi[2] - psi[0];
-    }
-    P00[gz] = (L0[0] + L0[1]) + L0[2];
-    P01[gz] = L0[2] - L0[0];
-    P10[gz] = (L1[0] + L1[1]) + L1[2];
-    P11[gz] = L1[2] - L1[0];
-  }
-  const T t1 = T(VF_TAU), t2 = T(VF_TAU * VF_TAU), t3 = T(VF_TAU * VF_TAU * VF_TAU);
-  T M[8];  // value moments sum psi P_a(tx) P_b(ty) P_c(tz)
-  M[0] = (P00[0] + P00[1]) + P00[2];
-  M[1] = t1 * ((P10[0] + P10[1]) + P10[2]);
-  M[2] = t1 * ((P01[0] + P01[1]) + P01[2]);
-  M[3] = t2 * ((P11[0] + P11[1]) + P11[2]);
-  M[4] = t1 * (P00[2] - P00[0]);
-  M[5] = t2 * (P10[2] - P10[0]);
-  M[6] = t2 * (P01[2] - P01[0]);
-  M[7] = t3 * (P11[2] - P11[0]);
-  // value part: sum_g psi prod_d (1/2 + s_d t_d) -> 3 inverse butterflies over M
-  T b1[8], b2[8], b3[8];
-#pragma unroll
-  for (int q = 0; q < 4; q++) {  // z: M[q] (mode 0), M[q+4] (mode 1) -> k = 0,1
-    b1[q] = T(0.5) * M[q] - M[q + 4];
-    b1[q + 4] = T(0.5) * M[q] + M[q + 4];
-  }
-#pragma unroll
-  for (int k = 0; k < 2; k++)
-#pragma unroll
-    for (int al = 0; al < 2; al++) {  // y
-      const T lo = b1[al + 4 * k], hi = b1[al + 2 + 4 * k];
-      b2[al + 4 * k] = T(0.5) * lo - hi;
-      b2[al + 2 + 4 * k] = T(0.5) * lo + hi;
-    }
-#pragma unroll
-  for (int p = 0; p < 4; p++) {  // x
-    const T lo = b2[2 * p], hi = b2[2 * p + 1];
-    b3[2 * p] = T(0.5) * lo - hi;
-    b3[2 * p + 1] = T(0.5) * lo + hi;
-  }
-#pragma unroll
-  for (int k = 0; k < 2; k++)
-#pragma unroll
-    for (int j = 0; j < 2; j++)
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const T ax_ = i ? AX[j][k] : -AX[j][k];
-        const T ay_ = j ? AY[i][k] : -AY[i][k];
-        const T az_ = k ? AZ[i][j] : -AZ[i][j];
-        y[i + 2 * j + 4 * k] = ((ax_ + ay_) + az_) + b3[i + 2 * j + 4 * k];
-      }
-}
-
-template <typename T_> struct VOp {
-  using T = T_;
-  using Args = VApplyArgs<T>;
-  static constexpr int NC = 1, NIN = 1, EPT = 1;
-  static constexpr int LIST = -1;
-  static constexpr bool PLANES_TMA = false;
-  static constexpr int CV = 27;  // per-cell values staged by the engine (the coefficient)
-  __device__ __forceinline__ static const CUtensorMap* cell_map(const Args& A) { return &A.cmap; }
-  __device__ __forceinline__ static unsigned* cell_err(const Args& A) { return A.cerr; }
-  __device__ __forceinline__ static void node_src(const Args& A, int64_t n, const T* (&src)[NIN]) {
-    src[0] = A.x + n;
-  }
-  // cc: the element's 27 coefficients in shared memory, cs apart
-  __device__ __forceinline__ static void element(const Args& A, const LayerTable& L, int ex,
-                                                 int ey, int ez, const T (&in)[8][NIN],
-                                                 T (&out)[8][NC], const T* cc, int cs) {
-    T xn[8], yn[8];
-#pragma unroll
-    for (int a = 0; a < 8; a++) xn[a] = in[a][0];
-    const int layer = A.elayer ? A.elayer[ez] : 0;
-    v_element<T>(xn, cc, cs, T(A.P->aeps[layer]), A.ihx, A.ihy, A.ihz, A.vol, yn);
-#pragma unroll
-    for (int a = 0; a < 8; a++) out[a][0] = yn[a];
-  }
-  __device__ __forceinline__ static unsigned node_flags(const Args& A, int64_t n) {
-    return A.mask ? A.mask[n] : 0u;
-  }
-  template <bool DOT>
-  __device__ __forceinline__ static double finish_node_in(const Args& A, int64_t n, const T (&val)[NC],
-                                                          unsigned m, const T (&xin)[NC]) {
-    const T y = m ? T(0) : val[0];
-    A.y[n] = y;
-    if constexpr (DOT) return (double)xin[0] * (double)y;
-    return 0.;
-  }
-  template <bool DOT>
-  __device__ __forceinline__ static double finish_node(const Args& A, int64_t n, const T (&val)[NC]) {
-    const T xin[NC] = {DOT ? A.x[n] : T(0)};
-    return finish_node_in<DOT>(A, n, val, node_flags(A, n), xin);
   }
 };
 

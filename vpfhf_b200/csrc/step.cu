@@ -6,6 +6,7 @@
 
 #include "abi_util.h"
 #include "solver.h"
+#include "vmat.h"
 #include "vec.h"
 
 using namespace vfgpu;
@@ -15,16 +16,16 @@ namespace vfgpu {
 void free_solver(vfgpu_ctx* c) {
   for (auto& p : c->p64) cudaFree(p), p = nullptr;
   for (auto& p : c->p32) cudaFree(p), p = nullptr;
-  cudaFree(c->coef64);
-  cudaFree(c->coef32);
+  cudaFree(c->vmat64);
+  cudaFree(c->vmat32);
   cudaFree(c->vmask);
   cudaFree(c->d_cg);
   cudaFree(c->d_red);
   cudaFree(c->d_out);
   if (c->h_cg) cudaFreeHost(c->h_cg);
   if (c->h_out) cudaFreeHost(c->h_out);
-  c->coef64 = nullptr;
-  c->coef32 = nullptr;
+  c->vmat64 = nullptr;
+  c->vmat32 = nullptr;
   c->vmask = nullptr;
   c->d_cg = nullptr;
   c->d_red = nullptr;
@@ -43,16 +44,9 @@ static int solve_buffers(vfgpu_ctx* c) {
     if (e == cudaSuccess) e = cudaMalloc((void**)&p, n3 * sizeof(double));
   for (auto& p : c->p32)
     if (e == cudaSuccess) e = cudaMalloc((void**)&p, n3 * sizeof(float));
-  const size_t ncoef = (size_t)vcoef_size(c->nx - 1, c->ny - 1, c->nz - 1);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&c->coef64, ncoef * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&c->coef32, ncoef * sizeof(float));
-  // row padding is copied but never used; keep it defined
-  if (e == cudaSuccess) e = cudaMemsetAsync(c->coef64, 0, ncoef * sizeof(double), c->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(c->coef32, 0, ncoef * sizeof(float), c->stream);
-  if (e == cudaSuccess)
-    e = vcoef_tensor_map(&c->vmap64, c->coef64, 8, c->nx - 1, c->ny - 1, c->nz - 1);
-  if (e == cudaSuccess)
-    e = vcoef_tensor_map(&c->vmap32, c->coef32, 4, c->nx - 1, c->ny - 1, c->nz - 1);
+  const size_t ncoef = (size_t)kVCouplings * vmat_stride(c->N);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&c->vmat64, ncoef * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&c->vmat32, ncoef * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc((void**)&c->vmask, (size_t)c->N);
   if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_cg, sizeof(CGState));
   if (e == cudaSuccess)
@@ -122,42 +116,6 @@ static cudaError_t u_load(vfgpu_ctx* c, const ElemArgs& E, double* f, const doub
                                u0);
   if (e == cudaSuccess && c->has_insitu) e = launch_insitu_load(insitu_args(c), f, c->stream);
   return e;
-}
-
-template <typename T>
-static VApplyArgs<T> v_args(vfgpu_ctx* c, const T* x, T* y, const uint8_t* mask,
-                            const CUtensorMap& cmap, T* seam, const TilePlan& p) {
-  VApplyArgs<T> A{};
-  A.cmap = cmap;
-  A.cerr = c->d_cerr;
-  A.x = x;
-  A.y = y;
-  A.mask = mask;
-  A.elayer = c->d_elayer;
-  A.seamX = seam;
-  A.seamY = seam + p.seamX;
-  A.nx = c->nx;
-  A.ny = c->ny;
-  A.nz = c->nz;
-  A.ihx = T(1.0 / c->hx);
-  A.ihy = T(1.0 / c->hy);
-  A.ihz = T(1.0 / c->hz);
-  A.vol = T(c->hx * c->hy * c->hz);
-  A.P = c->d_params;
-  return A;
-}
-
-// VFGPU_ERR_CUDA when a V apply gave up waiting for its coefficient copies (the
-// flag is cleared for the next solve).
-static int check_cell_copies(vfgpu_ctx* c) {
-  unsigned flag = 0;
-  cudaError_t e = cudaMemcpyAsync(&flag, c->d_cerr, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return cuda_fail(e, "V apply");
-  if (!flag) return VFGPU_OK;
-  cudaMemsetAsync(c->d_cerr, 0, sizeof(unsigned), c->stream);
-  return fail(VFGPU_ERR_CUDA, "operator apply: a tensor copy (V coefficients or U node planes) did not "
-                              "complete in time");
 }
 
 // Reads n doubles of d_out into h_out (synchronising the stream).
@@ -298,15 +256,13 @@ static int u_dots_of(const vfgpu_ctx* c, const TilePlan& p, int prec_bytes) {
 }
 
 // Which CG call sites let the operator apply accumulate p.w (bit k-1 for call site k:
-// 1 U FP64, 2 U FP32, 3 V FP64, 4 V FP32); the others use a separate p.w pass.  U in
-// both precisions and V in FP64: the 129^3 mixed StepU measured 37.07 ms with the FP32
-// U apply accumulating p.w (the packed FP32 fixed-weight wave has the registers for it)
-// against 37.78 ms with the separate pass; with the earlier single-wave FP32 kernel the
-// accumulator spilled (U FP32 0.064 s fused-off against 0.066 s fused-on; FP64 U 0.0957 s
-// fused, 0.0972 s separate).  V FP32 fused as well measured 6.44 against 6.50 ms per
-// mixed StepV: not taken.
+// 1 U FP64, 2 U FP32, 3 V FP64, 4 V FP32); the others use a separate p.w pass.  U in both
+// precisions: the 129^3 mixed StepU measured 37.07 ms with the FP32 U apply accumulating p.w
+// (the packed FP32 fixed-weight wave has the registers for it) against 37.78 ms with the
+// separate pass; FP64 U 0.0957 s against 0.0972 s.  V: a node's row is in registers when its
+// x.y is known.
 #ifndef VFGPU_FUSE_DOT_MASK
-#define VFGPU_FUSE_DOT_MASK 7
+#define VFGPU_FUSE_DOT_MASK 15
 #endif
 static double* dot_buf(vfgpu_ctx* c, int kind) {
   return ((VFGPU_FUSE_DOT_MASK >> (kind - 1)) & 1) ? c->d_dot : nullptr;
@@ -521,7 +477,6 @@ int vfgpu_step_u(vfgpu_ctx* c, const vfgpu_solve_opts* o_, vfgpu_solve_stats* st
     if (w.expired() && !reason) reason = -100;
   }
   if (!reason) reason = -5;  // SNES_DIVERGED_MAX_IT
-  if (int rc2 = check_cell_copies(c)) return rc2;
   S.reason = reason;
   S.fnorm = fnorm;
   S.seconds = w.seconds();
@@ -536,19 +491,28 @@ int vfgpu_step_u(vfgpu_ctx* c, const vfgpu_solve_opts* o_, vfgpu_solve_stats* st
 namespace vfgpu {
 
 // ---------------------------------------------------------------------------- V
-static cudaError_t v_apply64(vfgpu_ctx* c, const double* x, double* y, const uint8_t* mask,
-                             const int* skip, double* dot = nullptr) {
-  VApplyArgs<double> A = v_args<double>(c, x, y, mask, c->vmap64, c->seam64, c->vplan64);
+template <typename T>
+static cudaError_t v_apply(vfgpu_ctx* c, const T* a, const T* x, T* y, const uint8_t* mask,
+                           const int* skip, double* dot) {
+  VMatArgs<T> A{};
+  A.a = a;
+  A.x = x;
+  A.y = y;
+  A.mask = mask;
   A.skip = skip;
   A.dot = dot;
-  return launch_v_apply<double>(A, c->vplan64, c->layers, c->stream);
+  A.nx = c->nx;
+  A.ny = c->ny;
+  A.nz = c->nz;
+  return launch_vmat_apply<T>(A, c->stream);
+}
+static cudaError_t v_apply64(vfgpu_ctx* c, const double* x, double* y, const uint8_t* mask,
+                             const int* skip, double* dot = nullptr) {
+  return v_apply<double>(c, c->vmat64, x, y, mask, skip, dot);
 }
 static cudaError_t v_apply32(vfgpu_ctx* c, const float* x, float* y, const uint8_t* mask,
                              const int* skip, double* dot = nullptr) {
-  VApplyArgs<float> A = v_args<float>(c, x, y, mask, c->vmap32, c->seam32, c->vplan32);
-  A.skip = skip;
-  A.dot = dot;
-  return launch_v_apply<float>(A, c->vplan32, c->layers, c->stream);
+  return v_apply<float>(c, c->vmat32, x, y, mask, skip, dot);
 }
 
 // F_V (VF_VResidual, VFMech.c:2687-2879) at v.
@@ -596,11 +560,10 @@ int vfgpu_step_v(vfgpu_ctx* c, const vfgpu_solve_opts* o_, vfgpu_solve_stats* st
   c->v32_stale = c->ul_stale = true;  // V changes from here on, also on an error return
   cudaError_t e = dev_v_bounds(c->f[VFGPU_FIELD_VIRREV], c->vf.atnum == 1, lb, ub, V, N, c->stream);
   if (e == cudaSuccess)
-    e = launch_v_coef(E, c->f[VFGPU_FIELD_U], c->f[VFGPU_FIELD_THETA], c->f[VFGPU_FIELD_THETAREF],
-                      c->coef64, mixed ? c->coef32 : nullptr, c->stream);
+    e = launch_v_assemble(E, c->f[VFGPU_FIELD_U], c->f[VFGPU_FIELD_THETA], c->f[VFGPU_FIELD_THETAREF],
+                          c->vmat64, mixed ? c->vmat32 : nullptr, c->stream);
   if (e == cudaSuccess) e = launch_v_rhs(E, c->f[VFGPU_FIELD_U], c->f[VFGPU_FIELD_PRESSURE], b, c->stream);
-  if (e == cudaSuccess) e = launch_v_diag(E, c->coef64, tmp, c->stream);
-  if (e == cudaSuccess) e = dev_inv(tmp, dinv, mixed ? dinv32 : nullptr, N, c->stream);
+  if (e == cudaSuccess) e = dev_inv(c->vmat64, dinv, mixed ? dinv32 : nullptr, N, c->stream);
   if (e == cudaSuccess) e = v_residual(c, V, b, tmp, F);
   if (e == cudaSuccess) e = dev_vi_norm2(F, V, lb, ub, N, c->d_red, c->d_out, c->stream);
   if (e == cudaSuccess) e = fetch(c, 1);
@@ -623,7 +586,7 @@ int vfgpu_step_v(vfgpu_ctx* c, const vfgpu_solve_opts* o_, vfgpu_solve_stats* st
     int kits = 0, kreason = 0;
     bool tmo = false;
     if (!mixed) {
-      CGVecs<double> v{Y, R, P, Wv, dinv, F, mask, N, dot_buf(c, 3), dots_of(c, c->vplan64)};
+      CGVecs<double> v{Y, R, P, Wv, dinv, F, mask, N, dot_buf(c, 3), vmat_blocks(N)};
       rc = run_cg<double>(c, 3, v, apply64, o.ksp_rtol, o.ksp_atol, o.ksp_dtol, o.ksp_maxit, w, &kits,
                           &kreason, &tmo);
       if (rc) return rc;
@@ -641,7 +604,7 @@ int vfgpu_step_v(vfgpu_ctx* c, const vfgpu_solve_opts* o_, vfgpu_solve_stats* st
       for (int k = 0; k < o.max_refine && zr > target; k++) {
         e = dev_to_f32(R, b32, N, c->stream);
         if (e != cudaSuccess) return cuda_fail(e, "vfgpu_step_v");
-        CGVecs<float> v{x32, r32, pp32, w32, dinv32, b32, mask, N, dot_buf(c, 4), dots_of(c, c->vplan32)};
+        CGVecs<float> v{x32, r32, pp32, w32, dinv32, b32, mask, N, dot_buf(c, 4), vmat_blocks(N)};
         const double in_rtol = std::max(o.inner_rtol, 0.5 * target / zr);
         int its32 = 0, r32reason = 0;
         rc = run_cg<float>(c, 4, v, apply32, in_rtol, 0.0, o.ksp_dtol, o.ksp_maxit, w, &its32,
@@ -707,7 +670,6 @@ int vfgpu_step_v(vfgpu_ctx* c, const vfgpu_solve_opts* o_, vfgpu_solve_stats* st
   }
   if (!reason) reason = -5;
   c->v32_stale = c->ul_stale = true;
-  if (int rc2 = check_cell_copies(c)) return rc2;
   S.reason = reason;
   S.fnorm = fnorm;
   S.seconds = w.seconds();
@@ -811,18 +773,15 @@ int vfgpu_memory_estimate(const vfgpu_grid* g, long long* bytes) {
   if (g->nx < 2 || g->ny < 2 || g->nz < 2)
     return fail(VFGPU_ERR_INVALID, "vfgpu_memory_estimate: bad grid");
   const long long N = (long long)g->nx * g->ny * g->nz;
-  const long long NC = (long long)(g->nx - 1) * (g->ny - 1) * (g->nz - 1);
   const TilePlan p64 = u_plan(g->nx, g->ny, g->nz, 8, 148), p32 = u_plan(g->nx, g->ny, g->nz, 4, 148);
-  const TilePlan q64 = v_plan(g->nx, g->ny, g->nz, 8, 148), q32 = v_plan(g->nx, g->ny, g->nz, 4, 148);
   long long b = 0;
   b += (2 * 3 * N + 5 * N) * 8;                          // fields U, BCU, V, VIrrev, theta, thetaRef, p
   b += N * 4 + (g->nz - 1) + 3 * N + 3 * N;              // V32, layers, BC kinds and bits
   b += (long long)(unit_lists_bytes(p64, g->nz) + unit_lists_bytes(p32, g->nz));  // U unit lists
-  b += (long long)std::max(p64.seamX + p64.seamY, q64.seamX + q64.seamY) * 8 +
-       (long long)std::max(p32.seamX + p32.seamY, q32.seamX + q32.seamY) * 4;
+  b += (long long)(p64.seamX + p64.seamY) * 8 + (long long)(p32.seamX + p32.seamY) * 4;
   b += 3 * 3 * N * 8 + 2 * 3 * N * 4;                    // staging vectors
   b += vfgpu_ctx::NP64 * (3 * N + kPoolSlack) * 8 + vfgpu_ctx::NP32 * (3 * N + kPoolSlack) * 4;
-  b += vcoef_size(g->nx - 1, g->ny - 1, g->nz - 1) * 12 + N;  // V coefficient (FP64 + FP32), mask
+  b += kVCouplings * (long long)vmat_stride(N) * 12 + N;  // V couplings (FP64 + FP32), mask
   b += (RED_BLOCKS + energy_blocks()) * 4 * 8 + 4096;    // reductions, scalars
   *bytes = b;
   return VFGPU_OK;
@@ -856,14 +815,14 @@ int vfgpu_v_residual(vfgpu_ctx* c, double* F) {
   const int64_t N = c->N;
   const int64_t Na = pool_stride(N);
   double *b = c->p64[0], *tmp = c->p64[0] + Na, *Fd = c->p64[0] + 2 * Na;
-  cudaError_t e = launch_v_coef(E, c->f[VFGPU_FIELD_U], c->f[VFGPU_FIELD_THETA],
-                                c->f[VFGPU_FIELD_THETAREF], c->coef64, nullptr, c->stream);
+  cudaError_t e = launch_v_assemble(E, c->f[VFGPU_FIELD_U], c->f[VFGPU_FIELD_THETA],
+                                    c->f[VFGPU_FIELD_THETAREF], c->vmat64, nullptr, c->stream);
   if (e == cudaSuccess) e = launch_v_rhs(E, c->f[VFGPU_FIELD_U], c->f[VFGPU_FIELD_PRESSURE], b, c->stream);
   if (e == cudaSuccess) e = v_residual(c, c->f[VFGPU_FIELD_V], b, tmp, Fd);
   if (e == cudaSuccess) e = copy_out(c, F, Fd, N);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "vfgpu_v_residual");
-  return check_cell_copies(c);
+  return VFGPU_OK;
 }
 
 }  // extern "C"

@@ -32,20 +32,11 @@
 //   so that a queued batch of iterations costs nothing once it is done), LIST:
 //   -1, or the unit list (A.ur, A.ustart, A.utotal) the operator's launches take when
 //   the list is given -- the U operator's units split by phase field over two
-//   launches, each with its own wave of blocks (unit lists 0 and 1) -- and PLANES_TMA:
-//   node planes by cp.async values (false) or, for an operator with the U inputs
-//   (interlaced x, v) and tensor maps A.xmap / A.vmap, by 1-D tensor copies per tile
-//   row (PlaneBox), completion on one mbarrier per ring slot (bounded waits,
-//   A.plane_err).
-// An Op with CV > 0 per-cell values (the V operator's 27 Gauss-point coefficients)
-//   supplies cell_map(A) (a 3-D tensor map, box 32 x TY x CV over (ex, ey, CV ez + g))
-//   and cell_err(A), and element(..., cc, cs) reads its cell's values from shared
-//   memory (cc[g cs]): one thread issues the tensor copy of element layer k + 2 into a
-//   2-stage buffer while layer k is computed, completion tracked by an mbarrier per
-//   stage.  The wait is bounded: a thread whose wait gives up sets *cell_err, the
-//   block stops at that layer's barrier (no further copy is issued), thread 0 waits
-//   (bounded again) for the copies still in flight into its stages, and the block
-//   returns.
+//   optional A.skip flag that turns a launch into a no-op (set by a converged CG,
+//   so that a queued batch of iterations costs nothing once it is done), and LIST:
+//   -1, or the unit list (A.ur, A.ustart, A.utotal) the operator's launches take when
+//   the list is given -- the U operator's units split by phase field over two
+//   launches, each with its own wave of blocks (unit lists 0 and 1).
 #pragma once
 
 #include <algorithm>
@@ -72,54 +63,23 @@ template <int TY, int EPT = 1> struct Tile {
 // two (layer k + 1's elements are written while layer k's node sums still read) where
 // MINB blocks of that size fit an SM, else one, with a second barrier per layer.
 constexpr int kRing = 4;
-// Tensor-copied node planes (Op::PLANES_TMA: the interlaced x, 3 values per node, and v):
-// a ring slot holds BY rows of x, then BY rows of v; each row is one 1-D tensor box that
-// starts at the row's first value rounded down to 16 bytes (A values), so XBOX / VBOX
-// values cover the row's 33 nodes after that shift, at 128-byte row pitches XP / VP.
-template <typename T> struct PlaneBox {
-  static constexpr int A = 16 / (int)sizeof(T);
-  static constexpr int XBOX = (99 + A - 1 + A - 1) / A * A, VBOX = (33 + A - 1 + A - 1) / A * A;
-  static constexpr int XP = (XBOX * (int)sizeof(T) + 127) / 128 * 128 / (int)sizeof(T);
-  static constexpr int VP = (VBOX * (int)sizeof(T) + 127) / 128 * 128 / (int)sizeof(T);
-};
 template <class Op, int TY> constexpr size_t ring_bytes() {
-  using T = typename Op::T;
-  if constexpr (Op::PLANES_TMA)
-    return sizeof(T) * kRing * Tile<TY>::BY * (PlaneBox<T>::XP + PlaneBox<T>::VP);
-  else
-    return sizeof(T) * kRing * Op::NIN * Tile<TY>::BX * Tile<TY>::BY;
+  return sizeof(typename Op::T) * kRing * Op::NIN * Tile<TY>::BX * Tile<TY>::BY;
 }
 template <class Op, int TY, int SCS = 2> constexpr size_t sc_bytes() {
   return sizeof(typename Op::T) * SCS * 4 * Op::NC * 33 * TY;
 }
-// ring, corner buffers and (PLANES_TMA) one mbarrier per ring slot
-template <class Op, int TY, int SCS = 2> constexpr size_t tile_base_bytes() {
-  return ring_bytes<Op, TY>() + sc_bytes<Op, TY, SCS>() + (Op::PLANES_TMA ? 8 * kRing : 0);
-}
 template <class Op, int TY, int MINB> constexpr int sc_stages() {
-  return (Op::CV > 0 || MINB * (tile_base_bytes<Op, TY, 2>() + 1024) <= 228 * 1024) ? 2 : 1;
-}
-// Per-cell value stages (Op::CV > 0): [kCellStages][CV][TY][32] at a 128-byte aligned
-// offset, then one 8-byte mbarrier per stage.
-constexpr int kCellStages = 2;
-template <class Op, int TY> constexpr size_t cell_off() { return (tile_base_bytes<Op, TY>() + 127) & ~size_t(127); }
-template <class Op, int TY> constexpr size_t cell_stage_bytes() {
-  return sizeof(typename Op::T) * Op::CV * TY * 32;
+  return MINB * (ring_bytes<Op, TY>() + sc_bytes<Op, TY, 2>() + 1024) <= 228 * 1024 ? 2 : 1;
 }
 template <class Op, int TY, int MINB> constexpr size_t tile_smem_bytes() {
-  if constexpr (Op::CV > 0)
-    return cell_off<Op, TY>() + kCellStages * cell_stage_bytes<Op, TY>() + kCellStages * 8;
-  else
-    return tile_base_bytes<Op, TY, sc_stages<Op, TY, MINB>()>();
+  return ring_bytes<Op, TY>() + sc_bytes<Op, TY, sc_stages<Op, TY, MINB>()>();
 }
 
-// mbarrier and tensor-copy primitives (one thread issues; every thread may wait).
+// mbarrier primitives with a bounded wait (one thread arrives; every thread may wait).
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"((unsigned)__cvta_generic_to_shared(bar)),
                "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_inval(uint64_t* bar) {
-  asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"((unsigned)__cvta_generic_to_shared(bar)) : "memory");
 }
 __device__ __forceinline__ void mbar_fence_init() {
   asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -154,26 +114,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, unsign
     }
   }
 }
-// 3-D tiled tensor copy global -> shared (no multicast), completion on bar.
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
-                                            uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(z), "r"((unsigned)__cvta_generic_to_shared(bar))
-      : "memory");
-}
-
-// 1-D tiled tensor copy global -> shared (no multicast), completion on bar; x: the first
-// element of the box (its byte offset a multiple of 16).
-__device__ __forceinline__ void tma_load_1d(void* dst, const CUtensorMap* map, int x, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.1d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2}], [%3];\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-      "l"(map), "r"(x), "r"((unsigned)__cvta_generic_to_shared(bar))
-      : "memory");
-}
-
 // Asynchronous global -> shared copy of one 4- or 8-byte value (LDGSTS); with
 // valid == false nothing is read and the destination is zero-filled.
 template <typename T>
@@ -201,11 +141,8 @@ __global__ void __launch_bounds__(32 * TY / Op::EPT, MINB)
   constexpr int NC = Op::NC, NIN = Op::NIN;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   constexpr int SCS = sc_stages<Op, TY, MINB>();
-  T* sx = reinterpret_cast<T*>(smem_raw);  // [kRing][NIN][BY][BX], or the PlaneBox rows
+  T* sx = reinterpret_cast<T*>(smem_raw);  // [kRing][NIN][BY][BX]
   T* sc = reinterpret_cast<T*>(smem_raw + ring_bytes<Op, TY>());  // [SCS][4*NC][TY][33]
-  [[maybe_unused]] uint64_t* pbar = nullptr;  // PLANES_TMA: one mbarrier per ring slot
-  if constexpr (Op::PLANES_TMA)
-    pbar = reinterpret_cast<uint64_t*>(smem_raw + ring_bytes<Op, TY>() + sc_bytes<Op, TY, SCS>());
   const int lane = threadIdx.x, wy = threadIdx.y, tid = wy * 32 + lane;
   const int nx = A.nx, ny = A.ny, nz = A.nz, nex = nx - 1, ney = ny - 1;
   // This block's share of the work: node planes [U b / n, U (b + 1) / n) of the
@@ -227,16 +164,7 @@ __global__ void __launch_bounds__(32 * TY / Op::EPT, MINB)
   }
   if (A.skip && *A.skip) return;  // converged solve: uniform early exit, before any barrier
   double dacc = 0.;  // this thread's share of x.y over the nodes it finishes (A.dot)
-  [[maybe_unused]] T* cbuf = nullptr;
-  [[maybe_unused]] uint64_t* cbar = nullptr;
-  if constexpr (Op::CV > 0) {
-    cbuf = reinterpret_cast<T*>(smem_raw + cell_off<Op, TY>());
-    cbar = reinterpret_cast<uint64_t*>(smem_raw + cell_off<Op, TY>() + kCellStages * cell_stage_bytes<Op, TY>());
-  }
-
-  // Returns false if a bounded wait on the per-cell copies gave up (the block then
-  // stops: see the layer barrier).
-  auto run_segment = [&](const int bx, const int by, const int z0, const int z1) -> bool {
+  auto run_segment = [&](const int bx, const int by, const int z0, const int z1) {
   const int X0 = bx * 32, Y0 = by * TY;
   const int kf = max(z0 - 1, 0), kl = min(z1, nz - 1) - 1;
 
@@ -258,53 +186,18 @@ __global__ void __launch_bounds__(32 * TY / Op::EPT, MINB)
       }
   };
 
-  // input q of the node in tile row w, column l of plane kz, from ring slot buf (with
-  // PLANES_TMA: x component q < 3 or v, at the row's 16-byte shift, which only the low
-  // bits of the row's first node index decide)
-  auto rv = [&](int buf, int kz, int q, int w, int l) -> T {
-    if constexpr (Op::PLANES_TMA) {
-      using PB = PlaneBox<T>;
-      const unsigned n0 = ((unsigned)kz * (unsigned)ny + (unsigned)(Y0 + w)) * (unsigned)nx + (unsigned)X0;
-      if (q < 3) return sx[(buf * G::BY + w) * PB::XP + 3 * l + q + (int)((3u * n0) & (PB::A - 1))];
-      return sx[kRing * G::BY * PB::XP + (buf * G::BY + w) * PB::VP + l + (int)(n0 & (PB::A - 1))];
-    } else {
-      return SXA(buf, q, w, l);
-    }
-  };
-
-  // issue the copies of node plane kz into ring slot buf: one cp.async group, or
-  // (PLANES_TMA) two tensor copies per tile row from warp 0, completing on pbar[buf]
+  // issue the copies of node plane kz into ring slot buf: one cp.async group
   auto fetch_plane = [&](int buf, int kz) {
-    if constexpr (Op::PLANES_TMA) {
-      using PB = PlaneBox<T>;
-      if (wy == 0) {
-        const int rows = min(G::BY, ny - Y0);
-        if (lane == 0)
-          mbar_expect_tx(&pbar[buf], (unsigned)(rows * (PB::XBOX + PB::VBOX) * sizeof(T)));
-        __syncwarp();
-        if (lane < rows) {
-          const int64_t n0 = ((int64_t)kz * ny + Y0 + lane) * nx + X0, e0 = 3 * n0;
-          tma_load_1d(sx + (buf * G::BY + lane) * PB::XP, &A.xmap, (int)(e0 - (e0 & (PB::A - 1))),
-                      &pbar[buf]);
-          tma_load_1d(sx + kRing * G::BY * PB::XP + (buf * G::BY + lane) * PB::VP, &A.vmap,
-                      (int)(n0 - (n0 & (PB::A - 1))), &pbar[buf]);
-        }
-      }
-    } else {
-      for (int s = tid; s < G::BX * G::BY; s += G::NT) {
-        const int l = s % G::BX, w = s / G::BX, X = X0 + l, Y = Y0 + w;
-        const bool in = X < nx && Y < ny;
-        const T* src[NIN];
-        Op::node_src(A, in ? node_index(X, Y, kz, nx, ny) : 0, src);
+    for (int s = tid; s < G::BX * G::BY; s += G::NT) {
+      const int l = s % G::BX, w = s / G::BX, X = X0 + l, Y = Y0 + w;
+      const bool in = X < nx && Y < ny;
+      const T* src[NIN];
+      Op::node_src(A, in ? node_index(X, Y, kz, nx, ny) : 0, src);
 #pragma unroll
-        for (int q = 0; q < NIN; q++) cp_async_val(&SXA(buf, q, w, l), src[q], in);
-      }
-      cp_async_commit();
+      for (int q = 0; q < NIN; q++) cp_async_val(&SXA(buf, q, w, l), src[q], in);
     }
+    cp_async_commit();
   };
-  // PLANES_TMA: the slot and phase parity of plane kz's copy in this segment
-  [[maybe_unused]] auto pslot = [&](int kz) { return (kz - kf) % kRing; };
-  [[maybe_unused]] auto pphase = [&](int kz) { return (unsigned)(((kz - kf) / kRing) & 1); };
 
   // fl: the node's flags (loaded ahead), buf: the ring slot holding plane z
   auto emit = [&](int l, int w, int X, int Y, int z, const T (&val)[NC], unsigned fl, int buf) {
@@ -313,7 +206,7 @@ __global__ void __launch_bounds__(32 * TY / Op::EPT, MINB)
     if (!(left || right || bot || top)) {
       T xin[NC];
 #pragma unroll
-      for (int c = 0; c < NC; c++) xin[c] = rv(buf, z, c, w, l);
+      for (int c = 0; c < NC; c++) xin[c] = SXA(buf, c, w, l);
       dacc += Op::template finish_node_in<DOT>(A, node_index(X, Y, z, nx, ny), val, fl, xin);
     } else if (left || right) {
       const int i = left ? bx : bx + 1;
@@ -338,48 +231,10 @@ __global__ void __launch_bounds__(32 * TY / Op::EPT, MINB)
   // Pipeline: planes kf, kf+1 resident before the first layer; during layer k the
   // copy of plane k+2 is in flight; one barrier per layer publishes plane k+2 and
   // the corner contributions of layer k together.
-  [[maybe_unused]] bool gave_up = false;
-  if constexpr (Op::PLANES_TMA) {
-    if (tid == 0) {
-      for (int st = 0; st < kRing; st++) mbar_init(&pbar[st], 1);
-      mbar_fence_init();
-    }
-    __syncthreads();  // initialised before any copy or wait
-  }
   fetch_plane(0, kf);
   fetch_plane(1, kf + 1);
-  // per-cell values of layers kf, kf + 1 (CV > 0): issued before the first barrier,
-  // which also publishes the mbarrier initialisation
-  [[maybe_unused]] auto fetch_cells = [&](int st, int kz) {
-    if constexpr (Op::CV > 0) {
-      mbar_expect_tx(&cbar[st], (unsigned)cell_stage_bytes<Op, TY>());
-      tma_load_3d(cbuf + (size_t)st * Op::CV * TY * 32, Op::cell_map(A), X0, Y0, Op::CV * kz, &cbar[st]);
-    }
-  };
-  if constexpr (Op::CV > 0) {
-    if (tid == 0) {
-      for (int st = 0; st < kCellStages; st++) mbar_init(&cbar[st], 1);
-      mbar_fence_init();
-      for (int st = 0; st < kCellStages; st++)
-        if (kf + st <= kl) fetch_cells(st, kf + st);
-    }
-  }
-  if constexpr (Op::PLANES_TMA) {
-    // bounded waits; if one gives up the block stops (thread 0 first waits, bounded again,
-    // for the copies in flight into slots 0 and 1) and the launch's results are void
-    gave_up = !mbar_wait(&pbar[0], 0u, A.plane_err);
-    gave_up = !mbar_wait(&pbar[1], 0u, A.plane_err) || gave_up;
-    if (__syncthreads_or(gave_up)) {
-      if (tid == 0) {
-        mbar_wait(&pbar[0], 0u, nullptr);
-        mbar_wait(&pbar[1], 0u, nullptr);
-      }
-      return false;
-    }
-  } else {
-    cp_async_wait_all();
-    __syncthreads();
-  }
+  cp_async_wait_all();
+  __syncthreads();
   if (kf + 2 <= kl + 1) fetch_plane(2, kf + 2);
   for (int k = kf; k <= kl; k++) {
     const int r0 = (k - kf) % kRing, r1 = (k - kf + 1) % kRing, sb = SCS == 2 ? (k - kf) & 1 : 0;
@@ -396,8 +251,6 @@ __global__ void __launch_bounds__(32 * TY / Op::EPT, MINB)
     if constexpr (EPT == 1) {
       const int ey = Y0 + wy;
       T yc[8][NC];
-      if constexpr (Op::CV > 0)
-        gave_up = !mbar_wait(&cbar[(k - kf) % kCellStages], ((k - kf) / kCellStages) & 1, Op::cell_err(A));
       if (ex < nex && ey < ney) {
         T in[8][NIN];
 #pragma unroll
@@ -408,14 +261,9 @@ __global__ void __launch_bounds__(32 * TY / Op::EPT, MINB)
             for (int i = 0; i < 2; i++) {
               const int a = i + 2 * j + 4 * kk, buf = kk ? r1 : r0;
 #pragma unroll
-              for (int q = 0; q < NIN; q++) in[a][q] = rv(buf, k + kk, q, wy + j, lane + i);
+              for (int q = 0; q < NIN; q++) in[a][q] = SXA(buf, q, wy + j, lane + i);
             }
-        if constexpr (Op::CV > 0)
-          Op::element(A, L, ex, ey, k, in, yc,
-                      cbuf + (size_t)((k - kf) % kCellStages) * Op::CV * TY * 32 + wy * 32 + lane,
-                      TY * 32);
-        else
-          Op::element(A, L, ex, ey, k, in, yc);
+        Op::element(A, L, ex, ey, k, in, yc);
       } else {
 #pragma unroll
         for (int a = 0; a < 8; a++)
@@ -446,7 +294,7 @@ __global__ void __launch_bounds__(32 * TY / Op::EPT, MINB)
               for (int i = 0; i < 2; i++) {
                 const int a = i + 2 * j + 4 * kk, buf = kk ? r1 : r0;
 #pragma unroll
-                for (int q = 0; q < NIN; q++) in[e][a][q] = rv(buf, k + kk, q, EPT * wy + e + j, lane + i);
+                for (int q = 0; q < NIN; q++) in[e][a][q] = SXA(buf, q, EPT * wy + e + j, lane + i);
               }
         Op::element_multi(A, L, ex, ey, k, ok, in, yc);
       } else {
@@ -460,38 +308,9 @@ __global__ void __launch_bounds__(32 * TY / Op::EPT, MINB)
 #pragma unroll
       for (int e = 0; e < EPT; e++) store_xsums(sb, EPT * wy + e, yc[e]);
     }
-    if constexpr (Op::PLANES_TMA) {  // plane k+2 has landed (bounded)
-      if (k + 2 <= kl + 1 && !mbar_wait(&pbar[pslot(k + 2)], pphase(k + 2), A.plane_err)) gave_up = true;
-    } else {
-      cp_async_wait_all();  // this thread's copies of plane k+2 have landed
-    }
-    if constexpr (Op::CV > 0) {
-      // ... and everyone's; corner contributions of layer k visible.  If any thread's
-      // wait on layer k's values gave up, the whole block stops here: no further copy
-      // is issued, thread 0 waits (bounded) for the tensor copies still in flight into
-      // the stages of layers k and k + 1, and the launch's results are void (the host
-      // sees *cell_err).
-      if (__syncthreads_or(gave_up)) {
-        if (tid == 0) {
-          mbar_wait(&cbar[(k - kf) % kCellStages], ((k - kf) / kCellStages) & 1, nullptr);
-          if (k + 1 <= kl)
-            mbar_wait(&cbar[(k + 1 - kf) % kCellStages], ((k + 1 - kf) / kCellStages) & 1, nullptr);
-        }
-        return false;
-      }
-    } else if constexpr (Op::PLANES_TMA) {
-      // ... corner contributions of layer k visible; if a wait on plane k+2 gave up the
-      // block stops, thread 0 waiting (bounded) for that plane's copies in flight
-      if (__syncthreads_or(gave_up)) {
-        if (tid == 0 && k + 2 <= kl + 1) mbar_wait(&pbar[pslot(k + 2)], pphase(k + 2), nullptr);
-        return false;
-      }
-    } else {
-      __syncthreads();    // ... and everyone's; corner contributions of layer k visible
-    }
+    cp_async_wait_all();  // this thread's copies of plane k+2 have landed
+    __syncthreads();      // ... and everyone's; corner contributions of layer k visible
     if (k + 3 <= kl + 1) fetch_plane((k + 3 - kf) % kRing, k + 3);  // the slot of plane k - 1
-    if constexpr (Op::CV > 0)  // layer k's stage is no longer read
-      if (tid == 0 && k + kCellStages <= kl) fetch_cells((k - kf) % kCellStages, k + kCellStages);
 #pragma unroll
     for (int si = 0; si < G::NSLOT; si++) {
       const int s = tid + si * G::NT;
@@ -533,7 +352,6 @@ __global__ void __launch_bounds__(32 * TY / Op::EPT, MINB)
            (nz - 1 - kf) % kRing);
     }
   }
-  return true;
   };  // run_segment
 
   if constexpr (Op::LIST >= 0)
@@ -551,17 +369,9 @@ __global__ void __launch_bounds__(32 * TY / Op::EPT, MINB)
       const int64_t left = u_end - u;
       z1 = left < (int64_t)(nz - z0) ? z0 + (int)left : nz;
     }
-    if (!run_segment(col % A.ntx, col / A.ntx, z0, z1)) break;  // block-uniform
+    run_segment(col % A.ntx, col / A.ntx, z0, z1);
     u += z1 - z0;
-    if (u < u_end) {
-      __syncthreads();  // the next segment reuses the shared-memory buffers
-      if constexpr (Op::CV > 0)  // every phase of the stages completed: re-armed by the next init
-        if (tid == 0)
-          for (int st = 0; st < kCellStages; st++) mbar_inval(&cbar[st]);
-      if constexpr (Op::PLANES_TMA)  // every plane copied was waited for
-        if (tid == 0)
-          for (int st = 0; st < kRing; st++) mbar_inval(&pbar[st]);
-    }
+    if (u < u_end) __syncthreads();  // the next segment reuses the shared-memory buffers
   }
   if constexpr (DOT) {
     __syncthreads();  // the shared-memory buffers are no longer read

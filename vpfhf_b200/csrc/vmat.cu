@@ -1,0 +1,72 @@
+// vmat.cu -- y = K_V x with the assembled couplings (vmat.h).
+#include <algorithm>
+
+#include "vmat.h"
+
+namespace vfgpu {
+
+namespace {
+
+constexpr int VM_THREADS = 256;
+// 4 blocks of 256 threads on each of 148 SMs: one wave
+constexpr int VM_BLOCKS = 592;
+
+// One thread per node, nodes in memory order, one wave of blocks that sweeps the planes
+// together, so that the 13 couplings a node shares with the nodes behind it (the planes just
+// read) come from L1 and L2 and HBM sees each coupling once.  A masked node costs its mask
+// byte: where the bounds are active (most of the grid in an AT1 problem) whole warps leave
+// at once.  Indices are linear: a neighbour beyond an x or y face lands on the next row's or
+// plane's node, whose coupling (or whose own) in that direction is 0; only the first and last
+// nodes of the array need the range checked (CHECK).
+// Measured at 129^3 inside the AT1 penny crack's StepV (few nodes free): 7.9 us a launch in
+// FP64 and 4.4 us in FP32, where the element form with its staged coefficients took 63.5 + 4.5
+// (seams) and 33.7 + 2.8 us (averages over a solve's launches, finished ones included); with
+// every node free 97 us in FP64 (element form 96 + 8.7).
+template <typename T, bool CHECK>
+__device__ __forceinline__ T vmat_row(const VMatArgs<T>& A, int64_t n, int64_t N, int64_t st) {
+  const int64_t row = A.nx, pl = (int64_t)A.nx * A.ny;
+  T r = A.a[n] * A.x[n];
+#pragma unroll
+  for (int d = 1; d < kVCouplings; d++) {
+    const int64_t o = kVForward[d][0] + kVForward[d][1] * row + kVForward[d][2] * pl;
+    if (!CHECK || n + o < N) r = fma(A.a[d * st + n], A.x[n + o], r);
+    if (!CHECK || n - o >= 0) r = fma(A.a[d * st + n - o], A.x[n - o], r);
+  }
+  return r;
+}
+
+template <typename T, bool DOT>
+__global__ void __launch_bounds__(VM_THREADS, 4) vmat_apply_kernel(const __grid_constant__ VMatArgs<T> A) {
+  __shared__ double red[32];
+  if (A.skip && *A.skip) return;  // converged solve
+  const int64_t N = (int64_t)A.nx * A.ny * A.nz, st = vmat_stride(N);
+  const int64_t reach = (int64_t)A.nx * A.ny + A.nx + 1;
+  double acc = 0.;
+  for (int64_t n = (int64_t)blockIdx.x * VM_THREADS + threadIdx.x; n < N; n += (int64_t)gridDim.x * VM_THREADS) {
+    T y = T(0);
+    if (!(A.mask && A.mask[n])) {
+      y = n >= reach && n + reach < N ? vmat_row<T, false>(A, n, N, st) : vmat_row<T, true>(A, n, N, st);
+      if constexpr (DOT) acc += (double)A.x[n] * (double)y;
+    }
+    A.y[n] = y;
+  }
+  if constexpr (DOT) {
+    const double s = block_sum_dbl(acc, red);
+    if (threadIdx.x == 0) A.dot[blockIdx.x] = s;
+  }
+}
+
+}  // namespace
+
+int vmat_blocks(int64_t n) { return (int)std::min<int64_t>(VM_BLOCKS, (n + VM_THREADS - 1) / VM_THREADS); }
+
+template <typename T> cudaError_t launch_vmat_apply(const VMatArgs<T>& A, cudaStream_t s) {
+  const int b = vmat_blocks((int64_t)A.nx * A.ny * A.nz);
+  if (A.dot) vmat_apply_kernel<T, true><<<b, VM_THREADS, 0, s>>>(A);
+  else vmat_apply_kernel<T, false><<<b, VM_THREADS, 0, s>>>(A);
+  return cudaGetLastError();
+}
+template cudaError_t launch_vmat_apply<double>(const VMatArgs<double>&, cudaStream_t);
+template cudaError_t launch_vmat_apply<float>(const VMatArgs<float>&, cudaStream_t);
+
+}  // namespace vfgpu
