@@ -67,3 +67,59 @@ def test_v_residual_and_energies(cuda, oracle_mod, n, atnum, thermal, cellE, lay
     assert cov == pytest.approx(cov_o, rel=1e-10) and ctx.crack_opening() == cov
     assert np.abs(cc - cc_o).max() <= 1e-10 * np.abs(cc_o).max()
     ctx.close()
+
+
+# Grids that take the U stencil: the smallest that do in FP64 (2000 units of 32 x 8 x 1), one
+# column past a 32 x 16 tile and its multiples, a chunk of few planes, faces not a multiple of
+# 30 columns or 4 planes; the last one also in FP32 (6000 units).
+STENCIL = [((34, 40, 200), (1.0, 1.0, 5.0)), ((66, 18, 223), (2.0, 0.6, 6.0)), ((35, 129, 64), (34.0, 128.0, 63.0)),
+           ((97, 99, 161), (1.1, 0.9, 1.7))]
+
+
+@pytest.mark.parametrize("n,l", STENCIL)
+@pytest.mark.parametrize("field", ["intact", "blob", "scaled"])
+def test_u_stencil(cuda, oracle_mod, n, l, field):
+    """K(v) x with the stencil at homogeneous nodes, against the oracle (FP64 1e-12 of the
+    largest entry, FP32 2e-6 normwise: the bounds of the element operator's tests) and the
+    same bits in every split mode; Dirichlet rows on all faces and one vertex, a field that
+    is intact, that has a random blob across tile seams and faces, and that is constant at
+    0.4 with a blob."""
+    import vpfhf_b200 as vg
+    E, nu, eta = 1e10, 0.3, 1e-6
+    rng = np.random.default_rng(sum(n))
+    o = oracle_mod.Oracle(n, l, E=E, nu=nu, eta=eta)
+    ctx = vg.VFContext(n, l, dict(E=E, nu=nu), eta=eta)
+    bc = vg.rollers()
+    bc[0] = vg.BCSpec(X0=vg.BC_ZERO, X1=vg.BC_ZERO, X1Y1Z0=vg.BC_ONE)
+    bc[2] = vg.BCSpec(Z0=vg.BC_ZERO, Y1=vg.BC_ZERO)
+    ctx.set_bc(bc)
+    mask = np.zeros((n[2], n[1], n[0], 3), np.uint8)
+    mask[:, :, [0, -1], 0] = 1
+    mask[:, [0, -1], :, 1] = 1
+    mask[0, :, :, 2] = mask[:, -1, :, 2] = 1
+    mask = mask.reshape(-1)
+    v = np.full(o.N, 0.4 if field == "scaled" else 1.0)
+    if field != "intact":
+        vv = v.reshape(n[2], n[1], n[0])
+        a = vv[n[2] // 3: n[2] // 3 + 5, 10:21, 25:]
+        a[...] = rng.uniform(0, 1, a.shape)
+        vv[-2:, :3, :4] = 0.7
+    ctx.set_field("V", v)
+    x = rng.standard_normal(3 * o.N) * 1e-3
+    xd = cuda.from_numpy(x).cuda()
+    yref = o.u_apply(v, x, mask)
+    y = ctx.u_apply(xd, vg.FP64)
+    assert np.abs(y.cpu().numpy() - yref).max() <= 1e-12 * np.abs(yref).max()
+    y32 = ctx.u_apply(xd, vg.MIXED)
+    assert np.linalg.norm(y32.cpu().numpy() - yref) <= 2e-6 * np.linalg.norm(yref)
+    for mode in ("on", "off"):
+        ctx.set_u_split(mode)
+        assert cuda.equal(ctx.u_apply(xd, vg.FP64), y)
+        assert cuda.equal(ctx.u_apply(xd, vg.MIXED), y32)
+    # the Dirichlet rows move with the boundary conditions, also when v does not
+    ctx.set_bc([vg.BCSpec(), vg.BCSpec(), vg.BCSpec(Z1=vg.BC_ZERO)])
+    m2 = np.zeros((n[2], n[1], n[0], 3), np.uint8)
+    m2[-1, :, :, 2] = 1
+    yref = o.u_apply(v, x, m2.reshape(-1))
+    assert np.abs(ctx.u_apply(xd, vg.FP64).cpu().numpy() - yref).max() <= 1e-12 * np.abs(yref).max()
+    ctx.close()

@@ -46,4 +46,9 @@ cudaError_t u_lists_refresh(vfgpu_ctx* c);
 // Whether the ctx's U applies in this precision (8 or 4 bytes) take the unit lists (and
 // write the second wave's x.y partials).
 bool u_lists_on(const vfgpu_ctx* c, int prec_bytes);
+// Whether the ctx's U applies in this precision take the stencil at homogeneous nodes: one
+// material, no per-cell modulus, no NOCOMPRESSION, a grid for which it pays.
+bool u_stencil_on(const vfgpu_ctx* c, int prec_bytes);
+// The lists an apply on the ctx's grid runs with (empty: one wave).
+vfgpu::UnitLists u_lists_of(const vfgpu_ctx* c, int prec_bytes);
 }  // namespace vfgpu

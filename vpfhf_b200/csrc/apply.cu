@@ -1,9 +1,11 @@
 // apply.cu -- instantiations of the tile engine for the U operator.
+#include <atomic>
 #include <mutex>
 #include <type_traits>
 
 #include "kernels.h"
 #include "ops.cuh"
+#include "u_stencil.cuh"
 
 namespace vfgpu {
 
@@ -67,6 +69,24 @@ constexpr int U32_MINB = kU32Packed ? (VFGPU_U32_PACKED_TY == 16 ? 1 : 2) : VFGP
 using U32Op = std::conditional_t<kU32Packed, UOpF2, UOp<float>>;
 using U32OpC = std::conditional_t<kU32Packed, UOpF2, UOp<float, true>>;
 
+template <typename T, int MINB> cudaError_t set_stencil_attributes();
+
+// Blocks per SM of the stencil kernel.
+#ifndef VFGPU_ST64_MINB
+#define VFGPU_ST64_MINB 2
+#endif
+#ifndef VFGPU_ST32_MINB
+#define VFGPU_ST32_MINB 3
+#endif
+constexpr int ST64_MINB = VFGPU_ST64_MINB, ST32_MINB = VFGPU_ST32_MINB;
+// Smallest grids, in (tile, plane) units, whose homogeneous nodes take the stencil.
+#ifndef VFGPU_ST64_MIN_UNITS
+#define VFGPU_ST64_MIN_UNITS 2000
+#endif
+#ifndef VFGPU_ST32_MIN_UNITS
+#define VFGPU_ST32_MIN_UNITS 6000
+#endif
+
 // Cubic cells take the U element with every 1/h folded into the row weight.
 template <typename T> bool cubic(const UApplyArgs<T>& A) { return A.ihx == A.ihy && A.ihy == A.ihz; }
 
@@ -85,6 +105,14 @@ cudaError_t apply_kernel_attributes() {
   if (e == cudaSuccess) e = set_tile_attributes<U32OpC, U32_TY, U32_MINB>();
   if (e == cudaSuccess) e = set_tile_attributes<UOpNC<double>, U64_TY, 1>();
   if (e == cudaSuccess) e = set_tile_attributes<UOpNC<float>, U_TY, 2>();
+  if (e == cudaSuccess) e = set_tile_attributes<UOpMarked<double>, U64_TY, U64_MINB>();
+  if (e == cudaSuccess) e = set_tile_attributes<UOpMarked<double, true>, U64_TY, U64_MINB>();
+  if constexpr (!kU32Packed) {
+    if (e == cudaSuccess) e = set_tile_attributes<UOpMarked<float>, U32_TY, U32_MINB>();
+    if (e == cudaSuccess) e = set_tile_attributes<UOpMarked<float, true>, U32_TY, U32_MINB>();
+  }
+  if (e == cudaSuccess) e = set_stencil_attributes<double, ST64_MINB>();
+  if (e == cudaSuccess) e = set_stencil_attributes<float, ST32_MINB>();
   return e;
 }
 
@@ -197,9 +225,12 @@ __device__ int block_scan_excl(int* a, int n, int* wsum) {
   return total;
 }
 
-// Unit type of node plane z of a tile column from its layer flags f[0, nz - 1):
-// 0 when the element layers below and above are constant (or absent), else 1.
+// Unit type of node plane z of a tile column: from its layer flags f[0, nz - 1), 0 when the
+// element layers below and above are constant (or absent), else 1; or (PLANES) its own
+// flag f[z], 1 when the unit holds a node the stencil does not write.
+template <bool PLANES>
 __device__ __forceinline__ int unit_type(const uint8_t* f, int z, int nez) {
+  if (PLANES) return f[z];
   const bool below = z == 0 || f[z - 1], above = z == nez || f[z];
   return below && above ? 0 : 1;
 }
@@ -209,6 +240,7 @@ __device__ __forceinline__ int unit_type(const uint8_t* f, int z, int nez) {
 // counted, offset by prefix sums over the columns in tile order, written; then, per
 // list l and block b of its wave of ncta_l blocks, the run holding the list's unit
 // U b / ncta_l (binary search on the runs' unit offsets).
+template <bool PLANES>
 __global__ void __launch_bounds__(1024) unit_lists_kernel(const uint8_t* __restrict__ cls, int nz,
                                                           int ncol, int ncta0, int ncta1, int4* __restrict__ runs0,
                                                           int4* __restrict__ runs1, int* __restrict__ start0,
@@ -218,10 +250,10 @@ __global__ void __launch_bounds__(1024) unit_lists_kernel(const uint8_t* __restr
   int* wsum = sh + 4 * ncol;
   const int nez = nz - 1;
   for (int c = threadIdx.x; c < ncol; c += blockDim.x) {
-    const uint8_t* f = cls + (int64_t)c * nez;
+    const uint8_t* f = cls + (int64_t)c * (PLANES ? nz : nez);
     int nr[2] = {0, 0}, nu[2] = {0, 0}, prev = -1;
     for (int z = 0; z < nz; z++) {
-      const int t = unit_type(f, z, nez);
+      const int t = unit_type<PLANES>(f, z, nez);
       nu[t]++;
       if (t != prev) nr[t]++;
       prev = t;
@@ -237,11 +269,11 @@ __global__ void __launch_bounds__(1024) unit_lists_kernel(const uint8_t* __restr
   for (int a = 0; a < 4; a++) tot[a] = block_scan_excl(cnt + a * ncol, ncol, wsum);
   int4* runs[2] = {runs0, runs1};
   for (int c = threadIdx.x; c < ncol; c += blockDim.x) {
-    const uint8_t* f = cls + (int64_t)c * nez;
+    const uint8_t* f = cls + (int64_t)c * (PLANES ? nz : nez);
     int r[2] = {cnt[c], cnt[ncol + c]}, u[2] = {cnt[2 * ncol + c], cnt[3 * ncol + c]};
-    int z0 = 0, t0 = unit_type(f, 0, nez);
+    int z0 = 0, t0 = unit_type<PLANES>(f, 0, nez);
     for (int z = 1; z <= nz; z++) {
-      const int t = z < nz ? unit_type(f, z, nez) : -1;
+      const int t = z < nz ? unit_type<PLANES>(f, z, nez) : -1;
       if (t != t0) {
         runs[t0][r[t0]++] = make_int4(c, z0, z, u[t0]);
         u[t0] += z - z0;
@@ -290,7 +322,7 @@ size_t unit_lists_bytes(const TilePlan& p, int nz) {
   const int64_t ncol = (int64_t)p.ntx * p.nty;
   if (nz < 2 || ncol > kMaxListCols) return 0;
   auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
-  return up(ncol * (nz - 1)) + 2 * up(ncol * nz * sizeof(int4)) + up(p.ncta0 * sizeof(int)) +
+  return up(ncol * nz) + 2 * up(ncol * nz * sizeof(int4)) + up(p.ncta0 * sizeof(int)) +
          up(p.ncta * sizeof(int)) + up(2 * sizeof(int));
 }
 
@@ -301,7 +333,7 @@ UnitLists unit_lists_carve(void* base, const TilePlan& p, int nz) {
   auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
   char* q = static_cast<char*>(base);
   L.cls = reinterpret_cast<uint8_t*>(q);
-  q += up(ncol * (nz - 1));
+  q += up(ncol * nz);
   for (int l = 0; l < 2; l++) {
     L.runs[l] = reinterpret_cast<int4*>(q);
     q += up(ncol * nz * sizeof(int4));
@@ -335,9 +367,119 @@ cudaError_t build_unit_lists(const double* v, int nx, int ny, int nz, const Tile
   }
   if (e != cudaSuccess) return e;
   const int ncol = p.ntx * p.nty;
-  unit_lists_kernel<<<1, 1024, (4 * ncol + 32) * sizeof(int), s>>>(
+  unit_lists_kernel<false><<<1, 1024, (4 * ncol + 32) * sizeof(int), s>>>(
       L.cls, nz, ncol, p.ncta0, p.ncta, L.runs[0], L.runs[1], L.start[0], L.start[1], L.total);
   return cudaGetLastError();
+}
+
+// ------------------------------------------------------------------ node flags
+// node[n] = the Dirichlet bits, kNodeOne where v = 1, kNodeElement where one of the up to 26
+// neighbours has another v.
+__global__ void __launch_bounds__(256) u_node_kernel(const double* __restrict__ v, const uint8_t* __restrict__ bc,
+                                                     uint8_t* __restrict__ node, int nx, int ny, int nz) {
+  const int64_t plane = (int64_t)nx * ny, N = plane * nz;
+  const int64_t n = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (n >= N) return;
+  const int k = (int)(n / plane), r = (int)(n - k * plane), j = r / nx, i = r - j * nx;
+  const double a = v[n];
+  bool same = true;
+#pragma unroll
+  for (int c = -1; c < 2; c++)
+#pragma unroll
+    for (int b = -1; b < 2; b++)
+#pragma unroll
+      for (int d = -1; d < 2; d++)
+        same &= v[node_index(min(max(i + d, 0), nx - 1), min(max(j + b, 0), ny - 1), min(max(k + c, 0), nz - 1), nx,
+                             ny)] == a;
+  node[n] = (uint8_t)(bc[n] | (a == 1. ? kNodeOne : 0u) | (same ? 0u : kNodeElement));
+}
+
+// type[col nz + z] = 1 when the 33 x (TY + 1) nodes of tile col in plane z hold one of the
+// element operator's.
+template <int TY>
+__global__ void __launch_bounds__(32 * TY) u_unit_type_kernel(const uint8_t* __restrict__ node,
+                                                               uint8_t* __restrict__ type, int nx, int ny, int nz) {
+  const int tid = threadIdx.y * 32 + threadIdx.x, k0 = blockIdx.z * kClsLayers;
+  for (int k = k0; k < min(k0 + kClsLayers, nz); k++) {
+    bool any = false;
+    for (int s = tid; s < 33 * (TY + 1); s += 32 * TY) {
+      const int X = blockIdx.x * 32 + s % 33, Y = blockIdx.y * TY + s / 33;
+      if (X < nx && Y < ny) any = any || (node[node_index(X, Y, k, nx, ny)] & kNodeElement);
+    }
+    const int t = __syncthreads_or(any);
+    if (tid == 0) type[(int64_t)(blockIdx.y * gridDim.x + blockIdx.x) * nz + k] = t ? 1 : 0;
+  }
+}
+
+// A homogeneous node that only listed units hold goes to the element operator too (those
+// units run in any case): the stencil keeps the nodes of at least one unlisted unit.
+__global__ void __launch_bounds__(256) u_node_demote_kernel(const uint8_t* __restrict__ type,
+                                                            uint8_t* __restrict__ node, int nx, int ny, int nz,
+                                                            int ty, int ntx, int nty) {
+  const int64_t plane = (int64_t)nx * ny, n = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (n >= plane * nz) return;
+  const unsigned f = node[n];
+  if (f & kNodeElement) return;
+  const int k = (int)(n / plane), r = (int)(n - k * plane), j = r / nx, i = r - j * nx;
+  // the tiles whose boxes hold the node: the one it starts and, on a seam, the one before
+  const int bx1 = min(i / 32, ntx - 1), by1 = min(j / ty, nty - 1);
+  const int bx0 = i % 32 == 0 && i > 0 ? i / 32 - 1 : bx1, by0 = j % ty == 0 && j > 0 ? j / ty - 1 : by1;
+  bool all = true;
+  for (int by = by0; by <= by1; by++)
+    for (int bx = bx0; bx <= bx1; bx++) all = all && type[(int64_t)(by * ntx + bx) * nz + k];
+  if (all) node[n] = (uint8_t)(f | kNodeElement);
+}
+
+// range[b]: the planes [x, y) of stencil block b's chunk that hold nodes of the stencil.
+__global__ void __launch_bounds__(256) u_srange_kernel(const uint8_t* __restrict__ node, int2* __restrict__ range,
+                                                       int nx, int ny, int nz, StencilPlan p) {
+  const int b = blockIdx.x, bx = b % p.ntx, by = (b / p.ntx) % p.nty, bz = b / (p.ntx * p.nty);
+  const int ka = bz * p.zc, kb = min(ka + p.zc, nz);
+  int lo = kb, hi = ka;
+  for (int k = ka; k < kb; k++) {
+    bool hit = false;
+    for (int s = threadIdx.x; s < ST_X * ST_Y; s += 256) {
+      const int i = 1 + bx * ST_X + s % ST_X, j = 1 + by * ST_Y + s / ST_X;
+      if (i < nx - 1 && j < ny - 1) hit = hit || !(node[node_index(i, j, k, nx, ny)] & kNodeElement);
+    }
+    if (__syncthreads_or(hit)) {
+      lo = min(lo, k);
+      hi = k + 1;
+    }
+  }
+  if (threadIdx.x == 0) range[b] = make_int2(lo, hi);
+}
+
+cudaError_t build_node_flags(const double* v, const uint8_t* bc, int nx, int ny, int nz, uint8_t* node,
+                             cudaStream_t s) {
+  const int64_t N = (int64_t)nx * ny * nz;
+  u_node_kernel<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(v, bc, node, nx, ny, nz);
+  return cudaGetLastError();
+}
+
+cudaError_t build_stencil_lists(uint8_t* node, int2* range, int nx, int ny, int nz, const TilePlan& p,
+                                const UnitLists& L, cudaStream_t s) {
+  const int runs = (nz + kClsLayers - 1) / kClsLayers, ncol = p.ntx * p.nty;
+  const int64_t N = (int64_t)nx * ny * nz;
+  const dim3 grid(p.ntx, p.nty, runs);
+  switch (p.ty) {
+    case 4: u_unit_type_kernel<4><<<grid, dim3(32, 4), 0, s>>>(node, L.cls, nx, ny, nz); break;
+    case 8: u_unit_type_kernel<8><<<grid, dim3(32, 8), 0, s>>>(node, L.cls, nx, ny, nz); break;
+    case 16: u_unit_type_kernel<16><<<grid, dim3(32, 16), 0, s>>>(node, L.cls, nx, ny, nz); break;
+    default: return cudaErrorInvalidValue;
+  }
+  u_node_demote_kernel<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(L.cls, node, nx, ny, nz, p.ty, p.ntx, p.nty);
+  u_srange_kernel<<<p.st.blocks(), 256, 0, s>>>(node, range, nx, ny, nz, p.st);
+  unit_lists_kernel<true><<<1, 1024, (4 * ncol + 32) * sizeof(int), s>>>(
+      L.cls, nz, ncol, p.ncta0, p.ncta, L.runs[0], L.runs[1], L.start[0], L.start[1], L.total);
+  return cudaGetLastError();
+}
+
+bool stencil_pays(const TilePlan& p, int nx, int ny, int nz, int prec_bytes) {
+  if (U64_TY != U32_TY || (prec_bytes == 4 && kU32Packed)) return false;  // the plans share the node flags
+  const int64_t ncol = (int64_t)p.ntx * p.nty;
+  if (std::min(nx, std::min(ny, nz)) < 8 || ncol > kMaxListCols || ceil_div(nz, kClsLayers) > 65535) return false;
+  return ncol * nz >= (prec_bytes == 8 ? VFGPU_ST64_MIN_UNITS : VFGPU_ST32_MIN_UNITS);
 }
 
 TilePlan u_plan(int nx, int ny, int nz, int prec_bytes, int num_sms) {
@@ -345,13 +487,61 @@ TilePlan u_plan(int nx, int ny, int nz, int prec_bytes, int num_sms) {
                          prec_bytes == 8 ? U64_MINB : U32_MINB, num_sms);
   const TilePlan q = tile_plan(nx, ny, nz, p.ty, 3, prec_bytes == 8 ? U64C_MINB : U32C_MINB, num_sms);
   p.ncta0 = q.ncta;
+  p.st = stencil_plan(nx, ny, nz, num_sms * (prec_bytes == 8 ? ST64_MINB : ST32_MINB));
   return p;
+}
+
+template <typename T, int MINB> cudaError_t set_stencil_attributes() {
+  static std::atomic<unsigned long long> done{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  constexpr int smem = (int)stencil_smem<T>();
+  e = cudaFuncSetAttribute(u_stencil_kernel<T, MINB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(u_stencil_kernel<T, MINB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
+}
+
+// Homogeneous nodes by the stencil, then the others by the element operator over unit list
+// 1, then the faces with the element operator's seams.  With A.dot the x.y partials go to
+// A.dot[0, blocks) (stencil), then ncta (elements), then nface + seam_blocks.
+template <class OpG, int TY, int MINB, int STB>
+static cudaError_t launch_u_stencil(typename OpG::Args A, const TilePlan& p, const LayerTable& L, cudaStream_t s) {
+  using T = typename OpG::T;
+  A.ntx = p.ntx;
+  A.nty = p.nty;
+  cudaError_t e = set_stencil_attributes<T, STB>();
+  if (e == cudaSuccess) e = set_tile_attributes<OpG, TY, MINB>();
+  if (e != cudaSuccess) return e;
+  constexpr size_t smem = stencil_smem<T>(), smemG = tile_smem_bytes<OpG, TY, MINB>();
+  const int nb = p.st.blocks(), oblocks = p.st.nface + seam_blocks(p, A.nx, A.ny, A.nz);
+  const dim3 block(32, TY);
+  typename OpG::Args AG = A;
+  if (AG.dot) AG.dot += nb;
+  if (A.dot) {
+    u_stencil_kernel<T, STB, true><<<nb, ST_THREADS, smem, s>>>(A, p.st);
+    tile_apply_kernel<OpG, TY, MINB, true><<<p.ncta, block, smemG, s>>>(AG, L);
+    u_outer_kernel<OpG, true><<<oblocks, 256, 0, s>>>(AG, TY, p.ncta, p.st.nface);
+  } else {
+    u_stencil_kernel<T, STB, false><<<nb, ST_THREADS, smem, s>>>(A, p.st);
+    tile_apply_kernel<OpG, TY, MINB, false><<<p.ncta, block, smemG, s>>>(AG, L);
+    u_outer_kernel<OpG, false><<<oblocks, 256, 0, s>>>(AG, TY, p.ncta, p.st.nface);
+  }
+  return cudaGetLastError();
 }
 
 template <>
 cudaError_t launch_u_apply<double>(const UApplyArgs<double>& A, const TilePlan& p,
                                    const LayerTable& L, cudaStream_t s) {
   if (A.cflag) return launch_tile_apply<UOpNC<double>, U64_TY, 1>(A, p, L, s);
+  if (A.node) {
+    if (cubic(A)) return launch_u_stencil<UOpMarked<double, true>, U64_TY, U64_MINB, ST64_MINB>(A, p, L, s);
+    return launch_u_stencil<UOpMarked<double>, U64_TY, U64_MINB, ST64_MINB>(A, p, L, s);
+  }
   if (A.ur[0] && A.ur[1]) {
     if (cubic(A))
       return launch_tile_apply_split<UOpConst<double, true>, UOp<double, true>, U64_TY, U64C_MINB, U64_MINB>(
@@ -368,6 +558,10 @@ cudaError_t launch_u_apply<float>(const UApplyArgs<float>& A, const TilePlan& p,
   // scalar tile (the packed build option keeps the plain operator packed)
   if (A.cflag) return launch_tile_apply<UOpNC<float>, U_TY, 2>(A, p, L, s);
   if constexpr (!kU32Packed) {
+    if (A.node) {
+      if (cubic(A)) return launch_u_stencil<UOpMarked<float, true>, U32_TY, U32_MINB, ST32_MINB>(A, p, L, s);
+      return launch_u_stencil<UOpMarked<float>, U32_TY, U32_MINB, ST32_MINB>(A, p, L, s);
+    }
     if (A.ur[0] && A.ur[1]) {
       if (cubic(A))
         return launch_tile_apply_split<U32COpC, U32OpC, U32_TY, U32C_MINB, U32_MINB>(A, p, L, s);

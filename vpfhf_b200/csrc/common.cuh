@@ -25,6 +25,34 @@ struct LayerTable {
   double Gc[VF_MAXLAYER];
 };
 
+// Coefficients of the U operator's separable stencil (u_stencil.cuh) at spacing (h0, h1, h2)
+// for the axes (0, 1, 2): P, Q, R of the rows and, for a node on a face across axis 1, the
+// terms of the half that is missing.
+struct StencilCoefs {
+  double xx, xy, yx, yy, xd, q, qz, rx, ry;
+  double g;               // R's multiple on the lowest plane
+  double em, el, fl, fm;  // face: of P_0, P_1; of R_1, R_2
+};
+inline StencilCoefs stencil_coefs(double lam, double mu, double h0, double h1, double h2) {
+  const double l2 = lam + 2. * mu, lm = lam + mu, a0 = h1 * h2 / h0, a1 = h0 * h2 / h1, a2 = h0 * h1 / h2;
+  StencilCoefs c;
+  c.xx = -l2 * a0;
+  c.xy = -mu * a1;
+  c.yx = -mu * a0;
+  c.yy = -l2 * a1;
+  c.xd = -lm * .25 * h2;
+  c.q = -mu * a2;
+  c.qz = -l2 * a2;
+  c.rx = -lm * .25 * h1;
+  c.ry = -lm * .25 * h0;
+  c.g = (mu - lam) / lm;
+  c.em = mu * .5 * h2;
+  c.el = lam * .5 * h2;
+  c.fl = lam * .5 * h0;
+  c.fm = mu * .5 * h0;
+  return c;
+}
+
 // Per-problem parameters the operator kernels read through a device pointer, so
 // that captured CUDA graphs stay valid when a ctx is re-used for another problem
 // (set-up calls rewrite this block instead of the kernels' by-value arguments).
@@ -32,6 +60,7 @@ struct DevParams {
   LayerTable L;
   double eta;                  // eta (VFProp.eta)
   double aeps[VF_MAXLAYER];    // Gc/(2 c_w) * eps per layer (V operator gradient term)
+  StencilCoefs st[2];          // layer 0: axes x, y, z, and y, x, z (the U stencil)
 };
 
 template <typename T> struct Vec3 { T x, y, z; };
@@ -40,7 +69,7 @@ __host__ __device__ inline int64_t node_index(int i, int j, int k, int nx, int n
   return ((int64_t)k * ny + j) * nx + i;
 }
 
-inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
+__host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Deterministic sum of one double per thread over a block (any 1-3D shape with a
 // multiple of 32 threads): warp shuffle trees, then warp 0 sums the warp totals in

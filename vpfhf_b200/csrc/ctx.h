@@ -27,6 +27,10 @@ struct vfgpu_ctx {
   void* d_ul = nullptr;
   vfgpu::UnitLists ul64, ul32;
   bool ul_stale = true;
+  // per-node flags and per-block plane ranges of the stencil (UApplyArgs::node, srange), for
+  // grids that take it; built with the lists
+  uint8_t* d_unode = nullptr;
+  int2 *d_srange64 = nullptr, *d_srange32 = nullptr;
   int u_split = VFGPU_U_SPLIT_AUTO;
   vfgpu::DevParams* d_params = nullptr;  // device copy of layers / eta / aeps
   float* d_cellE = nullptr;     // NC or null

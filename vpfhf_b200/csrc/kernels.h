@@ -21,6 +21,10 @@ struct UnitLists {
   int4* runs[2] = {};      // [ntx nty nz] each
   int* start[2] = {};      // [ncta0], [ncta]
   int* total = nullptr;    // [2]
+  // The stencil's flags (UApplyArgs::node, srange), null where the grid or the problem takes
+  // the element operator alone; cls then holds a type per (tile, plane)
+  uint8_t* node = nullptr;
+  int2* srange = nullptr;
 };
 // Device bytes of a plan's unit lists; 0 when the grid has more tile columns than the
 // one-block list builder takes (its applies then split all units).
@@ -32,12 +36,25 @@ bool unit_lists_pay(const TilePlan& p, int nz, int prec_bytes);
 // Rebuilds the lists from the FP64 phase field v (two launches on s).
 cudaError_t build_unit_lists(const double* v, int nx, int ny, int nz, const TilePlan& p,
                              const UnitLists& L, cudaStream_t s);
+// Whether the plan's homogeneous nodes take the stencil in precision prec_bytes (a rule of
+// the grid alone, so that every apply of a grid gives the same bits).
+bool stencil_pays(const TilePlan& p, int nx, int ny, int nz, int prec_bytes);
+inline size_t stencil_range_bytes(const TilePlan& p) { return sizeof(int2) * (size_t)p.st.blocks(); }
+// The node flags from the FP64 phase field and the Dirichlet bits; then, per plan, the
+// unit lists from them (with the nodes of listed units alone handed to the elements) and the
+// stencil blocks' plane ranges.  Plans of the same tiles may share the node flags.
+cudaError_t build_node_flags(const double* v, const uint8_t* bc, int nx, int ny, int nz, uint8_t* node,
+                             cudaStream_t s);
+cudaError_t build_stencil_lists(uint8_t* node, int2* range, int nx, int ny, int nz, const TilePlan& p,
+                                const UnitLists& L, cudaStream_t s);
 template <typename T> void use_unit_lists(UApplyArgs<T>& A, const UnitLists& L) {
   for (int l = 0; l < 2; l++) {
     A.ur[l] = L.cls ? L.runs[l] : nullptr;
     A.ustart[l] = L.cls ? L.start[l] : nullptr;
   }
   A.utotal = L.cls ? L.total : nullptr;
+  A.node = L.cls ? L.node : nullptr;
+  A.srange = L.srange;
 }
 
 template <typename T>

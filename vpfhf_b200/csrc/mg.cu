@@ -638,7 +638,7 @@ template <typename T> LevelT<T> view(vfgpu_ctx* c, int l) {
     V.cellE = c->d_cellE;
     V.dinv = (const T*)c->mg_dinv0;
     V.cflag = c->unilateral ? c->d_cflag : nullptr;
-    V.ul = u_lists_on(c, (int)sizeof(T)) ? (sizeof(T) == 8 ? c->ul64 : c->ul32) : UnitLists{};
+    V.ul = u_lists_of(c, (int)sizeof(T));
     V.n3 = 3 * c->N;
   } else {
     V.nx = L.nx;
@@ -678,6 +678,9 @@ template <typename T> UApplyArgs<T> level_args(vfgpu_ctx* c, const LevelT<T>& V,
   A.ihy = T(1.0 / V.hy);
   A.ihz = T(1.0 / V.hz);
   A.vol = T(V.hx * V.hy * V.hz);
+  A.hx = V.hx;
+  A.hy = V.hy;
+  A.hz = V.hz;
   A.eta = T(c->vf.eta);
   A.P = c->d_params;
   A.cflag = V.cflag;
@@ -1048,7 +1051,7 @@ int mgcg(vfgpu_ctx* c, const double* b, double* x, double* r, double* p, double*
   outer.elayer = c->d_elayer;
   outer.cellE = c->d_cellE;
   outer.cflag = c->unilateral ? c->d_cflag : nullptr;
-  outer.ul = u_lists_on(c, 8) ? c->ul64 : UnitLists{};
+  outer.ul = u_lists_of(c, 8);
   while (!*reason && e == cudaSuccess) {
     e = level_apply<double>(c, outer, p, w);
     const double* pa[1] = {p};

@@ -83,6 +83,7 @@ template <typename T_, bool CUBIC = false> struct UOp {
   __device__ __forceinline__ static unsigned node_flags(const Args& A, int64_t n) {
     return A.bc ? A.bc[n] : 0u;
   }
+  __device__ __forceinline__ static bool skip_node(unsigned) { return false; }
   // Writes y of node n (Dirichlet rows: y = x) from the node's flags b and input
   // values xin; with DOT, returns x.y over its dofs (the launch accumulates the CG dot
   // into A.dot).
@@ -163,6 +164,7 @@ template <typename T_> struct UOpNC {
   __device__ __forceinline__ static unsigned node_flags(const Args& A, int64_t n) {
     return UOp<T>::node_flags(A, n);
   }
+  __device__ __forceinline__ static bool skip_node(unsigned) { return false; }
   template <bool DOT>
   __device__ __forceinline__ static double finish_node_in(const Args& A, int64_t n, const T (&val)[NC],
                                                           unsigned b, const T (&xin)[NC]) {
@@ -224,6 +226,7 @@ struct UOpF2 {
   __device__ __forceinline__ static unsigned node_flags(const Args& A, int64_t n) {
     return UOp<float>::node_flags(A, n);
   }
+  __device__ __forceinline__ static bool skip_node(unsigned) { return false; }
   template <bool DOT>
   __device__ __forceinline__ static double finish_node_in(const Args& A, int64_t n, const T (&val)[NC],
                                                           unsigned b, const T (&xin)[NC]) {
@@ -285,6 +288,7 @@ template <bool CUBIC = false> struct UOpF2Const {
   __device__ __forceinline__ static unsigned node_flags(const Args& A, int64_t n) {
     return UOp<float>::node_flags(A, n);
   }
+  __device__ __forceinline__ static bool skip_node(unsigned) { return false; }
   template <bool DOT>
   __device__ __forceinline__ static double finish_node_in(const Args& A, int64_t n, const T (&val)[NC],
                                                           unsigned b, const T (&xin)[NC]) {

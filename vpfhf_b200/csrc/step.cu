@@ -250,9 +250,9 @@ static cudaError_t u_apply32(vfgpu_ctx* c, const float* x, float* y, const int* 
   return launch_u_apply<float>(A, c->plan32, c->layers, c->stream);
 }
 static int dots_of(const vfgpu_ctx* c, const TilePlan& p) { return tile_dot_count(p, c->nx, c->ny, c->nz); }
-// The U applies of a split launch (unit lists) write a second wave's partials.
+// The U applies with unit lists or the stencil write a second wave's partials.
 static int u_dots_of(const vfgpu_ctx* c, const TilePlan& p, int prec_bytes) {
-  return dots_of(c, p) + (u_lists_on(c, prec_bytes) ? p.ncta0 : 0);
+  return dots_of(c, p) + (u_stencil_on(c, prec_bytes) ? p.st.blocks() + p.st.nface : u_lists_on(c, prec_bytes) ? p.ncta0 : 0);
 }
 
 // Which CG call sites let the operator apply accumulate p.w (bit k-1 for call site k:
@@ -778,6 +778,7 @@ int vfgpu_memory_estimate(const vfgpu_grid* g, long long* bytes) {
   b += (2 * 3 * N + 5 * N) * 8;                          // fields U, BCU, V, VIrrev, theta, thetaRef, p
   b += N * 4 + (g->nz - 1) + 3 * N + 3 * N;              // V32, layers, BC kinds and bits
   b += (long long)(unit_lists_bytes(p64, g->nz) + unit_lists_bytes(p32, g->nz));  // U unit lists
+  b += N + (long long)(stencil_range_bytes(p64) + stencil_range_bytes(p32));  // U node and block flags
   b += (long long)(p64.seamX + p64.seamY) * 8 + (long long)(p32.seamX + p32.seamY) * 4;
   b += 3 * 3 * N * 8 + 2 * 3 * N * 4;                    // staging vectors
   b += vfgpu_ctx::NP64 * (3 * N + kPoolSlack) * 8 + vfgpu_ctx::NP32 * (3 * N + kPoolSlack) * 4;

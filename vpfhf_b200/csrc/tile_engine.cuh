@@ -25,7 +25,8 @@
 //   element_multi(A, L, ex, ey[EPT], ez, ok[EPT], in[EPT][8][NIN], out[EPT][8][NC])
 //   (EPT > 1; out[e] must be 0 where ok[e] is false),
 //   finish_node<DOT>(A, n, val[NC]) (writes y, applying Dirichlet rows / masks; with
-//   DOT returns the node's x.y), node_flags(A, n) and finish_node_in<DOT>(A, n, val,
+//   DOT returns the node's x.y), skip_node(flags) (true: another kernel writes the node),
+//   node_flags(A, n) and finish_node_in<DOT>(A, n, val,
 //   flags, xin[NC]) (the same from flags loaded ahead and the node's inputs from the
 //   plane ring), and an
 //   optional A.skip flag that turns a launch into a no-op (set by a converged CG,
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(32 * TY / Op::EPT, MINB)
 
   // fl: the node's flags (loaded ahead), buf: the ring slot holding plane z
   auto emit = [&](int l, int w, int X, int Y, int z, const T (&val)[NC], unsigned fl, int buf) {
+    if (Op::skip_node(fl)) return;
     const bool left = (l == 0 && bx > 0), right = (l == 32 && bx < A.ntx - 1);
     const bool bot = (w == 0 && by > 0), top = (w == TY && by < A.nty - 1);
     if (!(left || right || bot || top)) {
@@ -386,48 +388,99 @@ __global__ void __launch_bounds__(32 * TY / Op::EPT, MINB)
 // seam node in a fixed order and finishes the node (Op::finish_node); with A.dot,
 // block b's share of x.y goes to A.dot[dot_base + b].
 template <class Op, bool DOT>
-__global__ void __launch_bounds__(256) seam_fixup_kernel(const typename Op::Args A, int TY, int dot_base) {
+__device__ __forceinline__ double seam_range(const typename Op::Args& A, int TY, int64_t first, int64_t step) {
   using T = typename Op::T;
   constexpr int NC = Op::NC;
-  __shared__ double red[32];
   const int nx = A.nx, ny = A.ny, nz = A.nz;
-  if (A.skip && *A.skip) return;
   double dacc = 0.;
   const int64_t nxs = (int64_t)(A.ntx - 1) * nz * ny;
   const int64_t nys = (int64_t)(A.nty - 1) * nz * nx;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nxs + nys;
-       t += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t t = first; t < nxs + nys; t += step) {
     T val[NC];
     int64_t n;
     if (t < nxs) {
       const int Y = (int)(t % ny);
       const int64_t r = t / ny;
       const int z = (int)(r % nz), i = (int)(r / nz) + 1;
+      n = node_index(32 * i, Y, z, nx, ny);
+      if (Op::skip_node(Op::node_flags(A, n))) continue;
       const bool onY = (Y % TY == 0) && (Y > 0) && (Y / TY < A.nty);
       const T* p = A.seamX + t * 4 * NC;
 #pragma unroll
       for (int c = 0; c < NC; c++)
         val[c] = onY ? ((p[c] + p[NC + c]) + p[2 * NC + c]) + p[3 * NC + c] : p[c] + p[NC + c];
-      n = node_index(32 * i, Y, z, nx, ny);
     } else {
       const int64_t u = t - nxs;
       const int X = (int)(u % nx);
       const int64_t r = u / nx;
       const int z = (int)(r % nz), j = (int)(r / nz) + 1;
       if (X % 32 == 0 && X > 0 && X / 32 < A.ntx) continue;
+      n = node_index(X, TY * j, z, nx, ny);
+      if (Op::skip_node(Op::node_flags(A, n))) continue;
       const T* p = A.seamY + u * 2 * NC;
 #pragma unroll
       for (int c = 0; c < NC; c++) val[c] = p[c] + p[NC + c];
-      n = node_index(X, TY * j, z, nx, ny);
     }
     dacc += Op::template finish_node<DOT>(A, n, val);
   }
+  return dacc;
+}
+template <class Op, bool DOT>
+__global__ void __launch_bounds__(256) seam_fixup_kernel(const typename Op::Args A, int TY, int dot_base) {
+  __shared__ double red[32];
+  if (A.skip && *A.skip) return;
+  const double dacc = seam_range<Op, DOT>(A, TY, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
+                                          (int64_t)gridDim.x * blockDim.x);
   if constexpr (DOT) {
     const double bs = block_sum_dbl(dacc, red);
     if (threadIdx.x == 0) A.dot[dot_base + blockIdx.x] = bs;
   }
 }
 
+
+#ifndef VFGPU_ST_RY
+#define VFGPU_ST_RY 4
+#endif
+#ifndef VFGPU_ST_W
+#define VFGPU_ST_W 4
+#endif
+constexpr int ST_X = 32, ST_RY = VFGPU_ST_RY, ST_W = VFGPU_ST_W, ST_Y = ST_RY * ST_W, ST_THREADS = 32 * ST_W;
+// Launch shape of the U operator's stencil (u_stencil.cuh): 32 x ST_Y column tiles in chunks
+// of zc planes, and the blocks of the x and y faces and the edges in its last launch,
+// 8 warps each.
+struct StencilPlan {
+  int ntx = 0, nty = 0, nchunk = 0, zc = 0;
+  int nface = 0;
+  __host__ __device__ int blocks() const { return ntx * nty * nchunk; }
+};
+constexpr int ST_FACE_Z = 4;  // nodes of a face column one thread does
+// Warps of the x and y faces: a warp does up to 30 columns of a face, ST_FACE_Z nodes of each.
+__host__ __device__ inline int face_groups(int nx, int ny) { return 2 * ceil_div(nx - 2, 30) + 2 * ceil_div(ny - 2, 30); }
+__host__ __device__ inline int face_warps(int nx, int ny, int nz) { return face_groups(nx, ny) * ceil_div(nz - 2, ST_FACE_Z); }
+// Nodes of the box's edges (grids of at least 3 nodes per axis).
+__host__ __device__ inline int edge_nodes(int nx, int ny, int nz) { return 4 * (nx - 2) + 4 * (ny - 2) + 4 * nz; }
+// slots: blocks the device holds at once.  The chunk count is the one whose waves of
+// (planes + 2 halo planes + about 2 planes of ring fill) end first.
+inline StencilPlan stencil_plan(int nx, int ny, int nz, int slots) {
+  StencilPlan p;
+  if (nx < 3 || ny < 3 || nz < 3) return p;  // such grids keep the element operator
+  p.ntx = ceil_div(nx - 2, ST_X);
+  p.nty = ceil_div(ny - 2, ST_Y);
+  p.nface = std::min(148 * 4, ceil_div(face_warps(nx, ny, nz), 8));
+  const int tiles = p.ntx * p.nty;
+  int64_t best = -1;
+  p.nchunk = 1;
+  for (int c = 1; c <= ceil_div(nz, 2); c++) {
+    const int64_t waves = ((int64_t)tiles * c + slots - 1) / slots, cost = waves * (ceil_div(nz, c) + 4);
+    if (best < 0 || cost < best) {
+      best = cost;
+      p.nchunk = c;
+    }
+  }
+  p.zc = ceil_div(nz, p.nchunk);
+  p.nchunk = ceil_div(nz, p.zc);
+  return p;
+}
 
 // Launch plan: xy tiles of 32 x ty elements, the blocks of one launch (one wave of
 // ctas_per_sm blocks per SM, or one unit per block on small grids) and the seam buffer
@@ -438,6 +491,7 @@ struct TilePlan {
   int ncta0;  // the wave of a split launch's unit list 0 (UOpConst), which may take more
               // blocks per SM; = ncta otherwise
   size_t seamX, seamY;
+  StencilPlan st;  // U plans only
 };
 
 inline TilePlan tile_plan(int nx, int ny, int nz, int ty, int nc, int ctas_per_sm, int num_sms) {

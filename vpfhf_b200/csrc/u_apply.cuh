@@ -29,11 +29,20 @@
 
 namespace vfgpu {
 
+// Bits of UApplyArgs::node: 0-2 Dirichlet components, then
+constexpr unsigned kNodeOne = 0x40;      // v == 1 exactly
+constexpr unsigned kNodeElement = 0x80;  // not homogeneous: an element-operator node
+
 template <typename T> struct UApplyArgs {
   const T* __restrict__ x;            // 3N interlaced input
   const T* __restrict__ v;            // N phase field
   T* __restrict__ y;                  // 3N output
   const uint8_t* __restrict__ bc;     // N: bit c => dof (node,c) is Dirichlet
+  const uint8_t* __restrict__ node;   // N: bc with kNodeOne / kNodeElement (u_stencil.cuh), or null;
+                                      // given: the stencil writes the homogeneous nodes and the
+                                      // element operator (unit list 1) the others
+  const int2* __restrict__ srange;    // with node: per stencil block the planes [x, y) of its chunk
+                                      // that hold nodes of the stencil
   const uint8_t* __restrict__ elayer; // nz-1: material layer of element layer ek (or null)
   const float* __restrict__ cellE;    // per-cell Young's modulus (or null)
   T* __restrict__ seamX;              // x-seam partials [(ntx-1)][nz][ny][4][3]
@@ -54,6 +63,7 @@ template <typename T> struct UApplyArgs {
   int nx, ny, nz;
   int ntx, nty;                       // tiles in x, y
   T ihx, ihy, ihz, vol, eta;
+  double hx, hy, hz;                  // (with node) the spacing
 };
 
 // Modal transform of nodal values f[a], a = i + 2j + 4k, into m[p], p = a + 2b + 4c

@@ -110,6 +110,8 @@ int upload_params(vfgpu_ctx* c) {
   DevParams P{};
   P.L = c->layers;
   P.eta = c->vf.eta;
+  P.st[0] = stencil_coefs(c->layers.lambda[0], c->layers.mu[0], c->hx, c->hy, c->hz);
+  P.st[1] = stencil_coefs(c->layers.lambda[0], c->layers.mu[0], c->hy, c->hx, c->hz);
   const double atcv = c->vf.atnum == 1 ? 2. / 3. : .5;  // VFCommon.c:482-492
   for (int l = 0; l < VF_MAXLAYER; l++) P.aeps[l] = c->layers.Gc[l] / atcv * .5 * c->vf.epsilon;
   cudaError_t e = cudaMemcpyAsync(c->d_params, &P, sizeof P, cudaMemcpyHostToDevice, c->stream);
@@ -136,17 +138,25 @@ UApplyArgs<T> u_args(vfgpu_ctx* c, const T* x, const T* v, T* y, T* seam, const 
   A.ihy = T(1.0 / c->hy);
   A.ihz = T(1.0 / c->hz);
   A.vol = T(c->hx * c->hy * c->hz);
+  A.hx = c->hx;
+  A.hy = c->hy;
+  A.hz = c->hz;
   A.eta = T(c->vf.eta);
   A.P = c->d_params;
   A.cflag = c->unilateral ? c->d_cflag : nullptr;
-  use_unit_lists(A, u_lists_on(c, (int)sizeof(T)) ? (sizeof(T) == 8 ? c->ul64 : c->ul32) : UnitLists{});
+  use_unit_lists(A, u_lists_of(c, (int)sizeof(T)));
   return A;
 }
-// The split mode and the grid call for the lists in this precision (NOCOMPRESSION aside).
+bool u_stencil_on(const vfgpu_ctx* c, int prec_bytes) {
+  return (prec_bytes == 8 ? c->d_srange64 : c->d_srange32) && c->nlayer == 1 && !c->d_cellE && !c->unilateral;
+}
+
+// The stencil, or the split mode and the grid, call for the lists in this precision
+// (NOCOMPRESSION aside).
 static bool u_lists_wanted(const vfgpu_ctx* c, int prec_bytes) {
   const TilePlan& p = prec_bytes == 8 ? c->plan64 : c->plan32;
   if (!(prec_bytes == 8 ? c->ul64.cls : c->ul32.cls)) return false;
-  if (c->u_split == VFGPU_U_SPLIT_ON) return true;
+  if (u_stencil_on(c, prec_bytes) || c->u_split == VFGPU_U_SPLIT_ON) return true;
   return c->u_split == VFGPU_U_SPLIT_AUTO && unit_lists_pay(p, c->nz, prec_bytes);
 }
 
@@ -154,15 +164,31 @@ cudaError_t u_lists_refresh(vfgpu_ctx* c) {
   if (!c->ul_stale) return cudaSuccess;
   const double* v = c->f[VFGPU_FIELD_V];
   cudaError_t e = cudaSuccess;
-  if (u_lists_wanted(c, 8)) e = build_unit_lists(v, c->nx, c->ny, c->nz, c->plan64, c->ul64, c->stream);
-  if (e == cudaSuccess && u_lists_wanted(c, 4))
-    e = build_unit_lists(v, c->nx, c->ny, c->nz, c->plan32, c->ul32, c->stream);
+  const bool s64 = u_stencil_on(c, 8), s32 = u_stencil_on(c, 4);
+  if (s64 || s32)
+    e = build_node_flags(v, c->bcU_bits, c->nx, c->ny, c->nz, c->d_unode, c->stream);
+  auto lists = [&](bool st, int2* range, const TilePlan& p, const UnitLists& L) {
+    return st ? build_stencil_lists(c->d_unode, range, c->nx, c->ny, c->nz, p, L, c->stream)
+              : build_unit_lists(v, c->nx, c->ny, c->nz, p, L, c->stream);
+  };
+  if (e == cudaSuccess && u_lists_wanted(c, 8)) e = lists(s64, c->d_srange64, c->plan64, c->ul64);
+  if (e == cudaSuccess && u_lists_wanted(c, 4)) e = lists(s32, c->d_srange32, c->plan32, c->ul32);
   if (e == cudaSuccess) c->ul_stale = false;
   return e;
 }
 
 bool u_lists_on(const vfgpu_ctx* c, int prec_bytes) {
   return !c->unilateral && u_lists_wanted(c, prec_bytes);
+}
+
+UnitLists u_lists_of(const vfgpu_ctx* c, int prec_bytes) {
+  if (!u_lists_on(c, prec_bytes)) return UnitLists{};
+  UnitLists L = prec_bytes == 8 ? c->ul64 : c->ul32;
+  if (u_stencil_on(c, prec_bytes)) {
+    L.node = c->d_unode;
+    L.srange = prec_bytes == 8 ? c->d_srange64 : c->d_srange32;
+  }
+  return L;
 }
 
 template UApplyArgs<double> u_args<double>(vfgpu_ctx*, const double*, const double*, double*,
@@ -196,7 +222,7 @@ int vfgpu_destroy(vfgpu_ctx* c) {
   if (c->s_in) cudaStreamDestroy(c->s_in);
   if (c->s_out) cudaStreamDestroy(c->s_out);
   cudaFree(c->t64c);
-  void* bufs[] = {c->d_tcB, c->d_tcerr, c->d_widthc, c->d_pmult, c->d_width, c->d_wpart, c->d_wstall, c->d_cflag, c->d_params, c->d_dot, c->d_elayer, c->d_ul, c->d_cellE, c->bcU_kind, c->bcU_bits, c->bcV_kind, c->bcV_bits,
+  void* bufs[] = {c->d_tcB, c->d_tcerr, c->d_widthc, c->d_pmult, c->d_width, c->d_wpart, c->d_wstall, c->d_cflag, c->d_params, c->d_dot, c->d_elayer, c->d_ul, c->d_unode, c->d_srange64, c->d_srange32, c->d_cellE, c->bcU_kind, c->bcU_bits, c->bcV_kind, c->bcV_bits,
                   c->V32, c->seam64, c->seam32, c->t64a, c->t64b, c->t32a, c->t32b};
   for (void* p : bufs) cudaFree(p);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -263,11 +289,18 @@ int vfgpu_create(const vfgpu_grid* g, vfgpu_ctx** out) {
       c->ul32 = unit_lists_carve(b32 ? static_cast<char*>(c->d_ul) + b64 : nullptr, c->plan32, c->nz);
     }
   }
+  {
+    const bool s64 = c->ul64.cls && stencil_pays(c->plan64, c->nx, c->ny, c->nz, 8);
+    const bool s32 = c->ul32.cls && stencil_pays(c->plan32, c->nx, c->ny, c->nz, 4);
+    if (s64 || s32) ALLOC(c->d_unode, c->N);
+    if (s64) ALLOC(c->d_srange64, stencil_range_bytes(c->plan64));
+    if (s32) ALLOC(c->d_srange32, stencil_range_bytes(c->plan32));
+  }
   ALLOC(c->d_params, sizeof(DevParams));
   {
     int nd = vmat_blocks(c->N);
     for (const TilePlan* p : {&c->plan64, &c->plan32})
-      nd = std::max(nd, tile_dot_count(*p, c->nx, c->ny, c->nz) + p->ncta0);  // U: split launch
+      nd = std::max(nd, tile_dot_count(*p, c->nx, c->ny, c->nz) + std::max(p->ncta0, p->st.blocks() + p->st.nface));
     ALLOC(c->d_dot, (size_t)nd * sizeof(double));
   }
   ALLOC(c->bcU_kind, 3 * c->N);
@@ -342,6 +375,10 @@ int vfgpu_set_matprop(vfgpu_ctx* c, int nlayer, const vfgpu_matprop* mp, const i
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "vfgpu_set_matprop");
   c->layers = L;
+  if ((c->nlayer == 1) != (nlayer == 1)) {  // the U applies' kernels may change
+    c->gen++;
+    c->ul_stale = true;
+  }
   c->nlayer = nlayer;
   c->have_mat = true;
   return upload_params(c);
@@ -353,7 +390,10 @@ int vfgpu_set_cell_modulus(vfgpu_ctx* c, const double* cellE) {
   // The cell-modulus pointer is captured by CG graphs: they are re-captured whenever it
   // appears, disappears or moves.
   if (!cellE) {
-    if (c->d_cellE) c->gen++;
+    if (c->d_cellE) {
+      c->gen++;
+      c->ul_stale = true;  // the U applies' kernels may change
+    }
     cudaFree(c->d_cellE);
     c->d_cellE = nullptr;
     return VFGPU_OK;
@@ -361,6 +401,7 @@ int vfgpu_set_cell_modulus(vfgpu_ctx* c, const double* cellE) {
   cudaError_t e = cudaSuccess;
   if (!c->d_cellE) {
     c->gen++;
+    c->ul_stale = true;
     e = cudaMalloc((void**)&c->d_cellE, c->NC * sizeof(float));
   }
   if (e != cudaSuccess) return cuda_fail(e, "vfgpu_set_cell_modulus");
@@ -397,7 +438,10 @@ int vfgpu_set_unilateral(vfgpu_ctx* c, int type) {
       return cuda_fail(e, "vfgpu_set_unilateral");
     }
   }
-  if (type != c->unilateral) c->gen++;  // captured CG graphs launch the other operator kernel
+  if (type != c->unilateral) {  // captured CG graphs launch the other operator kernel
+    c->gen++;
+    c->ul_stale = true;
+  }
   c->unilateral = type;
   return VFGPU_OK;
 }
@@ -437,6 +481,7 @@ int vfgpu_set_bc(vfgpu_ctx* c, const vfgpu_bc bcU[3], const vfgpu_bc* bcV) {
         return fail(VFGPU_ERR_INVALID, "vfgpu_set_bc: bad vertex type");
   }
   cudaSetDevice(c->dev);
+  c->ul_stale = true;  // the stencil's node flags carry the Dirichlet bits
   std::vector<uint8_t> ku, kv, bu(c->N, 0), bv(c->N, 0);
   build_bc_kind(c->nx, c->ny, c->nz, 3, bcU, ku);
   build_bc_kind(c->nx, c->ny, c->nz, 1, bcV, kv);
