@@ -23,7 +23,8 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 HOST_CXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
 # Per-file extra flags: the crack initialisers and the fracture width round like the
 # reference's C code.
-FILE_FLAGS = {"cracks.cu": ["-fmad=false"], "width.cu": ["-fmad=false"]}
+# cg_loop.cu sets graph conditions from the device (cudadevrt): relocatable device code.
+FILE_FLAGS = {"cracks.cu": ["-fmad=false"], "width.cu": ["-fmad=false"], "cg_loop.cu": ["-rdc=true"]}
 
 
 def _flags(debug: bool) -> list[str]:
@@ -63,7 +64,7 @@ def build(force: bool = False, debug: bool = False, verbose: bool = False) -> st
                     raise RuntimeError(f"nvcc failed on {src}")
     objs = [os.path.join(BUILD, os.path.basename(s)[:-3] + ".o") for s in srcs]
     if jobs or not os.path.exists(LIB) or os.path.getmtime(LIB) < max(map(os.path.getmtime, objs)):
-        cmd = [NVCC] + ARCH + ["-shared", "-ccbin", HOST_CXX, "-o", LIB] + objs + ["-cudart", "static"]
+        cmd = [NVCC] + ARCH + ["-shared", "-ccbin", HOST_CXX, "-o", LIB] + objs + ["-cudart", "static", "-lcudadevrt"]
         p = subprocess.run(cmd, capture_output=True, text=True)
         if p.returncode:
             raise RuntimeError("link failed:\n" + p.stdout + p.stderr)

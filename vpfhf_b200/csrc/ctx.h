@@ -125,7 +125,7 @@ struct vfgpu_ctx {
   cudaEvent_t ev_start = nullptr, ev_in[kPipeSlabs] = {}, ev_y[kPipeSlabs] = {},
               ev_out[kPipeSlabs] = {};
 
-  // Captured CUDA graphs of CG iteration batches, keyed by (call site, batch size).
+  // Captured CUDA graphs (CG loops, V-cycles), keyed by (call site, variant).
   // Kernels read the material table, eta and the AT gradient weights through
   // d_params, so new material / vfprop values leave the graphs valid; a set-up call
   // that changes a captured pointer (the cell-modulus array) bumps `gen` and stale
@@ -134,13 +134,18 @@ struct vfgpu_ctx {
     int kind, batch;
     uint64_t gen;
     cudaGraphExec_t exec;
+    cudaGraph_t src;  // kept with exec: a conditional node's handle, which the kernels of its
+                      // body write through, lives as long as the graph it was made in
+    void release() {
+      if (exec) cudaGraphExecDestroy(exec);
+      if (src) cudaGraphDestroy(src);
+      exec = nullptr;
+      src = nullptr;
+    }
   };
   std::vector<Graph> graphs;
   uint64_t gen = 1;
   bool use_graphs = true;
-  // per CG call site (run_cg kind 1..4): iterations of its last solve, the size of
-  // the first batch of the next one
-  int cg_last_its[8] = {0};
 };
 
 namespace vfgpu {

@@ -1092,7 +1092,7 @@ void free_mg(vfgpu_ctx* c) {
   for (size_t k = 0; k < c->graphs.size();) {  // the V-cycle graphs hold the old pointers
     auto& g = c->graphs[k];
     if (g.kind == kGraphMG64 || g.kind == kGraphMG32) {
-      if (g.exec) cudaGraphExecDestroy(g.exec);
+      g.release();
       c->graphs.erase(c->graphs.begin() + k);
     } else {
       k++;

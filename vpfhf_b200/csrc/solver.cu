@@ -1,4 +1,6 @@
 // solver.cu -- reductions, PCG kernels and the vector kernels of the U/V solves.
+#include <algorithm>
+#include <climits>
 #include <cmath>
 
 #include "cg.cuh"
@@ -8,43 +10,47 @@ namespace vfgpu {
 
 namespace {
 
-// Block-level fixed-order tree sum of K values per thread into partial[blockIdx*K + q].
+// Fixed-order sum of K values per thread over the block (shuffle trees, then the warps in
+// order), in every thread.
 template <int K>
-__device__ __forceinline__ void block_sum(double (&v)[K], double* __restrict__ partial) {
-  __shared__ double red[K][RED_THREADS];
+__device__ __forceinline__ void block_total(double (&v)[K]) {
+  __shared__ double red[K][RED_THREADS / 32];
 #pragma unroll
-  for (int q = 0; q < K; q++) red[q][threadIdx.x] = v[q];
+  for (int q = 0; q < K; q++)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+  __syncthreads();  // a previous call's totals have been read
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int q = 0; q < K; q++) red[q][threadIdx.x >> 5] = v[q];
   __syncthreads();
-  for (int st = RED_THREADS / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st)
 #pragma unroll
-      for (int q = 0; q < K; q++) red[q][threadIdx.x] += red[q][threadIdx.x + st];
-    __syncthreads();
+  for (int q = 0; q < K; q++) {
+    v[q] = red[q][0];
+#pragma unroll
+    for (int w = 1; w < RED_THREADS / 32; w++) v[q] += red[q][w];
   }
-  if (threadIdx.x < K) partial[blockIdx.x * K + threadIdx.x] = red[threadIdx.x][0];
 }
 
-// Fixed-order sum of the per-block partials (one block).
+// Block-level fixed-order sum of K values per thread into partial[blockIdx*K + q].
 template <int K>
-__device__ __forceinline__ void final_sum(const double* __restrict__ partial, double (&out)[K]) {
-  __shared__ double red[K][RED_THREADS];
-  double v[K];
+__device__ __forceinline__ void block_sum(double (&v)[K], double* __restrict__ partial) {
+  block_total<K>(v);
+  if (threadIdx.x == 0)
 #pragma unroll
-  for (int q = 0; q < K; q++) v[q] = 0.;
-  for (int b = threadIdx.x; b < RED_BLOCKS; b += RED_THREADS)
+    for (int q = 0; q < K; q++) partial[blockIdx.x * K + q] = v[q];
+}
+
+// Fixed-order sum of n blocks' partials by one block, in every thread (identical in every
+// block that calls it).  L1 is bypassed: an earlier kernel of the same graph wrote them.
+template <int K>
+__device__ __forceinline__ void final_sum(const double* __restrict__ partial, int n, double (&out)[K]) {
 #pragma unroll
-    for (int q = 0; q < K; q++) v[q] += partial[b * K + q];
+  for (int q = 0; q < K; q++) out[q] = 0.;
+  for (int b = threadIdx.x; b < n; b += RED_THREADS)
 #pragma unroll
-  for (int q = 0; q < K; q++) red[q][threadIdx.x] = v[q];
-  __syncthreads();
-  for (int st = RED_THREADS / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st)
-#pragma unroll
-      for (int q = 0; q < K; q++) red[q][threadIdx.x] += red[q][threadIdx.x + st];
-    __syncthreads();
-  }
-#pragma unroll
-  for (int q = 0; q < K; q++) out[q] = red[q][0];
+    for (int q = 0; q < K; q++) out[q] += __ldcg(partial + b * K + q);
+  block_total<K>(out);
 }
 
 #define GRID_LOOP(i, n)                                                                  \
@@ -74,6 +80,24 @@ __device__ __forceinline__ Pack<T> ld16(const T* __restrict__ a, int64_t c) {
   }
   return p;
 }
+// The same with evict-first caching: for a vector that is not read again before others push
+// it out of L2.
+template <typename T>
+__device__ __forceinline__ Pack<T> ld16s(const T* __restrict__ a, int64_t c) {
+  Pack<T> p;
+  if constexpr (sizeof(T) == 8) {
+    const double2 q = __ldcs(reinterpret_cast<const double2*>(a) + c);
+    p.e[0] = q.x;
+    p.e[1] = q.y;
+  } else {
+    const float4 q = __ldcs(reinterpret_cast<const float4*>(a) + c);
+    p.e[0] = q.x;
+    p.e[1] = q.y;
+    p.e[2] = q.z;
+    p.e[3] = q.w;
+  }
+  return p;
+}
 template <typename T>
 __device__ __forceinline__ void st16(T* __restrict__ a, int64_t c, const Pack<T>& p) {
   if constexpr (sizeof(T) == 8) {
@@ -93,19 +117,6 @@ __device__ __forceinline__ void pack_loop(int64_t n, FP fp, FT ft) {
   for (int64_t c = t0; c < np; c += st) fp(c);
   for (int64_t i = np * W + t0; i < n; i += st) ft(i);
 }
-// The same packs visited from the end of the vectors back (for an elementwise kernel
-// that follows a forward pass over some of the same vectors: it starts on the lines that
-// pass left in L2).
-template <typename T, class FP, class FT>
-__device__ __forceinline__ void pack_loop_rev(int64_t n, FP fp, FT ft) {
-  constexpr int W = Pack<T>::W;
-  const int64_t np = n / W;
-  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t st = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = np * W + t0; i < n; i += st) ft(i);
-  for (int64_t c = t0; c < np; c += st) fp(np - 1 - c);
-}
-
 template <typename T>
 __global__ void __launch_bounds__(RED_THREADS) cg_init_kernel(CGVecs<T> v, double* partial) {
   double acc[2] = {0., 0.};
@@ -125,9 +136,10 @@ __global__ void __launch_bounds__(RED_THREADS) cg_init_kernel(CGVecs<T> v, doubl
 __global__ void cg_init_final(CGState* st, const double* partial, double rtol, double atol,
                               double dtol, int maxit) {
   double s[2];
-  final_sum<2>(partial, s);
+  final_sum<2>(partial, RED_BLOCKS, s);
   if (threadIdx.x == 0) {
-    st->rz = s[0];
+    st->rz[0] = st->rz[1] = s[0];
+    st->itn[0] = st->itn[1] = 0;
     st->zz = s[1];
     st->rnorm0 = sqrt(s[1]);
     st->ttol = fmax(rtol * st->rnorm0, atol);
@@ -135,7 +147,7 @@ __global__ void cg_init_final(CGState* st, const double* partial, double rtol, d
     st->its = 0;
     st->xalpha = 0.;
     st->maxit = maxit;
-    st->arrive = 0;
+    st->yield = INT_MAX;
     st->done = 0;
     st->reason = CG_RUNNING;
     if (!(st->rnorm0 == st->rnorm0)) {
@@ -151,89 +163,40 @@ __global__ void cg_init_final(CGState* st, const double* partial, double rtol, d
   }
 }
 
-// Fixed-order sum of n block partials by one block; every thread gets the result
-// (identical in every block that calls it).  L1 is bypassed: the partials were
-// written by other blocks or by an earlier kernel.
-__device__ __forceinline__ double sum_partials(const double* __restrict__ p, int n) {
-  __shared__ double red[RED_THREADS];
-  double v = 0.;
-  for (int b = threadIdx.x; b < n; b += RED_THREADS) v += __ldcg(p + b);
-  red[threadIdx.x] = v;
-  __syncthreads();
-  for (int st = RED_THREADS / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) red[threadIdx.x] += red[threadIdx.x + st];
-    __syncthreads();
-  }
-  const double s = red[0];
-  __syncthreads();
-  return s;
-}
-
-// End of a CG iteration from the new (r, z) and (z, z): iteration count,
-// convergence tests (KSPConvergedDefault on the preconditioned norm) and beta.
-__device__ __forceinline__ void cg_finish_iteration(CGState* st, double rz, double zz) {
-  st->its += 1;
-  st->zz = zz;
-  const double dp = sqrt(zz);
-  if (!(dp == dp)) {
-    st->done = 1;
-    st->reason = CG_DIVERGED_NAN;
-  } else if (dp <= st->ttol) {
-    st->done = 1;
-    st->reason = CG_CONVERGED_RTOL;
-  } else if (dp >= st->dtol * st->rnorm0) {
-    st->done = 1;
-    st->reason = CG_DIVERGED_DTOL;
-  } else if (st->its >= st->maxit) {
-    st->done = 1;
-    st->reason = CG_DIVERGED_ITS;
-  } else {
-    st->beta = rz / st->rz;
-    st->rz = rz;
-    if (rz == 0.) {
-      st->done = 1;
-      st->reason = CG_CONVERGED_ATOL;
-    }
-  }
-}
-
-// p.w by blocks (for an operator apply that did not produce it).
-template <typename T>
-__global__ void __launch_bounds__(RED_THREADS) cg_pw_kernel(CGVecs<T> v, const CGState* st,
-                                                            double* partial) {
-  if (st->done) return;
-  double acc[1] = {0.};
-  pack_loop<T>(
-      v.n,
-      [&](int64_t c) {
-        const Pack<T> p = ld16(v.p, c), w = ld16(v.w, c);
-#pragma unroll
-        for (int k = 0; k < Pack<T>::W; k++) acc[0] += (double)p.e[k] * (double)w.e[k];
-      },
-      [&](int64_t i) { acc[0] += (double)v.p[i] * (double)v.w[i]; });
-  block_sum<1>(acc, partial);
-}
-
-// One CG step after w = A p: every block sums the operator's p.w partials (written
-// by the tile and seam kernels of the apply) to the same alpha = (r,z)/(p,w), updates
-// x and r, and adds its share of (r,z), (z,z) with z = D^-1 r; the last block to
-// finish sums those partials and ends the iteration (cg_finish_iteration).  The
-// arrival counter is the only atomic; every sum has a fixed order.
+// r -= alpha w and the block partials of (r, z), (z, z) with z = D^-1 r, after w = A p: every
+// block sums the operator's p.w partials (written by the apply's kernels) to the same
+// alpha = (r,z)/(p,w).  The block's first packets are on their way while it does: the sum is a
+// memory latency and a block reduction that would otherwise come before any of the kernel's
+// traffic.  w is not read again: evict-first, so that r and dinv stay in L2 for the
+// direction kernel (41.0 -> 37.2 us at 129^3 FP64 beside 43.1 -> 44.3 us there).
 template <typename T>
 __global__ void __launch_bounds__(RED_THREADS) cg_update_kernel(CGVecs<T> v, CGState* st,
-                                                                double* partial) {
-  if (st->done) return;
-  const double pw = sum_partials(v.dotp, v.ndot);
+                                                                double* partial, int par) {
+  // block 0 may set done while other blocks start: the whole block takes one view of it
+  if (__syncthreads_or(st->done)) return;
+  constexpr int W = Pack<T>::W;
+  const int64_t np = v.n / W, t0 = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x;
+  const int64_t step = (int64_t)gridDim.x * RED_THREADS;
+  Pack<T> r, w, d;
+  if (t0 < np) {
+    r = ld16(v.r, t0);
+    w = ld16s(v.w, t0);
+    d = ld16(v.dinv, t0);
+  }
+  double pws[1];
+  final_sum<1>(v.dotp, v.ndot, pws);
+  const double pw = pws[0];
   if (!(pw > 0.)) {  // same value in every block: all of them stop here
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       st->pw = pw;
       st->xalpha = 0.;  // no step of this iteration reaches x
+      st->its = st->itn[par];
       st->done = 1;
       st->reason = (pw == pw) ? CG_DIVERGED_INDEFINITE : CG_DIVERGED_NAN;
     }
     return;
   }
-  const double alpha = st->rz / pw;  // st->rz changes only after every block has arrived
+  const double alpha = st->rz[par] / pw;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->pw = pw;
     st->alpha = alpha;
@@ -241,85 +204,103 @@ __global__ void __launch_bounds__(RED_THREADS) cg_update_kernel(CGVecs<T> v, CGS
   }
   const T a = (T)alpha;
   double acc[2] = {0., 0.};
-  pack_loop<T>(
-      v.n,
-      [&](int64_t c) {
-        Pack<T> r = ld16(v.r, c);
-        const Pack<T> w = ld16(v.w, c), d = ld16(v.dinv, c);
+  for (int64_t c = t0; c < np;) {
 #pragma unroll
-        for (int k = 0; k < Pack<T>::W; k++) {
-          r.e[k] = r.e[k] - a * w.e[k];
-          const T z = r.e[k] * d.e[k];
-          acc[0] += (double)z * (double)r.e[k];
-          acc[1] += (double)z * (double)z;
-        }
-        st16(v.r, c, r);
-      },
-      [&](int64_t i) {
-        const T r = v.r[i] - a * v.w[i];
-        const T z = r * v.dinv[i];
-        v.r[i] = r;
-        acc[0] += (double)z * (double)r;
-        acc[1] += (double)z * (double)z;
-      });
+    for (int k = 0; k < W; k++) {
+      r.e[k] = r.e[k] - a * w.e[k];
+      const T z = r.e[k] * d.e[k];
+      acc[0] += (double)z * (double)r.e[k];
+      acc[1] += (double)z * (double)z;
+    }
+    st16(v.r, c, r);
+    c += step;
+    if (c < np) {
+      r = ld16(v.r, c);
+      w = ld16s(v.w, c);
+      d = ld16(v.dinv, c);
+    }
+  }
+  for (int64_t i = np * W + t0; i < v.n; i += step) {
+    const T ri = v.r[i] - a * v.w[i];
+    const T z = ri * v.dinv[i];
+    v.r[i] = ri;
+    acc[0] += (double)z * (double)ri;
+    acc[1] += (double)z * (double)z;
+  }
   block_sum<2>(acc, partial);
-  __shared__ bool last;
-  __threadfence();  // this block's partials are visible before it is counted
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&st->arrive, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double sum[2] = {0., 0.};
-  {
-    __shared__ double red[2][RED_THREADS];
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += RED_THREADS) {
-      sum[0] += __ldcg(partial + 2 * b);
-      sum[1] += __ldcg(partial + 2 * b + 1);
-    }
-    red[0][threadIdx.x] = sum[0];
-    red[1][threadIdx.x] = sum[1];
-    __syncthreads();
-    for (int s2 = RED_THREADS / 2; s2 > 0; s2 >>= 1) {
-      if (threadIdx.x < s2) {
-        red[0][threadIdx.x] += red[0][threadIdx.x + s2];
-        red[1][threadIdx.x] += red[1][threadIdx.x + s2];
-      }
-      __syncthreads();
-    }
-    sum[0] = red[0][0];
-    sum[1] = red[1][0];
-  }
-  if (threadIdx.x == 0) {
-    st->arrive = 0;
-    cg_finish_iteration(st, sum[0], sum[1]);
-  }
 }
 
-// x += alpha p and p = z + beta p in one pass (the iteration went on: not done),
-// back from the end of the vectors: the update kernel's forward pass left the tail of r
-// and dinv in L2.
+// End of a CG iteration: every block sums the update kernel's partials to the same (r, z),
+// (z, z) and takes the same decision -- convergence tests of KSPConvergedDefault on the
+// preconditioned norm, or beta -- of which block 0 keeps the record; then x += alpha p and
+// p = z + beta p in one pass, back from the end of the vectors: the update kernel's forward
+// pass left the tail of r and dinv in L2.  As there, the first packets are on their way while
+// the block sums.  (Ending the iteration in the update kernel's last block instead costs a
+// fence, an atomic and that block's serial reduction.)
 template <typename T>
-__global__ void cg_p_kernel(CGVecs<T> v, const CGState* st) {
-  if (st->done) return;
-  const T a = (T)st->alpha, b = (T)st->beta;
-  pack_loop_rev<T>(
-      v.n,
-      [&](int64_t c) {
-        Pack<T> p = ld16(v.p, c), x = ld16(v.x, c);
-        const Pack<T> r = ld16(v.r, c), d = ld16(v.dinv, c);
+__global__ void __launch_bounds__(RED_THREADS) cg_p_kernel(CGVecs<T> v, CGState* st, const double* partial,
+                                                           int nblk, int par) {
+  // done is set from an earlier iteration, or by block 0 of this launch (which then takes the
+  // same decision as this block would): the whole block takes one view of it
+  if (__syncthreads_or(st->done)) return;
+  constexpr int W = Pack<T>::W;
+  const int64_t np = v.n / W, t0 = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x;
+  const int64_t step = (int64_t)gridDim.x * RED_THREADS;
+  Pack<T> p, x, r, d;
+  int64_t c = np - 1 - t0;
+  auto load = [&]() {
+    p = ld16(v.p, c);
+    r = ld16(v.r, c);
+    d = ld16(v.dinv, c);
+    x = ld16(v.x, c);
+  };
+  if (c >= 0) load();
+  double s[2];
+  final_sum<2>(partial, nblk, s);
+  const double rz = s[0], zz = s[1], dp = sqrt(zz), rz0 = st->rz[par];
+  const int its = st->itn[par] + 1;
+  int reason = CG_RUNNING;
+  double beta = 0.;
+  if (!(dp == dp)) {
+    reason = CG_DIVERGED_NAN;
+  } else if (dp <= st->ttol) {
+    reason = CG_CONVERGED_RTOL;
+  } else if (dp >= st->dtol * st->rnorm0) {
+    reason = CG_DIVERGED_DTOL;
+  } else if (its >= st->maxit) {
+    reason = CG_DIVERGED_ITS;
+  } else {
+    beta = rz / rz0;
+    if (rz == 0.) reason = CG_CONVERGED_ATOL;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->its = its;
+    st->itn[par ^ 1] = its;
+    st->zz = zz;
+    st->beta = beta;
+    st->rz[par ^ 1] = rz;
+    if (reason) {
+      st->reason = reason;
+      st->done = 1;
+    }
+  }
+  if (reason) return;
+  const T a = (T)st->alpha, b = (T)beta;
+  while (c >= 0) {
 #pragma unroll
-        for (int k = 0; k < Pack<T>::W; k++) {
-          x.e[k] = x.e[k] + a * p.e[k];
-          p.e[k] = r.e[k] * d.e[k] + b * p.e[k];
-        }
-        st16(v.x, c, x);
-        st16(v.p, c, p);
-      },
-      [&](int64_t i) {
-        v.x[i] = v.x[i] + a * v.p[i];
-        v.p[i] = v.r[i] * v.dinv[i] + b * v.p[i];
-      });
+    for (int k = 0; k < W; k++) {
+      x.e[k] = x.e[k] + a * p.e[k];
+      p.e[k] = r.e[k] * d.e[k] + b * p.e[k];
+    }
+    st16(v.x, c, x);
+    st16(v.p, c, p);
+    c -= step;
+    if (c >= 0) load();
+  }
+  for (int64_t i = np * W + t0; i < v.n; i += step) {
+    v.x[i] = v.x[i] + a * v.p[i];
+    v.p[i] = v.r[i] * v.dinv[i] + b * v.p[i];
+  }
 }
 
 // The step of the iteration that stopped the solve (its cg_p_kernel did not run):
@@ -364,7 +345,7 @@ __global__ void __launch_bounds__(RED_THREADS) dots_kernel(PtrPack<K> a, PtrPack
 template <int K>
 __global__ void dots_final(const double* partial, double* out) {
   double s[K];
-  final_sum<K>(partial, s);
+  final_sum<K>(partial, RED_BLOCKS, s);
   if (threadIdx.x == 0)
 #pragma unroll
     for (int q = 0; q < K; q++) out[q] = s[q];
@@ -524,20 +505,20 @@ template <typename T> static bool aligned16(const CGVecs<T>& v) {
   return true;
 }
 
+// Blocks of the update and direction kernels: two packets per thread on small systems (fewer
+// partials to sum), one wave of 4 blocks per SM on large ones.
+template <typename T> static int cg_blocks(int64_t n) {
+  const int64_t per = 2 * RED_THREADS * Pack<T>::W;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(RED_BLOCKS, (n + per - 1) / per));
+}
+
 template <typename T>
-cudaError_t cg_after_apply(const CGVecs<T>& v, CGState* st, double* partial, cudaStream_t s) {
+cudaError_t cg_iteration(const CGVecs<T>& v, CGState* st, double* partial, int par, cudaStream_t s) {
   if (!aligned16(v)) return cudaErrorMisalignedAddress;  // caught on the host, nothing launched
-  if (!v.dotp) {  // the apply did not accumulate p.w: a separate pass into partial[2R, 3R)
-    cg_pw_kernel<T><<<RED_BLOCKS, RED_THREADS, 0, s>>>(v, st, partial + 2 * RED_BLOCKS);
-    CGVecs<T> u = v;
-    u.dotp = partial + 2 * RED_BLOCKS;
-    u.ndot = RED_BLOCKS;
-    cg_update_kernel<T><<<RED_BLOCKS, RED_THREADS, 0, s>>>(u, st, partial);
-  } else {
-    if (v.ndot <= 0) return cudaErrorInvalidValue;
-    cg_update_kernel<T><<<RED_BLOCKS, RED_THREADS, 0, s>>>(v, st, partial);
-  }
-  cg_p_kernel<T><<<RED_BLOCKS, RED_THREADS, 0, s>>>(v, st);
+  if (!v.dotp || v.ndot <= 0) return cudaErrorInvalidValue;
+  const int nb = cg_blocks<T>(v.n);
+  cg_update_kernel<T><<<nb, RED_THREADS, 0, s>>>(v, st, partial, par);
+  cg_p_kernel<T><<<nb, RED_THREADS, 0, s>>>(v, st, partial, nb, par);
   return cudaGetLastError();
 }
 
@@ -552,9 +533,8 @@ template cudaError_t cg_init<double>(const CGVecs<double>&, CGState*, double*, d
                                      double, int, cudaStream_t);
 template cudaError_t cg_init<float>(const CGVecs<float>&, CGState*, double*, double, double,
                                     double, int, cudaStream_t);
-template cudaError_t cg_after_apply<double>(const CGVecs<double>&, CGState*, double*,
-                                            cudaStream_t);
-template cudaError_t cg_after_apply<float>(const CGVecs<float>&, CGState*, double*, cudaStream_t);
+template cudaError_t cg_iteration<double>(const CGVecs<double>&, CGState*, double*, int, cudaStream_t);
+template cudaError_t cg_iteration<float>(const CGVecs<float>&, CGState*, double*, int, cudaStream_t);
 template cudaError_t cg_finish_x<double>(const CGVecs<double>&, const CGState*, cudaStream_t);
 template cudaError_t cg_finish_x<float>(const CGVecs<float>&, const CGState*, cudaStream_t);
 

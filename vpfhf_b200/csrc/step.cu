@@ -145,91 +145,129 @@ struct Watch {
   double seconds() const { return std::chrono::duration<double>(clk::now() - t0).count(); }
 };
 
-// PCG with device-side convergence: queues batches of iterations (every kernel of a
-// converged solve is a no-op), checks the flag between batches.
-// Graph of `batch` CG iterations for call site `kind`, captured on first use (the
-// kernels' pointers are fixed per call site; see vfgpu_ctx::Graph).
-template <class Body>
-static cudaGraphExec_t cg_graph(vfgpu_ctx* c, int kind, int batch, Body body) {
+// The ctx's graph for call site `kind` (and `batch`, a variant of it), built by `make` on first
+// use or when the ctx's generation moved (the kernels' pointers are fixed per call site; see
+// vfgpu_ctx::Graph); null if it cannot be built.
+template <class Make>
+static cudaGraphExec_t cached_graph(vfgpu_ctx* c, int kind, int batch, Make make) {
+  vfgpu_ctx::Graph* slot = nullptr;
   for (auto& g : c->graphs)
     if (g.kind == kind && g.batch == batch) {
-      if (g.gen == c->gen) return g.exec;
-      cudaGraphExecDestroy(g.exec);
-      g.exec = nullptr;
+      if (g.gen == c->gen && g.exec) return g.exec;
+      g.release();
+      slot = &g;
     }
-  cudaGraph_t graph = nullptr;
+  cudaGraph_t graph = make();
   cudaGraphExec_t exec = nullptr;
-  if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  const cudaError_t eb = body();
-  const cudaError_t ec = cudaStreamEndCapture(c->stream, &graph);
-  if (eb != cudaSuccess || ec != cudaSuccess || !graph ||
-      cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) {
+  if (!graph || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) {
     if (graph) cudaGraphDestroy(graph);
     cudaGetLastError();
     return nullptr;
   }
-  cudaGraphDestroy(graph);
-  bool stored = false;
-  for (auto& g : c->graphs)
-    if (g.kind == kind && g.batch == batch) {
-      g.exec = exec;
-      g.gen = c->gen;
-      stored = true;
-    }
-  if (!stored) c->graphs.push_back({kind, batch, c->gen, exec});
+  const vfgpu_ctx::Graph made{kind, batch, c->gen, exec, graph};
+  if (slot) *slot = made;
+  else c->graphs.push_back(made);
   return exec;
 }
 
 cudaGraphExec_t ctx_graph(vfgpu_ctx* c, int kind, int batch,
                           const std::function<cudaError_t()>& body) {
-  return cg_graph(c, kind, batch, body);
+  return cached_graph(c, kind, batch, [&]() -> cudaGraph_t {
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return nullptr;
+    const cudaError_t eb = body();
+    const cudaError_t ec = cudaStreamEndCapture(c->stream, &graph);
+    if (eb != cudaSuccess || ec != cudaSuccess) {
+      if (graph) cudaGraphDestroy(graph);
+      return nullptr;
+    }
+    return graph;
+  });
 }
 
+// A graph of one conditional while node whose body is what `body` launches; body gets the
+// handle whose condition its last kernel sets.
+static cudaGraph_t while_graph(vfgpu_ctx* c, const std::function<cudaError_t(cudaGraphConditionalHandle)>& body) {
+  cudaGraph_t graph = nullptr;
+  if (cudaGraphCreate(&graph, 0) != cudaSuccess) return nullptr;
+  cudaGraphConditionalHandle h{};
+  cudaGraphNode_t node{};
+  cudaGraphNodeParams np{};
+  np.type = cudaGraphNodeTypeConditional;
+  cudaError_t e = cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault);
+  if (e == cudaSuccess) {
+    np.conditional.handle = h;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    e = cudaGraphAddNode(&node, graph, nullptr, 0, &np);
+  }
+  if (e == cudaSuccess)
+    e = cudaStreamBeginCaptureToGraph(c->stream, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                      cudaStreamCaptureModeThreadLocal);
+  if (e == cudaSuccess) {
+    cudaGraph_t captured = nullptr;
+    const cudaError_t eb = body(h);
+    e = cudaStreamEndCapture(c->stream, &captured);
+    if (eb != cudaSuccess) e = eb;
+  }
+  if (e != cudaSuccess) {
+    cudaGraphDestroy(graph);
+    return nullptr;
+  }
+  return graph;
+}
+
+// PCG with device-side convergence.  The iterations run in a conditional while node of a
+// graph, four to a body, so a solve costs one launch and one host read whatever its length,
+// and at most three iterations are queued behind the last one.  (Batches of 4 to 64
+// queued iterations, checked in between, launched 580 iterations for 320 at 41^3 and 692 for
+// 486 at 129^3, each finished one a row of empty kernels.)  With a time limit the loop also
+// returns every kYieldIts iterations for the clock to be read.  Without graphs the same
+// iterations are launched in batches.
+constexpr int kYieldIts = 64, kBodyIts = 4;
 template <typename T, class Apply>
 static int run_cg(vfgpu_ctx* c, int kind, const CGVecs<T>& v, Apply apply, double rtol,
                   double atol, double dtol, int maxit, const Watch& w, int* its, int* reason,
                   bool* timeout) {
   cudaError_t e = cg_init<T>(v, c->d_cg, c->d_red, rtol, atol, dtol, maxit, c->stream);
-  // Batches of iterations are queued without a host round trip; a converged CG turns
-  // the rest of a batch into no-ops (skip flag), so the batch sizes do not change the
-  // result.  The first batch is the largest power of two (4..64) not above the call
-  // site's last iteration count, and is queued before the first host check.
-  int batch = 4;
-  while (batch < 64 && 2 * batch <= c->cg_last_its[kind & 7]) batch *= 2;
-  bool first = true;
   *timeout = false;
-  auto body = [&](int nb) {
+  // an even number of iterations: each launch starts at parity 0
+  auto body = [&](int n) {
     cudaError_t eb = cudaSuccess;
-    for (int b = 0; b < nb && eb == cudaSuccess; b++) {
+    for (int b = 0; b < n && eb == cudaSuccess; b++) {
       eb = apply(v.p, v.w, &c->d_cg->done, const_cast<double*>(v.dotp));
-      if (eb == cudaSuccess) eb = cg_after_apply<T>(v, c->d_cg, c->d_red, c->stream);
+      if (eb == cudaSuccess)
+        eb = cg_iteration<T>(v, c->d_cg, c->d_red, b & 1, c->stream);
     }
     return eb;
   };
-  while (e == cudaSuccess) {
-    if (!first) {
-      e = cudaMemcpyAsync(c->h_cg, c->d_cg, sizeof(CGState), cudaMemcpyDeviceToHost, c->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-      if (e != cudaSuccess || c->h_cg->done) break;
-      if (w.expired()) {
-        *timeout = true;
-        break;
-      }
-      batch = std::min(batch * 2, 64);
+  cudaGraphExec_t g = !c->use_graphs ? nullptr : cached_graph(c, kind, 0, [&] {
+    return while_graph(c, [&](cudaGraphConditionalHandle h) {
+      const cudaError_t eb = body(kBodyIts);
+      return eb == cudaSuccess ? cg_set_condition(c->d_cg, h, c->stream) : eb;
+    });
+  });
+  for (int from = 0; e == cudaSuccess; from = c->h_cg->its) {
+    if (g) {
+      if (w.limit > 0) e = cg_set_yield(c->d_cg, from + kYieldIts, c->stream);
+      if (e == cudaSuccess) e = cudaGraphLaunch(g, c->stream);
+    } else {
+      e = body(kYieldIts);
     }
-    first = false;
-    cudaGraphExec_t g = c->use_graphs ? cg_graph(c, kind, batch, [&] { return body(batch); }) : nullptr;
-    e = g ? cudaGraphLaunch(g, c->stream) : body(batch);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(c->h_cg, c->d_cg, sizeof(CGState), cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e != cudaSuccess || c->h_cg->done) break;
+    if (w.expired()) {
+      *timeout = true;
+      break;
+    }
   }
   // the step of the iteration that stopped the solve has not reached x yet
   if (e == cudaSuccess) e = cg_finish_x<T>(v, c->d_cg, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "CG");
   *its = c->h_cg->its;
   *reason = c->h_cg->reason;
-  c->cg_last_its[kind & 7] = *its;
   return VFGPU_OK;
 }
 
@@ -253,19 +291,6 @@ static int dots_of(const vfgpu_ctx* c, const TilePlan& p) { return tile_dot_coun
 // The U applies with unit lists or the stencil write a second wave's partials.
 static int u_dots_of(const vfgpu_ctx* c, const TilePlan& p, int prec_bytes) {
   return dots_of(c, p) + (u_stencil_on(c, prec_bytes) ? p.st.blocks() + p.st.nface : u_lists_on(c, prec_bytes) ? p.ncta0 : 0);
-}
-
-// Which CG call sites let the operator apply accumulate p.w (bit k-1 for call site k:
-// 1 U FP64, 2 U FP32, 3 V FP64, 4 V FP32); the others use a separate p.w pass.  U in both
-// precisions: the 129^3 mixed StepU measured 37.07 ms with the FP32 U apply accumulating p.w
-// (the packed FP32 fixed-weight wave has the registers for it) against 37.78 ms with the
-// separate pass; FP64 U 0.0957 s against 0.0972 s.  V: a node's row is in registers when its
-// x.y is known.
-#ifndef VFGPU_FUSE_DOT_MASK
-#define VFGPU_FUSE_DOT_MASK 15
-#endif
-static double* dot_buf(vfgpu_ctx* c, int kind) {
-  return ((VFGPU_FUSE_DOT_MASK >> (kind - 1)) & 1) ? c->d_dot : nullptr;
 }
 
 // F = K(V) U - f, Dirichlet rows U - ubc (VF_UResidual, VFMech.c:1456-1887).
@@ -371,7 +396,7 @@ int vfgpu_step_u(vfgpu_ctx* c, const vfgpu_solve_opts* o_, vfgpu_solve_stats* st
       S.ksp_its += kits;
       tmo = w.expired();
     } else if (!mixed) {
-      CGVecs<double> v{Y, R, P, W, dinv, F, nullptr, n3, dot_buf(c, 1), u_dots_of(c, c->plan64, 8)};
+      CGVecs<double> v{Y, R, P, W, dinv, F, nullptr, n3, c->d_dot, u_dots_of(c, c->plan64, 8)};
       rc = run_cg<double>(c, 1, v, apply64, o.ksp_rtol, o.ksp_atol, o.ksp_dtol, o.ksp_maxit, w, &kits,
                           &kreason, &tmo);
       if (rc) return rc;
@@ -391,7 +416,7 @@ int vfgpu_step_u(vfgpu_ctx* c, const vfgpu_solve_opts* o_, vfgpu_solve_stats* st
         float* b32 = reinterpret_cast<float*>(P);  // FP32 right-hand side staged in P
         e = dev_to_f32(R, b32, n3, c->stream);
         if (e != cudaSuccess) return cuda_fail(e, "vfgpu_step_u");
-        CGVecs<float> v{x32, r32, pp32, w32, c->p32[4], b32, nullptr, n3, dot_buf(c, 2), u_dots_of(c, c->plan32, 4)};
+        CGVecs<float> v{x32, r32, pp32, w32, c->p32[4], b32, nullptr, n3, c->d_dot, u_dots_of(c, c->plan32, 4)};
         const double in_rtol = std::max(o.inner_rtol, 0.5 * target / zr);
         int its32 = 0, r32reason = 0;
         rc = run_cg<float>(c, 2, v, apply32, in_rtol, 0.0, o.ksp_dtol, o.ksp_maxit, w, &its32,
@@ -586,7 +611,7 @@ int vfgpu_step_v(vfgpu_ctx* c, const vfgpu_solve_opts* o_, vfgpu_solve_stats* st
     int kits = 0, kreason = 0;
     bool tmo = false;
     if (!mixed) {
-      CGVecs<double> v{Y, R, P, Wv, dinv, F, mask, N, dot_buf(c, 3), vmat_blocks(N)};
+      CGVecs<double> v{Y, R, P, Wv, dinv, F, mask, N, c->d_dot, vmat_blocks(N)};
       rc = run_cg<double>(c, 3, v, apply64, o.ksp_rtol, o.ksp_atol, o.ksp_dtol, o.ksp_maxit, w, &kits,
                           &kreason, &tmo);
       if (rc) return rc;
@@ -604,7 +629,7 @@ int vfgpu_step_v(vfgpu_ctx* c, const vfgpu_solve_opts* o_, vfgpu_solve_stats* st
       for (int k = 0; k < o.max_refine && zr > target; k++) {
         e = dev_to_f32(R, b32, N, c->stream);
         if (e != cudaSuccess) return cuda_fail(e, "vfgpu_step_v");
-        CGVecs<float> v{x32, r32, pp32, w32, dinv32, b32, mask, N, dot_buf(c, 4), vmat_blocks(N)};
+        CGVecs<float> v{x32, r32, pp32, w32, dinv32, b32, mask, N, c->d_dot, vmat_blocks(N)};
         const double in_rtol = std::max(o.inner_rtol, 0.5 * target / zr);
         int its32 = 0, r32reason = 0;
         rc = run_cg<float>(c, 4, v, apply32, in_rtol, 0.0, o.ksp_dtol, o.ksp_maxit, w, &its32,

@@ -207,8 +207,7 @@ int vfgpu_destroy(vfgpu_ctx* c) {
   if (!c) return VFGPU_OK;
   cudaSetDevice(c->dev);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  for (auto& g : c->graphs)
-    if (g.exec) cudaGraphExecDestroy(g.exec);
+  for (auto& g : c->graphs) g.release();
   c->graphs.clear();
   free_solver(c);
   free_mg(c);
