@@ -123,3 +123,41 @@ def test_u_stencil(cuda, oracle_mod, n, l, field):
     yref = o.u_apply(v, x, m2.reshape(-1))
     assert np.abs(ctx.u_apply(xd, vg.FP64).cpu().numpy() - yref).max() <= 1e-12 * np.abs(yref).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("cellE,unilateral,layers", [(False, 1, False), (True, 0, False), (True, 1, False),
+                                                     (False, 0, True)])
+def test_u_tiles(cuda, oracle_mod, cellE, unilateral, layers):
+    """The tile engine past the sizes of the two-phase apply (86 x 87 x 88: more than 400,000
+    cells, ragged tiles), where the other forms' tests are on smaller grids: NOCOMPRESSION,
+    per-cell modulus, material layers; FP64 at 1e-12, FP32 at 2e-6 against the oracle."""
+    import vpfhf_b200 as vg
+    n, l = (86, 87, 88), (1.7, 1.6, 1.9)
+    rng = np.random.default_rng(21)
+    cE = None
+    if cellE:
+        cE = np.exp(np.log(1e10) + 0.5 * rng.standard_normal((n[0] - 1) * (n[1] - 1) * (n[2] - 1)))
+        cE = cE.astype(np.float32).astype(np.float64)
+    E, nu = ([1e10, 3e10], [0.25, 0.3]) if layers else ([1e10], [0.25])
+    lay = np.array([k // 40 % 2 for k in range(n[2] - 1)], np.int32) if layers else None
+    o = oracle_mod.Oracle(n, l, E=E, nu=nu, eta=1e-6, cellE=cE, unilateral=unilateral, layer=lay)
+    ctx = vg.VFContext(n, l, [dict(E=a, nu=b) for a, b in zip(E, nu)], eta=1e-6, layer=lay)
+    if cE is not None:
+        ctx.set_cell_modulus(cE)
+    ctx.set_bc(vg.rollers())
+    mask, _ = o.bc(oracle_mod.rollers_face())
+    v = np.ones(o.N)
+    vv = v.reshape(n[2], n[1], n[0])
+    vv[30:50, 20:60, 10:70] = rng.uniform(0, 1, (20, 40, 60))
+    u0 = rng.standard_normal(3 * o.N) * 1e-4
+    ctx.set_field("V", v)
+    if unilateral:
+        ctx.set_unilateral(1)
+        ctx.set_field("U", u0)
+    x = rng.standard_normal(3 * o.N) * 1e-3
+    yref = o.u_apply_u(u0, v, x, mask) if unilateral else o.u_apply(v, x, mask)
+    xd = cuda.from_numpy(x).cuda()
+    assert np.abs(ctx.u_apply(xd, vg.FP64).cpu().numpy() - yref).max() <= 1e-12 * np.abs(yref).max()
+    y32 = ctx.u_apply(xd, vg.MIXED).cpu().numpy()
+    assert np.linalg.norm(y32 - yref) <= 2e-6 * np.linalg.norm(yref)
+    ctx.close()

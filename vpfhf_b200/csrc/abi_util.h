@@ -46,6 +46,11 @@ cudaError_t u_lists_refresh(vfgpu_ctx* c);
 // Whether the ctx's U applies in this precision (8 or 4 bytes) take the unit lists (and
 // write the second wave's x.y partials).
 bool u_lists_on(const vfgpu_ctx* c, int prec_bytes);
+// Whether the ctx's U applies in this precision run in two phases.
+bool u_twophase_on(const vfgpu_ctx* c, int prec_bytes);
+// Makes the two-phase scratch hold one apply of this grid in this precision, if such applies
+// run in two phases (a grown one invalidates captured graphs).
+cudaError_t ensure_escr(vfgpu_ctx* c, int nx, int ny, int nz, int prec_bytes);
 // Whether the ctx's U applies in this precision take the stencil at homogeneous nodes: one
 // material, no per-cell modulus, no NOCOMPRESSION, a grid for which it pays.
 bool u_stencil_on(const vfgpu_ctx* c, int prec_bytes);

@@ -6,6 +6,7 @@
 #include "kernels.h"
 #include "ops.cuh"
 #include "u_stencil.cuh"
+#include "u_twophase.cuh"
 
 namespace vfgpu {
 
@@ -475,6 +476,26 @@ cudaError_t build_stencil_lists(uint8_t* node, int2* range, int nx, int ny, int 
   return cudaGetLastError();
 }
 
+// Largest grids, in cells, whose applies run in two phases.  Per apply, two cracks, tiles (with
+// the stencil where it is taken) against two phases, us AT1 / AT2: FP64 17^3 16.4 / 14.4 and
+// 9.3 / 9.3 (of which about 8 are the call), 41^3 22.6 / 21.6 and 14.4 / 14.7, 65^3 36.9 / 34.9
+// and 28.7 / 34.2, 81^3 47.0 / 71.7 and 59.3 / 69.7, 97^3 46.8 / 93.2 and 95.7 / 112.8; FP32 41^3
+// 18.5 / 20.5 and 11.3 / 11.3, 65^3 24.6 / 27.9 and 18.5 / 23.8, 81^3 42.0 / 48.5 and 28.7 / 39.0,
+// 97^3 52.3 / 65.0 and 53.6 / 70.9; 97 x 61 x 83 (tiles that fit) - / 31.6 and - / 33.2.
+#ifndef VFGPU_TWOPHASE64_CELLS
+#define VFGPU_TWOPHASE64_CELLS 300000
+#endif
+#ifndef VFGPU_TWOPHASE32_CELLS
+#define VFGPU_TWOPHASE32_CELLS 400000
+#endif
+bool twophase_pays(int nx, int ny, int nz, int prec_bytes) {
+  const int64_t most = prec_bytes == 8 ? VFGPU_TWOPHASE64_CELLS : VFGPU_TWOPHASE32_CELLS;
+  return (int64_t)(nx - 1) * (ny - 1) * (nz - 1) <= most;
+}
+
+size_t twophase_scratch(int nx, int ny, int nz) { return twophase_values(nx, ny, nz); }
+int twophase_dots(int nx, int ny, int nz) { return twophase_node_blocks(nx, ny, nz); }
+
 bool stencil_pays(const TilePlan& p, int nx, int ny, int nz, int prec_bytes) {
   if (U64_TY != U32_TY || (prec_bytes == 4 && kU32Packed)) return false;  // the plans share the node flags
   const int64_t ncol = (int64_t)p.ntx * p.nty;
@@ -537,6 +558,11 @@ static cudaError_t launch_u_stencil(typename OpG::Args A, const TilePlan& p, con
 template <>
 cudaError_t launch_u_apply<double>(const UApplyArgs<double>& A, const TilePlan& p,
                                    const LayerTable& L, cudaStream_t s) {
+  if (A.scr) {
+    if (A.cflag) return launch_u_twophase<UOpNC<double>>(A, L, s);
+    if (cubic(A)) return launch_u_twophase<UOp<double, true>>(A, L, s);
+    return launch_u_twophase<UOp<double>>(A, L, s);
+  }
   if (A.cflag) return launch_tile_apply<UOpNC<double>, U64_TY, 1>(A, p, L, s);
   if (A.node) {
     if (cubic(A)) return launch_u_stencil<UOpMarked<double, true>, U64_TY, U64_MINB, ST64_MINB>(A, p, L, s);
@@ -554,6 +580,11 @@ cudaError_t launch_u_apply<double>(const UApplyArgs<double>& A, const TilePlan& 
 template <>
 cudaError_t launch_u_apply<float>(const UApplyArgs<float>& A, const TilePlan& p,
                                   const LayerTable& L, cudaStream_t s) {
+  if (A.scr) {
+    if (A.cflag) return launch_u_twophase<UOpNC<float>>(A, L, s);
+    if (cubic(A)) return launch_u_twophase<UOp<float, true>>(A, L, s);
+    return launch_u_twophase<UOp<float>>(A, L, s);
+  }
   // NOCOMPRESSION needs the scalar layout: its plan is the FP32 plan only with the
   // scalar tile (the packed build option keeps the plain operator packed)
   if (A.cflag) return launch_tile_apply<UOpNC<float>, U_TY, 2>(A, p, L, s);

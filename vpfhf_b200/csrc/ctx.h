@@ -64,6 +64,9 @@ struct vfgpu_ctx {
   vfgpu::TilePlan plan64{}, plan32{};
   double* d_dot = nullptr;   // block partials of the CG's p.w written by the operator applies
   double* seam64 = nullptr;
+  // scratch of the two-phase U applies (of this grid or of multigrid levels), FP64 or FP32
+  void* d_escr = nullptr;
+  size_t escr_bytes = 0;
   float* seam32 = nullptr;
   double *t64a = nullptr, *t64b = nullptr;
   float *t32a = nullptr, *t32b = nullptr;

@@ -36,6 +36,11 @@ bool unit_lists_pay(const TilePlan& p, int nz, int prec_bytes);
 // Rebuilds the lists from the FP64 phase field v (two launches on s).
 cudaError_t build_unit_lists(const double* v, int nx, int ny, int nz, const TilePlan& p,
                              const UnitLists& L, cudaStream_t s);
+// Whether the grid's U applies run in two phases (u_twophase.cuh); the scratch of one, in values,
+// and the x.y partials it writes.
+bool twophase_pays(int nx, int ny, int nz, int prec_bytes);
+size_t twophase_scratch(int nx, int ny, int nz);
+int twophase_dots(int nx, int ny, int nz);
 // Whether the plan's homogeneous nodes take the stencil in precision prec_bytes (a rule of
 // the grid alone, so that every apply of a grid gives the same bits).
 bool stencil_pays(const TilePlan& p, int nx, int ny, int nz, int prec_bytes);

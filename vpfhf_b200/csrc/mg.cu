@@ -685,6 +685,7 @@ template <typename T> UApplyArgs<T> level_args(vfgpu_ctx* c, const LevelT<T>& V,
   A.P = c->d_params;
   A.cflag = V.cflag;
   use_unit_lists(A, V.ul);
+  A.scr = twophase_pays(V.nx, V.ny, V.nz, (int)sizeof(T)) ? static_cast<T*>(c->d_escr) : nullptr;
   return A;
 }
 
@@ -859,6 +860,7 @@ template <typename T> int mg_build(vfgpu_ctx* c) {
     etab_host(hx, hy, hz, &L.tab);
     L.coef = c->mg_coef + (int64_t)kCoefPerLevel * l;
     if (e == cudaSuccess) e = build_xfer(L, f);
+    if (e == cudaSuccess) e = ensure_escr(c, nx, ny, nz, (int)sizeof(T));
   }
   c->mg_bytes = (int)sizeof(T);
   c->mg_ready = false;
@@ -1121,6 +1123,8 @@ long long mg_memory_bytes(int nx, int ny, int nz, int bytes) {
   const long long nrd = bytes == 4 ? std::max(3 * N, 6 * N1) : 3 * N;
   long long b = (3 * 3 * N + 2 * nrd) * bytes + (bytes == 4 ? 3 * N * (4 + 8) : 0);  // fine vectors
   const int nlev = mg_levels(nx, ny, nz);
+  const bool fine_two = twophase_pays(nx, ny, nz, bytes);  // the ctx's scratch serves the levels
+  long long scr = 0;
   for (int l = 1; l < nlev; l++) {
     b += (long long)(nx + ny + nz) * (4 + 8);  // transfer tables
     nx = coarser(nx);
@@ -1131,9 +1135,11 @@ long long mg_memory_bytes(int nx, int ny, int nz, int bytes) {
     const TilePlan p = u_plan(nx, ny, nz, bytes, 148);
     b += (long long)(p.seamX + p.seamY) * bytes + 7 * 3 * Nl * bytes + Nl * 8 +
          (bytes == 4 ? Nl * 4 : 0) + Nl + (nz - 1) + NCl * 4;
+    if (!fine_two && twophase_pays(nx, ny, nz, bytes))
+      scr = std::max(scr, (long long)twophase_scratch(nx, ny, nz) * bytes);
   }
   if (nlev < 2) return 0;
-  return b + (long long)kCoefPerLevel * nlev * 8;
+  return b + scr + (long long)kCoefPerLevel * nlev * 8;
 }
 
 int run_mgcg(vfgpu_ctx* c, bool fp32, const double* b, double* x, double* r, double* p, double* w,

@@ -94,6 +94,8 @@ extern "C" int vfgpu_u_apply_noalloc(const vfgpu_grid* g, const vfgpu_matprop* m
   A.ihz = 1.0 / hz;
   A.vol = hx * hy * hz;
   A.eta = eta;
+  if (twophase_pays(g->nx, g->ny, g->nz, 8) && twophase_scratch(g->nx, g->ny, g->nz) <= kScratchDoubles)
+    A.scr = scratch;
   e = launch_u_apply<double>(A, p, L, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "vfgpu_u_apply_noalloc");
   return VFGPU_OK;

@@ -290,6 +290,7 @@ static cudaError_t u_apply32(vfgpu_ctx* c, const float* x, float* y, const int* 
 static int dots_of(const vfgpu_ctx* c, const TilePlan& p) { return tile_dot_count(p, c->nx, c->ny, c->nz); }
 // The U applies with unit lists or the stencil write a second wave's partials.
 static int u_dots_of(const vfgpu_ctx* c, const TilePlan& p, int prec_bytes) {
+  if (u_twophase_on(c, prec_bytes)) return twophase_dots(c->nx, c->ny, c->nz);
   return dots_of(c, p) + (u_stencil_on(c, prec_bytes) ? p.st.blocks() + p.st.nface : u_lists_on(c, prec_bytes) ? p.ncta0 : 0);
 }
 
@@ -803,6 +804,8 @@ int vfgpu_memory_estimate(const vfgpu_grid* g, long long* bytes) {
   b += (2 * 3 * N + 5 * N) * 8;                          // fields U, BCU, V, VIrrev, theta, thetaRef, p
   b += N * 4 + (g->nz - 1) + 3 * N + 3 * N;              // V32, layers, BC kinds and bits
   b += (long long)(unit_lists_bytes(p64, g->nz) + unit_lists_bytes(p32, g->nz));  // U unit lists
+  if (twophase_pays(g->nx, g->ny, g->nz, 8)) b += (long long)twophase_scratch(g->nx, g->ny, g->nz) * 8;
+  else if (twophase_pays(g->nx, g->ny, g->nz, 4)) b += (long long)twophase_scratch(g->nx, g->ny, g->nz) * 4;
   b += N + (long long)(stencil_range_bytes(p64) + stencil_range_bytes(p32));  // U node and block flags
   b += (long long)(p64.seamX + p64.seamY) * 8 + (long long)(p32.seamX + p32.seamY) * 4;
   b += 3 * 3 * N * 8 + 2 * 3 * N * 4;                    // staging vectors

@@ -60,6 +60,8 @@ template <typename T> struct UApplyArgs {
   const int4* __restrict__ ur[2];
   const int* __restrict__ ustart[2];
   const int* __restrict__ utotal;
+  T* __restrict__ scr;                // twophase_values(nx, ny, nz) of scratch, or null; given: the
+                                      // apply runs in two phases (u_twophase.cuh)
   int nx, ny, nz;
   int ntx, nty;                       // tiles in x, y
   T ihx, ihy, ihz, vol, eta;

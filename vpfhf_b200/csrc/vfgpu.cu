@@ -145,8 +145,24 @@ UApplyArgs<T> u_args(vfgpu_ctx* c, const T* x, const T* v, T* y, T* seam, const 
   A.P = c->d_params;
   A.cflag = c->unilateral ? c->d_cflag : nullptr;
   use_unit_lists(A, u_lists_of(c, (int)sizeof(T)));
+  A.scr = u_twophase_on(c, (int)sizeof(T)) ? static_cast<T*>(c->d_escr) : nullptr;
   return A;
 }
+bool u_twophase_on(const vfgpu_ctx* c, int prec_bytes) { return twophase_pays(c->nx, c->ny, c->nz, prec_bytes); }
+
+cudaError_t ensure_escr(vfgpu_ctx* c, int nx, int ny, int nz, int prec_bytes) {
+  if (!twophase_pays(nx, ny, nz, prec_bytes)) return cudaSuccess;
+  const size_t need = twophase_scratch(nx, ny, nz) * prec_bytes;
+  if (need <= c->escr_bytes) return cudaSuccess;
+  cudaFree(c->d_escr);
+  c->d_escr = nullptr;
+  c->escr_bytes = 0;
+  c->gen++;
+  const cudaError_t e = cudaMalloc(&c->d_escr, need);
+  if (e == cudaSuccess) c->escr_bytes = need;
+  return e;
+}
+
 bool u_stencil_on(const vfgpu_ctx* c, int prec_bytes) {
   return (prec_bytes == 8 ? c->d_srange64 : c->d_srange32) && c->nlayer == 1 && !c->d_cellE && !c->unilateral;
 }
@@ -155,6 +171,7 @@ bool u_stencil_on(const vfgpu_ctx* c, int prec_bytes) {
 // (NOCOMPRESSION aside).
 static bool u_lists_wanted(const vfgpu_ctx* c, int prec_bytes) {
   const TilePlan& p = prec_bytes == 8 ? c->plan64 : c->plan32;
+  if (u_twophase_on(c, prec_bytes)) return false;
   if (!(prec_bytes == 8 ? c->ul64.cls : c->ul32.cls)) return false;
   if (u_stencil_on(c, prec_bytes) || c->u_split == VFGPU_U_SPLIT_ON) return true;
   return c->u_split == VFGPU_U_SPLIT_AUTO && unit_lists_pay(p, c->nz, prec_bytes);
@@ -221,7 +238,7 @@ int vfgpu_destroy(vfgpu_ctx* c) {
   if (c->s_in) cudaStreamDestroy(c->s_in);
   if (c->s_out) cudaStreamDestroy(c->s_out);
   cudaFree(c->t64c);
-  void* bufs[] = {c->d_tcB, c->d_tcerr, c->d_widthc, c->d_pmult, c->d_width, c->d_wpart, c->d_wstall, c->d_cflag, c->d_params, c->d_dot, c->d_elayer, c->d_ul, c->d_unode, c->d_srange64, c->d_srange32, c->d_cellE, c->bcU_kind, c->bcU_bits, c->bcV_kind, c->bcV_bits,
+  void* bufs[] = {c->d_tcB, c->d_tcerr, c->d_widthc, c->d_pmult, c->d_width, c->d_wpart, c->d_wstall, c->d_cflag, c->d_params, c->d_dot, c->d_elayer, c->d_ul, c->d_escr, c->d_unode, c->d_srange64, c->d_srange32, c->d_cellE, c->bcU_kind, c->bcU_bits, c->bcV_kind, c->bcV_bits,
                   c->V32, c->seam64, c->seam32, c->t64a, c->t64b, c->t32a, c->t32b};
   for (void* p : bufs) cudaFree(p);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -289,15 +306,21 @@ int vfgpu_create(const vfgpu_grid* g, vfgpu_ctx** out) {
     }
   }
   {
-    const bool s64 = c->ul64.cls && stencil_pays(c->plan64, c->nx, c->ny, c->nz, 8);
-    const bool s32 = c->ul32.cls && stencil_pays(c->plan32, c->nx, c->ny, c->nz, 4);
+    for (int b : {8, 4})
+      if (e == cudaSuccess) e = ensure_escr(c, c->nx, c->ny, c->nz, b);
+    if (e != cudaSuccess) {
+      vfgpu_destroy(c);
+      return cuda_fail(e, "vfgpu_create: cudaMalloc");
+    }
+    const bool s64 = !u_twophase_on(c, 8) && c->ul64.cls && stencil_pays(c->plan64, c->nx, c->ny, c->nz, 8);
+    const bool s32 = !u_twophase_on(c, 4) && c->ul32.cls && stencil_pays(c->plan32, c->nx, c->ny, c->nz, 4);
     if (s64 || s32) ALLOC(c->d_unode, c->N);
     if (s64) ALLOC(c->d_srange64, stencil_range_bytes(c->plan64));
     if (s32) ALLOC(c->d_srange32, stencil_range_bytes(c->plan32));
   }
   ALLOC(c->d_params, sizeof(DevParams));
   {
-    int nd = vmat_blocks(c->N);
+    int nd = std::max(vmat_blocks(c->N), twophase_dots(c->nx, c->ny, c->nz));
     for (const TilePlan* p : {&c->plan64, &c->plan32})
       nd = std::max(nd, tile_dot_count(*p, c->nx, c->ny, c->nz) + std::max(p->ncta0, p->st.blocks() + p->st.nface));
     ALLOC(c->d_dot, (size_t)nd * sizeof(double));
