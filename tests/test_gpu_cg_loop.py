@@ -1,5 +1,5 @@
-"""GPU: the device-side CG loop -- iteration caps and time limits that end it anywhere in its
-body of four iterations, systems of a few unknowns, and many solves side by side."""
+"""GPU: the device-side CG loops -- iteration caps and time limits that end them anywhere in
+their body, systems of a few unknowns, and many solves side by side."""
 import numpy as np
 import pytest
 
@@ -69,3 +69,23 @@ def test_solves_side_by_side_keep_their_bits(cuda):
             a = alone[r["tag"] % 4]
             for key in ("elastic", "pressure_work", "surface", "cov", "am_err", "ksp_its_u", "ksp_its_v"):
                 assert r[key] == a[key], (r["tag"], key)
+
+
+@pytest.mark.parametrize("precision,n", [("fp64", (17, 9, 13)), ("mixed", (17, 9, 13)), ("mixed", (18, 18, 10))])
+@pytest.mark.parametrize("maxit", [1, 2, 5])
+def test_multigrid_iteration_cap(cuda, precision, n, maxit):
+    """The multigrid PCG's loop ends at the cap (odd and even unknown counts) with the last step
+    in x: the same bits each time, and a residual that Jacobi CG needs more iterations for."""
+    out = []
+    for pc in ("mg", "mg", "jacobi"):
+        ctx = _ctx(n, 2)
+        rc, st = ctx.step_u(dict(pc=pc, precision="fp64" if pc == "jacobi" else precision, ksp_maxit=maxit,
+                                 snes_maxit=1, ksp_rtol=1e-14))
+        assert st["ksp_its"] == maxit, st
+        out.append((ctx.get_field("U"), st["fnorm"]))
+        ctx.close()
+    assert np.array_equal(out[0][0], out[1][0])
+    assert out[0][1] == out[1][1] and np.isfinite(out[0][1])
+    if maxit == 5:
+        assert out[0][1] < out[2][1]
+

@@ -34,6 +34,12 @@ int run_mgcg(vfgpu_ctx* c, bool fp32, const double* b, double* x, double* r, dou
 // ctx->gen moves on (null: capture failed, run the body directly).
 cudaGraphExec_t ctx_graph(vfgpu_ctx* c, int kind, int batch,
                           const std::function<cudaError_t()>& body);
+// The same for a conditional while node whose body is what `body` launches: it gets the handle
+// whose condition its last kernel sets.
+cudaGraphExec_t ctx_while_graph(vfgpu_ctx* c, int kind, int batch,
+                                const std::function<cudaError_t(cudaGraphConditionalHandle)>& body);
+// x.y partials an apply of the ctx's U operator writes in this precision.
+int u_dot_count(const vfgpu_ctx* c, int prec_bytes);
 void free_mg(vfgpu_ctx* c);
 // Device bytes of the multigrid hierarchy of a grid in V-cycle precision `bytes` (4 or 8),
 // a per-cell modulus included; 0 when the grid has no coarse level.

@@ -112,7 +112,6 @@ struct vfgpu_ctx {
   bool mg_ev = false;             // the levels' ev vectors hold earlier eigenvector estimates
   bool mg_layers = false;         // the coarse levels' element layers match d_elayer
   double* mg_coef = nullptr;      // 64 doubles per level (MGLevel::coef points into it)
-  double* mg_z = nullptr;         // FP32 V-cycle: the preconditioned residual in FP64 (3N)
   const void* mg_dinv0 = nullptr; // fine inverse diagonal in the V-cycle's precision
 
   // Flow-coupling boundary (width.cu): cell width, permeability multiplier, node width,

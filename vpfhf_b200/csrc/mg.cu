@@ -17,8 +17,11 @@
 // estimate of 12 power iterations per level, 4 from the previous vector once there is
 // one), pre and post; the coarsest level runs degree kCoarseDeg on [lmax/100, lmax].  Every step is a fixed sequence of
 // deterministic kernels reading its Chebyshev coefficients from device memory, so
-// the V-cycle is a fixed symmetric linear operator (plain PCG applies) and is
-// replayed as one CUDA graph.
+// the V-cycle is a fixed symmetric linear operator (plain PCG applies).  A PCG iteration is the
+// body of a graph's while node: cycle, vector kernels (cg.cuh) and stopping test without the
+// host.  A host-driven iteration cost two round trips, a copy of r and z each way in mixed
+// precision and, at the last one, a cycle that nothing used: AM step at 129^3 mixed 19.3 ->
+// 18.0 ms, 65^3 FP64 26.1 -> 22.1 ms, 257 x 257 x 129 per-cell modulus 101.6 -> 85.8 ms.
 //
 // Precision: the V-cycle runs in FP64 (solve precision FP64) or FP32 (MIXED); the
 // outer CG, its residual and its stopping test stay FP64 in both.
@@ -404,23 +407,6 @@ __global__ void __launch_bounds__(kCoarseThreads, 1)
 
 template <typename Op> size_t coarse_smem_bytes(int ncell) {
   return (size_t)ncell * 8 * 3 * sizeof(typename Op::T);
-}
-
-// The PCG step x += alpha p, r -= alpha w with alpha = rz / (p.w) formed on the device
-// (pw = the dot product just reduced into *pw_in); nothing changes unless p.w > 0 (the
-// host then stops on the indefinite or NaN p.w it reads back from pw_out).
-__global__ void pcg_step_kernel(double* __restrict__ x, double* __restrict__ r,
-                                const double* __restrict__ p, const double* __restrict__ w,
-                                const double* __restrict__ pw_in, double* __restrict__ pw_out,
-                                double rz, int64_t n) {
-  const double pw = *pw_in;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *pw_out = pw;
-  if (!(pw > 0.)) return;
-  const double alpha = rz / pw;
-  GRID_STRIDE(i, n) {
-    x[i] += alpha * p[i];
-    r[i] += (-alpha) * w[i];
-  }
 }
 
 // Deterministic start vector of the power iteration in (-1/2, 1/2), 0 on Dirichlet dofs.
@@ -827,10 +813,7 @@ template <typename T> int mg_build(vfgpu_ctx* c) {
     L0.r = dalloc<T>(nrd, e);
     L0.d = dalloc<T>(nrd, e);
     L0.t = dalloc<T>(n3, e);
-    if (f32) {
-      L0.b = dalloc<T>(n3, e);
-      c->mg_z = (double*)dalloc<double>(n3, e);
-    }
+    if (f32) L0.b = dalloc<T>(n3, e);
     L0.coef = c->mg_coef;
   }
   int nx = c->nx, ny = c->ny, nz = c->nz;
@@ -983,25 +966,6 @@ template <typename T> int mg_setup(vfgpu_ctx* c) {
   return VFGPU_OK;
 }
 
-// One preconditioner application z = M^-1 r (FP64 in and out), as a graph replay.
-template <typename T> cudaError_t precondition(vfgpu_ctx* c, const double* r, double* z);
-template <> cudaError_t precondition<double>(vfgpu_ctx* c, const double* r, double* z) {
-  auto body = [c, r, z]() { return vcycle<double>(c, 0, r, z); };
-  cudaGraphExec_t g = c->use_graphs ? ctx_graph(c, kGraphMG64, 0, body) : nullptr;
-  return g ? cudaGraphLaunch(g, c->stream) : body();
-}
-template <> cudaError_t precondition<float>(vfgpu_ctx* c, const double* r, double* z) {
-  auto body = [c, r, z]() {
-    const LevelT<float> V = view<float>(c, 0);
-    cudaError_t e = convert_f64_f32(r, V.b, V.n3, c->stream);
-    if (e == cudaSuccess) e = vcycle<float>(c, 0, V.b, V.x);
-    if (e == cudaSuccess) e = convert_f32_f64(V.x, z, V.n3, c->stream);
-    return e;
-  };
-  cudaGraphExec_t g = c->use_graphs ? ctx_graph(c, kGraphMG32, 0, body) : nullptr;
-  return g ? cudaGraphLaunch(g, c->stream) : body();
-}
-
 template <typename T>
 int mgcg(vfgpu_ctx* c, const double* b, double* x, double* r, double* p, double* w,
          const double* dinv0, bool reuse, double rtol, double atol, double dtol, int maxit,
@@ -1014,31 +978,9 @@ int mgcg(vfgpu_ctx* c, const double* b, double* x, double* r, double* p, double*
   }
   *levels = (int)c->mg.size();
   const int64_t n3 = 3 * c->N;
-  // the preconditioned residual: the V-cycle's own output vector in FP64
-  double* z = sizeof(T) == 8 ? (double*)c->mg[0].x : c->mg_z;
-  cudaError_t e = cudaMemsetAsync(x, 0, n3 * sizeof(double), c->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(r, b, n3 * sizeof(double), cudaMemcpyDeviceToDevice, c->stream);
-  // h[0] = r.z, h[2] = ||D^-1 r||^2, h[8] = the step's p.w (one host read per iteration)
-  double h[9] = {0., 0., 0., 0., 0., 0., 0., 0., 0.};
-  auto scalars = [&]() {
-    const double* pa[1] = {r};
-    const double* pb[1] = {z};
-    if (e == cudaSuccess) e = dev_dots(pa, pb, 1, n3, c->d_red, c->d_out, c->stream);
-    if (e == cudaSuccess) e = dev_znorm2(r, dinv0, n3, c->d_red, c->d_out + 2, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, c->d_out, 9 * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  };
-  if (e == cudaSuccess) e = precondition<T>(c, r, z);
-  scalars();
-  if (e != cudaSuccess) return cuda_fail(e, "multigrid PCG");
-  double rz = h[0];
-  const double rnorm0 = sqrt(h[2]), ttol = std::max(rtol * rnorm0, atol);
-  *its = 0;
-  *reason = 0;
-  if (!(rnorm0 == rnorm0)) *reason = CG_DIVERGED_NAN;
-  else if (rnorm0 <= ttol) *reason = rnorm0 <= atol ? CG_CONVERGED_ATOL : CG_CONVERGED_RTOL;
-  else if (!(rz > 0.)) *reason = rz == 0. ? CG_CONVERGED_ATOL : CG_DIVERGED_INDEFINITE;
-  if (!*reason) e = cudaMemcpyAsync(p, z, n3 * sizeof(double), cudaMemcpyDeviceToDevice, c->stream);
+  const LevelT<T> V = view<T>(c, 0);
+  constexpr bool f32 = sizeof(T) == 4;
+  MgcgVecs<T> m{x, r, p, w, dinv0, b, V.x, f32 ? (float*)V.b : nullptr, n3, c->d_dot, u_dot_count(c, 8)};
   LevelT<double> outer{};  // the FP64 Jacobian whatever the V-cycle's precision
   outer.nx = c->nx;
   outer.ny = c->ny;
@@ -1054,36 +996,40 @@ int mgcg(vfgpu_ctx* c, const double* b, double* x, double* r, double* p, double*
   outer.cellE = c->d_cellE;
   outer.cflag = c->unilateral ? c->d_cflag : nullptr;
   outer.ul = u_lists_of(c, 8);
-  while (!*reason && e == cudaSuccess) {
-    e = level_apply<double>(c, outer, p, w);
-    const double* pa[1] = {p};
-    const double* pb[1] = {w};
-    if (e == cudaSuccess) e = dev_dots(pa, pb, 1, n3, c->d_red, c->d_out, c->stream);
-    if (e == cudaSuccess) {
-      pcg_step_kernel<<<blocks_for(n3), 256, 0, c->stream>>>(x, r, p, w, c->d_out, c->d_out + 8, rz, n3);
-      e = cudaGetLastError();
+  // one iteration (cg.cuh), in a while node of a graph: no host round trip until the end
+  auto body = [&](const cudaGraphConditionalHandle* loop) {
+    cudaError_t eb = vcycle<T>(c, 0, f32 ? V.b : (const T*)(const void*)r, V.x);
+    if (eb == cudaSuccess) eb = mgcg_direction<T>(m, c->d_cg, c->d_red, c->stream);
+    if (eb == cudaSuccess) {
+      UApplyArgs<double> A = level_args<double>(c, outer, p, w);
+      A.skip = &c->d_cg->done;
+      A.dot = c->d_dot;
+      eb = launch_u_apply<double>(A, c->plan64, c->layers, c->stream);
     }
-    if (e == cudaSuccess) e = precondition<T>(c, r, z);
-    scalars();
-    if (e != cudaSuccess) break;
-    const double pw = h[8];
-    if (!(pw > 0.)) {  // x and r were left unchanged
-      *reason = (pw == pw) ? CG_DIVERGED_INDEFINITE : CG_DIVERGED_NAN;
-      break;
-    }
-    *its += 1;
-    const double dp = sqrt(h[2]);
-    if (!(dp == dp)) *reason = CG_DIVERGED_NAN;
-    else if (dp <= ttol) *reason = CG_CONVERGED_RTOL;
-    else if (dp >= dtol * rnorm0) *reason = CG_DIVERGED_DTOL;
-    else if (*its >= maxit) *reason = CG_DIVERGED_ITS;
-    else if (!(h[0] > 0.)) *reason = h[0] == 0. ? CG_CONVERGED_ATOL : CG_DIVERGED_INDEFINITE;
-    else {
-      const double beta = h[0] / rz;
-      rz = h[0];
-      e = dev_axpby(p, z, beta, p, n3, c->stream);  // p = z + beta p
-    }
+    if (eb == cudaSuccess) eb = mgcg_update<T>(m, c->d_cg, c->d_red, c->stream);
+    if (eb == cudaSuccess) eb = mgcg_end(c->d_cg, c->d_red, n3, loop, c->stream);
+    return eb;
+  };
+  auto read_state = [&]() {
+    cudaError_t eb = cudaMemcpyAsync(c->h_cg, c->d_cg, sizeof(CGState), cudaMemcpyDeviceToHost, c->stream);
+    return eb == cudaSuccess ? cudaStreamSynchronize(c->stream) : eb;
+  };
+  cudaError_t e = mgcg_init<T>(m, c->d_cg, c->d_red, rtol, atol, dtol, maxit, c->stream);
+  if (e == cudaSuccess) e = read_state();
+  cudaGraphExec_t g = !c->use_graphs ? nullptr
+                                     : ctx_while_graph(c, f32 ? kGraphMG32 : kGraphMG64, 0,
+                                                       [&](cudaGraphConditionalHandle h) { return body(&h); });
+  while (e == cudaSuccess && !c->h_cg->done) {
+    e = g ? cudaGraphLaunch(g, c->stream) : body(nullptr);
+    if (e == cudaSuccess) e = read_state();
   }
+  CGVecs<double> fin{};
+  fin.x = x;
+  fin.p = p;
+  fin.n = n3;
+  if (e == cudaSuccess) e = cg_finish_x<double>(fin, c->d_cg, c->stream);
+  *its = c->h_cg->its;
+  *reason = c->h_cg->reason;
   if (e != cudaSuccess) return cuda_fail(e, "multigrid PCG");
   return VFGPU_OK;
 }
@@ -1109,9 +1055,7 @@ void free_mg(vfgpu_ctx* c) {
   }
   c->mg.clear();
   cudaFree(c->mg_coef);
-  cudaFree(c->mg_z);
   c->mg_coef = nullptr;
-  c->mg_z = nullptr;
   c->mg_bytes = 0;
   c->mg_ready = false;
   c->mg_ev = false;
@@ -1121,7 +1065,7 @@ long long mg_memory_bytes(int nx, int ny, int nz, int bytes) {
   const long long N = (long long)nx * ny * nz;
   const long long N1 = (long long)coarser(nx) * coarser(ny) * coarser(nz);
   const long long nrd = bytes == 4 ? std::max(3 * N, 6 * N1) : 3 * N;
-  long long b = (3 * 3 * N + 2 * nrd) * bytes + (bytes == 4 ? 3 * N * (4 + 8) : 0);  // fine vectors
+  long long b = (3 * 3 * N + 2 * nrd) * bytes + (bytes == 4 ? 3 * N * 4 : 0);  // fine vectors
   const int nlev = mg_levels(nx, ny, nz);
   const bool fine_two = twophase_pays(nx, ny, nz, bytes);  // the ctx's scratch serves the levels
   long long scr = 0;

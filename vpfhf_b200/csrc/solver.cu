@@ -10,28 +10,6 @@ namespace vfgpu {
 
 namespace {
 
-// Fixed-order sum of K values per thread over the block (shuffle trees, then the warps in
-// order), in every thread.
-template <int K>
-__device__ __forceinline__ void block_total(double (&v)[K]) {
-  __shared__ double red[K][RED_THREADS / 32];
-#pragma unroll
-  for (int q = 0; q < K; q++)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-  __syncthreads();  // a previous call's totals have been read
-  if ((threadIdx.x & 31) == 0)
-#pragma unroll
-    for (int q = 0; q < K; q++) red[q][threadIdx.x >> 5] = v[q];
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < K; q++) {
-    v[q] = red[q][0];
-#pragma unroll
-    for (int w = 1; w < RED_THREADS / 32; w++) v[q] += red[q][w];
-  }
-}
-
 // Block-level fixed-order sum of K values per thread into partial[blockIdx*K + q].
 template <int K>
 __device__ __forceinline__ void block_sum(double (&v)[K], double* __restrict__ partial) {
@@ -39,18 +17,6 @@ __device__ __forceinline__ void block_sum(double (&v)[K], double* __restrict__ p
   if (threadIdx.x == 0)
 #pragma unroll
     for (int q = 0; q < K; q++) partial[blockIdx.x * K + q] = v[q];
-}
-
-// Fixed-order sum of n blocks' partials by one block, in every thread (identical in every
-// block that calls it).  L1 is bypassed: an earlier kernel of the same graph wrote them.
-template <int K>
-__device__ __forceinline__ void final_sum(const double* __restrict__ partial, int n, double (&out)[K]) {
-#pragma unroll
-  for (int q = 0; q < K; q++) out[q] = 0.;
-  for (int b = threadIdx.x; b < n; b += RED_THREADS)
-#pragma unroll
-    for (int q = 0; q < K; q++) out[q] += __ldcg(partial + b * K + q);
-  block_total<K>(out);
 }
 
 #define GRID_LOOP(i, n)                                                                  \
@@ -303,6 +269,167 @@ __global__ void __launch_bounds__(RED_THREADS) cg_p_kernel(CGVecs<T> v, CGState*
   }
 }
 
+// ---- PCG around the multigrid V-cycle (cg.cuh)
+template <typename TZ>
+__global__ void __launch_bounds__(RED_THREADS) mgcg_init_kernel(MgcgVecs<TZ> v, double* partial) {
+  double acc[1] = {0.};
+  GRID_LOOP(i, v.n) {
+    const double r = v.b[i], z = r * v.dinv[i];
+    v.x[i] = 0.;
+    v.r[i] = r;
+    if (v.r32) v.r32[i] = (float)r;
+    acc[0] += z * z;
+  }
+  block_sum<1>(acc, partial);
+}
+
+__global__ void __launch_bounds__(RED_THREADS) mgcg_init_final(CGState* st, const double* partial, int nblk,
+                                                               double rtol, double atol, double dtol, int maxit) {
+  double s[1];
+  final_sum<1>(partial, nblk, s);
+  if (threadIdx.x) return;
+  st->rnorm0 = sqrt(s[0]);
+  st->zz = s[0];
+  st->ttol = fmax(rtol * st->rnorm0, atol);
+  st->dtol = dtol;
+  st->its = 0;
+  st->xalpha = 0.;
+  st->maxit = maxit;
+  st->yield = INT_MAX;
+  st->done = 0;
+  st->reason = CG_RUNNING;
+  if (!(st->rnorm0 == st->rnorm0)) {
+    st->done = 1;
+    st->reason = CG_DIVERGED_NAN;
+  } else if (st->rnorm0 <= st->ttol) {
+    st->done = 1;
+    st->reason = st->rnorm0 <= atol ? CG_CONVERGED_ATOL : CG_CONVERGED_RTOL;
+  }
+}
+
+__device__ __forceinline__ double2 ld2(const double* a, int64_t c) { return reinterpret_cast<const double2*>(a)[c]; }
+__device__ __forceinline__ double2 ld2(const float* a, int64_t c) {
+  const float2 q = reinterpret_cast<const float2*>(a)[c];
+  return make_double2(q.x, q.y);
+}
+
+template <typename TZ>
+__global__ void __launch_bounds__(RED_THREADS) mgcg_rz_kernel(MgcgVecs<TZ> v, const CGState* st, double* partial) {
+  if (__syncthreads_or(st->done)) return;
+  double acc[1] = {0.};
+  const int64_t np = v.n / 2, t0 = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x;
+  const int64_t step = (int64_t)gridDim.x * RED_THREADS;
+  for (int64_t c = t0; c < np; c += step) {
+    const double2 r = ld2(v.r, c), z = ld2(v.z, c);
+    acc[0] += r.x * z.x;
+    acc[0] += r.y * z.y;
+  }
+  for (int64_t i = 2 * np + t0; i < v.n; i += step) acc[0] += v.r[i] * (double)v.z[i];
+  block_sum<1>(acc, partial);
+}
+
+// x += alpha p (the iteration before) and p = z + beta p; the first iteration has neither.  The
+// parity of the finished iterations, which only the end of an iteration moves, picks the
+// (r, z) that every block reads and the one that block 0 leaves.
+template <typename TZ>
+__global__ void __launch_bounds__(RED_THREADS) mgcg_p_kernel(MgcgVecs<TZ> v, CGState* st, const double* partial,
+                                                             int nblk) {
+  if (__syncthreads_or(st->done)) return;
+  const int64_t np = v.n / 2, t0 = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x;
+  const int64_t step = (int64_t)gridDim.x * RED_THREADS;
+  const int its = st->its, par = its & 1;
+  double2 p = make_double2(0., 0.), x = p, z = p;
+  auto load = [&](int64_t c) {
+    z = ld2(v.z, c);
+    if (its) {
+      p = ld2(v.p, c);
+      x = ld2(v.x, c);
+    }
+  };
+  if (t0 < np) load(t0);
+  double s[1];
+  final_sum<1>(partial, nblk, s);
+  const double rz = s[0];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->rz[par ^ 1] = rz;
+    if (!(rz > 0.)) {
+      st->reason = rz == 0. ? CG_CONVERGED_ATOL : CG_DIVERGED_INDEFINITE;
+      st->done = 1;
+    }
+  }
+  if (!(rz > 0.)) return;
+  const double b = its ? rz / st->rz[par] : 0., a = st->xalpha;
+  for (int64_t c = t0; c < np;) {
+    double2 q = z;
+    if (its) {
+      x.x += a * p.x;
+      x.y += a * p.y;
+      q.x += b * p.x;
+      q.y += b * p.y;
+      reinterpret_cast<double2*>(v.x)[c] = x;
+    }
+    reinterpret_cast<double2*>(v.p)[c] = q;
+    c += step;
+    if (c < np) load(c);
+  }
+  for (int64_t i = 2 * np + t0; i < v.n; i += step) {
+    const double zi = v.z[i];
+    if (its) v.x[i] += a * v.p[i];
+    v.p[i] = its ? zi + b * v.p[i] : zi;
+  }
+}
+
+template <typename TZ>
+__global__ void __launch_bounds__(RED_THREADS) mgcg_update_kernel(MgcgVecs<TZ> v, CGState* st, double* partial) {
+  if (__syncthreads_or(st->done)) return;
+  const int64_t np = v.n / 2, t0 = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x;
+  const int64_t step = (int64_t)gridDim.x * RED_THREADS;
+  double2 r = make_double2(0., 0.), w = r, d = r;
+  auto load = [&](int64_t c) {
+    r = ld2(v.r, c);
+    w = ld2(v.w, c);
+    d = ld2(v.dinv, c);
+  };
+  if (t0 < np) load(t0);
+  double pws[1];
+  final_sum<1>(v.dotp, v.ndot, pws);
+  const double pw = pws[0];
+  if (!(pw > 0.)) {  // same value in every block; x and r stay as they are
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      st->pw = pw;
+      st->xalpha = 0.;
+      st->done = 1;
+      st->reason = (pw == pw) ? CG_DIVERGED_INDEFINITE : CG_DIVERGED_NAN;
+    }
+    return;
+  }
+  const double alpha = st->rz[(st->its & 1) ^ 1] / pw;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->pw = pw;
+    st->alpha = alpha;
+    st->xalpha = alpha;
+  }
+  double acc[1] = {0.};
+  for (int64_t c = t0; c < np;) {
+    r.x += -alpha * w.x;
+    r.y += -alpha * w.y;
+    const double zx = r.x * d.x, zy = r.y * d.y;
+    acc[0] += zx * zx;
+    acc[0] += zy * zy;
+    reinterpret_cast<double2*>(v.r)[c] = r;
+    if (v.r32) reinterpret_cast<float2*>(v.r32)[c] = make_float2((float)r.x, (float)r.y);
+    c += step;
+    if (c < np) load(c);
+  }
+  for (int64_t i = 2 * np + t0; i < v.n; i += step) {
+    const double ri = v.r[i] - alpha * v.w[i], zi = ri * v.dinv[i];
+    v.r[i] = ri;
+    if (v.r32) v.r32[i] = (float)ri;
+    acc[0] += zi * zi;
+  }
+  block_sum<1>(acc, partial);
+}
+
 // The step of the iteration that stopped the solve (its cg_p_kernel did not run):
 // x += xalpha p; nothing after an indefinite p.w (xalpha = 0) or while the solve is
 // still going (a watchdog stop between iterations: every step has reached x).
@@ -505,18 +632,11 @@ template <typename T> static bool aligned16(const CGVecs<T>& v) {
   return true;
 }
 
-// Blocks of the update and direction kernels: two packets per thread on small systems (fewer
-// partials to sum), one wave of 4 blocks per SM on large ones.
-template <typename T> static int cg_blocks(int64_t n) {
-  const int64_t per = 2 * RED_THREADS * Pack<T>::W;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(RED_BLOCKS, (n + per - 1) / per));
-}
-
 template <typename T>
 cudaError_t cg_iteration(const CGVecs<T>& v, CGState* st, double* partial, int par, cudaStream_t s) {
   if (!aligned16(v)) return cudaErrorMisalignedAddress;  // caught on the host, nothing launched
   if (!v.dotp || v.ndot <= 0) return cudaErrorInvalidValue;
-  const int nb = cg_blocks<T>(v.n);
+  const int nb = cg_blocks(v.n, (int)sizeof(T));
   cg_update_kernel<T><<<nb, RED_THREADS, 0, s>>>(v, st, partial, par);
   cg_p_kernel<T><<<nb, RED_THREADS, 0, s>>>(v, st, partial, nb, par);
   return cudaGetLastError();
@@ -524,7 +644,7 @@ cudaError_t cg_iteration(const CGVecs<T>& v, CGState* st, double* partial, int p
 
 template <typename T>
 cudaError_t cg_finish_x(const CGVecs<T>& v, const CGState* st, cudaStream_t s) {
-  if (!aligned16(v)) return cudaErrorMisalignedAddress;
+  if (reinterpret_cast<uintptr_t>(v.x) % 16 || reinterpret_cast<uintptr_t>(v.p) % 16) return cudaErrorMisalignedAddress;
   cg_finish_x_kernel<T><<<RED_BLOCKS, RED_THREADS, 0, s>>>(v, st);
   return cudaGetLastError();
 }
@@ -533,6 +653,39 @@ template cudaError_t cg_init<double>(const CGVecs<double>&, CGState*, double*, d
                                      double, int, cudaStream_t);
 template cudaError_t cg_init<float>(const CGVecs<float>&, CGState*, double*, double, double,
                                     double, int, cudaStream_t);
+// r.z partials in partial[0, RED_BLOCKS), those of the stopping test in the next RED_BLOCKS
+template <typename TZ>
+cudaError_t mgcg_init(const MgcgVecs<TZ>& v, CGState* st, double* partial, double rtol, double atol, double dtol,
+                      int maxit, cudaStream_t s) {
+  for (const void* q : {(const void*)v.x, (const void*)v.r, (const void*)v.p, (const void*)v.w, (const void*)v.dinv,
+                        (const void*)v.z, (const void*)v.r32})
+    if (reinterpret_cast<uintptr_t>(q) % 16) return cudaErrorMisalignedAddress;
+  if (!v.dotp || v.ndot <= 0) return cudaErrorInvalidValue;
+  mgcg_init_kernel<TZ><<<RED_BLOCKS, RED_THREADS, 0, s>>>(v, partial);
+  mgcg_init_final<<<1, RED_THREADS, 0, s>>>(st, partial, RED_BLOCKS, rtol, atol, dtol, maxit);
+  return cudaGetLastError();
+}
+template <typename TZ>
+cudaError_t mgcg_direction(const MgcgVecs<TZ>& v, CGState* st, double* partial, cudaStream_t s) {
+  const int nb = cg_blocks(v.n, 8);
+  mgcg_rz_kernel<TZ><<<nb, RED_THREADS, 0, s>>>(v, st, partial);
+  mgcg_p_kernel<TZ><<<nb, RED_THREADS, 0, s>>>(v, st, partial, nb);
+  return cudaGetLastError();
+}
+template <typename TZ>
+cudaError_t mgcg_update(const MgcgVecs<TZ>& v, CGState* st, double* partial, cudaStream_t s) {
+  mgcg_update_kernel<TZ><<<cg_blocks(v.n, 8), RED_THREADS, 0, s>>>(v, st, partial + RED_BLOCKS);
+  return cudaGetLastError();
+}
+template cudaError_t mgcg_init<double>(const MgcgVecs<double>&, CGState*, double*, double, double, double, int,
+                                       cudaStream_t);
+template cudaError_t mgcg_init<float>(const MgcgVecs<float>&, CGState*, double*, double, double, double, int,
+                                      cudaStream_t);
+template cudaError_t mgcg_direction<double>(const MgcgVecs<double>&, CGState*, double*, cudaStream_t);
+template cudaError_t mgcg_direction<float>(const MgcgVecs<float>&, CGState*, double*, cudaStream_t);
+template cudaError_t mgcg_update<double>(const MgcgVecs<double>&, CGState*, double*, cudaStream_t);
+template cudaError_t mgcg_update<float>(const MgcgVecs<float>&, CGState*, double*, cudaStream_t);
+
 template cudaError_t cg_iteration<double>(const CGVecs<double>&, CGState*, double*, int, cudaStream_t);
 template cudaError_t cg_iteration<float>(const CGVecs<float>&, CGState*, double*, int, cudaStream_t);
 template cudaError_t cg_finish_x<double>(const CGVecs<double>&, const CGState*, cudaStream_t);

@@ -217,6 +217,11 @@ static cudaGraph_t while_graph(vfgpu_ctx* c, const std::function<cudaError_t(cud
   return graph;
 }
 
+cudaGraphExec_t ctx_while_graph(vfgpu_ctx* c, int kind, int batch,
+                                const std::function<cudaError_t(cudaGraphConditionalHandle)>& body) {
+  return cached_graph(c, kind, batch, [&] { return while_graph(c, body); });
+}
+
 // PCG with device-side convergence.  The iterations run in a conditional while node of a
 // graph, four to a body, so a solve costs one launch and one host read whatever its length,
 // and at most three iterations are queued behind the last one.  (Batches of 4 to 64
@@ -241,11 +246,9 @@ static int run_cg(vfgpu_ctx* c, int kind, const CGVecs<T>& v, Apply apply, doubl
     }
     return eb;
   };
-  cudaGraphExec_t g = !c->use_graphs ? nullptr : cached_graph(c, kind, 0, [&] {
-    return while_graph(c, [&](cudaGraphConditionalHandle h) {
-      const cudaError_t eb = body(kBodyIts);
-      return eb == cudaSuccess ? cg_set_condition(c->d_cg, h, c->stream) : eb;
-    });
+  cudaGraphExec_t g = !c->use_graphs ? nullptr : ctx_while_graph(c, kind, 0, [&](cudaGraphConditionalHandle h) {
+    const cudaError_t eb = body(kBodyIts);
+    return eb == cudaSuccess ? cg_set_condition(c->d_cg, h, c->stream) : eb;
   });
   for (int from = 0; e == cudaSuccess; from = c->h_cg->its) {
     if (g) {
@@ -287,11 +290,12 @@ static cudaError_t u_apply32(vfgpu_ctx* c, const float* x, float* y, const int* 
   A.dot = dot;
   return launch_u_apply<float>(A, c->plan32, c->layers, c->stream);
 }
-static int dots_of(const vfgpu_ctx* c, const TilePlan& p) { return tile_dot_count(p, c->nx, c->ny, c->nz); }
 // The U applies with unit lists or the stencil write a second wave's partials.
-static int u_dots_of(const vfgpu_ctx* c, const TilePlan& p, int prec_bytes) {
+int u_dot_count(const vfgpu_ctx* c, int prec_bytes) {
+  const TilePlan& p = prec_bytes == 8 ? c->plan64 : c->plan32;
   if (u_twophase_on(c, prec_bytes)) return twophase_dots(c->nx, c->ny, c->nz);
-  return dots_of(c, p) + (u_stencil_on(c, prec_bytes) ? p.st.blocks() + p.st.nface : u_lists_on(c, prec_bytes) ? p.ncta0 : 0);
+  return tile_dot_count(p, c->nx, c->ny, c->nz) + (u_stencil_on(c, prec_bytes) ? p.st.blocks() + p.st.nface
+                                                   : u_lists_on(c, prec_bytes) ? p.ncta0 : 0);
 }
 
 // F = K(V) U - f, Dirichlet rows U - ubc (VF_UResidual, VFMech.c:1456-1887).
@@ -397,7 +401,7 @@ int vfgpu_step_u(vfgpu_ctx* c, const vfgpu_solve_opts* o_, vfgpu_solve_stats* st
       S.ksp_its += kits;
       tmo = w.expired();
     } else if (!mixed) {
-      CGVecs<double> v{Y, R, P, W, dinv, F, nullptr, n3, c->d_dot, u_dots_of(c, c->plan64, 8)};
+      CGVecs<double> v{Y, R, P, W, dinv, F, nullptr, n3, c->d_dot, u_dot_count(c, 8)};
       rc = run_cg<double>(c, 1, v, apply64, o.ksp_rtol, o.ksp_atol, o.ksp_dtol, o.ksp_maxit, w, &kits,
                           &kreason, &tmo);
       if (rc) return rc;
@@ -417,7 +421,7 @@ int vfgpu_step_u(vfgpu_ctx* c, const vfgpu_solve_opts* o_, vfgpu_solve_stats* st
         float* b32 = reinterpret_cast<float*>(P);  // FP32 right-hand side staged in P
         e = dev_to_f32(R, b32, n3, c->stream);
         if (e != cudaSuccess) return cuda_fail(e, "vfgpu_step_u");
-        CGVecs<float> v{x32, r32, pp32, w32, c->p32[4], b32, nullptr, n3, c->d_dot, u_dots_of(c, c->plan32, 4)};
+        CGVecs<float> v{x32, r32, pp32, w32, c->p32[4], b32, nullptr, n3, c->d_dot, u_dot_count(c, 4)};
         const double in_rtol = std::max(o.inner_rtol, 0.5 * target / zr);
         int its32 = 0, r32reason = 0;
         rc = run_cg<float>(c, 2, v, apply32, in_rtol, 0.0, o.ksp_dtol, o.ksp_maxit, w, &its32,
