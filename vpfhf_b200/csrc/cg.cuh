@@ -106,22 +106,25 @@ cudaError_t cg_iteration(const CGVecs<T>& v, CGState* st, double* partial, int p
 template <typename T>
 cudaError_t cg_finish_x(const CGVecs<T>& v, const CGState* st, cudaStream_t s);
 // The PCG around a multigrid preconditioner (FP64 vectors; z = M^-1 r in TZ = double or
-// float, which the V-cycle leaves in its own vector).  One iteration is: the V-cycle;
-// mgcg_direction (block partials of r.z, then beta, x += alpha p of the iteration before and
+// float, the V-cycle's own vector).  One iteration is: the V-cycle without its first and last
+// smoothing steps on the fine level; mgcg_direction (the last step z += zdinv (r - t) / theta
+// with the block partials of r.z; then beta, x += alpha p of the iteration before and
 // p = z + beta p); the operator apply w = A p with the partials of p.w; mgcg_update
-// (r -= alpha w, the V-cycle's FP32 copy of r, block partials of (D^-1 r).(D^-1 r), the Jacobi
-// solve's stopping test); and the end of the iteration from those partials, which also sets
+// (r -= alpha w, the V-cycle's FP32 copy of r and its first step z = zdinv r / theta, block
+// partials of (D^-1 r).(D^-1 r), the Jacobi solve's stopping test); and the end of the iteration from those partials, which also sets
 // the while node's condition (mgcg_end in cg_loop.cu; loop null: no condition).  So the test
-// comes before the next V-cycle, and the iteration's vector traffic is r, w, dinv, the copy;
-// r, z; z, p, x.  cg_finish_x adds the last step to x.
+// comes before the next V-cycle, and no vector is passed over for a dot alone.  cg_finish_x
+// adds the last step to x.
 template <typename TZ> struct MgcgVecs {
   double *x, *r, *p, *w;
   const double *dinv, *b;
-  const TZ* z;
+  TZ* z;
   float* r32;  // the V-cycle's right-hand side (FP32), or null: it reads r
   int64_t n;
   const double* dotp;
   int ndot;
+  const TZ *t, *zdinv;  // fine level: K z, the smoother's inverse diagonal and coefficients
+  const double* zcoef;  // (zcoef[1] = 1 / theta)
 };
 template <typename TZ>
 cudaError_t mgcg_init(const MgcgVecs<TZ>& v, CGState* st, double* partial, double rtol, double atol, double dtol,

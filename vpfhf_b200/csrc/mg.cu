@@ -13,7 +13,7 @@
 // and, for a per-cell modulus, the mean of the fine cells whose centres it holds
 // (nested: the 8 children).  Transfers: trilinear prolongation and its exact
 // transpose, Dirichlet dofs excluded on both sides.  Smoother: Chebyshev
-// iteration of D^-1 K (degree kSmoothDeg) on [lmax/10, lmax] (lmax = 1.1 x the
+// iteration of D^-1 K (degree 1: a weighted Jacobi step) on [lmax/10, lmax] (lmax = 1.1 x the
 // estimate of 12 power iterations per level, 4 from the previous vector once there is
 // one), pre and post; the coarsest level runs degree kCoarseDeg on [lmax/100, lmax].  Every step is a fixed sequence of
 // deterministic kernels reading its Chebyshev coefficients from device memory, so
@@ -21,13 +21,16 @@
 // body of a graph's while node: cycle, vector kernels (cg.cuh) and stopping test without the
 // host.  A host-driven iteration cost two round trips, a copy of r and z each way in mixed
 // precision and, at the last one, a cycle that nothing used: AM step at 129^3 mixed 19.3 ->
-// 18.0 ms, 65^3 FP64 26.1 -> 22.1 ms, 257 x 257 x 129 per-cell modulus 101.6 -> 85.8 ms.
+// 18.0 ms, 65^3 FP64 26.1 -> 22.1 ms, 257 x 257 x 129 per-cell modulus 101.6 -> 85.8 ms.  The
+// smoothing steps inside the passes that make or read their vectors, and the transfers below:
+// 18.0 -> 17.6, 22.1 -> 20.5, 85.8 -> 85.1 ms.
 //
 // Precision: the V-cycle runs in FP64 (solve precision FP64) or FP32 (MIXED); the
 // outer CG, its residual and its stopping test stay FP64 in both.
 #include <algorithm>
 #include <cmath>
 #include <functional>
+#include <type_traits>
 #include <vector>
 
 #include "abi_util.h"
@@ -47,7 +50,7 @@ namespace {
 // with 20 iterations against 0.181 s / 15 for degree 2 and 0.209 s / 13 for degree 3).
 // 2 warm power iterations instead of 4 cost one more CG iteration per StepU in the
 // 129^3 AM loop (4 AM steps: 87.3 against 85.9 ms mixed).
-constexpr int kSmoothDeg = 1, kCoarseDeg = 15, kPowerIts = 12, kWarmPowerIts = 4;
+constexpr int kCoarseDeg = 15, kPowerIts = 12, kWarmPowerIts = 4;
 constexpr double kSmoothLo = 0.1, kCoarseLo = 0.01, kLmaxSafety = 1.1;
 constexpr int kCoefPerLevel = 64;  // [0] lmax [1] 1/theta [2..59] (c1, c2) [62..63] scratch
 constexpr int kPowBlocks = 296, kPowThreads = 256;
@@ -98,19 +101,25 @@ struct Xfer {
   XferAxis a[3];
 };
 
+// The type of the weights: double, or where no axis has a table (TABLE = false) the level's own
+// (1, 1/2 and their products are exact).
+template <typename T, bool TABLE> using XferWeight = std::conditional_t<TABLE, double, T>;
 // Weight of coarse node I at fine node i of its support (the prolongation's entry).
-__device__ __forceinline__ double hat(const XferAxis& A, int i, int I) {
-  if (A.mode == kXferNested) return i == 2 * I ? 1.0 : 0.5;
-  if (A.mode == kXferIdentity) return 1.0;
-  const double w = A.pw[i];
-  return A.pI[i] == I ? 1.0 - w : w;
+template <bool TABLE, typename W> __device__ __forceinline__ W hat(const XferAxis& A, int i, int I) {
+  if (A.mode == kXferNested) return i == 2 * I ? W(1) : W(0.5);
+  if (A.mode == kXferIdentity) return W(1);
+  if constexpr (TABLE) {
+    const W w = A.pw[i];
+    return A.pI[i] == I ? W(1) - w : w;
+  }
+  return W(0);  // not reached
 }
 // The support [lo, lo + n) of coarse node I.
-__device__ __forceinline__ void support_of(const XferAxis& A, int I, int& lo, int& n) {
+template <bool TABLE> __device__ __forceinline__ void support_of(const XferAxis& A, int I, int& lo, int& n) {
   if (A.mode == kXferNested) {
     lo = max(2 * I - 1, 0);
     n = min(2 * I + 1, A.nf - 1) - lo + 1;
-  } else if (A.mode == kXferIdentity) {
+  } else if (!TABLE || A.mode == kXferIdentity) {
     lo = I;
     n = 1;
   } else {
@@ -119,99 +128,180 @@ __device__ __forceinline__ void support_of(const XferAxis& A, int I, int& lo, in
   }
 }
 // The coarse cell of fine node i and its upper weight.
-__device__ __forceinline__ void cell_of(const XferAxis& A, int i, int& I, double& whi) {
+template <bool TABLE, typename W> __device__ __forceinline__ void cell_of(const XferAxis& A, int i, int& I, W& whi) {
   if (A.mode == kXferNested) {
     I = i >> 1;
-    whi = (i & 1) ? 0.5 : 0.0;
-  } else if (A.mode == kXferIdentity) {
+    whi = (i & 1) ? W(0.5) : W(0);
+  } else if (!TABLE || A.mode == kXferIdentity) {
     I = i;
-    whi = 0.0;
+    whi = W(0);
   } else {
     I = A.pI[i];
-    whi = A.pw[i];
+    whi = W(A.pw[i]);
   }
 }
 
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// Both transfers run the written level's planes along the grid's y and the nodes of a plane in
+// memory order (32-bit index arithmetic), Q = 3 components to a thread where that fills the
+// chip, else one: the coarse levels are latencies, and get three times the warps.
+constexpr int64_t kXferWide = 148 * 512;
+inline dim3 transfer_grid(int nx, int ny, int nz, int q) {
+  const int64_t b = ((int64_t)(3 / q) * nx * ny + 255) / 256;
+  return dim3((unsigned)b, (unsigned)std::min(nz, 65535));
+}
+inline bool transfer_wide(int nx, int ny, int nz) { return (int64_t)nx * ny * nz >= kXferWide; }
+inline bool has_table(const Xfer& X) {
+  return X.a[0].mode == kXferTable || X.a[1].mode == kXferTable || X.a[2].mode == kXferTable;
+}
+
 // Restriction of the residual b - t (the transpose of prolong_add_kernel): coarse node I
-// gathers the fine nodes of its hat function's support with the same weights, skipping
-// fine Dirichlet dofs; coarse Dirichlet dofs are zeroed.
+// gathers the fine nodes of its hat function's support with the same weights, leaving out
+// fine Dirichlet dofs; coarse Dirichlet dofs are zeroed.  With zc also the coarse level's
+// pre-smoothing step from 0, zc = dinv_c rc / theta_c.  Supports of up to 3 nodes per axis where
+// no axis needs a table, else 4.  Every point of the support is loaded, clamped and Dirichlet
+// ones too, and then left out: nothing waits for a mask before it loads.  Measured per launch,
+// before (one thread per node, masked loads, double weights, 64-bit divisions) and now: onto
+// 17^3 FP32 11.2 -> 4.0 us, FP64 12.7 -> 6.4, onto 33^3 FP64 14.8 -> 13.6, from 257 x 257 x 129
+// FP32 101 -> 92 us; the prolongation 4.2 -> 2.7, 129^3 FP32 28.6 -> 20.8, 257 x 257 x 129 106 ->
+// 76 us.  One component per thread throughout: 165 and 252 us at the largest.
+template <typename T, bool TABLE, int Q>
+__global__ void __launch_bounds__(256)
+    restrict_kernel(const T* __restrict__ bf, const T* __restrict__ tf, const uint8_t* __restrict__ bc_f, int fx,
+                    int fy, const Xfer X, T* __restrict__ rc, int cx, int cy, int cz,
+                    const uint8_t* __restrict__ bc_c, T* __restrict__ zc, const T* __restrict__ dinv_c,
+                    const double* __restrict__ coef_c) {
+  using W = XferWeight<T, TABLE>;
+  constexpr int S = TABLE ? 4 : 3, Z = Q == 3 || TABLE || sizeof(T) == 8 ? 1 : S;  // planes loaded at once
+  const unsigned q = blockIdx.x * 256u + threadIdx.x, m = Q == 3 ? q : q / 3u;
+  const int c0 = Q == 3 ? 0 : (int)(q - 3u * m);
+  if (m >= (unsigned)cx * (unsigned)cy) return;
+  const int J = (int)(m / (unsigned)cx), I = (int)(m - (unsigned)J * (unsigned)cx);
+  int x0, nxs, y0, nys;
+  support_of<TABLE>(X.a[0], I, x0, nxs);
+  support_of<TABLE>(X.a[1], J, y0, nys);
+  W wx[S], wy[S];
+#pragma unroll
+  for (int s = 0; s < S; s++) {
+    wx[s] = s < nxs ? hat<TABLE, W>(X.a[0], x0 + s, I) : W(0);
+    wy[s] = s < nys ? hat<TABLE, W>(X.a[1], y0 + s, J) : W(0);
+  }
+  for (int K = blockIdx.y; K < cz; K += gridDim.y) {
+    int z0, nzs;
+    support_of<TABLE>(X.a[2], K, z0, nzs);
+    W wz[S];
+#pragma unroll
+    for (int s = 0; s < S; s++) wz[s] = s < nzs ? hat<TABLE, W>(X.a[2], z0 + s, K) : W(0);
+    T acc[Q];
+#pragma unroll
+    for (int c = 0; c < Q; c++) acc[c] = T(0);
+    T res[Z * S * S][Q];
+    unsigned bits[Z * S * S];
+#pragma unroll
+    for (int z = 0; z < S; z += Z) {
+#pragma unroll
+      for (int s = 0; s < Z * S * S; s++) {
+        const int c1 = s % S, c2 = s / S % S, c3 = z + s / (S * S);
+        const int64_t n = node_index(x0 + min(c1, nxs - 1), y0 + min(c2, nys - 1), z0 + min(c3, nzs - 1), fx, fy);
+        bits[s] = (unsigned)bc_f[n] >> c0;
+#pragma unroll
+        for (int c = 0; c < Q; c++) res[s][c] = bf[3 * n + c0 + c] - tf[3 * n + c0 + c];
+      }
+#pragma unroll
+      for (int s = 0; s < Z * S * S; s++) {
+        const int c1 = s % S, c2 = s / S % S, c3 = z + s / (S * S);
+        const T w = T(wz[c3] * wy[c2] * wx[c1]);
+        const bool in = c1 < nxs && c2 < nys && c3 < nzs;
+#pragma unroll
+        for (int c = 0; c < Q; c++) {
+          const T next = acc[c] + w * res[s][c];
+          acc[c] = in && !((bits[s] >> c) & 1u) ? next : acc[c];
+        }
+      }
+    }
+    const int64_t o = (int64_t)K * cx * cy + m;
+    const unsigned fixed = (unsigned)bc_c[o] >> c0;
+#pragma unroll
+    for (int c = 0; c < Q; c++) {
+      const int64_t i = 3 * o + c0 + c;
+      const T r = (fixed >> c) & 1u ? T(0) : acc[c];
+      rc[i] = r;
+      if (zc) zc[i] = mul_rn(dinv_c[i] * r, T(coef_c[1]));
+    }
+  }
+}
 template <typename T>
-__global__ void restrict_kernel(const T* __restrict__ bf, const T* __restrict__ tf,
-                                const uint8_t* __restrict__ bc_f, int fx, int fy, const Xfer X,
-                                T* __restrict__ rc, int cx, int cy, int cz,
-                                const uint8_t* __restrict__ bc_c) {
-  const int64_t Nc = (int64_t)cx * cy * cz;
-  GRID_STRIDE(q, Nc) {
-    const int I = (int)(q % cx), J = (int)((q / cx) % cy), K = (int)(q / ((int64_t)cx * cy));
-    int x0, nxs, y0, nys, z0, nzs;
-    support_of(X.a[0], I, x0, nxs);
-    support_of(X.a[1], J, y0, nys);
-    support_of(X.a[2], K, z0, nzs);
-    double wx[4];
+cudaError_t launch_restrict(const T* bf, const T* tf, const uint8_t* bc_f, int fx, int fy, const Xfer& X, T* rc,
+                            int cx, int cy, int cz, const uint8_t* bc_c, T* zc, const T* dinv_c,
+                            const double* coef_c, cudaStream_t s) {
+  const bool wide = transfer_wide(cx, cy, cz), table = has_table(X);
+  const auto kernel = wide ? (table ? restrict_kernel<T, true, 3> : restrict_kernel<T, false, 3>)
+                           : (table ? restrict_kernel<T, true, 1> : restrict_kernel<T, false, 1>);
+  kernel<<<transfer_grid(cx, cy, cz, wide ? 3 : 1), 256, 0, s>>>(bf, tf, bc_f, fx, fy, X, rc, cx, cy, cz, bc_c, zc,
+                                                                 dinv_c, coef_c);
+  return cudaGetLastError();
+}
+
+// x_f += trilinear interpolation of e_c; fine Dirichlet dofs untouched.
+template <typename T, bool TABLE, int Q>
+__global__ void __launch_bounds__(256)
+    prolong_add_kernel(const T* __restrict__ ec, int cx, int cy, const Xfer X, T* __restrict__ xf, int fx, int fy,
+                       int fz, const uint8_t* __restrict__ bc_f) {
+  using W = XferWeight<T, TABLE>;
+  const unsigned q = blockIdx.x * 256u + threadIdx.x, m = Q == 3 ? q : q / 3u;
+  const int c0 = Q == 3 ? 0 : (int)(q - 3u * m);
+  if (m >= (unsigned)fx * (unsigned)fy) return;
+  const int j = (int)(m / (unsigned)fx), i = (int)(m - (unsigned)j * (unsigned)fx);
+  int Ix, Iy;
+  W hx, hy;
+  cell_of<TABLE, W>(X.a[0], i, Ix, hx);
+  cell_of<TABLE, W>(X.a[1], j, Iy, hy);
+  for (int k = blockIdx.y; k < fz; k += gridDim.y) {
+    int Iz;
+    W hz;
+    cell_of<TABLE, W>(X.a[2], k, Iz, hz);
+    const int64_t o = (int64_t)k * fx * fy + m;
+    const unsigned bits = (unsigned)bc_f[o] >> c0;
+    const T* e = ec + 3 * node_index(Ix, Iy, Iz, cx, cy) + c0;
+    T x[Q], acc[Q];
 #pragma unroll
-    for (int c1 = 0; c1 < 4; c1++) wx[c1] = c1 < nxs ? hat(X.a[0], x0 + c1, I) : 0.0;
-    T acc[3] = {T(0), T(0), T(0)};
-    // fully unrolled (predicated) so that the row loads of the support issue together
+    for (int c = 0; c < Q; c++) {
+      x[c] = xf[3 * o + c0 + c];
+      acc[c] = T(0);
+    }
 #pragma unroll
-    for (int c3 = 0; c3 < 4; c3++) {
-      if (c3 >= nzs) continue;
-      const double wz = hat(X.a[2], z0 + c3, K);
+    for (int dk = 0; dk < 2; dk++) {
+      const W wzk = dk ? hz : W(1) - hz;
 #pragma unroll
-      for (int c2 = 0; c2 < 4; c2++) {
-        if (c2 >= nys) continue;
-        const double wzy = wz * hat(X.a[1], y0 + c2, J);
-        const int64_t row = node_index(x0, y0 + c2, z0 + c3, fx, fy);
+      for (int dj = 0; dj < 2; dj++) {
+        const W wyj = dj ? hy : W(1) - hy;
 #pragma unroll
-        for (int c1 = 0; c1 < 4; c1++) {
-          if (c1 < nxs) {
-            const T w = T(wzy * wx[c1]);
-            const int64_t n = row + c1;
-            const unsigned bf_bits = bc_f[n];
+        for (int di = 0; di < 2; di++) {
+          const W wxi = di ? hx : W(1) - hx;
+          if (wzk != W(0) && wyj != W(0) && wxi != W(0)) {
+            const T w = T(wzk * wyj * wxi);
+            const int64_t a = 3 * ((int64_t)(dk * cy + dj) * cx + di);
 #pragma unroll
-            for (int c = 0; c < 3; c++)
-              if (!((bf_bits >> c) & 1u)) acc[c] += w * (bf[3 * n + c] - tf[3 * n + c]);
+            for (int c = 0; c < Q; c++) acc[c] += w * e[a + c];
           }
         }
       }
     }
-    const unsigned b = bc_c[q];
-    for (int c = 0; c < 3; c++) rc[3 * q + c] = ((b >> c) & 1u) ? T(0) : acc[c];
+#pragma unroll
+    for (int c = 0; c < Q; c++)
+      if (!((bits >> c) & 1u)) xf[3 * o + c0 + c] = x[c] + acc[c];
   }
 }
-
-// x_f += trilinear interpolation of e_c; fine Dirichlet dofs untouched.
 template <typename T>
-__global__ void prolong_add_kernel(const T* __restrict__ ec, int cx, int cy, const Xfer X,
-                                   T* __restrict__ xf, int fx, int fy, int fz,
-                                   const uint8_t* __restrict__ bc_f) {
-  const int64_t Nf = (int64_t)fx * fy * fz;
-  GRID_STRIDE(q, Nf) {
-    const int i = (int)(q % fx), j = (int)((q / fx) % fy), k = (int)(q / ((int64_t)fx * fy));
-    int Ix, Iy, Iz;
-    double hx, hy, hz;
-    cell_of(X.a[0], i, Ix, hx);
-    cell_of(X.a[1], j, Iy, hy);
-    cell_of(X.a[2], k, Iz, hz);
-    T acc[3] = {T(0), T(0), T(0)};
-    for (int dk = 0; dk < 2; dk++) {
-      const double wzk = dk ? hz : 1.0 - hz;
-      if (wzk == 0.0) continue;
-      for (int dj = 0; dj < 2; dj++) {
-        const double wyj = dj ? hy : 1.0 - hy;
-        if (wyj == 0.0) continue;
-        for (int di = 0; di < 2; di++) {
-          const double wxi = di ? hx : 1.0 - hx;
-          if (wxi == 0.0) continue;
-          const T w = T(wzk * wyj * wxi);
-          const int64_t n = node_index(Ix + di, Iy + dj, Iz + dk, cx, cy);
-          for (int c = 0; c < 3; c++) acc[c] += w * ec[3 * n + c];
-        }
-      }
-    }
-    const unsigned b = bc_f[q];
-    for (int c = 0; c < 3; c++)
-      if (!((b >> c) & 1u)) xf[3 * q + c] += acc[c];
-  }
+cudaError_t launch_prolong(const T* ec, int cx, int cy, const Xfer& X, T* xf, int fx, int fy, int fz,
+                           const uint8_t* bc_f, cudaStream_t s) {
+  const bool wide = transfer_wide(fx, fy, fz), table = has_table(X);
+  const auto kernel = wide ? (table ? prolong_add_kernel<T, true, 3> : prolong_add_kernel<T, false, 3>)
+                           : (table ? prolong_add_kernel<T, true, 1> : prolong_add_kernel<T, false, 1>);
+  kernel<<<transfer_grid(fx, fy, fz, wide ? 3 : 1), 256, 0, s>>>(ec, cx, cy, X, xf, fx, fy, fz, bc_f);
+  return cudaGetLastError();
 }
 
 // Coarse node I takes v interpolated at its position (in the nested case: fine node 2I)
@@ -278,14 +368,13 @@ __global__ void cell_mean_kernel(const float* __restrict__ ef, int fcx, int fcy,
   }
 }
 
-// r = dinv * (b - t), or dinv * b when t is null (x = 0); d = r / theta.
+// r = dinv * b (x = 0); d = r / theta.
 template <typename T>
-__global__ void cheb_init_kernel(const T* __restrict__ b, const T* __restrict__ t,
-                                 const T* __restrict__ dinv, T* __restrict__ r, T* __restrict__ d,
-                                 const double* __restrict__ coef, int64_t n) {
+__global__ void cheb_init_kernel(const T* __restrict__ b, const T* __restrict__ dinv, T* __restrict__ r,
+                                 T* __restrict__ d, const double* __restrict__ coef, int64_t n) {
   const T inv_theta = T(coef[1]);
   GRID_STRIDE(i, n) {
-    const T ri = dinv[i] * (t ? b[i] - t[i] : b[i]);
+    const T ri = dinv[i] * b[i];
     r[i] = ri;
     d[i] = ri * inv_theta;
   }
@@ -308,25 +397,19 @@ __global__ void cheb_step_kernel(T* __restrict__ x, T* __restrict__ d, T* __rest
   }
 }
 
-// Degree 1 (a Jacobi step weighted 1/theta) in one pass: x += dinv (b - t) / theta, or
-// x = dinv b / theta from x = 0 (t null) -- cheb_init_kernel and the last
-// cheb_step_kernel's arithmetic (the product rounded before the add, as there) without
-// the r and d vectors.
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+// Post-smoothing of degree 1 in one pass: x += dinv (b - t) / theta (the product rounded before
+// the add).  Pre-smoothing from x = 0, x = dinv b / theta, is part of the kernel that writes b
+// (restrict_kernel, and the outer PCG on the fine level), as the fine level's post-smoothing
+// is of the PCG's pass over (r, z).
 template <typename T>
-__global__ void jacobi1_kernel(const T* __restrict__ b, const T* __restrict__ t,
-                               const T* __restrict__ dinv, T* __restrict__ x,
-                               const double* __restrict__ coef, int64_t n) {
+__global__ void jacobi1_kernel(const T* __restrict__ b, const T* __restrict__ t, const T* __restrict__ dinv,
+                               T* __restrict__ x, const double* __restrict__ coef, int64_t n) {
   const T inv_theta = T(coef[1]);
-  GRID_STRIDE(i, n) {
-    const T di = mul_rn(dinv[i] * (t ? b[i] - t[i] : b[i]), inv_theta);
-    x[i] = t ? x[i] + di : di;
-  }
+  GRID_STRIDE(i, n) x[i] = x[i] + mul_rn(dinv[i] * (b[i] - t[i]), inv_theta);
 }
 
 // The coarsest level's Chebyshev solve from x = 0 in one CTA (the level has <= 8 nodes
-// per axis): the same iteration as chebyshev() with zero_start, its operator applied as
+// per axis): the same iteration as chebyshev(), its operator applied as
 // one element per thread into shared memory (ncell x 8 x 3 values) and gathered per node
 // in a fixed order, so the result is deterministic.  Replaces 2 deg launches.
 constexpr int kCoarseThreads = 256, kCoarseMaxNodes = 8 * 8 * 8;
@@ -680,28 +763,15 @@ cudaError_t level_apply(vfgpu_ctx* c, const LevelT<T>& V, const T* x, T* y) {
   return launch_u_apply<T>(level_args<T>(c, V, x, y), *V.plan, c->layers, c->stream);
 }
 
-// Chebyshev iteration on D^-1 K x = D^-1 b with the level's coefficients; x updated in
-// place (zero_start: x = 0 on entry and no initial residual apply).  (Carrying the
-// update in the operator's epilogue instead of a separate pass measured slower on B200:
-// StepU 257^3 0.250 s against 0.225 s mixed, 0.378 s against 0.328 s FP64 -- the extra
+// Chebyshev iteration on D^-1 K x = D^-1 b from x = 0 with the level's coefficients.
+// (Carrying the update in the operator's epilogue instead of a separate pass measured slower on
+// B200: StepU 257^3 0.250 s against 0.225 s mixed, 0.378 s against 0.328 s FP64 -- the extra
 // loads stall the compute-bound z-march.)
-template <typename T>
-cudaError_t chebyshev(vfgpu_ctx* c, const LevelT<T>& V, const T* b, T* x, int deg, bool zero_start) {
+template <typename T> cudaError_t chebyshev(vfgpu_ctx* c, const LevelT<T>& V, const T* b, T* x, int deg) {
   const int64_t n3 = V.n3;
-  if (deg == 1) {
-    cudaError_t e = zero_start ? cudaSuccess : level_apply<T>(c, V, x, V.t);
-    if (e == cudaSuccess) {
-      jacobi1_kernel<T><<<blocks_for(n3), 256, 0, c->stream>>>(b, zero_start ? nullptr : V.t, V.dinv,
-                                                              x, V.coef, n3);
-      e = cudaGetLastError();
-    }
-    return e;
-  }
-  cudaError_t e =
-      zero_start ? cudaMemsetAsync(x, 0, n3 * sizeof(T), c->stream) : level_apply<T>(c, V, x, V.t);
+  cudaError_t e = cudaMemsetAsync(x, 0, n3 * sizeof(T), c->stream);
   if (e == cudaSuccess) {
-    cheb_init_kernel<T><<<blocks_for(n3), 256, 0, c->stream>>>(b, zero_start ? nullptr : V.t, V.dinv,
-                                                              V.r, V.d, V.coef, n3);
+    cheb_init_kernel<T><<<blocks_for(n3), 256, 0, c->stream>>>(b, V.dinv, V.r, V.d, V.coef, n3);
     e = cudaGetLastError();
   }
   for (int k = 0; k < deg && e == cudaSuccess; k++) {
@@ -718,7 +788,7 @@ cudaError_t chebyshev(vfgpu_ctx* c, const LevelT<T>& V, const T* b, T* x, int de
 
 // The coarsest level's solve: kCoarseDeg Chebyshev steps from x = 0, in one CTA.
 template <typename T> cudaError_t coarse_solve(vfgpu_ctx* c, const LevelT<T>& V, const T* b, T* x) {
-  if (V.n3 / 3 > kCoarseMaxNodes || V.cflag) return chebyshev<T>(c, V, b, x, kCoarseDeg, true);
+  if (V.n3 / 3 > kCoarseMaxNodes || V.cflag) return chebyshev<T>(c, V, b, x, kCoarseDeg);
   const UApplyArgs<T> A = level_args<T>(c, V, V.d, V.t);
   const int ncell = (V.nx - 1) * (V.ny - 1) * (V.nz - 1);
   if (A.ihx == A.ihy && A.ihy == A.ihz)
@@ -743,25 +813,25 @@ template <typename T> cudaError_t coarse_attributes() {
   return e;
 }
 
-// z = V-cycle(b) from level l down.
+// z = V-cycle(b) from level l down; above the coarsest level z = dinv b / theta on entry, and at
+// level 0 the last step, z += dinv (b - t) / theta with t = K z, is left to the caller.
 template <typename T> cudaError_t vcycle(vfgpu_ctx* c, int l, const T* b, T* z) {
   const LevelT<T> V = view<T>(c, l);
-  if (l == (int)c->mg.size() - 1) return coarse_solve<T>(c, V, b, z);
+  const int levels = (int)c->mg.size();
+  if (l == levels - 1) return coarse_solve<T>(c, V, b, z);
   const LevelT<T> C = view<T>(c, l + 1);
-  cudaError_t e = chebyshev<T>(c, V, b, z, kSmoothDeg, true);
-  if (e == cudaSuccess) e = level_apply<T>(c, V, z, V.t);
-  if (e == cudaSuccess) {
-    restrict_kernel<T><<<blocks_for(C.n3 / 3), 256, 0, c->stream>>>(
-        b, V.t, V.bc, V.nx, V.ny, xfer_of(c, l + 1), C.b, C.nx, C.ny, C.nz, C.bc);
-    e = cudaGetLastError();
-  }
+  cudaError_t e = level_apply<T>(c, V, z, V.t);
+  if (e == cudaSuccess)
+    e = launch_restrict<T>(b, V.t, V.bc, V.nx, V.ny, xfer_of(c, l + 1), C.b, C.nx, C.ny, C.nz, C.bc,
+                           l + 2 < levels ? C.x : nullptr, C.dinv, C.coef, c->stream);
   if (e == cudaSuccess) e = vcycle<T>(c, l + 1, C.b, C.x);
-  if (e == cudaSuccess) {
-    prolong_add_kernel<T><<<blocks_for(V.n3 / 3), 256, 0, c->stream>>>(
-        C.x, C.nx, C.ny, xfer_of(c, l + 1), z, V.nx, V.ny, V.nz, V.bc);
+  if (e == cudaSuccess)
+    e = launch_prolong<T>(C.x, C.nx, C.ny, xfer_of(c, l + 1), z, V.nx, V.ny, V.nz, V.bc, c->stream);
+  if (e == cudaSuccess) e = level_apply<T>(c, V, z, V.t);
+  if (e == cudaSuccess && l > 0) {
+    jacobi1_kernel<T><<<blocks_for(V.n3), 256, 0, c->stream>>>(b, V.t, V.dinv, z, V.coef, V.n3);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = chebyshev<T>(c, V, b, z, kSmoothDeg, false);
   return e;
 }
 
@@ -946,7 +1016,7 @@ template <typename T> int mg_setup(vfgpu_ctx* c) {
     }
     if (e == cudaSuccess) {
       const bool last = l == nlev - 1;
-      cheb_coef_kernel<<<1, 32, 0, c->stream>>>(V.coef, last ? kCoarseDeg : kSmoothDeg,
+      cheb_coef_kernel<<<1, 32, 0, c->stream>>>(V.coef, last ? kCoarseDeg : 1,
                                                 last ? kCoarseLo : kSmoothLo, kLmaxSafety);
       e = cudaGetLastError();
     }
@@ -980,7 +1050,8 @@ int mgcg(vfgpu_ctx* c, const double* b, double* x, double* r, double* p, double*
   const int64_t n3 = 3 * c->N;
   const LevelT<T> V = view<T>(c, 0);
   constexpr bool f32 = sizeof(T) == 4;
-  MgcgVecs<T> m{x, r, p, w, dinv0, b, V.x, f32 ? (float*)V.b : nullptr, n3, c->d_dot, u_dot_count(c, 8)};
+  MgcgVecs<T> m{x, r, p, w, dinv0, b, V.x, f32 ? (float*)V.b : nullptr, n3, c->d_dot, u_dot_count(c, 8),
+                V.t, V.dinv, V.coef};
   LevelT<double> outer{};  // the FP64 Jacobian whatever the V-cycle's precision
   outer.nx = c->nx;
   outer.ny = c->ny;

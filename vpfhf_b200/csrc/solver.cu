@@ -270,14 +270,31 @@ __global__ void __launch_bounds__(RED_THREADS) cg_p_kernel(CGVecs<T> v, CGState*
 }
 
 // ---- PCG around the multigrid V-cycle (cg.cuh)
+// The V-cycle's first smoothing step from z = 0 (the product rounded).
+__device__ __forceinline__ double presmooth(double dinv, double r, double inv_theta) {
+  return __dmul_rn(dinv * r, inv_theta);
+}
+__device__ __forceinline__ float presmooth(float dinv, double r, float inv_theta) {
+  return __fmul_rn(dinv * (float)r, inv_theta);
+}
+// Its last one, z + dinv (r - t) / theta.
+__device__ __forceinline__ double postsmooth(double z, double dinv, double r, double t, double inv_theta) {
+  return z + __dmul_rn(dinv * (r - t), inv_theta);
+}
+__device__ __forceinline__ float postsmooth(float z, float dinv, double r, float t, float inv_theta) {
+  return z + __fmul_rn(dinv * ((float)r - t), inv_theta);
+}
+
 template <typename TZ>
 __global__ void __launch_bounds__(RED_THREADS) mgcg_init_kernel(MgcgVecs<TZ> v, double* partial) {
+  const TZ th = TZ(v.zcoef[1]);
   double acc[1] = {0.};
   GRID_LOOP(i, v.n) {
     const double r = v.b[i], z = r * v.dinv[i];
     v.x[i] = 0.;
     v.r[i] = r;
     if (v.r32) v.r32[i] = (float)r;
+    v.z[i] = presmooth(v.zdinv[i], r, th);
     acc[0] += z * z;
   }
   block_sum<1>(acc, partial);
@@ -307,24 +324,45 @@ __global__ void __launch_bounds__(RED_THREADS) mgcg_init_final(CGState* st, cons
   }
 }
 
-__device__ __forceinline__ double2 ld2(const double* a, int64_t c) { return reinterpret_cast<const double2*>(a)[c]; }
-__device__ __forceinline__ double2 ld2(const float* a, int64_t c) {
+template <typename TZ> struct Two {
+  TZ x, y;
+};
+__device__ __forceinline__ Two<double> ld2(const double* a, int64_t c) {
+  const double2 q = reinterpret_cast<const double2*>(a)[c];
+  return {q.x, q.y};
+}
+__device__ __forceinline__ Two<float> ld2(const float* a, int64_t c) {
   const float2 q = reinterpret_cast<const float2*>(a)[c];
-  return make_double2(q.x, q.y);
+  return {q.x, q.y};
+}
+__device__ __forceinline__ void st2(double* a, int64_t c, double x, double y) {
+  reinterpret_cast<double2*>(a)[c] = make_double2(x, y);
+}
+__device__ __forceinline__ void st2(float* a, int64_t c, float x, float y) {
+  reinterpret_cast<float2*>(a)[c] = make_float2(x, y);
 }
 
 template <typename TZ>
-__global__ void __launch_bounds__(RED_THREADS) mgcg_rz_kernel(MgcgVecs<TZ> v, const CGState* st, double* partial) {
+__global__ void __launch_bounds__(RED_THREADS) mgcg_smooth_rz_kernel(MgcgVecs<TZ> v, const CGState* st,
+                                                                     double* partial) {
   if (__syncthreads_or(st->done)) return;
+  const TZ th = TZ(v.zcoef[1]);
   double acc[1] = {0.};
   const int64_t np = v.n / 2, t0 = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x;
   const int64_t step = (int64_t)gridDim.x * RED_THREADS;
   for (int64_t c = t0; c < np; c += step) {
-    const double2 r = ld2(v.r, c), z = ld2(v.z, c);
-    acc[0] += r.x * z.x;
-    acc[0] += r.y * z.y;
+    const Two<double> r = ld2(v.r, c);
+    const Two<TZ> z = ld2(v.z, c), t = ld2(v.t, c), d = ld2(v.zdinv, c);
+    const TZ zx = postsmooth(z.x, d.x, r.x, t.x, th), zy = postsmooth(z.y, d.y, r.y, t.y, th);
+    st2(v.z, c, zx, zy);
+    acc[0] += r.x * (double)zx;
+    acc[0] += r.y * (double)zy;
   }
-  for (int64_t i = 2 * np + t0; i < v.n; i += step) acc[0] += v.r[i] * (double)v.z[i];
+  for (int64_t i = 2 * np + t0; i < v.n; i += step) {
+    const TZ z = postsmooth(v.z[i], v.zdinv[i], v.r[i], v.t[i], th);
+    v.z[i] = z;
+    acc[0] += v.r[i] * (double)z;
+  }
   block_sum<1>(acc, partial);
 }
 
@@ -338,7 +376,8 @@ __global__ void __launch_bounds__(RED_THREADS) mgcg_p_kernel(MgcgVecs<TZ> v, CGS
   const int64_t np = v.n / 2, t0 = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x;
   const int64_t step = (int64_t)gridDim.x * RED_THREADS;
   const int its = st->its, par = its & 1;
-  double2 p = make_double2(0., 0.), x = p, z = p;
+  Two<double> p{0., 0.}, x = p;
+  Two<TZ> z{TZ(0), TZ(0)};
   auto load = [&](int64_t c) {
     z = ld2(v.z, c);
     if (its) {
@@ -360,15 +399,13 @@ __global__ void __launch_bounds__(RED_THREADS) mgcg_p_kernel(MgcgVecs<TZ> v, CGS
   if (!(rz > 0.)) return;
   const double b = its ? rz / st->rz[par] : 0., a = st->xalpha;
   for (int64_t c = t0; c < np;) {
-    double2 q = z;
+    double qx = z.x, qy = z.y;
     if (its) {
-      x.x += a * p.x;
-      x.y += a * p.y;
-      q.x += b * p.x;
-      q.y += b * p.y;
-      reinterpret_cast<double2*>(v.x)[c] = x;
+      st2(v.x, c, x.x + a * p.x, x.y + a * p.y);
+      qx += b * p.x;
+      qy += b * p.y;
     }
-    reinterpret_cast<double2*>(v.p)[c] = q;
+    st2(v.p, c, qx, qy);
     c += step;
     if (c < np) load(c);
   }
@@ -384,11 +421,14 @@ __global__ void __launch_bounds__(RED_THREADS) mgcg_update_kernel(MgcgVecs<TZ> v
   if (__syncthreads_or(st->done)) return;
   const int64_t np = v.n / 2, t0 = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x;
   const int64_t step = (int64_t)gridDim.x * RED_THREADS;
-  double2 r = make_double2(0., 0.), w = r, d = r;
+  Two<double> r{0., 0.}, w = r, d = r;
+  Two<TZ> zd{TZ(0), TZ(0)};
+  const TZ th = TZ(v.zcoef[1]);
   auto load = [&](int64_t c) {
     r = ld2(v.r, c);
     w = ld2(v.w, c);
     d = ld2(v.dinv, c);
+    zd = ld2(v.zdinv, c);
   };
   if (t0 < np) load(t0);
   double pws[1];
@@ -416,8 +456,9 @@ __global__ void __launch_bounds__(RED_THREADS) mgcg_update_kernel(MgcgVecs<TZ> v
     const double zx = r.x * d.x, zy = r.y * d.y;
     acc[0] += zx * zx;
     acc[0] += zy * zy;
-    reinterpret_cast<double2*>(v.r)[c] = r;
-    if (v.r32) reinterpret_cast<float2*>(v.r32)[c] = make_float2((float)r.x, (float)r.y);
+    st2(v.r, c, r.x, r.y);
+    if (v.r32) st2(v.r32, c, (float)r.x, (float)r.y);
+    st2(v.z, c, presmooth(zd.x, r.x, th), presmooth(zd.y, r.y, th));
     c += step;
     if (c < np) load(c);
   }
@@ -425,6 +466,7 @@ __global__ void __launch_bounds__(RED_THREADS) mgcg_update_kernel(MgcgVecs<TZ> v
     const double ri = v.r[i] - alpha * v.w[i], zi = ri * v.dinv[i];
     v.r[i] = ri;
     if (v.r32) v.r32[i] = (float)ri;
+    v.z[i] = presmooth(v.zdinv[i], ri, th);
     acc[0] += zi * zi;
   }
   block_sum<1>(acc, partial);
@@ -658,7 +700,7 @@ template <typename TZ>
 cudaError_t mgcg_init(const MgcgVecs<TZ>& v, CGState* st, double* partial, double rtol, double atol, double dtol,
                       int maxit, cudaStream_t s) {
   for (const void* q : {(const void*)v.x, (const void*)v.r, (const void*)v.p, (const void*)v.w, (const void*)v.dinv,
-                        (const void*)v.z, (const void*)v.r32})
+                        (const void*)v.z, (const void*)v.r32, (const void*)v.t, (const void*)v.zdinv})
     if (reinterpret_cast<uintptr_t>(q) % 16) return cudaErrorMisalignedAddress;
   if (!v.dotp || v.ndot <= 0) return cudaErrorInvalidValue;
   mgcg_init_kernel<TZ><<<RED_BLOCKS, RED_THREADS, 0, s>>>(v, partial);
@@ -668,7 +710,7 @@ cudaError_t mgcg_init(const MgcgVecs<TZ>& v, CGState* st, double* partial, doubl
 template <typename TZ>
 cudaError_t mgcg_direction(const MgcgVecs<TZ>& v, CGState* st, double* partial, cudaStream_t s) {
   const int nb = cg_blocks(v.n, 8);
-  mgcg_rz_kernel<TZ><<<nb, RED_THREADS, 0, s>>>(v, st, partial);
+  mgcg_smooth_rz_kernel<TZ><<<nb, RED_THREADS, 0, s>>>(v, st, partial);
   mgcg_p_kernel<TZ><<<nb, RED_THREADS, 0, s>>>(v, st, partial, nb);
   return cudaGetLastError();
 }
