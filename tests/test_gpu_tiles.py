@@ -69,6 +69,44 @@ def test_v_residual_and_energies(cuda, oracle_mod, n, atnum, thermal, cellE, lay
     ctx.close()
 
 
+@pytest.mark.parametrize("n,atnum,thermal,cellE,layers,unilateral", CASES)
+def test_u_load(cuda, oracle_mod, n, atnum, thermal, cellE, layers, unilateral):
+    """F_U at U = 0 is minus the load: entries of at most 216 Gauss terms, 1e-11 of the largest as
+    above."""
+    o, ctx, u, v, p, theta = _setup(oracle_mod, n, atnum, thermal, cellE, layers, unilateral)
+    u = np.zeros(3 * o.N)
+    ctx.set_field("U", u)
+    mask, val = o.bc(oracle_mod.rollers_face())
+    F = ctx.u_residual()
+    Fr = o.u_residual_ref(u, v, theta, None, p, mask, val)
+    assert np.abs(F - Fr).max() <= 1e-11 * np.abs(Fr).max()
+    ctx.close()
+
+
+@pytest.mark.parametrize("case", [CASES[1], CASES[3]])
+def test_u_diagonal(cuda, oracle_mod, case):
+    """One Jacobi CG iteration from U = 0 moves along z = D^-1 r, D the diagonal of the oracle's
+    operator (the step lengths, CG's and Newton's, are the solver's): a handful of roundings of
+    sums of one sign, 1e-10."""
+    o, ctx, u, v, p, theta = _setup(oracle_mod, *case)
+    n3 = 3 * o.N
+    ctx.set_field("U", np.zeros(n3))
+    mask, val = o.bc(oracle_mod.rollers_face())
+    rc, st = ctx.step_u(dict(ksp_maxit=1, snes_maxit=1))
+    assert st["ksp_its"] == 1, st
+    F = o.u_residual_ref(np.zeros(n3), v, theta, None, p, mask, val)
+    D, e = np.empty(n3), np.zeros(n3)
+    for i in range(n3):
+        e[i] = 1.0
+        D[i] = o.u_apply(v, e, mask)[i]
+        e[i] = 0.0
+    z, U = F / D, ctx.get_field("U")
+    i = np.abs(z).argmax()
+    assert U[i] / z[i] < 0.0
+    assert np.abs(U / U[i] - z / z[i]).max() <= 1e-10
+    ctx.close()
+
+
 # Grids that take the U stencil: the smallest that do in FP64 (2000 units of 32 x 8 x 1), one
 # column past a 32 x 16 tile and its multiples, a chunk of few planes, faces not a multiple of
 # 30 columns or 4 planes; the last one also in FP32 (6000 units).

@@ -1,9 +1,9 @@
-// elem.cu -- once-per-solve element kernels, written per Gauss point after the
-// reference's element routines.  Scatter to nodes is done in 8 parity colours of
-// elements so that no two threads of a launch touch the same node: deterministic, no
-// atomics.  The element tables travel by value in the kernel parameters
-// (__grid_constant__): every thread of a warp reads the same entry, which the
-// constant bank broadcasts.
+// elem.cu -- once-per-solve element kernels, after the reference's element routines.  The plain
+// operator's element vectors are summed in one pass (cell_gather_kernel); the NOCOMPRESSION
+// forms are written per Gauss point and scattered to nodes in 8 parity colours of elements, so
+// that no two threads of a launch touch the same node.  Both are deterministic, without
+// atomics.  The element tables travel by value in the kernel parameters (__grid_constant__):
+// every thread of a warp reads the same entry, which the constant bank broadcasts.
 #include <algorithm>
 #include <cmath>
 
@@ -222,77 +222,26 @@ __device__ __forceinline__ void face_moments(const double (&q)[27], double (&F)[
     }
 }
 
-// u_diag_kernel in tensor form (plain operator): diag of node (i,j,k), component x, is
+// The U diagonal in tensor form (plain operator): diag of node (i,j,k), component x, is
 //   (lambda + 2 mu) Jx[j][k] / hx^2 + mu (Jy[i][k] / hy^2 + Jz[i][j] / hz^2)
 // with J_d the integrals of w (v^2 + eta) against the squared basis functions of the
 // other two axes (and similarly for y, z).
-__global__ void u_diag_tp_kernel(const __grid_constant__ ElemArgs E, int color,
-                                 const double* __restrict__ v, double* __restrict__ d) {
-  int ei, ej, ek;
-  if (!colour_cell(E, color, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, ei, ej, ek)) return;
-  int64_t n[8];
-  cell_nodes(E, ei, ej, ek, n);
-  double v8[8], v27[27], s27[27];
+struct UDiagCell {
+  static constexpr int NF = 1, NV = 3, MINB = 2;  // nodal fields, values per corner, blocks per SM
+  const double* __restrict__ v;
+  const uint8_t* __restrict__ bc;  // Dirichlet bits or null
+  double* __restrict__ d;
+  __device__ __forceinline__ void load(int64_t n, double (&q)[NF]) const { q[0] = v[n]; }
+  __device__ __forceinline__ void put(int64_t n, const double (&y)[NV]) const {
+    const unsigned b = bc ? bc[n] : 0u;
 #pragma unroll
-  for (int a = 0; a < 8; a++) v8[a] = v[n[a]];
-  interp27(v8, v27);
-  const double vol = E.hx * E.hy * E.hz;
-#pragma unroll
-  for (int gz = 0; gz < 3; gz++)
-#pragma unroll
-    for (int gy = 0; gy < 3; gy++)
-#pragma unroll
-      for (int gx = 0; gx < 3; gx++) {
-        const int g = gx + 3 * gy + 9 * gz;
-        s27[g] = (vol * (w1(gx) * w1(gy) * w1(gz))) * fma(v27[g], v27[g], E.eta);
-      }
-  double J[3][2][2];
-  face_moments<true>(s27, J);
-  const CellMat m = cell_mat(E, ei, ej, ek);
-  const double l2m = m.lambda + 2. * m.mu;
-  const double ih2[3] = {1. / (E.hx * E.hx), 1. / (E.hy * E.hy), 1. / (E.hz * E.hz)};
-#pragma unroll
-  for (int k = 0; k < 2; k++)
-#pragma unroll
-    for (int j = 0; j < 2; j++)
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const double jx = J[0][j][k] * ih2[0], jy = J[1][i][k] * ih2[1], jz = J[2][i][j] * ih2[2];
-        const int64_t q = 3 * n[i + 2 * j + 4 * k];
-        d[q + 0] += fma(l2m, jx, m.mu * (jy + jz));
-        d[q + 1] += fma(l2m, jy, m.mu * (jx + jz));
-        d[q + 2] += fma(l2m, jz, m.mu * (jx + jy));
-      }
-}
-
-// u_rhs_kernel in tensor form (plain operator): the thermo-poro load
-// sum_g w dphi_a,c S_g, S = 3 kappa alpha (theta - thetaRef)(v^2 + eta) + beta p v, as
-// face moments of w S times -+1/h_c, and the crack-pressure load
-// sum_g w p grad_c v phi_a as a full contraction.
-__global__ void u_rhs_tp_kernel(const __grid_constant__ ElemArgs E, int color,
-                                const double* __restrict__ v, const double* __restrict__ theta,
-                                const double* __restrict__ thetaRef, const double* __restrict__ p,
-                                double* __restrict__ f) {
-  int ei, ej, ek;
-  if (!colour_cell(E, color, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, ei, ej, ek)) return;
-  int64_t n[8];
-  cell_nodes(E, ei, ej, ek, n);
-  double v8[8], th8[8], p8[8];
-#pragma unroll
-  for (int a = 0; a < 8; a++) {
-    v8[a] = v[n[a]];
-    th8[a] = theta ? theta[n[a]] - (thetaRef ? thetaRef[n[a]] : 0.) : 0.;
-    p8[a] = p ? p[n[a]] : 0.;
+    for (int c = 0; c < 3; c++) d[3 * n + c] = (b >> c) & 1u ? 1. : y[c];
   }
-  const CellMat m = cell_mat(E, ei, ej, ek);
-  const double coefalpha = (3. * m.lambda + 2. * m.mu) * m.alpha, beta = m.beta;
-  const double vol = E.hx * E.hy * E.hz;
-  double ve[27], pe[27], ws[27];
-  interp27(v8, ve);
-  interp27(p8, pe);
-  {
-    double te[27];
-    interp27(th8, te);
+  __device__ __forceinline__ void cell(const ElemArgs& E, int ei, int ej, int ek, const double (&q)[NF][8],
+                                       double (&out)[8][NV]) const {
+    double v27[27], s27[27];
+    interp27(q[0], v27);
+    const double vol = E.hx * E.hy * E.hz;
 #pragma unroll
     for (int gz = 0; gz < 3; gz++)
 #pragma unroll
@@ -300,48 +249,59 @@ __global__ void u_rhs_tp_kernel(const __grid_constant__ ElemArgs E, int color,
 #pragma unroll
         for (int gx = 0; gx < 3; gx++) {
           const int g = gx + 3 * gy + 9 * gz;
-          const double s = coefalpha * te[g] * (ve[g] * ve[g] + E.eta) + beta * pe[g] * ve[g];
-          ws[g] = (vol * (w1(gx) * w1(gy) * w1(gz))) * s;
+          s27[g] = (vol * (w1(gx) * w1(gy) * w1(gz))) * fma(v27[g], v27[g], E.eta);
+        }
+    double J[3][2][2];
+    face_moments<true>(s27, J);
+    const CellMat m = cell_mat(E, ei, ej, ek);
+    const double l2m = m.lambda + 2. * m.mu;
+    const double ih2[3] = {1. / (E.hx * E.hx), 1. / (E.hy * E.hy), 1. / (E.hz * E.hz)};
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          const double jx = J[0][j][k] * ih2[0], jy = J[1][i][k] * ih2[1], jz = J[2][i][j] * ih2[2];
+          const int a = i + 2 * j + 4 * k;
+          out[a][0] = fma(l2m, jx, m.mu * (jy + jz));
+          out[a][1] = fma(l2m, jy, m.mu * (jx + jz));
+          out[a][2] = fma(l2m, jz, m.mu * (jx + jy));
         }
   }
-  double F[3][2][2];
-  face_moments<false>(ws, F);
-  const double ih[3] = {1. / E.hx, 1. / E.hy, 1. / E.hz};
-  double rl[8][3];
+};
+
+// The U load in tensor form (plain operator): the thermo-poro load
+// sum_g w dphi_a,c S_g, S = 3 kappa alpha (theta - thetaRef)(v^2 + eta) + beta p v, as
+// face moments of w S times -+1/h_c, and the crack-pressure load
+// sum_g w p grad_c v phi_a as a full contraction.
+// The crack-pressure term of an element with 8 equal nodal v (and finite p) is 0 and not
+// evaluated: grad v is exactly 0 there.
+struct URhsCell {
+  static constexpr int NF = 3, NV = 3, MINB = 1;
+  const double *__restrict__ v, *__restrict__ theta, *__restrict__ thetaRef, *__restrict__ p;
+  double* __restrict__ f;
+  __device__ __forceinline__ void load(int64_t n, double (&q)[NF]) const {
+    q[0] = v[n];
+    q[1] = theta ? theta[n] - (thetaRef ? thetaRef[n] : 0.) : 0.;
+    q[2] = p ? p[n] : 0.;
+  }
+  __device__ __forceinline__ void put(int64_t n, const double (&y)[NV]) const {
 #pragma unroll
-  for (int k = 0; k < 2; k++)
-#pragma unroll
-    for (int j = 0; j < 2; j++)
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const int a = i + 2 * j + 4 * k;
-        rl[a][0] = (i ? ih[0] : -ih[0]) * F[0][j][k];
-        rl[a][1] = (j ? ih[1] : -ih[1]) * F[1][i][k];
-        rl[a][2] = (k ? ih[2] : -ih[2]) * F[2][i][j];
-      }
-  if (E.hasCrackPressure) {
-    // grad v at the points: each component depends on the two other axes only
-    double gv[3][9];  // gv[d][a + 3 b], (a, b) the other axes' point indices
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-      for (int b = 0; b < 3; b++) {
-        double sx = 0., sy = 0., sz = 0.;
-#pragma unroll
-        for (int q = 0; q < 2; q++)
-#pragma unroll
-          for (int r = 0; r < 2; r++) {
-            sx += bas(q, a) * bas(r, b) * (v8[1 + 2 * q + 4 * r] - v8[2 * q + 4 * r]);
-            sy += bas(q, a) * bas(r, b) * (v8[q + 2 + 4 * r] - v8[q + 4 * r]);
-            sz += bas(q, a) * bas(r, b) * (v8[q + 2 * r + 4] - v8[q + 2 * r]);
-          }
-        gv[0][a + 3 * b] = sx * ih[0];
-        gv[1][a + 3 * b] = sy * ih[1];
-        gv[2][a + 3 * b] = sz * ih[2];
-      }
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      double qc[27], oc[8];
+    for (int c = 0; c < 3; c++) f[3 * n + c] = y[c];
+  }
+  __device__ __forceinline__ void cell(const ElemArgs& E, int ei, int ej, int ek, const double (&fld)[NF][8],
+                                       double (&rl)[8][NV]) const {
+    const double (&v8)[8] = fld[0], (&th8)[8] = fld[1], (&p8)[8] = fld[2];
+    const CellMat m = cell_mat(E, ei, ej, ek);
+    const double coefalpha = (3. * m.lambda + 2. * m.mu) * m.alpha, beta = m.beta;
+    const double vol = E.hx * E.hy * E.hz;
+    double ve[27], pe[27], ws[27];
+    interp27(v8, ve);
+    interp27(p8, pe);
+    {
+      double te[27];
+      interp27(th8, te);
 #pragma unroll
       for (int gz = 0; gz < 3; gz++)
 #pragma unroll
@@ -349,19 +309,71 @@ __global__ void u_rhs_tp_kernel(const __grid_constant__ ElemArgs E, int color,
 #pragma unroll
           for (int gx = 0; gx < 3; gx++) {
             const int g = gx + 3 * gy + 9 * gz;
-            const double gvc = c == 0 ? gv[0][gy + 3 * gz] : (c == 1 ? gv[1][gx + 3 * gz] : gv[2][gx + 3 * gy]);
-            qc[g] = (vol * (w1(gx) * w1(gy) * w1(gz))) * pe[g] * gvc;
+            const double s = coefalpha * te[g] * (ve[g] * ve[g] + E.eta) + beta * pe[g] * ve[g];
+            ws[g] = (vol * (w1(gx) * w1(gy) * w1(gz))) * s;
           }
-      contract27(qc, oc);
+    }
+    double F[3][2][2];
+    face_moments<false>(ws, F);
+    const double ih[3] = {1. / E.hx, 1. / E.hy, 1. / E.hz};
 #pragma unroll
-      for (int a = 0; a < 8; a++) rl[a][c] += oc[a];
+    for (int k = 0; k < 2; k++)
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          const int a = i + 2 * j + 4 * k;
+          rl[a][0] = (i ? ih[0] : -ih[0]) * F[0][j][k];
+          rl[a][1] = (j ? ih[1] : -ih[1]) * F[1][i][k];
+          rl[a][2] = (k ? ih[2] : -ih[2]) * F[2][i][j];
+        }
+    bool flat = true;
+    double ps = 0.;
+#pragma unroll
+    for (int a = 0; a < 8; a++) {
+      flat = flat && v8[a] == v8[0];
+      ps += fabs(p8[a]);
+    }
+    if (E.hasCrackPressure && !(flat && ps - ps == 0.)) {
+      // grad v at the points: each component depends on the two other axes only
+      double gv[3][9];  // gv[d][a + 3 b], (a, b) the other axes' point indices
+#pragma unroll
+      for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+          double sx = 0., sy = 0., sz = 0.;
+#pragma unroll
+          for (int q = 0; q < 2; q++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+              sx += bas(q, a) * bas(r, b) * (v8[1 + 2 * q + 4 * r] - v8[2 * q + 4 * r]);
+              sy += bas(q, a) * bas(r, b) * (v8[q + 2 + 4 * r] - v8[q + 4 * r]);
+              sz += bas(q, a) * bas(r, b) * (v8[q + 2 * r + 4] - v8[q + 2 * r]);
+            }
+          gv[0][a + 3 * b] = sx * ih[0];
+          gv[1][a + 3 * b] = sy * ih[1];
+          gv[2][a + 3 * b] = sz * ih[2];
+        }
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        double qc[27], oc[8];
+#pragma unroll
+        for (int gz = 0; gz < 3; gz++)
+#pragma unroll
+          for (int gy = 0; gy < 3; gy++)
+#pragma unroll
+            for (int gx = 0; gx < 3; gx++) {
+              const int g = gx + 3 * gy + 9 * gz;
+              const double gvc = c == 0 ? gv[0][gy + 3 * gz] : (c == 1 ? gv[1][gx + 3 * gz] : gv[2][gx + 3 * gy]);
+              qc[g] = (vol * (w1(gx) * w1(gy) * w1(gz))) * pe[g] * gvc;
+            }
+        contract27(qc, oc);
+#pragma unroll
+        for (int a = 0; a < 8; a++) rl[a][c] += oc[a];
+      }
     }
   }
-#pragma unroll
-  for (int a = 0; a < 8; a++)
-#pragma unroll
-    for (int c = 0; c < 3; c++) f[3 * n[a] + c] += rl[a][c];
-}
+};
 
 __global__ void u_rhs_kernel(const __grid_constant__ ElemArgs E, int color, const double* __restrict__ v,
                              const double* __restrict__ theta, const double* __restrict__ thetaRef,
@@ -597,14 +609,15 @@ __global__ void __launch_bounds__(256, 1) v_assemble_kernel(const __grid_constan
                                                             const double* __restrict__ theta,
                                                             const double* __restrict__ thetaRef,
                                                             double* __restrict__ a64,
-                                                            float* __restrict__ a32, int64_t stride, int zc) {
+                                                            float* __restrict__ a32, int64_t stride, int gx,
+                                                            int zc) {
   extern __shared__ double vm_s[];  // [27][8][32]
   const int l = threadIdx.x, w = threadIdx.y;
   const int nx = E.nx, ny = E.ny, nz = E.nz;
-  const int ex = blockIdx.x * VM_NX - 1 + l, ey = blockIdx.y * VM_NY - 1 + w;
+  const int ex = (int)(blockIdx.x % gx) * VM_NX - 1 + l, ey = (int)(blockIdx.x / gx) * VM_NY - 1 + w;
   const bool cell = ex >= 0 && ex < nx - 1 && ey >= 0 && ey < ny - 1;
   const bool node = l > 0 && w > 0 && ex < nx && ey < ny;  // owns node column (ex, ey)
-  const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);
+  const int z0 = blockIdx.y * zc, z1 = min(z0 + zc, nz);
   const int64_t plane = (int64_t)nx * ny;
   const int64_t base = cell ? (int64_t)ey * nx + ex : 0;
   double f[3][8], th8[8], carry[5];
@@ -689,55 +702,144 @@ __global__ void __launch_bounds__(256, 1) v_assemble_kernel(const __grid_constan
 // V load (VF_ResidualVAT1/AT23D_local and VF_ResidualVCrackPressure3D_local,
 // VFMech.c:2294-2384) in tensor form: the AT term coef sum_g w phi_a = coef vol / 8 per
 // node, the crack-pressure term sum_g w p (u . grad phi_a) as face moments of w p u_c.
-__global__ void v_rhs_tp_kernel(const __grid_constant__ ElemArgs E, int color,
-                                const double* __restrict__ u, const double* __restrict__ p,
-                                double* __restrict__ b) {
-  int ei, ej, ek;
-  if (!colour_cell(E, color, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, ei, ej, ek)) return;
-  int64_t n[8];
-  cell_nodes(E, ei, ej, ek, n);
-  const CellMat m = cell_mat(E, ei, ej, ek);
-  const double vol = E.hx * E.hy * E.hz;
-  const double coef = m.Gc / E.atcv / E.epsilon * (E.atnum == 1 ? .25 : .5);
-  double rl[8];
+struct VRhsCell {
+  static constexpr int NF = 4, NV = 1, MINB = 1;
+  const double *__restrict__ u, *__restrict__ p;
+  double* __restrict__ b;
+  bool pressure;  // p given and crack pressure on
+  __device__ __forceinline__ void load(int64_t n, double (&q)[NF]) const {
 #pragma unroll
-  for (int a = 0; a < 8; a++) rl[a] = coef * vol * 0.125;
-  if (E.hasCrackPressure && p) {
-    double p8[8], pe[27];
+    for (int c = 0; c < 3; c++) q[c] = pressure ? u[3 * n + c] : 0.;
+    q[3] = pressure ? p[n] : 0.;
+  }
+  __device__ __forceinline__ void put(int64_t n, const double (&y)[NV]) const { b[n] = y[0]; }
+  __device__ __forceinline__ void cell(const ElemArgs& E, int ei, int ej, int ek, const double (&fld)[NF][8],
+                                       double (&out)[8][NV]) const {
+    const CellMat m = cell_mat(E, ei, ej, ek);
+    const double vol = E.hx * E.hy * E.hz;
+    const double coef = m.Gc / E.atcv / E.epsilon * (E.atnum == 1 ? .25 : .5);
 #pragma unroll
-    for (int a = 0; a < 8; a++) p8[a] = p[n[a]];
-    interp27(p8, pe);
-    const double ih[3] = {1. / E.hx, 1. / E.hy, 1. / E.hz};
+    for (int a = 0; a < 8; a++) out[a][0] = coef * vol * 0.125;
+    if (pressure) {
+      double pe[27];
+      interp27(fld[3], pe);
+      const double ih[3] = {1. / E.hx, 1. / E.hy, 1. / E.hz};
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      double u8[8], q[27], F[3][2][2];
+      for (int c = 0; c < 3; c++) {
+        double q[27], F[3][2][2];
+        interp27(fld[c], q);
 #pragma unroll
-      for (int a = 0; a < 8; a++) u8[a] = u[3 * n[a] + c];
-      interp27(u8, q);
+        for (int gz = 0; gz < 3; gz++)
 #pragma unroll
-      for (int gz = 0; gz < 3; gz++)
+          for (int gy = 0; gy < 3; gy++)
 #pragma unroll
-        for (int gy = 0; gy < 3; gy++)
+            for (int gx = 0; gx < 3; gx++) {
+              const int g = gx + 3 * gy + 9 * gz;
+              q[g] = (vol * (w1(gx) * w1(gy) * w1(gz))) * pe[g] * q[g];
+            }
+        face_moments<false>(q, F);
 #pragma unroll
-          for (int gx = 0; gx < 3; gx++) {
-            const int g = gx + 3 * gy + 9 * gz;
-            q[g] = (vol * (w1(gx) * w1(gy) * w1(gz))) * pe[g] * q[g];
-          }
-      face_moments<false>(q, F);
+        for (int k = 0; k < 2; k++)
 #pragma unroll
-      for (int k = 0; k < 2; k++)
+          for (int j = 0; j < 2; j++)
 #pragma unroll
-        for (int j = 0; j < 2; j++)
-#pragma unroll
-          for (int i = 0; i < 2; i++) {
-            const int sgn = c == 0 ? i : (c == 1 ? j : k);
-            const double fm = c == 0 ? F[0][j][k] : (c == 1 ? F[1][i][k] : F[2][i][j]);
-            rl[i + 2 * j + 4 * k] += (sgn ? ih[c] : -ih[c]) * fm;
-          }
+            for (int i = 0; i < 2; i++) {
+              const int sgn = c == 0 ? i : (c == 1 ? j : k);
+              const double fm = c == 0 ? F[0][j][k] : (c == 1 ? F[1][i][k] : F[2][i][j]);
+              out[i + 2 * j + 4 * k][0] += (sgn ? ih[c] : -ih[c]) * fm;
+            }
+      }
     }
   }
+};
+
+// One pass of an element vector: a block owns 31 x 7 node columns and the 32 x 8 cell columns
+// around them, and marches up a chunk of node planes.  Per element layer each thread evaluates
+// its cell (C::cell); its corners' values are summed over x by a shuffle, over y through
+// shared memory (two buffers, one barrier per layer) and over z in registers, so every node is
+// written once, in one fixed order.  The cells on the seams of the blocks are computed
+// twice.  8 launches of a parity colour each read and wrote the result 8 times, a cache line
+// for every second node: at 129^3 U load 466 us, diagonal 234, V load 215; now 275, 118 and 214
+// (bound by FP64 issue, V's at one block of 8 warps per SM); 65^3 74 -> 80, 47 -> 27, 50 -> 45; the
+// diagonals of the coarse levels 47 -> 6 to 9.
+constexpr int CG_NX = 31, CG_NY = 7;
+template <class C>
+__global__ void __launch_bounds__(256, C::MINB)
+    cell_gather_kernel(const __grid_constant__ ElemArgs E, const C op, int gx, int zc) {
+  constexpr int NF = C::NF, NV = C::NV;
+  __shared__ double sh[2][2 * NV][256];
+  const int l = threadIdx.x, w = threadIdx.y, t = w * 32 + l;
+  const int nx = E.nx, ny = E.ny, nz = E.nz;
+  const int bx = blockIdx.x % gx, by = blockIdx.x / gx;
+  const int ex = bx * CG_NX - 1 + l, ey = by * CG_NY - 1 + w;
+  const bool cell = ex >= 0 && ex < nx - 1 && ey >= 0 && ey < ny - 1;
+  const bool node = l > 0 && w > 0 && ex < nx && ey < ny;  // owns node column (ex, ey)
+  const int z0 = blockIdx.y * zc, z1 = min(z0 + zc, nz), k0 = max(z0 - 1, 0);
+  const int64_t plane = (int64_t)nx * ny, base = cell ? (int64_t)ey * nx + ex : 0;
+  double q[NF][8], carry[NV];
 #pragma unroll
-  for (int a = 0; a < 8; a++) b[n[a]] += rl[a];
+  for (int c = 0; c < NV; c++) carry[c] = 0.;
+  auto load4 = [&](int k) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      double f[NF];
+      op.load(cell ? base + k * plane + (j >> 1) * nx + (j & 1) : 0, f);
+#pragma unroll
+      for (int i = 0; i < NF; i++) q[i][4 + j] = f[i];
+    }
+  };
+  load4(k0);
+  for (int k = k0; k < z1; k++) {
+    const int b = (k - k0) & 1;
+    const bool layer = k < nz - 1;
+    double xs[2][2][NV];  // [j][kk]: this cell's and its left neighbour's share of column ex
+    if (layer) {
+#pragma unroll
+      for (int i = 0; i < NF; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) q[i][j] = q[i][4 + j];
+      load4(k + 1);
+      double out[8][NV];
+      if (cell) {
+        op.cell(E, ex, ey, k, q, out);
+      } else {
+#pragma unroll
+        for (int a = 0; a < 8; a++)
+#pragma unroll
+          for (int c = 0; c < NV; c++) out[a][c] = 0.;
+      }
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+#pragma unroll
+        for (int kk = 0; kk < 2; kk++)
+#pragma unroll
+          for (int c = 0; c < NV; c++)
+            xs[j][kk][c] = __shfl_up_sync(0xffffffffu, out[1 + 2 * j + 4 * kk][c], 1) + out[2 * j + 4 * kk][c];
+#pragma unroll
+      for (int kk = 0; kk < 2; kk++)
+#pragma unroll
+        for (int c = 0; c < NV; c++) sh[b][kk * NV + c][t] = xs[1][kk][c];
+    }
+    __syncthreads();
+    if (!node) continue;
+    double y[NV], up[NV];
+#pragma unroll
+    for (int c = 0; c < NV; c++) {
+      y[c] = layer ? carry[c] + (sh[b][c][t - 32] + xs[0][0][c]) : carry[c];
+      up[c] = layer ? sh[b][NV + c][t - 32] + xs[0][1][c] : 0.;
+    }
+    if (k >= z0) op.put((int64_t)k * plane + (int64_t)ey * nx + ex, y);
+#pragma unroll
+    for (int c = 0; c < NV; c++) carry[c] = up[c];
+  }
+}
+
+// Node planes of a marching block's chunk: four waves of one block per SM on large grids
+// (each chunk evaluates the layer below it again), at least `least` planes on small ones, at
+// most 65535 chunks.
+int march_planes(int64_t columns, int nz, int least) {
+  const int zc = (int)std::max<int64_t>(least, (columns * nz + 591) / 592);
+  return std::max(std::min(zc, nz), ceil_div(nz, 65535));
 }
 
 // Neumaier-compensated accumulation.
@@ -1128,6 +1230,13 @@ __global__ void __launch_bounds__(EN_THREADS, (WANT & kEnElastic) ? 3 : 4) energ
   if (threadIdx.x < 4) partial[blockIdx.x * 4 + threadIdx.x] = red[threadIdx.x][0];
 }
 
+template <class C> cudaError_t cell_gather(const ElemArgs& E, const C& op, cudaStream_t s) {
+  const int gx = ceil_div(E.nx, CG_NX), gy = ceil_div(E.ny, CG_NY);
+  const int zc = march_planes((int64_t)gx * gy, E.nz, 2);
+  cell_gather_kernel<C><<<dim3(gx * gy, ceil_div(E.nz, zc)), dim3(32, 8), 0, s>>>(E, op, gx, zc);
+  return cudaGetLastError();
+}
+
 template <typename K, typename... Args>
 cudaError_t colours(const ElemArgs& E, K kernel, cudaStream_t s, Args... args) {
   for (int color = 0; color < 8; color++) {
@@ -1145,10 +1254,10 @@ cudaError_t colours(const ElemArgs& E, K kernel, cudaStream_t s, Args... args) {
 cudaError_t launch_u_rhs(const ElemArgs& E, const double* v, const double* theta,
                          const double* thetaRef, const double* p, double* f, cudaStream_t s,
                          const double* u0) {
+  if (!E.unilateral) return cell_gather(E, URhsCell{v, theta, thetaRef, p, f}, s);
   const int64_t N = (int64_t)E.nx * E.ny * E.nz;
   cudaError_t e = cudaMemsetAsync(f, 0, 3 * N * sizeof(double), s);
   if (e != cudaSuccess) return e;
-  if (!E.unilateral) return colours(E, u_rhs_tp_kernel, s, v, theta, thetaRef, p, f);
   return colours(E, u_rhs_kernel, s, v, theta, thetaRef, p, f, u0);
 }
 
@@ -1160,10 +1269,10 @@ cudaError_t launch_nc_flags(const ElemArgs& E, const double* u, uint32_t* flags,
 
 cudaError_t launch_u_diag(const ElemArgs& E, const double* v, const uint8_t* bcbits, double* d,
                           cudaStream_t s, const double* u0) {
+  if (!E.unilateral) return cell_gather(E, UDiagCell{v, bcbits, d}, s);
   const int64_t N = (int64_t)E.nx * E.ny * E.nz;
   cudaError_t e = cudaMemsetAsync(d, 0, 3 * N * sizeof(double), s);
-  if (e == cudaSuccess)
-    e = E.unilateral ? colours(E, u_diag_kernel, s, v, d, u0) : colours(E, u_diag_tp_kernel, s, v, d);
+  if (e == cudaSuccess) e = colours(E, u_diag_kernel, s, v, d, u0);
   if (e == cudaSuccess && bcbits) {
     bc_diag_kernel<<<(int)std::min<int64_t>((N + 255) / 256, 2368), 256, 0, s>>>(bcbits, d, N);
     e = cudaGetLastError();
@@ -1177,22 +1286,15 @@ cudaError_t launch_v_assemble(const ElemArgs& E, const double* u, const double* 
   cudaError_t e = cudaFuncSetAttribute(v_assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int gx = ceil_div(E.nx, VM_NX), gy = ceil_div(E.ny, VM_NY);
-  if (gy > 65535) return cudaErrorInvalidValue;
-  // planes of a chunk: four waves of one block per SM on large grids (each chunk computes the
-  // layer below it again), at least 4 planes on small ones, at most 65535 chunks
-  int zc = (int)std::max<int64_t>(4, ((int64_t)gx * gy * E.nz + 591) / 592);
-  zc = std::max(std::min(zc, E.nz), ceil_div(E.nz, 65535));
-  v_assemble_kernel<<<dim3(gx, gy, ceil_div(E.nz, zc)), dim3(32, 8), smem, s>>>(
-      E, u, theta, thetaRef, a64, a32, vmat_stride((int64_t)E.nx * E.ny * E.nz), zc);
+  const int zc = march_planes((int64_t)gx * gy, E.nz, 4);
+  v_assemble_kernel<<<dim3(gx * gy, ceil_div(E.nz, zc)), dim3(32, 8), smem, s>>>(
+      E, u, theta, thetaRef, a64, a32, vmat_stride((int64_t)E.nx * E.ny * E.nz), gx, zc);
   return cudaGetLastError();
 }
 
 cudaError_t launch_v_rhs(const ElemArgs& E, const double* u, const double* p, double* b,
                          cudaStream_t s) {
-  const int64_t N = (int64_t)E.nx * E.ny * E.nz;
-  cudaError_t e = cudaMemsetAsync(b, 0, N * sizeof(double), s);
-  if (e != cudaSuccess) return e;
-  return colours(E, v_rhs_tp_kernel, s, u, p, b);
+  return cell_gather(E, VRhsCell{u, p, b, E.hasCrackPressure && p}, s);
 }
 
 int energy_blocks() { return EN_BLOCKS; }
