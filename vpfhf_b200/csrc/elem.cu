@@ -166,33 +166,57 @@ __device__ __forceinline__ void interp27(const double (&f)[8], double (&o)[27]) 
         o[gx + 3 * gy + 9 * gz] = bas(0, gz) * fy[0][gy][gx] + bas(1, gz) * fy[1][gy][gx];
 }
 
-// out[i + 2j + 4k] = sum_g q_g b_i(gx) b_j(gy) b_k(gz)
-__device__ __forceinline__ void contract27(const double (&q)[27], double (&out)[8]) {
-  double cx[2][3][3], cy[2][2][3];
+// Products of two trilinear fields against the basis, in closed form (the 3-point rule is exact
+// for their degrees).  For axis d the other two, in increasing order, are bits ax1 and ax2 of a
+// modal index (modal_of), and a field's 4 transverse coefficients at power 0 or 1 of t_d are
+// m[(P ? d's bit : 0) + ...].
+__device__ __forceinline__ constexpr int ax1(int d) { return d == 0 ? 2 : 1; }
+__device__ __forceinline__ constexpr int ax2(int d) { return d == 2 ? 2 : 4; }
+template <int P> __device__ __forceinline__ void transverse(const double (&m)[8], int d, double (&f)[4]) {
 #pragma unroll
-  for (int i = 0; i < 2; i++)
+  for (int q = 0; q < 4; q++) f[q] = m[(P ? 1 << d : 0) + ((q & 1) ? ax1(d) : 0) + ((q & 2) ? ax2(d) : 0)];
+}
+// X[a][b] (+)= coefficient of t1^a t2^b in the product of two bilinear fields.
+template <bool ADD>
+__device__ __forceinline__ void bilinear_product(const double (&f)[4], const double (&g)[4], double (&X)[3][3]) {
+  const double q[3][3] = {{f[0] * g[0], fma(f[0], g[2], f[2] * g[0]), f[2] * g[2]},
+                          {fma(f[0], g[1], f[1] * g[0]),
+                           fma(f[0], g[3], f[3] * g[0]) + fma(f[1], g[2], f[2] * g[1]), fma(f[2], g[3], f[3] * g[2])},
+                          {f[1] * g[1], fma(f[1], g[3], f[3] * g[1]), f[3] * g[3]}};
 #pragma unroll
-    for (int gz = 0; gz < 3; gz++)
+  for (int a = 0; a < 3; a++)
 #pragma unroll
-      for (int gy = 0; gy < 3; gy++) {
-        const int b = 3 * gy + 9 * gz;
-        cx[i][gy][gz] = (bas(i, 0) * q[b] + bas(i, 1) * q[b + 1]) + bas(i, 2) * q[b + 2];
-      }
+    for (int b = 0; b < 3; b++) X[a][b] = ADD ? X[a][b] + q[a][b] : q[a][b];
+}
+// F[p][q] = integral of sum X[a][b] t1^a t2^b against b_p(t1) b_q(t2), b = 1/2 -+ t.
+__device__ __forceinline__ void bilinear_moments(const double (&X)[3][3], double (&F)[2][2]) {
+  double C[2][3];
 #pragma unroll
-  for (int i = 0; i < 2; i++)
+  for (int b = 0; b < 3; b++) {
+    const double e = .5 * fma(X[2][b], 1. / 12., X[0][b]), o = X[1][b] * (1. / 12.);
+    C[0][b] = e - o;
+    C[1][b] = e + o;
+  }
 #pragma unroll
-    for (int j = 0; j < 2; j++)
+  for (int p = 0; p < 2; p++) {
+    const double e = .5 * fma(C[p][2], 1. / 12., C[p][0]), o = C[p][1] * (1. / 12.);
+    F[p][0] = e - o;
+    F[p][1] = e + o;
+  }
+}
+// F[p][q]: the product of two fields (modal) integrated over axis d and against the basis along
+// the other two.
+__device__ __forceinline__ void product_face(const double (&f)[8], const double (&g)[8], int d, double (&F)[2][2]) {
+  double a[4], b[4], X[3][3];
+  transverse<0>(f, d, a);
+  transverse<0>(g, d, b);
+  bilinear_product<false>(a, b, X);
+  transverse<1>(f, d, a);
+  transverse<1>(g, d, b);
 #pragma unroll
-      for (int gz = 0; gz < 3; gz++)
-        cy[i][j][gz] = (bas(j, 0) * cx[i][0][gz] + bas(j, 1) * cx[i][1][gz]) + bas(j, 2) * cx[i][2][gz];
-#pragma unroll
-  for (int k = 0; k < 2; k++)
-#pragma unroll
-    for (int j = 0; j < 2; j++)
-#pragma unroll
-      for (int i = 0; i < 2; i++)
-        out[i + 2 * j + 4 * k] =
-            (bas(k, 0) * cy[i][j][0] + bas(k, 1) * cy[i][j][1]) + bas(k, 2) * cy[i][j][2];
+  for (int q = 0; q < 4; q++) b[q] *= 1. / 12.;
+  bilinear_product<true>(a, b, X);
+  bilinear_moments(X, F);
 }
 
 // Integrals of q against the squared or plain basis products that carry no factor
@@ -273,10 +297,10 @@ struct UDiagCell {
 
 // The U load in tensor form (plain operator): the thermo-poro load
 // sum_g w dphi_a,c S_g, S = 3 kappa alpha (theta - thetaRef)(v^2 + eta) + beta p v, as
-// face moments of w S times -+1/h_c, and the crack-pressure load
-// sum_g w p grad_c v phi_a as a full contraction.
-// The crack-pressure term of an element with 8 equal nodal v (and finite p) is 0 and not
-// evaluated: grad v is exactly 0 there.
+// face moments of w S times -+1/h_c (the beta term in closed form, the thermal one point by point
+// and only where theta differs from thetaRef at a node), and the crack-pressure load
+// sum_g w p grad_c v phi_a in closed form.  The crack-pressure term of an element with 8 equal
+// nodal v (and finite p) is 0 and not evaluated: grad v is exactly 0 there.
 struct URhsCell {
   static constexpr int NF = 3, NV = 3, MINB = 1;
   const double *__restrict__ v, *__restrict__ theta, *__restrict__ thetaRef, *__restrict__ p;
@@ -296,11 +320,16 @@ struct URhsCell {
     const CellMat m = cell_mat(E, ei, ej, ek);
     const double coefalpha = (3. * m.lambda + 2. * m.mu) * m.alpha, beta = m.beta;
     const double vol = E.hx * E.hy * E.hz;
-    double ve[27], pe[27], ws[27];
-    interp27(v8, ve);
-    interp27(p8, pe);
-    {
-      double te[27];
+    const double ih[3] = {1. / E.hx, 1. / E.hy, 1. / E.hz};
+    double vm[8], pm[8], F[3][2][2];
+    modal_of(v8, vm);
+    modal_of(p8, pm);
+    bool thermal = false;
+#pragma unroll
+    for (int a = 0; a < 8; a++) thermal = thermal || !(th8[a] == 0.);
+    if (thermal) {
+      double ve[27], ws[27], te[27];
+      interp27(v8, ve);
       interp27(th8, te);
 #pragma unroll
       for (int gz = 0; gz < 3; gz++)
@@ -309,13 +338,22 @@ struct URhsCell {
 #pragma unroll
           for (int gx = 0; gx < 3; gx++) {
             const int g = gx + 3 * gy + 9 * gz;
-            const double s = coefalpha * te[g] * (ve[g] * ve[g] + E.eta) + beta * pe[g] * ve[g];
-            ws[g] = (vol * (w1(gx) * w1(gy) * w1(gz))) * s;
+            ws[g] = (vol * (w1(gx) * w1(gy) * w1(gz))) * (coefalpha * te[g] * (ve[g] * ve[g] + E.eta));
           }
+      face_moments<false>(ws, F);
+    } else {
+#pragma unroll
+      for (int d = 0; d < 3; d++) F[d][0][0] = F[d][0][1] = F[d][1][0] = F[d][1][1] = 0.;
     }
-    double F[3][2][2];
-    face_moments<false>(ws, F);
-    const double ih[3] = {1. / E.hx, 1. / E.hy, 1. / E.hz};
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      double G[2][2];
+      product_face(pm, vm, d, G);
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+#pragma unroll
+        for (int k = 0; k < 2; k++) F[d][j][k] = fma(vol * beta, G[j][k], F[d][j][k]);
+    }
 #pragma unroll
     for (int k = 0; k < 2; k++)
 #pragma unroll
@@ -335,41 +373,28 @@ struct URhsCell {
       ps += fabs(p8[a]);
     }
     if (E.hasCrackPressure && !(flat && ps - ps == 0.)) {
-      // grad v at the points: each component depends on the two other axes only
-      double gv[3][9];  // gv[d][a + 3 b], (a, b) the other axes' point indices
-#pragma unroll
-      for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = 0; b < 3; b++) {
-          double sx = 0., sy = 0., sz = 0.;
-#pragma unroll
-          for (int q = 0; q < 2; q++)
-#pragma unroll
-            for (int r = 0; r < 2; r++) {
-              sx += bas(q, a) * bas(r, b) * (v8[1 + 2 * q + 4 * r] - v8[2 * q + 4 * r]);
-              sy += bas(q, a) * bas(r, b) * (v8[q + 2 + 4 * r] - v8[q + 4 * r]);
-              sz += bas(q, a) * bas(r, b) * (v8[q + 2 * r + 4] - v8[q + 2 * r]);
-            }
-          gv[0][a + 3 * b] = sx * ih[0];
-          gv[1][a + 3 * b] = sy * ih[1];
-          gv[2][a + 3 * b] = sz * ih[2];
-        }
+      // d_c v has no power of t_c: transverse products with p at powers 0 and 1 of t_c
 #pragma unroll
       for (int c = 0; c < 3; c++) {
-        double qc[27], oc[8];
+        double g[4], q[4], X[3][3], F0[2][2], F1[2][2];
+        transverse<1>(vm, c, g);
+        transverse<0>(pm, c, q);
+        bilinear_product<false>(q, g, X);
+        bilinear_moments(X, F0);
+        transverse<1>(pm, c, q);
+        bilinear_product<false>(q, g, X);
+        bilinear_moments(X, F1);
+        const double w = vol * ih[c];
 #pragma unroll
-        for (int gz = 0; gz < 3; gz++)
+        for (int k = 0; k < 2; k++)
 #pragma unroll
-          for (int gy = 0; gy < 3; gy++)
+          for (int j = 0; j < 2; j++)
 #pragma unroll
-            for (int gx = 0; gx < 3; gx++) {
-              const int g = gx + 3 * gy + 9 * gz;
-              const double gvc = c == 0 ? gv[0][gy + 3 * gz] : (c == 1 ? gv[1][gx + 3 * gz] : gv[2][gx + 3 * gy]);
-              qc[g] = (vol * (w1(gx) * w1(gy) * w1(gz))) * pe[g] * gvc;
+            for (int i = 0; i < 2; i++) {
+              const int t = c == 0 ? i : (c == 1 ? j : k), p = c == 0 ? j : i, r = c == 2 ? j : k;
+              const double m = fma(t ? 1. / 12. : -1. / 12., F1[p][r], .5 * F0[p][r]);
+              rl[i + 2 * j + 4 * k][c] = fma(w, m, rl[i + 2 * j + 4 * k][c]);
             }
-        contract27(qc, oc);
-#pragma unroll
-        for (int a = 0; a < 8; a++) rl[a][c] += oc[a];
       }
     }
   }
@@ -701,9 +726,9 @@ __global__ void __launch_bounds__(256, 1) v_assemble_kernel(const __grid_constan
 
 // V load (VF_ResidualVAT1/AT23D_local and VF_ResidualVCrackPressure3D_local,
 // VFMech.c:2294-2384) in tensor form: the AT term coef sum_g w phi_a = coef vol / 8 per
-// node, the crack-pressure term sum_g w p (u . grad phi_a) as face moments of w p u_c.
+// node, the crack-pressure term sum_g w p (u . grad phi_a) as face moments of p u_c in closed form.
 struct VRhsCell {
-  static constexpr int NF = 4, NV = 1, MINB = 1;
+  static constexpr int NF = 4, NV = 1, MINB = 2;
   const double *__restrict__ u, *__restrict__ p;
   double* __restrict__ b;
   bool pressure;  // p given and crack pressure on
@@ -721,32 +746,24 @@ struct VRhsCell {
 #pragma unroll
     for (int a = 0; a < 8; a++) out[a][0] = coef * vol * 0.125;
     if (pressure) {
-      double pe[27];
-      interp27(fld[3], pe);
+      double pm[8];
+      modal_of(fld[3], pm);
       const double ih[3] = {1. / E.hx, 1. / E.hy, 1. / E.hz};
 #pragma unroll
       for (int c = 0; c < 3; c++) {
-        double q[27], F[3][2][2];
-        interp27(fld[c], q);
-#pragma unroll
-        for (int gz = 0; gz < 3; gz++)
-#pragma unroll
-          for (int gy = 0; gy < 3; gy++)
-#pragma unroll
-            for (int gx = 0; gx < 3; gx++) {
-              const int g = gx + 3 * gy + 9 * gz;
-              q[g] = (vol * (w1(gx) * w1(gy) * w1(gz))) * pe[g] * q[g];
-            }
-        face_moments<false>(q, F);
+        double um[8], F[2][2];
+        modal_of(fld[c], um);
+        product_face(pm, um, c, F);
+        const double w = vol * ih[c];
 #pragma unroll
         for (int k = 0; k < 2; k++)
 #pragma unroll
           for (int j = 0; j < 2; j++)
 #pragma unroll
             for (int i = 0; i < 2; i++) {
-              const int sgn = c == 0 ? i : (c == 1 ? j : k);
-              const double fm = c == 0 ? F[0][j][k] : (c == 1 ? F[1][i][k] : F[2][i][j]);
-              out[i + 2 * j + 4 * k][0] += (sgn ? ih[c] : -ih[c]) * fm;
+              const int t = c == 0 ? i : (c == 1 ? j : k);
+              const double m = F[c == 0 ? j : i][c == 2 ? j : k];
+              out[i + 2 * j + 4 * k][0] = fma(t ? w : -w, m, out[i + 2 * j + 4 * k][0]);
             }
       }
     }
@@ -759,9 +776,10 @@ struct VRhsCell {
 // shared memory (two buffers, one barrier per layer) and over z in registers, so every node is
 // written once, in one fixed order.  The cells on the seams of the blocks are computed
 // twice.  8 launches of a parity colour each read and wrote the result 8 times, a cache line
-// for every second node: at 129^3 U load 466 us, diagonal 234, V load 215; now 275, 118 and 214
-// (bound by FP64 issue, V's at one block of 8 warps per SM); 65^3 74 -> 80, 47 -> 27, 50 -> 45; the
-// diagonals of the coarse levels 47 -> 6 to 9.
+// for every second node: at 129^3 U load 466 us, diagonal 234, V load 215; now 206, 118 and 125
+// (a chain of loads, element and exchange per layer at 8 or 16 warps per SM; fetching a plane
+// further ahead changed nothing); 65^3 74 -> 54, 47 -> 27, 50 -> 30; the diagonals of the coarse
+// levels 47 -> 6 to 9.
 constexpr int CG_NX = 31, CG_NY = 7;
 template <class C>
 __global__ void __launch_bounds__(256, C::MINB)
