@@ -313,11 +313,11 @@ def run_gpu(args):
     nodes, cells = ctx.N, (n - 1) ** 3
     # algorithmic traffic per apply: read u (24 B) + v (8 B), write y (24 B) per node
     alg_bytes = 56.0 * nodes
-    # FP64 instructions per element of the apply on this workload (nearly every element
-    # has a constant nodal phase field and takes the fixed-weight element), counted by ncu
-    # (smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on / cells, the
-    # fixed-weight launch of this workload under ncu --set full); an FMA is 2 flops
-    dfma_el, dadd_el, dmul_el = 44.1, 163.7, 25.6
+    # FP64 instructions per element of the apply on this workload (nearly every node lies in
+    # a homogeneous patch and takes the stencil), counted by ncu
+    # (smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on / cells, the stencil
+    # launch of this workload); an FMA is 2 flops
+    dfma_el, dadd_el, dmul_el = 31.1, 62.1, 13.1
     instr_el = dfma_el + dadd_el + dmul_el
     flops_el = 2 * dfma_el + dadd_el + dmul_el
     f64_peak = fp_peak_tflops(torch, "f64")
@@ -339,20 +339,18 @@ def run_gpu(args):
                    "parallelism": f"replicas x{world}", "l2": "flushed between timed steps"},
         "e2e": {"value": round(N3 * world / (e2e_ms * 1e-3) / 1e9, 3), "unit": "GDOF/s",
                 "h2d_bytes_per_step": N3 * 8, "d2h_bytes_per_step": N3 * 8},
-        "gpu_launches": 3 * args.steps,  # per apply: the two unit-list waves and the seam fix-up
+        "gpu_launches": 3 * args.steps,  # per apply: stencil, element tiles, faces and seams
         "roofline": {"bound": "hbm", "achieved": round(alg_bytes / (ms64 * 1e-3) / 1e9, 1),
                      "peak": hbm, "unit": "GB/s",
                      "frac": round(alg_bytes / (ms64 * 1e-3) / 1e9 / hbm, 4),
-                     "traffic": 108.7e6 if n == N_EDGE else None,
+                     "traffic": 61.0e6 if n == N_EDGE else None,
                      "note": "achieved: algorithmic bytes over the whole apply (three launches: "
-                             "the fixed-weight wave over the intact (tile, plane) units, the "
-                             "general wave over the rest, the seam fix-up); traffic: ncu dram "
-                             "read+write of the fixed-weight launch at 129^3 (84.3 + 24.4 MB; "
-                             "part of the output is still in the 126 MB L2 when it ends).  The "
-                             "kernel is bound by neither HBM nor the FP64 pipe "
-                             "(compute_roofline) but by the latency of its tile schedule "
-                             "(ncu: 16 warps per SM, issue active 54 %, FP64 pipe 34 %, top "
-                             "stalls fixed-latency dependencies)"},
+                             "the stencil over the homogeneous nodes, the element tiles over the "
+                             "(tile, plane) units with others, the faces with the tiles' seams); "
+                             "traffic: ncu dram read+write of the stencil launch at 129^3 (55.7 + 5.3 "
+                             "MB: most of the output is still in the 126 MB L2 when it ends).  The "
+                             "stencil is bound by latency at 8 warps per SM (ncu: issue active "
+                             "47 %, FP64 pipe 46 %, top stall fixed-latency dependencies)"},
         "compute_roofline": {
             "pipe": "fp64 CUDA cores",
             "fp64_instructions_per_element": {"dfma": dfma_el, "dadd": dadd_el, "dmul": dmul_el},

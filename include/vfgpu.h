@@ -165,7 +165,9 @@ int vfgpu_set_unilateral(vfgpu_ctx* ctx, int type);
  * elements all have a constant nodal phase field on a kernel with the fixed-weight element
  * alone, the rest on the general one; OFF: one wave over all units; AUTO (the default):
  * ON from a grid size per precision where it measured faster.  Grids with more than 2048
- * 32 x 8 element tiles per plane and NOCOMPRESSION always take one wave. */
+ * 32 x 8 element tiles per plane and NOCOMPRESSION always take one wave.  Grids whose applies
+ * run in two phases (small ones) or, with one material, on the stencil (large ones) have no
+ * such choice. */
 #define VFGPU_U_SPLIT_AUTO 0
 #define VFGPU_U_SPLIT_OFF 1
 #define VFGPU_U_SPLIT_ON 2

@@ -30,10 +30,6 @@
 //   flags, xin[NC]) (the same from flags loaded ahead and the node's inputs from the
 //   plane ring), and an
 //   optional A.skip flag that turns a launch into a no-op (set by a converged CG,
-//   so that a queued batch of iterations costs nothing once it is done), LIST:
-//   -1, or the unit list (A.ur, A.ustart, A.utotal) the operator's launches take when
-//   the list is given -- the U operator's units split by phase field over two
-//   optional A.skip flag that turns a launch into a no-op (set by a converged CG,
 //   so that a queued batch of iterations costs nothing once it is done), and LIST:
 //   -1, or the unit list (A.ur, A.ustart, A.utotal) the operator's launches take when
 //   the list is given -- the U operator's units split by phase field over two
