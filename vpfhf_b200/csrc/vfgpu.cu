@@ -562,7 +562,8 @@ cudaError_t pipe_resources(vfgpu_ctx* c) {
 // y = K x with x and y in host memory (FP64), as a pipeline over z-slabs of node planes:
 // slab s's planes go up on s_in, the slab with one halo plane on each side is applied
 // as a sub-grid on the ctx stream (same xy tiles and per-node sum order as the whole-grid
-// apply, so its interior planes carry the same bits; the halo planes' values are
+// element operator, so its interior planes carry that operator's bits (the device-buffer
+// apply's, where that does not take the stencil; there to rounding); the halo planes' values are
 // discarded), and its interior planes come back on s_out while later slabs are still
 // going up, so that both copy directions and the compute overlap.  Slabs alternate
 // between two output staging vectors, because a slab's apply also writes its halo
