@@ -5,9 +5,12 @@
 // the other at 8 warps per SM, so the apply is a chain of element latencies whatever the size.
 // Here one thread computes one element and leaves its 24 nodal values in scratch (one array
 // per value, so that loads and stores are coalesced), and a second launch sums the up to 8
-// values of each node component, in the tile engine's order inside a tile: the elements left
-// and right, then the rows, then the layers.  The price is 48 values per element through L2,
-// which is why large grids keep the tiles.
+// values of each node component in the tile engine's order: inside a tile the elements left
+// and right, then the rows, then the layers; on a seam of the tiles each tile's share that way,
+// then the shares.  So an apply has the same bits on either path, and the entry points that
+// take tiles where a ctx takes two phases (the fixed-scratch apply, launches without
+// scratch) agree with it bit for bit.  The price is 48 values per element through L2, which is
+// why large grids keep the tiles.
 #pragma once
 
 #include "ops.cuh"
@@ -52,7 +55,7 @@ __global__ void __launch_bounds__(TP_THREADS, sizeof(typename Op::T) == 8 ? 2 : 
 
 template <class Op, bool DOT>
 __global__ void __launch_bounds__(TP_NODE_THREADS)
-    u_node_sum_kernel(const __grid_constant__ typename Op::Args A) {
+    u_node_sum_kernel(const __grid_constant__ typename Op::Args A, int TY) {
   using T = typename Op::T;
   __shared__ double red[32];
   if (A.skip && *A.skip) return;
@@ -72,16 +75,30 @@ __global__ void __launch_bounds__(TP_NODE_THREADS)
 #pragma unroll
       for (int c = 0; c < 3; c++) e[a][c] = in ? A.scr[(a * 3 + c) * st + q] : T(0);
     }
+    // tile seams (seam_range in tile_engine.cuh)
+    const bool sx = i % 32 == 0 && i > 0 && i / 32 < A.ntx, sy = j % TY == 0 && j > 0 && j / TY < A.nty;
     T val[3], xin[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      T p[2];  // layer below (corners 4..7), above
-#pragma unroll
-      for (int z = 0; z < 2; z++) {
-        const int b = z ? 0 : 4;
-        p[z] = ((e[b + 3][c] + e[b + 2][c])) + (e[b + 1][c] + e[b][c]);
+      // e[a]: corners 0..3 of the layer above, 4..7 of the one below; odd a: the element to the
+      // left, a & 2: the row before
+      T l, r;
+      if (sx && sy) {  // four tiles: row before left, right, row after left, right
+        l = (e[7][c] + e[3][c]) + (e[6][c] + e[2][c]);
+        val[c] = (l + (e[5][c] + e[1][c])) + (e[4][c] + e[0][c]);
+      } else {
+        if (sx) {  // left and right tile
+          l = (e[7][c] + e[5][c]) + (e[3][c] + e[1][c]);
+          r = (e[6][c] + e[4][c]) + (e[2][c] + e[0][c]);
+        } else if (sy) {  // tiles of the row before and after
+          l = (e[7][c] + e[6][c]) + (e[3][c] + e[2][c]);
+          r = (e[5][c] + e[4][c]) + (e[1][c] + e[0][c]);
+        } else {  // layer below and above
+          l = (e[7][c] + e[6][c]) + (e[5][c] + e[4][c]);
+          r = (e[3][c] + e[2][c]) + (e[1][c] + e[0][c]);
+        }
+        val[c] = l + r;
       }
-      val[c] = p[0] + p[1];
       xin[c] = (DOT || ((fl >> c) & 1u)) ? A.x[3 * (int64_t)n + c] : T(0);
     }
     dacc += Op::template finish_node_in<DOT>(A, n, val, fl, xin);
@@ -92,13 +109,15 @@ __global__ void __launch_bounds__(TP_NODE_THREADS)
   }
 }
 
-// Both launches; with A.dot, twophase_node_blocks partials of x.y.
+// Both launches; with A.dot, twophase_node_blocks partials of x.y.  p: the grid's tiles.
 template <class Op>
-cudaError_t launch_u_twophase(const typename Op::Args& A, const LayerTable& L, cudaStream_t s) {
+cudaError_t launch_u_twophase(typename Op::Args A, const TilePlan& p, const LayerTable& L, cudaStream_t s) {
+  A.ntx = p.ntx;
+  A.nty = p.nty;
   const int ncell = (A.nx - 1) * (A.ny - 1) * (A.nz - 1), nb = twophase_node_blocks(A.nx, A.ny, A.nz);
   u_element_kernel<Op><<<(ncell + TP_THREADS - 1) / TP_THREADS, TP_THREADS, 0, s>>>(A, L);
-  if (A.dot) u_node_sum_kernel<Op, true><<<nb, TP_NODE_THREADS, 0, s>>>(A);
-  else u_node_sum_kernel<Op, false><<<nb, TP_NODE_THREADS, 0, s>>>(A);
+  if (A.dot) u_node_sum_kernel<Op, true><<<nb, TP_NODE_THREADS, 0, s>>>(A, p.ty);
+  else u_node_sum_kernel<Op, false><<<nb, TP_NODE_THREADS, 0, s>>>(A, p.ty);
   return cudaGetLastError();
 }
 
