@@ -164,10 +164,11 @@ int vfgpu_set_unilateral(vfgpu_ctx* ctx, int type);
  * choice with bit-identical results).  ON: two waves -- the (tile, plane) units whose
  * elements all have a constant nodal phase field on a kernel with the fixed-weight element
  * alone, the rest on the general one; OFF: one wave over all units; AUTO (the default):
+ * two phases (every element, then every node) on small grids, on larger ones one wave, and
  * ON from a grid size per precision where it measured faster.  Grids with more than 2048
- * 32 x 8 element tiles per plane and NOCOMPRESSION always take one wave.  Grids whose applies
- * run in two phases (small ones) or, with one material, on the stencil (large ones) have no
- * such choice. */
+ * 32 x 8 element tiles per plane and NOCOMPRESSION always take one wave (or, in AUTO, two
+ * phases).  Large grids of one material run their homogeneous nodes on a stencil whatever the
+ * mode. */
 #define VFGPU_U_SPLIT_AUTO 0
 #define VFGPU_U_SPLIT_OFF 1
 #define VFGPU_U_SPLIT_ON 2

@@ -52,7 +52,8 @@ cudaError_t u_lists_refresh(vfgpu_ctx* c);
 // Whether the ctx's U applies in this precision (8 or 4 bytes) take the unit lists (and
 // write the second wave's x.y partials).
 bool u_lists_on(const vfgpu_ctx* c, int prec_bytes);
-// Whether the ctx's U applies in this precision run in two phases.
+// Whether the ctx's U applies in this precision run in two phases (split mode AUTO, and the
+// scratch is there).
 bool u_twophase_on(const vfgpu_ctx* c, int prec_bytes);
 // Makes the two-phase scratch hold one apply of this grid in this precision, if such applies
 // run in two phases (a grown one invalidates captured graphs).

@@ -668,6 +668,7 @@ template <typename T> struct LevelT {
   const T* dinv;
   const uint32_t* cflag;  // fine level under NOCOMPRESSION: the Jacobian's bits
   vfgpu::UnitLists ul;    // fine level: the ctx's unit lists of its plan (else none)
+  bool two;               // applies in two phases
   T *x, *b, *r, *d, *t;
   double* coef;
   int64_t n3;
@@ -708,6 +709,7 @@ template <typename T> LevelT<T> view(vfgpu_ctx* c, int l) {
     V.dinv = (const T*)c->mg_dinv0;
     V.cflag = c->unilateral ? c->d_cflag : nullptr;
     V.ul = u_lists_of(c, (int)sizeof(T));
+    V.two = u_twophase_on(c, (int)sizeof(T));
     V.n3 = 3 * c->N;
   } else {
     V.nx = L.nx;
@@ -725,6 +727,8 @@ template <typename T> LevelT<T> view(vfgpu_ctx* c, int l) {
     V.dinv = (const T*)L.dinv;
     V.cflag = nullptr;
     V.ul = UnitLists{};
+    V.two = twophase_pays(L.nx, L.ny, L.nz, (int)sizeof(T)) &&
+            c->escr_bytes >= twophase_scratch(L.nx, L.ny, L.nz) * sizeof(T);
     V.n3 = 3 * L.N;
   }
   return V;
@@ -754,7 +758,7 @@ template <typename T> UApplyArgs<T> level_args(vfgpu_ctx* c, const LevelT<T>& V,
   A.P = c->d_params;
   A.cflag = V.cflag;
   use_unit_lists(A, V.ul);
-  A.scr = twophase_pays(V.nx, V.ny, V.nz, (int)sizeof(T)) ? static_cast<T*>(c->d_escr) : nullptr;
+  A.scr = V.two ? static_cast<T*>(c->d_escr) : nullptr;
   return A;
 }
 
@@ -1067,6 +1071,7 @@ int mgcg(vfgpu_ctx* c, const double* b, double* x, double* r, double* p, double*
   outer.cellE = c->d_cellE;
   outer.cflag = c->unilateral ? c->d_cflag : nullptr;
   outer.ul = u_lists_of(c, 8);
+  outer.two = u_twophase_on(c, 8);
   // one iteration (cg.cuh), in a while node of a graph: no host round trip until the end
   auto body = [&](const cudaGraphConditionalHandle* loop) {
     cudaError_t eb = vcycle<T>(c, 0, f32 ? V.b : (const T*)(const void*)r, V.x);

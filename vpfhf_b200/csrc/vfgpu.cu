@@ -148,7 +148,10 @@ UApplyArgs<T> u_args(vfgpu_ctx* c, const T* x, const T* v, T* y, T* seam, const 
   A.scr = u_twophase_on(c, (int)sizeof(T)) ? static_cast<T*>(c->d_escr) : nullptr;
   return A;
 }
-bool u_twophase_on(const vfgpu_ctx* c, int prec_bytes) { return twophase_pays(c->nx, c->ny, c->nz, prec_bytes); }
+bool u_twophase_on(const vfgpu_ctx* c, int prec_bytes) {
+  return c->u_split == VFGPU_U_SPLIT_AUTO && twophase_pays(c->nx, c->ny, c->nz, prec_bytes) &&
+         c->escr_bytes >= twophase_scratch(c->nx, c->ny, c->nz) * prec_bytes;
+}
 
 cudaError_t ensure_escr(vfgpu_ctx* c, int nx, int ny, int nz, int prec_bytes) {
   if (!twophase_pays(nx, ny, nz, prec_bytes)) return cudaSuccess;
