@@ -362,15 +362,16 @@ int vfgpu_server_destroy(vfgpu_server* s);
  * bit c set = component c of the node is Dirichlet; may be NULL) are device
  * arrays of the current device, the work is queued on `stream` (a
  * cudaStream_t, NULL = legacy default stream) and the call returns without
- * waiting.  The only scratch (the seam partial sums) is a fixed 32 MiB array
- * inside the library (VFGPU_NOALLOC_SCRATCH_DOUBLES doubles; every GPU that
+ * waiting.  The only scratch (the seam partial sums, or on small grids with seams the
+ * element values of a two-phase apply) is a fixed 32 MiB array inside the library (VFGPU_NOALLOC_SCRATCH_DOUBLES doubles; every GPU that
  * loads the library holds it until exit); grids whose seams need more are
  * rejected with VFGPU_ERR_INVALID (129^3 fits, 161^3 does not), and so are x and y
  * that overlap (the apply is out of place).  Every call looks up the array's device
  * address in the current context (cudaGetSymbolAddress, host-side) and, on the first
  * call on a device, opts the kernels in to their shared memory: make that first call
  * before any stream capture.  All calls share the one array, so calls whose work
- * overlaps on the GPU (different streams, different threads) race; serialise them.
+ * overlaps on the GPU (different streams, different threads) race; serialise them --
+ * except on grids of one 32 x 8 element tile (nx <= 33, ny <= 9), which use none of it.
  * Every scratch slot read is written earlier in the same call, so no clearing is
  * needed between calls. */
 #define VFGPU_NOALLOC_SCRATCH_DOUBLES 4194304

@@ -145,3 +145,30 @@ def test_two_phases_and_tiles_have_the_same_bits(cuda, n):
         assert torch.equal(_noalloc(torch, n, l, torch.from_numpy(v).cuda(), bits, xd), y)
         assert np.array_equal(ctx.u_apply(x, vg.FP64), y.cpu().numpy())
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [(33, 9, 60), (9, 8, 300), (2, 2, 2)])
+def test_one_tile_noalloc_calls_may_overlap(cuda, n):
+    """Grids of one tile use nothing of the fixed scratch: calls on four streams at once, on
+    different vectors, each give the bits they give alone."""
+    from vpfhf_b200 import _abi
+    torch = cuda
+    L, N = _abi.lib(), n[0] * n[1] * n[2]
+    rng = np.random.default_rng(3)
+    l = tuple(0.125 * (k - 1) for k in n)
+    v = torch.from_numpy(rng.uniform(0, 1, N)).cuda()
+    bits = torch.from_numpy(rng.integers(0, 8, N).astype(np.uint8)).cuda()
+    xs = [torch.from_numpy(rng.standard_normal(3 * N)).cuda() for _ in range(4)]
+    alone = [_noalloc(torch, n, l, v, bits, x) for x in xs]
+    g, mp = _abi.Grid(*n, *l), _abi.MatProp(1e10, 0.25, 0.0, 0.0, 1.0)
+    streams = [torch.cuda.Stream() for _ in xs]
+    ys = [[torch.full_like(x, float("nan")) for _ in range(50)] for x in xs]
+    torch.cuda.synchronize()
+    for k in range(50):
+        for s, x, y in zip(streams, xs, ys):
+            rc = L.vfgpu_u_apply_noalloc(C.byref(g), C.byref(mp), 1e-8, v.data_ptr(), bits.data_ptr(), x.data_ptr(),
+                                         y[k].data_ptr(), s.cuda_stream)
+            assert rc == 0, L.vfgpu_last_error().decode()
+    torch.cuda.synchronize()
+    for y, a in zip(ys, alone):
+        assert all(torch.equal(q, a) for q in y)

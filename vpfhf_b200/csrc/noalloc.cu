@@ -6,9 +6,10 @@
 // that cannot afford cudaMalloc's implicit device-wide synchronisation.  Such a
 // caller cannot create a vfgpu_ctx (vfgpu_create allocates the fields and work
 // space), so this entry point takes every array from the caller and keeps its
-// only scratch -- the seam partial sums of the tiled apply -- in one fixed,
-// file-scope device array.  That array is part of the loaded module: every GPU
-// that loads the library holds its 32 MiB until the process exits.
+// only scratch in one fixed, file-scope device array: the seam partial sums of the
+// tiled apply or, on small grids with seams whose 24 values per element fit it, those
+// of the two-phase apply (the same bits).  That array is part of the loaded
+// module: every GPU that loads the library holds its 32 MiB until the process exits.
 #include <cstring>
 
 #include "abi_util.h"
@@ -18,7 +19,7 @@ namespace {
 
 constexpr size_t kScratchDoubles = VFGPU_NOALLOC_SCRATCH_DOUBLES;
 
-// Seam partials of the last call; every slot the fix-up kernel reads is written
+// Seam partials or element values of the last call; every slot that is read is written
 // earlier in the same call, so nothing has to be cleared between calls.
 static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 
@@ -94,7 +95,10 @@ extern "C" int vfgpu_u_apply_noalloc(const vfgpu_grid* g, const vfgpu_matprop* m
   A.ihz = 1.0 / hz;
   A.vol = hx * hy * hz;
   A.eta = eta;
-  if (twophase_pays(g->nx, g->ny, g->nz, 8) && twophase_scratch(g->nx, g->ny, g->nz) <= kScratchDoubles)
+  // a grid of one tile has no seams and takes the tiles, which touch no scratch there: calls on
+  // such grids may overlap
+  if (p.seamX + p.seamY > 0 && twophase_pays(g->nx, g->ny, g->nz, 8) &&
+      twophase_scratch(g->nx, g->ny, g->nz) <= kScratchDoubles)
     A.scr = scratch;
   e = launch_u_apply<double>(A, p, L, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "vfgpu_u_apply_noalloc");
