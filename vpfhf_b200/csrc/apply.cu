@@ -559,9 +559,9 @@ template <>
 cudaError_t launch_u_apply<double>(const UApplyArgs<double>& A, const TilePlan& p,
                                    const LayerTable& L, cudaStream_t s) {
   if (A.scr) {
-    if (A.cflag) return launch_u_twophase<UOpNC<double>>(A, p, L, s);
-    if (cubic(A)) return launch_u_twophase<UOp<double, true>>(A, p, L, s);
-    return launch_u_twophase<UOp<double>>(A, p, L, s);
+    if (A.cflag) return launch_u_twophase<UOpNC<double>, U64_TY>(A, L, s);
+    if (cubic(A)) return launch_u_twophase<UOp<double, true>, U64_TY>(A, L, s);
+    return launch_u_twophase<UOp<double>, U64_TY>(A, L, s);
   }
   if (A.cflag) return launch_tile_apply<UOpNC<double>, U64_TY, 1>(A, p, L, s);
   if (A.node) {
@@ -581,9 +581,9 @@ template <>
 cudaError_t launch_u_apply<float>(const UApplyArgs<float>& A, const TilePlan& p,
                                   const LayerTable& L, cudaStream_t s) {
   if (A.scr) {
-    if (A.cflag) return launch_u_twophase<UOpNC<float>>(A, p, L, s);
-    if (cubic(A)) return launch_u_twophase<UOp<float, true>>(A, p, L, s);
-    return launch_u_twophase<UOp<float>>(A, p, L, s);
+    if (A.cflag) return launch_u_twophase<UOpNC<float>, U_TY>(A, L, s);
+    if (cubic(A)) return launch_u_twophase<UOp<float, true>, U32_TY>(A, L, s);
+    return launch_u_twophase<UOp<float>, U32_TY>(A, L, s);
   }
   // NOCOMPRESSION needs the scalar layout: its plan is the FP32 plan only with the
   // scalar tile (the packed build option keeps the plain operator packed)

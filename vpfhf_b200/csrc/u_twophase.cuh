@@ -53,9 +53,9 @@ __global__ void __launch_bounds__(TP_THREADS, sizeof(typename Op::T) == 8 ? 2 : 
     for (int c = 0; c < 3; c++) A.scr[(a * 3 + c) * st + cell] = out[a][c];
 }
 
-template <class Op, bool DOT>
+template <class Op, int TY, bool DOT>
 __global__ void __launch_bounds__(TP_NODE_THREADS)
-    u_node_sum_kernel(const __grid_constant__ typename Op::Args A, int TY) {
+    u_node_sum_kernel(const __grid_constant__ typename Op::Args A) {
   using T = typename Op::T;
   __shared__ double red[32];
   if (A.skip && *A.skip) return;
@@ -75,31 +75,27 @@ __global__ void __launch_bounds__(TP_NODE_THREADS)
 #pragma unroll
       for (int c = 0; c < 3; c++) e[a][c] = in ? A.scr[(a * 3 + c) * st + q] : T(0);
     }
-    // tile seams (seam_range in tile_engine.cuh)
-    const bool sx = i % 32 == 0 && i > 0 && i / 32 < A.ntx, sy = j % TY == 0 && j > 0 && j / TY < A.nty;
+    // e[a]: corners 0..3 of the layer above, 4..7 of the one below; odd a: the element to the left,
+    // a & 2: the row before
     T val[3], xin[3];
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      // e[a]: corners 0..3 of the layer above, 4..7 of the one below; odd a: the element to the
-      // left, a & 2: the row before
-      T l, r;
-      if (sx && sy) {  // four tiles: row before left, right, row after left, right
-        l = (e[7][c] + e[3][c]) + (e[6][c] + e[2][c]);
-        val[c] = (l + (e[5][c] + e[1][c])) + (e[4][c] + e[0][c]);
-      } else {
-        if (sx) {  // left and right tile
-          l = (e[7][c] + e[5][c]) + (e[3][c] + e[1][c]);
-          r = (e[6][c] + e[4][c]) + (e[2][c] + e[0][c]);
-        } else if (sy) {  // tiles of the row before and after
-          l = (e[7][c] + e[6][c]) + (e[3][c] + e[2][c]);
-          r = (e[5][c] + e[4][c]) + (e[1][c] + e[0][c]);
-        } else {  // layer below and above
-          l = (e[7][c] + e[6][c]) + (e[5][c] + e[4][c]);
-          r = (e[3][c] + e[2][c]) + (e[1][c] + e[0][c]);
-        }
-        val[c] = l + r;
-      }
+    for (int c = 0; c < 3; c++) {  // layer below and above
+      val[c] = ((e[7][c] + e[6][c]) + (e[5][c] + e[4][c])) + ((e[3][c] + e[2][c]) + (e[1][c] + e[0][c]));
       xin[c] = (DOT || ((fl >> c) & 1u)) ? A.x[3 * (int64_t)n + c] : T(0);
+    }
+    // tile seams (seam_range in tile_engine.cuh)
+    const bool sx = i % 32 == 0 && i > 0 && i < nx - 1, sy = j % TY == 0 && j > 0 && j < ny - 1;
+    if (sx || sy) {
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        // the four columns of elements, both layers of each
+        if (sx && sy)
+          val[c] = (((e[7][c] + e[3][c]) + (e[6][c] + e[2][c])) + (e[5][c] + e[1][c])) + (e[4][c] + e[0][c]);
+        else if (sx)  // left and right tile
+          val[c] = ((e[7][c] + e[5][c]) + (e[3][c] + e[1][c])) + ((e[6][c] + e[4][c]) + (e[2][c] + e[0][c]));
+        else  // tiles of the rows before and after
+          val[c] = ((e[7][c] + e[6][c]) + (e[3][c] + e[2][c])) + ((e[5][c] + e[4][c]) + (e[1][c] + e[0][c]));
+      }
     }
     dacc += Op::template finish_node_in<DOT>(A, n, val, fl, xin);
   }
@@ -109,15 +105,14 @@ __global__ void __launch_bounds__(TP_NODE_THREADS)
   }
 }
 
-// Both launches; with A.dot, twophase_node_blocks partials of x.y.  p: the grid's tiles.
-template <class Op>
-cudaError_t launch_u_twophase(typename Op::Args A, const TilePlan& p, const LayerTable& L, cudaStream_t s) {
-  A.ntx = p.ntx;
-  A.nty = p.nty;
+// Both launches; with A.dot, twophase_node_blocks partials of x.y.  TY: element rows of the
+// operator's tiles.
+template <class Op, int TY>
+cudaError_t launch_u_twophase(const typename Op::Args& A, const LayerTable& L, cudaStream_t s) {
   const int ncell = (A.nx - 1) * (A.ny - 1) * (A.nz - 1), nb = twophase_node_blocks(A.nx, A.ny, A.nz);
   u_element_kernel<Op><<<(ncell + TP_THREADS - 1) / TP_THREADS, TP_THREADS, 0, s>>>(A, L);
-  if (A.dot) u_node_sum_kernel<Op, true><<<nb, TP_NODE_THREADS, 0, s>>>(A, p.ty);
-  else u_node_sum_kernel<Op, false><<<nb, TP_NODE_THREADS, 0, s>>>(A, p.ty);
+  if (A.dot) u_node_sum_kernel<Op, TY, true><<<nb, TP_NODE_THREADS, 0, s>>>(A);
+  else u_node_sum_kernel<Op, TY, false><<<nb, TP_NODE_THREADS, 0, s>>>(A);
   return cudaGetLastError();
 }
 
