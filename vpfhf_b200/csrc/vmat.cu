@@ -15,22 +15,26 @@ constexpr int VM_BLOCKS = 592;
 // together, so that the 13 couplings a node shares with the nodes behind it (the planes just
 // read) come from L1 and L2 and HBM sees each coupling once.  A masked node costs its mask
 // byte: where the bounds are active (most of the grid in an AT1 problem) whole warps leave
-// at once.  Indices are linear: a neighbour beyond an x or y face lands on the next row's or
-// plane's node, whose coupling (or whose own) in that direction is 0; only the first and last
-// nodes of the array need the range checked (CHECK).
+// at once.  On the faces of the box (FACE) the neighbours that do not exist are left out by
+// their coordinates, not by their zero couplings: in memory order the node one past a row's end
+// is the next row's first, and 0 times a value that is not finite there would reach this row.
 // Measured at 129^3 inside the AT1 penny crack's StepV (few nodes free): 7.9 us a launch in
 // FP64 and 4.4 us in FP32, where the element form with its staged coefficients took 63.5 + 4.5
 // (seams) and 33.7 + 2.8 us (averages over a solve's launches, finished ones included); with
 // every node free 97 us in FP64 (element form 96 + 8.7).
-template <typename T, bool CHECK>
-__device__ __forceinline__ T vmat_row(const VMatArgs<T>& A, int64_t n, int64_t N, int64_t st) {
+template <typename T, bool FACE>
+__device__ __forceinline__ T vmat_row(const VMatArgs<T>& A, int64_t n, int i, int j, int k, int64_t st) {
   const int64_t row = A.nx, pl = (int64_t)A.nx * A.ny;
+  // whether the neighbour one step along -, 0, + of an axis exists
+  const bool ex[3] = {i > 0, true, i < A.nx - 1}, ey[3] = {j > 0, true, j < A.ny - 1},
+             ez[3] = {k > 0, true, k < A.nz - 1};
   T r = A.a[n] * A.x[n];
 #pragma unroll
   for (int d = 1; d < kVCouplings; d++) {
-    const int64_t o = kVForward[d][0] + kVForward[d][1] * row + kVForward[d][2] * pl;
-    if (!CHECK || n + o < N) r = fma(A.a[d * st + n], A.x[n + o], r);
-    if (!CHECK || n - o >= 0) r = fma(A.a[d * st + n - o], A.x[n - o], r);
+    const int dx = kVForward[d][0], dy = kVForward[d][1], dz = kVForward[d][2];
+    const int64_t o = dx + dy * row + dz * pl;
+    if (!FACE || (ex[1 + dx] && ey[1 + dy] && ez[1 + dz])) r = fma(A.a[d * st + n], A.x[n + o], r);
+    if (!FACE || (ex[1 - dx] && ey[1 - dy] && ez[1 - dz])) r = fma(A.a[d * st + n - o], A.x[n - o], r);
   }
   return r;
 }
@@ -40,12 +44,16 @@ __global__ void __launch_bounds__(VM_THREADS, 4) vmat_apply_kernel(const __grid_
   __shared__ double red[32];
   if (A.skip && *A.skip) return;  // converged solve
   const int64_t N = (int64_t)A.nx * A.ny * A.nz, st = vmat_stride(N);
-  const int64_t reach = (int64_t)A.nx * A.ny + A.nx + 1;
+  const unsigned nx = A.nx, ny = A.ny;
   double acc = 0.;
   for (int64_t n = (int64_t)blockIdx.x * VM_THREADS + threadIdx.x; n < N; n += (int64_t)gridDim.x * VM_THREADS) {
     T y = T(0);
     if (!(A.mask && A.mask[n])) {
-      y = n >= reach && n + reach < N ? vmat_row<T, false>(A, n, N, st) : vmat_row<T, true>(A, n, N, st);
+      // (N < 2^32: 14 couplings of 2^32 nodes do not fit a device)
+      const unsigned m = (unsigned)n, rows = m / nx;
+      const int i = (int)(m - rows * nx), k = (int)(rows / ny), j = (int)(rows - (unsigned)k * ny);
+      const bool face = i == 0 || i == A.nx - 1 || j == 0 || j == A.ny - 1 || k == 0 || k == A.nz - 1;
+      y = face ? vmat_row<T, true>(A, n, i, j, k, st) : vmat_row<T, false>(A, n, i, j, k, st);
       if constexpr (DOT) acc += (double)A.x[n] * (double)y;
     }
     A.y[n] = y;
