@@ -27,3 +27,43 @@ def test_values_that_are_not_finite_stay_with_their_neighbours(cuda, n, bad):
         assert np.isfinite(F[~near]).all()
         assert not np.isfinite(F[at[2], at[1], at[0]])
     ctx.close()
+
+
+def test_smooth_v_keeps_the_accuracy_of_differences(cuda):
+    """K_V v for a smooth v without strain (AT1: the stiffness part alone) against extended
+    precision.  The rows are differences of neighbours: of the order of sum |a_ij| times the
+    largest difference d between a node and its neighbours, not times v itself.  30 roundings
+    (27 products, their sum) of 2^-53 of that, and four of the load subtracted from it; plain
+    products would leave about 3 roundings of sum |a_ij| max v, a hundred times as much."""
+    import vpfhf_b200 as vg
+    n, h = (40, 33, 36), 1.0 / 32
+    Gc, eps = 100.0, 20.0 / 32
+    l = tuple(h * (k - 1) for k in n)
+    ctx = vg.VFContext(n, l, dict(E=1e10, nu=0.25, Gc=Gc), epsilon=eps, eta=1e-6, atnum=1)
+    ctx.set_bc(vg.rollers())
+    Z, Y, X = np.meshgrid(*(np.arange(k) * h for k in n[::-1]), indexing="ij")
+    v = 0.7 + 0.2 * np.sin(0.8 * X) * np.cos(0.5 * Y + 0.3 * Z)
+    ctx.set_field("V", np.zeros(ctx.N))
+    F0 = ctx.v_residual().reshape(v.shape)  # minus the load
+    ctx.set_field("V", v.reshape(-1))
+    F = ctx.v_residual().reshape(v.shape)
+    ctx.close()
+    ld = np.longdouble
+    aeps, hl = ld(Gc) / (ld(2) / 3) / 2 * ld(eps), ld(h)
+
+    def along(f, axis, mass):
+        f = np.moveaxis(f, axis, -1)
+        d = f[..., 1:] - f[..., :-1]
+        out = np.zeros_like(f)
+        if mass:  # h (f_i / 2 + d / 6) from each element
+            out[..., :-1] += hl * (f[..., :-1] / 2 + d / 6)
+            out[..., 1:] += hl * (f[..., 1:] / 2 - d / 6)
+        else:
+            out[..., :-1] -= d / hl
+            out[..., 1:] += d / hl
+        return np.moveaxis(out, -1, axis)
+    K = sum(along(along(along(v.astype(ld), 0, q != 0), 1, q != 1), 2, q != 2) for q in range(3))
+    err = np.abs(F.astype(ld) - (aeps * K + F0.astype(ld)))
+    d = max(np.abs(np.diff(v, axis=a)).max() for a in range(3)) * 3
+    suma = float(aeps * hl) * 16 / 3  # of a cube's 27 couplings
+    assert err.max() <= 2.0 ** -53 * (30 * suma * d + 4 * np.abs(F0).max())

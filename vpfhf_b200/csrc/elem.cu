@@ -522,11 +522,12 @@ __global__ void bc_diag_kernel(const uint8_t* __restrict__ bcbits, double* __res
 // 3-point sums.  Products of two 1-D basis functions are 1/4 - t + t^2 (both at the low
 // node), 1/4 - t^2 (one each) and 1/4 + t + t^2 (both high), so the cell's element matrix has
 // 27 distinct entries, one per product type and axis, built by sum factorisation; the
-// stiffness part (Gc / 2 c_w) eps grad . grad is a constant per type.  NOCOMPRESSION
+// stiffness part (Gc / 2 c_w) eps grad . grad is a constant per type.  A corner's row sum R is
+// the sum of the mass part over the 8 types it is in (the stiffness part's row sums are 0).  NOCOMPRESSION
 // (VFMech.c:115-218, 2125-2153) evaluates the row's three points instead (sign per point).
 __device__ __forceinline__ void v_cell_types(const ElemArgs& E, const CellMat& mat,
                                              const double (&m)[3][8], const double (&mth)[8],
-                                             double (&M)[27]) {
+                                             double (&M)[27], double (&R)[8]) {
   const double ih[3] = {1. / E.hx, 1. / E.hy, 1. / E.hz};
   const double vol = E.hx * E.hy * E.hz;
   const double mass = E.atnum == 2 ? mat.Gc / E.atcv * .5 / E.epsilon : 0.;
@@ -606,6 +607,17 @@ __device__ __forceinline__ void v_cell_types(const ElemArgs& E, const CellMat& m
         for (int x = 0; x < 3; x++)
           M[x + 3 * py + 9 * pz] = fma(w1(gz) * bb(pz, gz), cxy[py][x], M[x + 3 * py + 9 * pz]);
   }
+  double Rx[2][9], Ry[4][3];  // a corner low or high along an axis is in two of its three types
+#pragma unroll
+  for (int q = 0; q < 9; q++)
+#pragma unroll
+    for (int i = 0; i < 2; i++) Rx[i][q] = M[3 * q + i] + M[3 * q + i + 1];
+#pragma unroll
+  for (int pz = 0; pz < 3; pz++)
+#pragma unroll
+    for (int a = 0; a < 4; a++) Ry[a][pz] = Rx[a & 1][3 * pz + (a >> 1)] + Rx[a & 1][3 * pz + (a >> 1) + 1];
+#pragma unroll
+  for (int a = 0; a < 8; a++) R[a] = vol * (Ry[a & 3][a >> 2] + Ry[a & 3][(a >> 2) + 1]);
   const double kx = mat.Gc / E.atcv * .5 * E.epsilon * vol;
   const double ix = kx * ih[0] * ih[0], iy = kx * ih[1] * ih[1], iz = kx * ih[2] * ih[2];
   constexpr double st[3] = {1., -1., 1.}, ms[3] = {1. / 3., 1. / 6., 1. / 3.};
@@ -636,7 +648,7 @@ __global__ void __launch_bounds__(256, 1) v_assemble_kernel(const __grid_constan
                                                             double* __restrict__ a64,
                                                             float* __restrict__ a32, int64_t stride, int gx,
                                                             int zc) {
-  extern __shared__ double vm_s[];  // [27][8][32]
+  extern __shared__ double vm_s[];  // [27 + 8][8][32]
   const int l = threadIdx.x, w = threadIdx.y;
   const int nx = E.nx, ny = E.ny, nz = E.nz;
   const int ex = (int)(blockIdx.x % gx) * VM_NX - 1 + l, ey = (int)(blockIdx.x / gx) * VM_NY - 1 + w;
@@ -645,9 +657,9 @@ __global__ void __launch_bounds__(256, 1) v_assemble_kernel(const __grid_constan
   const int z0 = blockIdx.y * zc, z1 = min(z0 + zc, nz);
   const int64_t plane = (int64_t)nx * ny;
   const int64_t base = cell ? (int64_t)ey * nx + ex : 0;
-  double f[3][8], th8[8], carry[5];
+  double f[3][8], th8[8], carry[6];  // of the couplings within the plane, and of the row sum
 #pragma unroll
-  for (int q = 0; q < 5; q++) carry[q] = 0.;
+  for (int q = 0; q < 6; q++) carry[q] = 0.;
   auto load4 = [&](int k) {
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -669,19 +681,23 @@ __global__ void __launch_bounds__(256, 1) v_assemble_kernel(const __grid_constan
         th8[j] = th8[4 + j];
       }
       load4(k + 1);
-      double M[27];
+      double M[27], R[8];
       if (cell) {
         double m[3][8], mth[8];
 #pragma unroll
         for (int c = 0; c < 3; c++) modal_of(f[c], m[c]);
         modal_of(th8, mth);
-        v_cell_types(E, cell_mat(E, ex, ey, k), m, mth, M);
+        v_cell_types(E, cell_mat(E, ex, ey, k), m, mth, M, R);
       } else {
 #pragma unroll
         for (int t = 0; t < 27; t++) M[t] = 0.;
+#pragma unroll
+        for (int a = 0; a < 8; a++) R[a] = 0.;
       }
 #pragma unroll
       for (int t = 0; t < 27; t++) s[t * 256] = M[t];
+#pragma unroll
+      for (int a = 0; a < 8; a++) s[(27 + a) * 256] = R[a];
     }
     __syncthreads();
     if (node) {
@@ -702,6 +718,11 @@ __global__ void __launch_bounds__(256, 1) v_assemble_kernel(const __grid_constan
         }
         return r;
       };
+      // the row sum's share of the 4 cells in which the node is low (0) or high (1) in z
+      auto gather_sum = [&](int hz) {
+        return (s[(27 + 3 + 4 * hz) * 256 - 33] + s[(27 + 2 + 4 * hz) * 256 - 32]) +
+               (s[(27 + 1 + 4 * hz) * 256 - 1] + s[(27 + 4 * hz) * 256]);
+      };
       const bool layer = k < nz - 1;
       if (k >= z0) {
         const int64_t n = (int64_t)k * plane + (int64_t)ey * nx + ex;
@@ -715,10 +736,13 @@ __global__ void __launch_bounds__(256, 1) v_assemble_kernel(const __grid_constan
 #pragma unroll
         for (int q = 5; q < kVCouplings; q++)
           put(q, layer ? gather(kVForward[q][0], kVForward[q][1], 1) : 0.);
+        put(kVRowSum, carry[5] + (layer ? gather_sum(0) : 0.));
       }
-      if (layer)
+      if (layer) {
 #pragma unroll
         for (int q = 0; q < 5; q++) carry[q] = gather(kVForward[q][0], kVForward[q][1], 2);
+        carry[5] = gather_sum(1);
+      }
     }
     __syncthreads();  // the next layer rewrites the entries
   }
@@ -1300,7 +1324,7 @@ cudaError_t launch_u_diag(const ElemArgs& E, const double* v, const uint8_t* bcb
 
 cudaError_t launch_v_assemble(const ElemArgs& E, const double* u, const double* theta,
                               const double* thetaRef, double* a64, float* a32, cudaStream_t s) {
-  constexpr size_t smem = 27 * 256 * sizeof(double);
+  constexpr size_t smem = (27 + 8) * 256 * sizeof(double);
   cudaError_t e = cudaFuncSetAttribute(v_assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int gx = ceil_div(E.nx, VM_NX), gy = ceil_div(E.ny, VM_NY);

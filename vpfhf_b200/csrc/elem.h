@@ -38,8 +38,8 @@ cudaError_t launch_u_diag(const ElemArgs& E, const double* v, const uint8_t* bcb
                           cudaStream_t s, const double* u0 = nullptr);
 // NOCOMPRESSION sign pattern: flags[cell] bit g = (tr(eps(u)) < 0 at Gauss point g).
 cudaError_t launch_nc_flags(const ElemArgs& E, const double* u, uint32_t* flags, cudaStream_t s);
-// The V operator's couplings (vmat.h) at u, in FP64 and, if a32 is not null, FP32; the
-// first array is the operator's diagonal.
+// The V operator's couplings and row sums (vmat.h) at u, in FP64 and, if a32 is not null, FP32;
+// the first array is the operator's diagonal.
 cudaError_t launch_v_assemble(const ElemArgs& E, const double* u, const double* theta,
                               const double* thetaRef, double* a64, float* a32, cudaStream_t s);
 // b (N) = AT linear term + crack pressure term (VFMech.c:2294-2384).  Overwrites b.

@@ -44,7 +44,7 @@ static int solve_buffers(vfgpu_ctx* c) {
     if (e == cudaSuccess) e = cudaMalloc((void**)&p, n3 * sizeof(double));
   for (auto& p : c->p32)
     if (e == cudaSuccess) e = cudaMalloc((void**)&p, n3 * sizeof(float));
-  const size_t ncoef = (size_t)kVCouplings * vmat_stride(c->N);
+  const size_t ncoef = (size_t)kVArrays * vmat_stride(c->N);
   if (e == cudaSuccess) e = cudaMalloc((void**)&c->vmat64, ncoef * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc((void**)&c->vmat32, ncoef * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc((void**)&c->vmask, (size_t)c->N);
@@ -814,7 +814,7 @@ int vfgpu_memory_estimate(const vfgpu_grid* g, long long* bytes) {
   b += (long long)(p64.seamX + p64.seamY) * 8 + (long long)(p32.seamX + p32.seamY) * 4;
   b += 3 * 3 * N * 8 + 2 * 3 * N * 4;                    // staging vectors
   b += vfgpu_ctx::NP64 * (3 * N + kPoolSlack) * 8 + vfgpu_ctx::NP32 * (3 * N + kPoolSlack) * 4;
-  b += kVCouplings * (long long)vmat_stride(N) * 12 + N;  // V couplings (FP64 + FP32), mask
+  b += kVArrays * (long long)vmat_stride(N) * 12 + N;    // V couplings (FP64 + FP32), mask
   b += (RED_BLOCKS + energy_blocks()) * 4 * 8 + 4096;    // reductions, scalars
   *bytes = b;
   return VFGPU_OK;
