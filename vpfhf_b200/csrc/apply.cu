@@ -80,7 +80,10 @@ template <typename T, int MINB> cudaError_t set_stencil_attributes();
 #define VFGPU_ST32_MINB 3
 #endif
 constexpr int ST64_MINB = VFGPU_ST64_MINB, ST32_MINB = VFGPU_ST32_MINB;
-// Smallest grids, in (tile, plane) units, whose homogeneous nodes take the stencil.
+// Smallest grids, in (tile, plane) units, whose homogeneous nodes take the stencil.  Per apply, two
+// cracks, tiles split by phase field against stencil, us: FP64 75^3 (2250 units) 46.2 / 46.5,
+// 81^3 (2430) 52.4 / 48.3, 70 x 70 x 128 (3456) 65.3 / 59.3, 97^3 (3492) 61.2 / 50.4, 129^3 (8256)
+// 108 / 63; FP32 113^3 (6328) 65.7 / 61.8, 129^3 76 / 55 (below 6000 the FP32 tiles run one wave).
 #ifndef VFGPU_ST64_MIN_UNITS
 #define VFGPU_ST64_MIN_UNITS 2000
 #endif
@@ -479,7 +482,7 @@ cudaError_t build_stencil_lists(uint8_t* node, int2* range, int nx, int ny, int 
 // Largest grids, in cells, whose applies run in two phases.  Per apply, two cracks, tiles (with
 // the stencil where it is taken) against two phases, us AT1 / AT2: FP64 17^3 16.4 / 14.4 and
 // 9.3 / 9.3 (of which about 8 are the call), 41^3 22.6 / 21.6 and 14.4 / 14.7, 65^3 36.9 / 34.9
-// and 28.7 / 34.2, 81^3 47.0 / 71.7 and 59.3 / 69.7, 97^3 46.8 / 93.2 and 95.7 / 112.8; FP32 41^3
+// and 28.7 / 34.2, 81^3 48.3 / 71.7 and 59.3 / 69.7, 97^3 50.4 / 93.2 and 95.7 / 112.8; FP32 41^3
 // 18.5 / 20.5 and 11.3 / 11.3, 65^3 24.6 / 27.9 and 18.5 / 23.8, 81^3 42.0 / 48.5 and 28.7 / 39.0,
 // 97^3 52.3 / 65.0 and 53.6 / 70.9; 97 x 61 x 83 (tiles that fit) - / 31.6 and - / 33.2.
 #ifndef VFGPU_TWOPHASE64_CELLS

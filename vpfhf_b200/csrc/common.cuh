@@ -26,30 +26,30 @@ struct LayerTable {
 };
 
 // Coefficients of the U operator's separable stencil (u_stencil.cuh) at spacing (h0, h1, h2)
-// for the axes (0, 1, 2): P, Q, R of the rows and, for a node on a face across axis 1, the
-// terms of the half that is missing.
+// for the axes (0, 1, 2), rounded once: of 6 P, 36 Q and 36 R from sums over 6 m and 36 m m.
 struct StencilCoefs {
   double xx, xy, yx, yy, xd, q, qz, rx, ry;
   double g;               // R's multiple on the lowest plane
-  double em, el, fl, fm;  // face: of P_0, P_1; of R_1, R_2
+  double em, el, fl, fm;  // a face across axis 1, its missing half: of P_0, P_1; of R_1, R_2
 };
-inline StencilCoefs stencil_coefs(double lam, double mu, double h0, double h1, double h2) {
-  const double l2 = lam + 2. * mu, lm = lam + mu, a0 = h1 * h2 / h0, a1 = h0 * h2 / h1, a2 = h0 * h1 / h2;
+inline StencilCoefs stencil_coefs(double lambda, double mu_, double d0, double d1, double d2) {
+  const long double lam = lambda, mu = mu_, h0 = d0, h1 = d1, h2 = d2, l2 = lam + 2 * mu, lm = lam + mu;
+  const long double a0 = h1 * h2 / h0, a1 = h0 * h2 / h1, a2 = h0 * h1 / h2;
   StencilCoefs c;
-  c.xx = -l2 * a0;
-  c.xy = -mu * a1;
-  c.yx = -mu * a0;
-  c.yy = -l2 * a1;
-  c.xd = -lm * .25 * h2;
-  c.q = -mu * a2;
-  c.qz = -l2 * a2;
-  c.rx = -lm * .25 * h1;
-  c.ry = -lm * .25 * h0;
-  c.g = (mu - lam) / lm;
-  c.em = mu * .5 * h2;
-  c.el = lam * .5 * h2;
-  c.fl = lam * .5 * h0;
-  c.fm = mu * .5 * h0;
+  c.xx = (double)(-l2 * a0);
+  c.xy = (double)(-mu * a1);
+  c.yx = (double)(-mu * a0);
+  c.yy = (double)(-l2 * a1);
+  c.xd = (double)(-1.5L * lm * h2);
+  c.q = (double)(-mu * a2);
+  c.qz = (double)(-l2 * a2);
+  c.rx = (double)(-1.5L * lm * h1);
+  c.ry = (double)(-1.5L * lm * h0);
+  c.g = (double)((mu - lam) / lm);
+  c.em = (double)(3 * mu * h2);
+  c.el = (double)(3 * lam * h2);
+  c.fl = (double)(3 * lam * h0);
+  c.fm = (double)(3 * mu * h0);
   return c;
 }
 

@@ -14,18 +14,33 @@
 //   Q_z = -(lam + 2 mu) (hx hy / hz) m_x m_y u_z,
 //   R_z = -(lam + mu) ((hy / 4) d_x m_y u_x + (hx / 4) m_x d_y u_y):
 // what the element sums give there (the 3-point Gauss rule is exact for these degrees), in
-// about 95 operations per node against 234 per element plus the exchange and summation of
-// its 24 nodal values.  Every difference is taken before it is averaged, as in the
-// element's modal form.
+// about 115 operations per node against 234 per element plus the exchange and summation of
+// its 24 nodal values.
+//
+// Rounding.  K(v) maps a constant to 0, so every sum is of values less the node's own: e = d2_x u and the
+// second difference u2 across y (differences of neighbours) give 6 d2_y m_x u = 6 u2 + d2_y e and
+// G = 36 (m_x m_y u - u) = 6 e + 6 d2_y m_x u; from plane to plane the own value moves by du, of
+// which G takes 36.  Averages of full-size values would cancel for smooth u.  In FP64 the own value is
+// taken without its low bits, which G gets back, so that du is exact (its rounding would be the
+// largest of all for random u).  The 36 is left to S, which is held in two parts: one factor for all
+// rows, whose rounding does not average out; then the coefficients are the rows' own.  P +- R are formed
+// before the larger q G.  Passes in the vectors' type, rows in FP64 in both types: in FP32 alone the rows'
+// chain of sums rounds random u more than the element sums do (7.4e-8).  Normwise error of one apply,
+// element form / averages of u in the vectors' type / this form, x random and smooth (about a wave per box):
+// FP32 129^3 5.5 / 6.6 / 5.1 and 1690 / 3320 / 20 in 1e-8; FP64 86 x 87 x 88 cubic cells 2.0 / 2.9 / 1.3
+// and 160 / 293 / 8.4 in 1e-16, cells of 47 x 36 x 25 1.33 / 1.39 / 1.32.  Time of an apply in a loop
+// (two cracks), same order: FP32 129^3 76 / 44 / 55 us, 161^3 136 / 68 / 93, 257 x 257 x 129 279 / 115 /
+// 168; FP64 129^3 108 / 55 / 63, 97^3 60 / 47 / 51.  With FP32's passes in FP64 too (2.5e-8, the
+// rounding of the result alone) 57.5, 97 and 176 us.
 //
 // Columns inside the box in x and y: a block owns 32 x 16 of them and marches up a chunk of
 // planes, 4 rows of one column per thread.  Planes of 34 x 18 nodes stream through a 5-slot
 // shared-memory ring by asynchronous copies three planes ahead, one barrier per plane; a
-// thread makes the x-passes of the 6 rows its 4 outputs need (13.5 shared reads per node) and
+// thread makes the x-passes of the 6 rows its 4 outputs need (16.5 shared reads per node) and
 // keeps per row what planes k - 1 and k give to node k, so nothing is exchanged between
 // threads and no seam is summed.  127 = 4 x 32 - 1 = 8 x 16 - 1: the inside of the 2^k + 1 grids
 // fills the tiles.  On the lowest and highest plane M is h (f / 2 + (f' - f) / 6), K is
-// (f - f') / h, C = (f' - f) / 2 and T = -C -+ f: the node keeps P / 3 - Q and a multiple of R.
+// (f - f') / h, C = (f' - f) / 2 and T = -C -+ f: the node keeps 2 P - Q and a multiple of R.
 // x and y faces (their edges aside): runs of 4 nodes up a column, 30 columns per warp, with the
 // one-sided operators across the face; an x face is a y face with x and y exchanged.  The
 // box's 12 edges: 9 lanes per node from the 27 neighbours and the 1-D coefficients.  Both
@@ -40,6 +55,7 @@ namespace vfgpu {
 
 constexpr int ST_ROW = 3 * (ST_X + 2), ST_PLANE = ST_ROW * (ST_Y + 2), ST_RING = 5;
 template <typename T> constexpr size_t stencil_smem() { return sizeof(T) * ST_RING * ST_PLANE; }
+using StencilReal = double;  // the arithmetic of the rows (the passes are in the vectors' type)
 
 // 1-D operators of node i of n at spacing h: coefficients at i - 1, i, i + 1.
 template <typename T> struct Axis1D {
@@ -62,31 +78,33 @@ template <typename T> struct Axis1D {
 };
 
 // The share of node (i, j, k)'s rows (without S) that the three neighbours i - 1 .. i + 1 of
-// row j + b - 1, plane k + c - 1 give, for any node of the box (used on its edges).
-template <typename T>
-__device__ __forceinline__ void stencil_edge_row(const UApplyArgs<T>& A, int i, int j, int k, int b, int c, T lam,
-                                                 T mu, T hx, T hy, T hz, T (&y)[3]) {
-  const Axis1D<T> X(i, A.nx, hx), Y(j, A.ny, hy), Z(k, A.nz, hz);
-  const T l2 = lam + T(2) * mu;
+// row j + b - 1, plane k + c - 1 give, as values less the node's own, for any node of the box
+// (used on its edges).
+template <typename T, typename W>
+__device__ __forceinline__ void stencil_edge_row(const UApplyArgs<T>& A, int i, int j, int k, int b, int c, W lam,
+                                                 W mu, W hx, W hy, W hz, W (&y)[3]) {
+  const Axis1D<W> X(i, A.nx, hx), Y(j, A.ny, hy), Z(k, A.nz, hz);
+  const W l2 = lam + W(2) * mu;
   const int kk = min(max(k + c - 1, 0), A.nz - 1), jj = min(max(j + b - 1, 0), A.ny - 1);  // beyond: weight 0
-  T M[3], K[3], C[3], D[3];
+  const T* own = A.x + 3 * node_index(i, j, k, A.nx, A.ny);
+  W M[3], K[3], C[3], D[3];
 #pragma unroll
-  for (int q = 0; q < 3; q++) M[q] = K[q] = C[q] = D[q] = T(0);
+  for (int q = 0; q < 3; q++) M[q] = K[q] = C[q] = D[q] = W(0);
 #pragma unroll
   for (int a = 0; a < 3; a++) {
     const T* u = A.x + 3 * node_index(min(max(i + a - 1, 0), A.nx - 1), jj, kk, A.nx, A.ny);
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-      const T v = __ldg(u + q);
+      const W v = W(__ldg(u + q)) - W(__ldg(own + q));
       M[q] = fma(X.M[a], v, M[q]);
       K[q] = fma(X.K[a], v, K[q]);
       C[q] = fma(X.C[a], v, C[q]);
       D[q] = fma(X.D[a], v, D[q]);
     }
   }
-  auto at = [](const T (&f)[3], int q) { return q == 0 ? f[0] : q == 1 ? f[1] : f[2]; };
-  const T My = at(Y.M, b), Ky = at(Y.K, b), Cy = at(Y.C, b), Dy = at(Y.D, b);
-  const T Mz = at(Z.M, c), Kz = at(Z.K, c), Cz = at(Z.C, c), Dz = at(Z.D, c);
+  auto at = [](const W (&f)[3], int q) { return q == 0 ? f[0] : q == 1 ? f[1] : f[2]; };
+  const W My = at(Y.M, b), Ky = at(Y.K, b), Cy = at(Y.C, b), Dy = at(Y.D, b);
+  const W Mz = at(Z.M, c), Kz = at(Z.K, c), Cz = at(Z.C, c), Dz = at(Z.D, c);
   y[0] = Mz * (l2 * (K[0] * My) + mu * (M[0] * Ky) + lam * (D[1] * Cy) + mu * (C[1] * Dy)) +
          Kz * (mu * (M[0] * My)) + My * (lam * (D[2] * Cz) + mu * (C[2] * Dz));
   y[1] = Mz * (mu * (K[1] * My) + l2 * (M[1] * Ky) + lam * (C[0] * Dy) + mu * (D[0] * Cy)) +
@@ -95,49 +113,49 @@ __device__ __forceinline__ void stencil_edge_row(const UApplyArgs<T>& A, int i, 
          My * (lam * (C[0] * Dz) + mu * (D[0] * Cz)) + M[1] * (lam * (Cy * Dz) + mu * (Dy * Cz));
 }
 
-// StencilCoefs in the kernel's type (rounded once each).
-template <typename T> struct StencilCoef {
-  T xx, xy, yx, yy, xd, q, qz, rx, ry, g;
-  __device__ __forceinline__ explicit StencilCoef(const StencilCoefs& c)
-      : xx(T(c.xx)), xy(T(c.xy)), yx(T(c.yx)), yy(T(c.yy)), xd(T(c.xd)), q(T(c.q)), qz(T(c.qz)), rx(T(c.rx)),
-        ry(T(c.ry)), g(T(c.g)) {}
+// u without its low 32 bits (FP64): the difference of two of them near one another is exact.  FP32 as it is.
+__device__ __forceinline__ double stencil_high(double u) { return __hiloint2double(__double2hiint(u), 0); }
+__device__ __forceinline__ float stencil_high(float u) { return u; }
+
+// Takes in plane k of a row: fin = its share of node k - 1, whose rest acc holds; then acc = what planes
+// k - 1 and k give to node k, up = what plane k gives to node k + 1.  P is 6 times, q G and R 36 times
+// the rows' P, Q, R; G and R of the values less the plane's own reference, which changes by du from plane k - 1
+// (M: G's multiple of a constant; on a FACE R changes by f dr).
+template <int M, bool FACE, typename W>
+__device__ __forceinline__ void stencil_march(W P, W q, W G, W R, W du, W f, W dr, W& acc, W& up, W& rest, W& fin) {
+  rest = acc;
+  fin = fma(q, fma(W(M), du, G), P + (FACE ? fma(f, dr, R) : R));
+  acc = fma(W(4), P, fma(W(-2) * q, fma(W(M / 2), du, G), FACE ? fma(f, dr, up) : up));
+  up = fma(q, G, P - R);
+}
+
+// v^2 + eta, or its 36th, as a rounded value and the rest: one factor for every row of a homogeneous
+// patch, so its rounding would not average out.
+struct StencilScale {
+  double hi, lo;
+  __device__ __forceinline__ StencilScale(double v, double eta, bool over36) {
+    const double s = fma(v, v, eta), b = s - eta, r = fma(v, v, -b) + (eta - (s - b));
+    hi = s;
+    lo = r;
+    if (over36) {
+      const double c = 1.0 / 36.0, q = s * c;
+      hi = fma(fma(-36., q, s), c, q);
+      lo = (fma(-36., hi, s) + r) * c;
+    }
+  }
 };
 
-// Takes in plane k's P, Q, R of a row: fin = node k - 1, then acc = what planes k - 1 and k give
-// to node k, up = what plane k gives to node k + 1.
-template <typename T>
-__device__ __forceinline__ void stencil_march(const T (&P)[3], const T (&Q)[3], const T (&R)[3], T (&acc)[3],
-                                              T (&up)[3], T (&fin)[3]) {
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    const T t = fma(P[c], T(1.0 / 6.0), Q[c]);
-    fin[c] = acc[c] + (t + R[c]);
-    acc[c] = fma(T(2.0 / 3.0), P[c], fma(T(-2), Q[c], up[c]));
-    up[c] = t - R[c];
-  }
-}
-// acc on the lowest (g) or highest (-g) plane, from the rows' P, Q, R and what the plane below
-// gave (0 on the lowest).
-template <typename T>
-__device__ __forceinline__ void stencil_end(const T (&P)[3], const T (&Q)[3], const T (&R)[3], T g,
-                                            const T (&below)[3], T (&acc)[3]) {
-#pragma unroll
-  for (int c = 0; c < 3; c++) acc[c] = below[c] + fma(c < 2 ? g : -g, R[c], fma(P[c], T(1.0 / 3.0), -Q[c]));
-}
-
-// Writes a finished node from its rows (without S), flags and x; with DOT returns its x.y.
-// S1 = 1 + eta.
-template <typename T, bool DOT>
-__device__ __forceinline__ double stencil_put(const UApplyArgs<T>& A, T S1, T eta, int64_t n, unsigned f,
-                                              const T (&r)[3], const T* xin) {
-  T S = S1;
-  if (!(f & kNodeOne)) {
-    const T v = A.v[n];
-    S = fma(v, v, eta);
-  }
+// Writes a node from the two parts of its rows (without S; 36 times them where OVER36), flags and x; with
+// DOT returns its x.y.  S1: the scale at v = 1.
+template <typename T, bool DOT, bool OVER36, typename W>
+__device__ __forceinline__ double stencil_put(const UApplyArgs<T>& A, const StencilScale& S1, double eta, int64_t n, unsigned f,
+                                              const W (&r)[3], const W (&r2)[3], const T* xin) {
+  StencilScale S = S1;
+  if (!(f & kNodeOne)) S = StencilScale(A.v[n], eta, OVER36);
   T y[3];
 #pragma unroll
-  for (int c = 0; c < 3; c++) y[c] = S * r[c];
+  for (int c = 0; c < 3; c++)
+    y[c] = T(fma(S.hi, r[c], sizeof(T) == 8 ? fma(S.lo, r[c] + r2[c], S.hi * r2[c]) : S.hi * r2[c]));
   if (f & 7u)
 #pragma unroll
     for (int c = 0; c < 3; c++)
@@ -167,11 +185,11 @@ __global__ void __launch_bounds__(ST_THREADS, MINB)
     if (DOT && tid == 0) A.dot[blockIdx.x] = 0.;
     return;
   }
-  const T eta = T(A.P->eta);
+  using W = StencilReal;
+  const double eta = A.P->eta;
+  const StencilScale S1(1., eta, true);
   const int64_t plane = (int64_t)nx * ny;
-  const T sixth = T(1.0 / 6.0), S1 = T(1) + eta;
   double dacc = 0.;
-  auto put = [&](int64_t n, unsigned f, const T (&r)[3], const T* xin) { dacc += stencil_put<T, DOT>(A, S1, eta, n, f, r, xin); };
   const int bx = b % p.ntx, by = (b / p.ntx) % p.nty;
   const int X0 = bx * ST_X, Y0 = by * ST_Y;  // the halo corner: first inner column X0 + 1
   const int ka = zr.x, kb = zr.y;                       // planes [ka, kb) are written,
@@ -203,21 +221,22 @@ __global__ void __launch_bounds__(ST_THREADS, MINB)
     fs = fs == ST_RING - 1 ? 0 : fs + 1;
     cp_async_commit();  // also when empty: the waits count groups
   };
-  const StencilCoef<T> C(A.P->st[0]);
+  const StencilCoefs C = A.P->st[0];
+  const T rx = T(C.rx), ry = T(C.ry);
   const int i = X0 + 1 + lane, j0 = Y0 + 1 + wy * ST_RY;
   // rows of this thread whose nodes lie inside the x and y faces
   const int rows = i < nx - 1 ? min(max(ny - 1 - j0, 0), ST_RY) : 0;
   int64_t nk = (int64_t)j0 * nx + i + kf * plane;  // node of row 0 in plane k
-  T acc[ST_RY][3], up[ST_RY][3];
+  W acc[ST_RY][3], up[ST_RY][3];
 #pragma unroll
   for (int r = 0; r < ST_RY; r++)
 #pragma unroll
-    for (int c = 0; c < 3; c++) acc[r][c] = up[r][c] = T(0);
+    for (int c = 0; c < 3; c++) acc[r][c] = up[r][c] = W(0);
   unsigned fl[ST_RY];
 #pragma unroll
   for (int r = 0; r < ST_RY; r++) fl[r] = kNodeElement;
   // writes row r of the plane whose row 0 is node n and whose ring slot starts at xr
-  auto finish = [&](int r, int64_t n, const T (&fin)[3], const T* xr) {
+  auto finish = [&](int r, int64_t n, const W (&rest)[3], const W (&fin)[3], const T* xr) {
     if (fl[r] & kNodeElement) return;
     T xin[3];
 #pragma unroll
@@ -225,7 +244,7 @@ __global__ void __launch_bounds__(ST_THREADS, MINB)
     if (DOT || (fl[r] & 7u))
 #pragma unroll
       for (int c = 0; c < 3; c++) xin[c] = xr[(r + 1) * ST_ROW + 3 + c];
-    put(n + r * nx, fl[r], fin, xin);
+    dacc += stencil_put<T, DOT, true>(A, S1, eta, n + r * nx, fl[r], rest, fin, xin);
   };
   fetch();
   fetch();
@@ -247,50 +266,52 @@ __global__ void __launch_bounds__(ST_THREADS, MINB)
       if (r < live) nf[r] = A.node[nk + r * nx];
     }
     const bool end = k == 0 || k == nz - 1;
-    T d2[3][3], m[3][3], d[3][3];  // [row mod 3][component]: x-passes
+    T u[3][3], e[3][3], d[3][3];  // [row mod 3][component]: x-passes
 #pragma unroll
     for (int q = 0; q < ST_RY + 2; q++) {
 #pragma unroll
       for (int c = 0; c < 3; c++) {
-        const T lo = s[q * ST_ROW + c], u = s[q * ST_ROW + 3 + c], hi = s[q * ST_ROW + 6 + c];
-        const T e = (lo - u) + (hi - u);
-        d2[q % 3][c] = e;
-        m[q % 3][c] = fma(e, sixth, u);
+        const T lo = s[q * ST_ROW + c], at = s[q * ST_ROW + 3 + c], hi = s[q * ST_ROW + 6 + c];
+        u[q % 3][c] = at;
+        e[q % 3][c] = (lo - at) + (hi - at);
         d[q % 3][c] = hi - lo;
       }
       if (q < 2) continue;
       const int r = q - 2, lo = (q - 2) % 3, mid = (q - 1) % 3, hi = q % 3;
-      auto D2 = [&](const T (&f)[3][3], int c) { return (f[lo][c] - f[mid][c]) + (f[hi][c] - f[mid][c]); };
-      auto Mm = [&](const T (&f)[3][3], int c, T dd) { return fma(dd, sixth, f[mid][c]); };
+      auto M6 = [&](const T (&f)[3][3], int c) { return fma(T(4), f[mid][c], f[lo][c] + f[hi][c]); };  // 6 m_y f
       auto Dd = [&](const T (&f)[3][3], int c) { return f[hi][c] - f[lo][c]; };
-      T P[3], Q[3], R[3], fin[3];
+      auto Dm = [&](int c) { return fma(T(6), Dd(u, c), Dd(e, c)); };  // 6 d_y m_x u
+      T G[3], du[3];
+      W P[3], R[3], rest[3], fin[3];
       {
-        const T y2 = D2(m, 0);
-        P[0] = fma(C.xd, Dd(d, 1), fma(C.xy, y2, C.xx * Mm(d2, 0, D2(d2, 0))));
-        Q[0] = C.q * Mm(m, 0, y2);
-      }
-      {
-        const T y2 = D2(m, 1);
-        P[1] = fma(C.xd, Dd(d, 0), fma(C.yy, y2, C.yx * Mm(d2, 1, D2(d2, 1))));
-        Q[1] = C.q * Mm(m, 1, y2);
-      }
-      {
-        const T y2 = D2(m, 2);
-        P[2] = fma(C.xy, y2, C.yx * Mm(d2, 2, D2(d2, 2)));
-        Q[2] = C.qz * Mm(m, 2, y2);
-      }
-      R[0] = C.rx * Mm(d, 2, D2(d, 2));
-      R[1] = C.ry * Dd(m, 2);
-      R[2] = fma(C.ry, Dd(m, 1), C.rx * Mm(d, 0, D2(d, 0)));
-      T below[3];
+        T y2[3], me[3];
 #pragma unroll
-      for (int c = 0; c < 3; c++) below[c] = up[r][c];
-      stencil_march<T>(P, Q, R, acc[r], up[r], fin);
-      if (end) {
-        asm volatile("");  // a branch, not selects: it is taken on two planes
-        stencil_end<T>(P, Q, R, k == 0 ? C.g : -C.g, below, acc[r]);
+        for (int c = 0; c < 3; c++) {
+          const T u2 = (u[lo][c] - u[mid][c]) + (u[hi][c] - u[mid][c]), es = e[lo][c] + e[hi][c];
+          y2[c] = fma(T(6), u2, fma(T(-2), e[mid][c], es));  // 6 d2_y m_x u
+          me[c] = fma(T(4), e[mid][c], es);                  // 6 m_y d2_x u
+          const T own = stencil_high(u[mid][c]);
+          du[c] = own - stencil_high(sp[(r + 1) * ST_ROW + 3 + c]);  // 0 at the first plane
+          G[c] = fma(T(6), u2, sizeof(T) == 8 ? fma(T(36), u[mid][c] - own, me[c]) : me[c]);
+        }
+        P[0] = fma(C.xd, W(Dd(d, 1)), fma(C.xy, W(y2[0]), C.xx * W(me[0])));
+        P[1] = fma(C.xd, W(Dd(d, 0)), fma(C.yy, W(y2[1]), C.yx * W(me[1])));
+        P[2] = fma(C.xy, W(y2[2]), C.yx * W(me[2]));
       }
-      finish(r, nk - plane, fin, sp);
+      R[0] = W(rx * M6(d, 2));
+      R[1] = W(ry * Dm(2));
+      R[2] = W(fma(ry, Dm(1), rx * M6(d, 0)));
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const W qc = c < 2 ? C.q : C.qz, below = up[r][c];
+        stencil_march<36, false, W>(P[c], qc, G[c], R[c], du[c], W(0), W(0), acc[r][c], up[r][c], rest[c], fin[c]);
+        if (end) {
+          asm volatile("");  // a branch, not selects: it is taken on two planes
+          const W g = (k == 0) == (c < 2) ? C.g : -C.g;
+          acc[r][c] = fma(-qc, fma(W(36), W(du[c]), W(G[c])), fma(W(2), P[c], fma(g, R[c], below)));
+        }
+      }
+      finish(r, nk - plane, rest, fin, sp);
     }
 #pragma unroll
     for (int r = 0; r < ST_RY; r++) fl[r] = nf[r];
@@ -299,9 +320,11 @@ __global__ void __launch_bounds__(ST_THREADS, MINB)
     slot = slot == ST_RING - 1 ? 0 : slot + 1;
     s = mine + slot * ST_PLANE;
   }
-  if (kb == nz)  // the highest plane takes nothing from above
+  if (kb == nz) {  // the highest plane takes nothing from above
+    const W none[3] = {W(0), W(0), W(0)};
 #pragma unroll
-    for (int r = 0; r < ST_RY; r++) finish(r, nk - plane, acc[r], sp);
+    for (int r = 0; r < ST_RY; r++) finish(r, nk - plane, acc[r], none, sp);
+  }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   if constexpr (DOT) {
     const double s = block_sum_dbl(dacc, red);
@@ -311,43 +334,48 @@ __global__ void __launch_bounds__(ST_THREADS, MINB)
 
 // A face across axis n with tangential axis t: node strides along t and inward, components of
 // t and n, sg with d_n f = sg (inner - face), and the terms of the missing half (of P, of R).
-template <typename T> struct FaceAxes {
+template <typename W> struct FaceAxes {
   int st, sn, ct, cn;
-  T sg, em, el, fl, fm;
+  W sg, em, el, fl, fm;
 };
-// P, Q, R of the face node with index n in its plane; the lanes of a warp hold consecutive nodes
-// along t, so that the x-passes along t take their neighbours from the lanes beside (6 loads
-// instead of 18: on an x face every lane's load is a cache line of its own).  Components t, n, z.
-template <typename T>
-__device__ __forceinline__ void stencil_face_plane(const T* __restrict__ x, int64_t n, const FaceAxes<T>& F,
-                                                   const StencilCoef<T>& C, T (&P)[3], T (&Q)[3], T (&R)[3]) {
-  const T sixth = T(1.0 / 6.0);
-  T e2[2][3], m[2][3], d[2][3];
+// P, G, R of the face node with index n in its plane, and its references; the lanes of a warp hold
+// consecutive nodes along t, so that the x-passes along t take their neighbours from the lanes
+// beside (6 loads instead of 18: on an x face every lane's load is a cache line of its own).
+// Components t, n, z.
+template <typename T, typename W>
+__device__ __forceinline__ void stencil_face_plane(const T* __restrict__ x, int64_t n, const FaceAxes<W>& F,
+                                                   const StencilCoefs& C, W (&P)[3], W (&G)[3], W (&R)[3],
+                                                   W (&u0)[3]) {
+  W e[2][3], d[2][3], u[2][3];
 #pragma unroll
   for (int r = 0; r < 2; r++) {
-    const T* u = x + 3 * (n + r * (int64_t)F.sn);
+    const T* a = x + 3 * (n + r * (int64_t)F.sn);
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-      const T mi = __ldg(u + (q == 0 ? F.ct : q == 1 ? F.cn : 2));
-      const T lo = __shfl_up_sync(0xffffffffu, mi, 1), hi = __shfl_down_sync(0xffffffffu, mi, 1);
-      const T e = (lo - mi) + (hi - mi);
-      e2[r][q] = e;
-      m[r][q] = fma(e, sixth, mi);
+      const T mi = __ldg(a + (q == 0 ? F.ct : q == 1 ? F.cn : 2));
+      const W lo = __shfl_up_sync(0xffffffffu, mi, 1), hi = __shfl_down_sync(0xffffffffu, mi, 1);
+      u[r][q] = mi;
+      e[r][q] = (lo - u[r][q]) + (hi - u[r][q]);
       d[r][q] = hi - lo;
     }
   }
   // across the face: mass f / 3 + f' / 6, second difference f' - f, d = sg (f' - f)
-  auto Mn = [&](const T (&f)[2][3], int q) { return fma(f[1][q], sixth, f[0][q] * T(1.0 / 3.0)); };
-  auto Dn = [&](const T (&f)[2][3], int q) { return f[1][q] - f[0][q]; };
-  P[0] = fma(F.em, d[0][1], fma(C.xd * F.sg, Dn(d, 1), fma(C.xy, Dn(m, 0), C.xx * Mn(e2, 0))));
-  P[1] = fma(F.el, d[0][0], fma(C.xd * F.sg, Dn(d, 0), fma(C.yy, Dn(m, 1), C.yx * Mn(e2, 1))));
-  P[2] = fma(C.xy, Dn(m, 2), C.yx * Mn(e2, 2));
-  Q[0] = C.q * Mn(m, 0);
-  Q[1] = C.q * Mn(m, 1);
-  Q[2] = C.qz * Mn(m, 2);
-  R[0] = C.rx * Mn(d, 2);
-  R[1] = fma(F.fl, m[0][2], C.ry * F.sg * Dn(m, 2));
-  R[2] = fma(F.fm, m[0][1], fma(C.ry * F.sg, Dn(m, 1), C.rx * Mn(d, 0)));
+  auto M6 = [&](const W (&f)[2][3], int q) { return fma(W(2), f[0][q], f[1][q]); };
+  auto Dn = [&](const W (&f)[2][3], int q) { return f[1][q] - f[0][q]; };
+  W dm[3], m0[3];  // 6 (m_t u' - m_t u) and 6 (m_t u - u0)
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    dm[q] = fma(W(6), Dn(u, q), Dn(e, q));
+    u0[q] = stencil_high(u[0][q]);
+    m0[q] = fma(W(6), u[0][q] - u0[q], e[0][q]);
+    G[q] = fma(W(3), m0[q], dm[q]);
+  }
+  P[0] = fma(F.em, d[0][1], fma(C.xd * F.sg, Dn(d, 1), fma(C.xy, dm[0], C.xx * M6(e, 0))));
+  P[1] = fma(F.el, d[0][0], fma(C.xd * F.sg, Dn(d, 0), fma(C.yy, dm[1], C.yx * M6(e, 1))));
+  P[2] = fma(C.xy, dm[2], C.yx * M6(e, 2));
+  R[0] = C.rx * M6(d, 2);
+  R[1] = fma(F.fl, m0[2], C.ry * F.sg * dm[2]);
+  R[2] = fma(F.fm, m0[1], fma(C.ry * F.sg, dm[1], C.rx * M6(d, 0)));
 }
 
 // The x and y faces and the edges, by threads first, first + step, ... (whole warps); returns
@@ -357,7 +385,10 @@ __device__ __forceinline__ double stencil_outer(const UApplyArgs<T>& A, int64_t 
   double dacc = 0.;
   const int nx = A.nx, ny = A.ny, nz = A.nz, ncx = nx - 2, ncy = ny - 2;
   const int64_t plane = (int64_t)nx * ny;
-  const T eta = T(A.P->eta), S1 = T(1) + eta;
+  using W = StencilReal;
+  const double eta = A.P->eta;
+  const StencilScale S1(1., eta, true);
+  const W none[3] = {W(0), W(0), W(0)};
   const int lane = (int)(first & 31);
   // faces: groups of 30 columns (lanes 1 .. 30; 0 and 31 hold their neighbours), y and x faces in
   // turn, then runs of planes
@@ -383,35 +414,41 @@ __device__ __forceinline__ double stencil_outer(const UApplyArgs<T>& A, int64_t 
       any = any || !(f[c] & kNodeElement);
     }
     if (!__any_sync(0xffffffffu, any)) continue;
-    const StencilCoefs& cc = A.P->st[yf ? 0 : 1];
-    const StencilCoef<T> C(cc);
-    FaceAxes<T> F;
+    const StencilCoefs& C = A.P->st[yf ? 0 : 1];
+    FaceAxes<W> F;
     F.st = yf ? 1 : nx;
     F.sn = (yf ? nx : 1) * (high ? -1 : 1);
     F.ct = yf ? 0 : 1;
     F.cn = 1 - F.ct;
-    F.sg = high ? T(-1) : T(1);
-    F.em = -F.sg * T(cc.em);
-    F.el = -F.sg * T(cc.el);
-    F.fl = -F.sg * T(cc.fl);
-    F.fm = -F.sg * T(cc.fm);
-    T acc[3] = {T(0), T(0), T(0)}, up[3] = {T(0), T(0), T(0)}, out[ST_FACE_Z + 1][3];
+    F.sg = high ? W(-1) : W(1);
+    F.em = -F.sg * C.em;
+    F.el = -F.sg * C.el;
+    F.fl = -F.sg * C.fl;
+    F.fm = -F.sg * C.fm;
+    const W cR[3] = {W(0), W(6) * F.fl, W(6) * F.fm};
+    W acc[3] = {W(0), W(0), W(0)}, up[3] = {W(0), W(0), W(0)}, last[3];
     // every plane is evaluated (those beyond the run again its last one), so that the loads
     // of one plane do not wait for the others
 #pragma unroll
     for (int c = -1; c <= ST_FACE_Z; c++) {
-      T P[3], Q[3], R[3], fin[3];
-      stencil_face_plane<T>(A.x, n0 + min(c, cnt) * plane, F, C, P, Q, R);
-      stencil_march<T>(P, Q, R, acc, up, fin);
+      W P[3], G[3], R[3], u[3], du[3], rest[3], fin[3];
+      stencil_face_plane<T>(A.x, n0 + min(c, cnt) * plane, F, C, P, G, R, u);
 #pragma unroll
-      for (int q = 0; q < 3; q++) out[c > 0 ? c - 1 : ST_FACE_Z][q] = fin[q];
-    }
-#pragma unroll
-    for (int c = 0; c < ST_FACE_Z; c++)
-      if (!(f[c] & kNodeElement)) {
-        const T r3[3] = {yf ? out[c][0] : out[c][1], yf ? out[c][1] : out[c][0], out[c][2]};
-        dacc += stencil_put<T, DOT>(A, S1, eta, n0 + c * plane, f[c], r3, A.x + 3 * (n0 + c * plane));
+      for (int q = 0; q < 3; q++) {
+        du[q] = c >= 0 ? u[q] - last[q] : W(0);
+        last[q] = u[q];
       }
+#pragma unroll
+      for (int q = 0; q < 3; q++)
+        stencil_march<18, true, W>(P[q], q < 2 ? C.q : C.qz, G[q], R[q], du[q], cR[q], du[q == 1 ? 2 : 1], acc[q],
+                                   up[q], rest[q], fin[q]);
+      if (c > 0 && !(f[c - 1] & kNodeElement)) {
+        const W a[3] = {yf ? rest[0] : rest[1], yf ? rest[1] : rest[0], rest[2]};
+        const W b[3] = {yf ? fin[0] : fin[1], yf ? fin[1] : fin[0], fin[2]};
+        const int64_t n = n0 + (c - 1) * plane;
+        dacc += stencil_put<T, DOT, true>(A, S1, eta, n, f[c - 1], a, b, A.x + 3 * n);
+      }
+    }
   }
   // edges: 9 lanes per node, one per row of neighbours, three nodes per warp; summed in a fixed
   // order (one thread per node is a chain of 1500 dependent operations)
@@ -435,18 +472,17 @@ __device__ __forceinline__ double stencil_outer(const UApplyArgs<T>& A, int64_t 
     }
     const int64_t n = on ? node_index(i, j, k, nx, ny) : 0;
     const unsigned f = on ? A.node[n] : kNodeElement;
-    T r[3] = {T(0), T(0), T(0)};
+    W r[3] = {W(0), W(0), W(0)};
     if (!(f & kNodeElement))
-      stencil_edge_row<T>(A, i, j, k, rc % 3, rc / 3, T(A.P->L.lambda[0]), T(A.P->L.mu[0]), T(A.hx), T(A.hy),
-                          T(A.hz), r);
-    T sum[3];
+      stencil_edge_row<T, W>(A, i, j, k, rc % 3, rc / 3, A.P->L.lambda[0], A.P->L.mu[0], A.hx, A.hy, A.hz, r);
+    W sum[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       sum[c] = r[c];
 #pragma unroll
       for (int s = 1; s < 9; s++) sum[c] += __shfl_sync(0xffffffffu, r[c], min(9 * g + s, 31));
     }
-    if (rc == 0 && !(f & kNodeElement)) dacc += stencil_put<T, DOT>(A, S1, eta, n, f, sum, A.x + 3 * n);
+    if (rc == 0 && !(f & kNodeElement)) dacc += stencil_put<T, DOT, false>(A, StencilScale(1., eta, false), eta, n, f, sum, none, A.x + 3 * n);
   }
   return dacc;
 }
@@ -471,8 +507,8 @@ template <typename T_, bool CUBIC = false> struct UOpMarked : UOp<T_, CUBIC> {
 // The apply's last launch: blocks [0, nface) the stencil's faces and edges, the rest the element
 // operator's seams; x.y partials to A.dot[dot_base + block].
 template <class Op, bool DOT>
-__global__ void __launch_bounds__(256, sizeof(typename Op::T) == 8 ? 2 : 3) u_outer_kernel(const __grid_constant__ typename Op::Args A, int TY,
-                                                         int dot_base, int nface) {
+__global__ void __launch_bounds__(256, 2) u_outer_kernel(const __grid_constant__ typename Op::Args A, int TY, int dot_base,
+                                                         int nface) {
   __shared__ double red[32];
   if (A.skip && *A.skip) return;
   double dacc;
