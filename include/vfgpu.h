@@ -404,8 +404,8 @@ int vfgpu_tc_tables(double hx, double hy, double hz, double* B1, double* B2);
  * roofline). */
 int vfgpu_fma_peak(int bytes, double* tflops);
 
-/* Diagnostic, no counterpart in the reference: runs the library's bounded mbarrier wait
- * on a phase that completes (complete = 1) or never
+/* Diagnostic, no counterpart in the reference: runs the bounded mbarrier wait of the
+ * tensor-core apply on a phase that completes (complete = 1) or never
  * does (complete = 0) with a limit of `cycles` (<= 4e9) SM clock cycles, and sets
  * *timed_out to whether the wait gave up (the kernel then returns normally and the
  * device stays usable).  Returns 0, or < 0 on a bad argument or CUDA error. */

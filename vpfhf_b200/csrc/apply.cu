@@ -4,6 +4,7 @@
 #include <type_traits>
 
 #include "kernels.h"
+#include "mbar.cuh"
 #include "ops.cuh"
 #include "u_stencil.cuh"
 #include "u_twophase.cuh"
@@ -122,17 +123,18 @@ cudaError_t apply_kernel_attributes() {
 
 // One CTA waits on an mbarrier whose phase completes (complete = 1: the arrival is
 // made) or never does (complete = 0: 16 transaction bytes are expected and no copy is
-// issued); the bounded wait sets *err when it gives up.
+// issued); *err is set when the bounded wait gives up.
 __global__ void wait_selftest_kernel(unsigned* err, long long limit, int complete) {
   __shared__ uint64_t bar;
+  const uint32_t b = smem_u32(&bar);
   if (threadIdx.x == 0) {
-    mbar_init(&bar, 1);
+    mbar_init(b, 1);
     mbar_fence_init();
-    if (complete) mbar_arrive(&bar);
-    else mbar_expect_tx(&bar, 16);
+    if (complete) mbar_arrive(b);
+    else mbar_expect_tx(b, 16);
   }
   __syncthreads();
-  mbar_wait(&bar, 0, err, limit);
+  if (!mbar_wait(b, 0, limit)) atomicOr(err, 1u);
 }
 
 cudaError_t wait_selftest(long long cycles, int complete, int* timed_out) {

@@ -36,6 +36,7 @@
 
 #include "abi_util.h"
 #include "kernels.h"
+#include "mbar.cuh"
 
 namespace vfgpu {
 namespace {
@@ -84,8 +85,7 @@ struct TcArgs {
   long long ntiles;
 };
 
-// ---- tcgen05 / mbarrier primitives --------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// ---- tcgen05 primitives --------------------------------------------------------------
 
 __device__ __forceinline__ uint32_t to_tf32(float a) {
   uint32_t r;
@@ -131,25 +131,6 @@ __device__ __forceinline__ void tmem_ld8(uint32_t addr, float (&r)[8]) {
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-__device__ __forceinline__ void bar_init(uint32_t bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-}
-// Bounded parity wait (~1 s at the top clock); false if it gave up.
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
-  const long long t0 = clock64();
-  for (;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if (clock64() - t0 > 2000000000ll) return false;
-  }
-}
-
 // Splits a into TF32 hi/lo and stores both at byte offset off of the two buffers.
 __device__ __forceinline__ void put_split(unsigned char* sm, uint32_t off_hi, uint32_t off_lo, uint32_t o,
                                           float a) {
@@ -178,9 +159,9 @@ __global__ void __launch_bounds__(128, 1) tc_u_apply_kernel(const TcArgs A) {
     }
   }
   if (tid == 0) {
-    bar_init(bar1);
-    bar_init(bar2);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_init(bar1, 1);
+    mbar_init(bar2, 1);
+    mbar_fence_init();
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -253,7 +234,7 @@ __global__ void __launch_bounds__(128, 1) tc_u_apply_kernel(const TcArgs A) {
       mma_commit(bar1);
     }
     issued1++;
-    if (__syncthreads_or(!bar_wait(bar1, ph1 & 1))) {
+    if (__syncthreads_or(!mbar_wait(bar1, ph1 & 1))) {
       ok = false;
       break;
     }
@@ -263,7 +244,7 @@ __global__ void __launch_bounds__(128, 1) tc_u_apply_kernel(const TcArgs A) {
     // ---- three passes of 9 Gauss points: pointwise stress -> A2 -> GEMM2
     for (int pass = 0; pass < 3 && ok; pass++) {
       if (pass > 0) {  // the previous pass's MMAs still read A2
-        if (__syncthreads_or(!bar_wait(bar2, ph2 & 1))) {
+        if (__syncthreads_or(!mbar_wait(bar2, ph2 & 1))) {
           ok = false;
           break;
         }
@@ -304,7 +285,7 @@ __global__ void __launch_bounds__(128, 1) tc_u_apply_kernel(const TcArgs A) {
       issued2++;
     }
     if (!ok) break;
-    if (__syncthreads_or(!bar_wait(bar2, ph2 & 1))) {
+    if (__syncthreads_or(!mbar_wait(bar2, ph2 & 1))) {
       ok = false;
       break;
     }
@@ -336,9 +317,9 @@ __global__ void __launch_bounds__(128, 1) tc_u_apply_kernel(const TcArgs A) {
     if (tid == 0) {
       atomicOr(A.err, 1u);
       // the MMAs this block issued: wait (bounded) for their commits before freeing
-      if (issued1 > 0) bar_wait(bar1, ph1 & 1);
+      if (issued1 > 0) mbar_wait(bar1, ph1 & 1);
       for (int k = 0; k < issued2; k++) {
-        bar_wait(bar2, ph2 & 1);
+        mbar_wait(bar2, ph2 & 1);
         ph2++;
       }
     }

@@ -1,5 +1,5 @@
-// tile_engine.cuh -- the z-marching tile schedule shared by the matrix-free
-// operators (U: 3 dofs per node, V: 1 dof per node).
+// tile_engine.cuh -- the z-marching tile schedule of the matrix-free U operator's forms (plain,
+// fixed-weight, packed FP32, NOCOMPRESSION, and the nodes the stencil leaves).
 //
 // The grid's elements are cut into xy tiles of 32 (x, one warp) x TY (y, TY warps)
 // elements; a (tile, node plane) pair is one unit of work, and the ntx nty nz units,
@@ -73,44 +73,6 @@ template <class Op, int TY, int MINB> constexpr size_t tile_smem_bytes() {
   return ring_bytes<Op, TY>() + sc_bytes<Op, TY, sc_stages<Op, TY, MINB>()>();
 }
 
-// mbarrier primitives with a bounded wait (one thread arrives; every thread may wait).
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"((unsigned)__cvta_generic_to_shared(bar)),
-               "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_fence_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(bar)),
-               "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"((unsigned)__cvta_generic_to_shared(bar))
-               : "memory");
-}
-// Waits for the phase with the given parity to complete; gives up after `limit` cycles
-// (by default ~2e9, about a second), flags *err and returns false.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, unsigned* err,
-                                          long long limit = 2000000000ll) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
-  const long long t0 = clock64();
-  for (;;) {
-    unsigned done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if (clock64() - t0 > limit) {
-      if (err) atomicOr(err, 1u);
-      return false;
-    }
-  }
-}
 // Asynchronous global -> shared copy of one 4- or 8-byte value (LDGSTS); with
 // valid == false nothing is read and the destination is zero-filled.
 template <typename T>
