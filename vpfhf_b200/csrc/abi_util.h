@@ -30,12 +30,9 @@ cudaError_t nc_flags(vfgpu_ctx* c, const double* u);
 int run_mgcg(vfgpu_ctx* c, bool fp32, const double* b, double* x, double* r, double* p, double* w,
              const double* dinv0, const float* dinv0_32, bool reuse, double rtol, double atol,
              double dtol, int maxit, int* its, int* reason, int* levels);
-// Graph of one call site's launch sequence, captured on first use and re-captured when
+// Graph of one call site, a conditional while node whose body is what `body` launches (it gets
+// the handle whose condition its last kernel sets), captured on first use and re-captured when
 // ctx->gen moves on (null: capture failed, run the body directly).
-cudaGraphExec_t ctx_graph(vfgpu_ctx* c, int kind, int batch,
-                          const std::function<cudaError_t()>& body);
-// The same for a conditional while node whose body is what `body` launches: it gets the handle
-// whose condition its last kernel sets.
 cudaGraphExec_t ctx_while_graph(vfgpu_ctx* c, int kind, int batch,
                                 const std::function<cudaError_t(cudaGraphConditionalHandle)>& body);
 // x.y partials an apply of the ctx's U operator writes in this precision.

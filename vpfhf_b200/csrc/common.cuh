@@ -59,7 +59,6 @@ inline StencilCoefs stencil_coefs(double lambda, double mu_, double d0, double d
 struct DevParams {
   LayerTable L;
   double eta;                  // eta (VFProp.eta)
-  double aeps[VF_MAXLAYER];    // Gc/(2 c_w) * eps per layer (V operator gradient term)
   StencilCoefs st[2];          // layer 0: axes x, y, z, and y, x, z (the U stencil)
 };
 

@@ -32,7 +32,7 @@ struct vfgpu_ctx {
   uint8_t* d_unode = nullptr;
   int2 *d_srange64 = nullptr, *d_srange32 = nullptr;
   int u_split = VFGPU_U_SPLIT_AUTO;
-  vfgpu::DevParams* d_params = nullptr;  // device copy of layers / eta / aeps
+  vfgpu::DevParams* d_params = nullptr;  // device copy of layers / eta / stencil coefficients
   float* d_cellE = nullptr;     // NC or null
   bool have_mat = false;
   vfgpu_vfprop vf{0.2, 1e-5, 5e-2, 2, 0};  // VFPropGet defaults (VFCommon.c:468-480)

@@ -400,6 +400,7 @@ struct URhsCell {
   }
 };
 
+// The U load under NOCOMPRESSION, one colour of elements.
 __global__ void u_rhs_kernel(const __grid_constant__ ElemArgs E, int color, const double* __restrict__ v,
                              const double* __restrict__ theta, const double* __restrict__ thetaRef,
                              const double* __restrict__ p, double* __restrict__ f,
@@ -422,7 +423,7 @@ __global__ void u_rhs_kernel(const __grid_constant__ ElemArgs E, int color, cons
   // (VFMech.c:456-524): undegraded thermal term and p instead of p v where tr < 0
   const double coefalpha = (3. * m.lambda + 2. * m.mu) * m.alpha, beta = m.beta;
   double u8[8][3];
-  if (E.unilateral) gather_u8(n, u0, u8);
+  gather_u8(n, u0, u8);
   for (int g = 0; g < 27; g++) {
     double te = 0., pe = 0., ve = 0.;
     for (int a = 0; a < 8; a++) {
@@ -430,7 +431,7 @@ __global__ void u_rhs_kernel(const __grid_constant__ ElemArgs E, int color, cons
       pe += e.phi[a][g] * p8[a];
       ve += e.phi[a][g] * v8[a];
     }
-    const bool comp = E.unilateral && trace_at(e, u8, g) < 0.;
+    const bool comp = trace_at(e, u8, g) < 0.;
     const double s = comp ? coefalpha * te * (1. + E.eta) + beta * pe
                           : coefalpha * te * (ve * ve + E.eta) + beta * pe * ve;
     for (int a = 0; a < 8; a++)
@@ -452,6 +453,7 @@ __global__ void u_rhs_kernel(const __grid_constant__ ElemArgs E, int color, cons
     for (int c = 0; c < 3; c++) f[3 * n[a] + c] += rl[3 * a + c];
 }
 
+// The U diagonal under NOCOMPRESSION, one colour of elements.
 __global__ void u_diag_kernel(const __grid_constant__ ElemArgs E, int color, const double* __restrict__ v,
                               double* __restrict__ d, const double* __restrict__ u0) {
   int ei, ej, ek;
@@ -465,14 +467,14 @@ __global__ void u_diag_kernel(const __grid_constant__ ElemArgs E, int color, con
   for (int l = 0; l < 24; l++) dg[l] = 0.;
   const CellMat m = cell_mat(E, ei, ej, ek);
   double u8[8][3];
-  if (E.unilateral) gather_u8(n, u0, u8);
+  gather_u8(n, u0, u8);
   const double kappa = m.lambda + 2. * m.mu / 3.;
   for (int g = 0; g < 27; g++) {
     double s = 0.;
     for (int a = 0; a < 8; a++) s += v8[a] * e.phi[a][g];
     const double sv = s * s + E.eta, ws = e.w[g] * sv;
     // spherical coefficient: lambda s, or kappa (1 + eta) - 2 mu s / 3 in compression
-    const bool comp = E.unilateral && trace_at(e, u8, g) < 0.;
+    const bool comp = trace_at(e, u8, g) < 0.;
     const double lw = comp ? e.w[g] * (kappa * (1. + E.eta) - 2. * m.mu * sv / 3.) : ws * m.lambda;
     for (int a = 0; a < 8; a++) {
       const double d0 = e.dphi[a][0][g], d1 = e.dphi[a][1][g], d2 = e.dphi[a][2][g];
@@ -979,7 +981,7 @@ __global__ void __launch_bounds__(EN_THREADS, 3) energy_kernel(
             (1. + E.eta) * m.mu * w;
       // NOCOMPRESSION (VF_ElasticEnergyNoCompression3D_local, VFMech.c:819-908): the
       // spherical factor is 1 instead of v where tr < 0
-      const double sph = (E.unilateral && tr < 0.) ? 1. : ve;
+      const double sph = tr < 0. ? 1. : ve;
       const double WD = (tr / 3. - m.alpha * te) * sph - coefbeta * pe;
       el += 3. * threekappa / 2. * WD * WD * w;
       el += threekappa / 6. * tr * tr * E.eta * w;

@@ -170,21 +170,6 @@ static cudaGraphExec_t cached_graph(vfgpu_ctx* c, int kind, int batch, Make make
   return exec;
 }
 
-cudaGraphExec_t ctx_graph(vfgpu_ctx* c, int kind, int batch,
-                          const std::function<cudaError_t()>& body) {
-  return cached_graph(c, kind, batch, [&]() -> cudaGraph_t {
-    cudaGraph_t graph = nullptr;
-    if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return nullptr;
-    const cudaError_t eb = body();
-    const cudaError_t ec = cudaStreamEndCapture(c->stream, &graph);
-    if (eb != cudaSuccess || ec != cudaSuccess) {
-      if (graph) cudaGraphDestroy(graph);
-      return nullptr;
-    }
-    return graph;
-  });
-}
-
 // A graph of one conditional while node whose body is what `body` launches; body gets the
 // handle whose condition its last kernel sets.
 static cudaGraph_t while_graph(vfgpu_ctx* c, const std::function<cudaError_t(cudaGraphConditionalHandle)>& body) {

@@ -112,8 +112,6 @@ int upload_params(vfgpu_ctx* c) {
   P.eta = c->vf.eta;
   P.st[0] = stencil_coefs(c->layers.lambda[0], c->layers.mu[0], c->hx, c->hy, c->hz);
   P.st[1] = stencil_coefs(c->layers.lambda[0], c->layers.mu[0], c->hy, c->hx, c->hz);
-  const double atcv = c->vf.atnum == 1 ? 2. / 3. : .5;  // VFCommon.c:482-492
-  for (int l = 0; l < VF_MAXLAYER; l++) P.aeps[l] = c->layers.Gc[l] / atcv * .5 * c->vf.epsilon;
   cudaError_t e = cudaMemcpyAsync(c->d_params, &P, sizeof P, cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "parameter upload");
