@@ -27,7 +27,9 @@ constexpr int VM_BLOCKS = 592;
 // Measured at 129^3 inside the AT1 penny crack's StepV (few nodes free): 7.9 us a launch in
 // FP64 and 4.4 us in FP32, where the element form with its staged coefficients took 63.5 + 4.5
 // (seams) and 33.7 + 2.8 us (averages over a solve's launches, finished ones included); with
-// every node free 97 us in FP64 (element form 96 + 8.7).
+// every node free 102 us in FP64 (element form 96 + 8.7; the plain products 96).  A warp takes one form
+// of the row: with a branch per node nearly every warp of a 65^3 grid ran both (AT2 multigrid AM step 65^3
+// 21.5 -> 21.1 ms).
 template <typename T, bool FACE>
 __device__ __forceinline__ T vmat_row(const VMatArgs<T>& A, int64_t n, int i, int j, int k, int64_t st) {
   const int64_t row = A.nx, pl = (int64_t)A.nx * A.ny;
@@ -69,7 +71,8 @@ __global__ void __launch_bounds__(VM_THREADS, 4) vmat_apply_kernel(const __grid_
       const unsigned m = (unsigned)n, rows = m / nx;
       const int i = (int)(m - rows * nx), k = (int)(rows / ny), j = (int)(rows - (unsigned)k * ny);
       const bool face = i == 0 || i == A.nx - 1 || j == 0 || j == A.ny - 1 || k == 0 || k == A.nz - 1;
-      y = face ? vmat_row<T, true>(A, n, i, j, k, st) : vmat_row<T, false>(A, n, i, j, k, st);
+      // one form for the whole warp (the same bits where no neighbour is missing)
+      y = __any_sync(__activemask(), face) ? vmat_row<T, true>(A, n, i, j, k, st) : vmat_row<T, false>(A, n, i, j, k, st);
       if constexpr (DOT) acc += (double)A.x[n] * (double)y;
     }
     A.y[n] = y;
