@@ -317,7 +317,7 @@ def run_gpu(args):
     # a homogeneous patch and takes the stencil), counted by ncu
     # (smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on / cells, the stencil
     # launch of this workload); an FMA is 2 flops
-    dfma_el, dadd_el, dmul_el = 31.1, 62.1, 13.1
+    dfma_el, dadd_el, dmul_el = 54.1, 59.2, 10.0
     instr_el = dfma_el + dadd_el + dmul_el
     flops_el = 2 * dfma_el + dadd_el + dmul_el
     f64_peak = fp_peak_tflops(torch, "f64")
@@ -343,14 +343,14 @@ def run_gpu(args):
         "roofline": {"bound": "hbm", "achieved": round(alg_bytes / (ms64 * 1e-3) / 1e9, 1),
                      "peak": hbm, "unit": "GB/s",
                      "frac": round(alg_bytes / (ms64 * 1e-3) / 1e9 / hbm, 4),
-                     "traffic": 61.0e6 if n == N_EDGE else None,
+                     "traffic": 61.9e6 if n == N_EDGE else None,
                      "note": "achieved: algorithmic bytes over the whole apply (three launches: "
                              "the stencil over the homogeneous nodes, the element tiles over the "
                              "(tile, plane) units with others, the faces with the tiles' seams); "
-                             "traffic: ncu dram read+write of the stencil launch at 129^3 (55.7 + 5.3 "
+                             "traffic: ncu dram read+write of the stencil launch at 129^3 (56.2 + 5.7 "
                              "MB: most of the output is still in the 126 MB L2 when it ends).  The "
                              "stencil is bound by latency at 8 warps per SM (ncu: issue active "
-                             "47 %, FP64 pipe 46 %, top stall fixed-latency dependencies)"},
+                             "46 %, FP64 pipe 47 %, top stall fixed-latency dependencies)"},
         "compute_roofline": {
             "pipe": "fp64 CUDA cores",
             "fp64_instructions_per_element": {"dfma": dfma_el, "dadd": dadd_el, "dmul": dmul_el},

@@ -191,7 +191,10 @@ int vfgpu_get_field(vfgpu_ctx* ctx, int field, double* data);
 /* y = J_U x: the U Jacobian K(V) of VF_UIJacobian (VFMech.c:1897-2029) applied
  * matrix-free, Dirichlet rows identity (MatApplyDirichletBC, VFCartFE.c:1147-1296),
  * with the resident V.  x, y: 3N.  precision: VFGPU_FP64 or VFGPU_MIXED (FP32
- * kernel; x is rounded to FP32, y returned in FP64). */
+ * kernel; x is rounded to FP32, y returned in FP64).  With x and y in host memory an FP64
+ * apply runs in slabs of the element operator: the device-buffer apply's bits, except on
+ * large grids of one material, whose device-buffer applies run the homogeneous nodes on a
+ * stencil; there the two agree to rounding. */
 int vfgpu_u_apply(vfgpu_ctx* ctx, int precision, const double* x, double* y);
 
 /* Stream-ordered variant for device-resident data: x, y are device arrays of
@@ -362,9 +365,11 @@ int vfgpu_server_destroy(vfgpu_server* s);
  * bit c set = component c of the node is Dirichlet; may be NULL) are device
  * arrays of the current device, the work is queued on `stream` (a
  * cudaStream_t, NULL = legacy default stream) and the call returns without
- * waiting.  The only scratch (the seam partial sums, or on small grids with seams the
- * element values of a two-phase apply) is a fixed 32 MiB array inside the library (VFGPU_NOALLOC_SCRATCH_DOUBLES doubles; every GPU that
- * loads the library holds it until exit); grids whose seams need more are
+ * waiting.  The result has the bits of a ctx's host-buffer apply (vfgpu_u_apply).  The
+ * only scratch (the seam partial sums, or on small grids with seams the element values of a
+ * two-phase apply) is a fixed 32 MiB array inside the library
+ * (VFGPU_NOALLOC_SCRATCH_DOUBLES doubles; every GPU that loads the library holds it until
+ * exit); grids whose seams need more are
  * rejected with VFGPU_ERR_INVALID (129^3 fits, 161^3 does not), and so are x and y
  * that overlap (the apply is out of place).  Every call looks up the array's device
  * address in the current context (cudaGetSymbolAddress, host-side) and, on the first

@@ -41,8 +41,10 @@ cudaError_t build_unit_lists(const double* v, int nx, int ny, int nz, const Tile
 bool twophase_pays(int nx, int ny, int nz, int prec_bytes);
 size_t twophase_scratch(int nx, int ny, int nz);
 int twophase_dots(int nx, int ny, int nz);
-// Whether the plan's homogeneous nodes take the stencil in precision prec_bytes (a rule of
-// the grid alone, so that every apply of a grid gives the same bits).
+// Whether the plan's homogeneous nodes take the stencil in precision prec_bytes: the part of the
+// rule that the grid decides.  u_stencil_on adds the problem's (one material, no per-cell modulus,
+// no NOCOMPRESSION); the ctx's device-buffer applies and solves follow it, the host-buffer and
+// fixed-scratch applies keep the element operator.
 bool stencil_pays(const TilePlan& p, int nx, int ny, int nz, int prec_bytes);
 inline size_t stencil_range_bytes(const TilePlan& p) { return sizeof(int2) * (size_t)p.st.blocks(); }
 // The node flags from the FP64 phase field and the Dirichlet bits; then, per plan, the
